@@ -53,11 +53,11 @@ int dispatch(int precision, int64_t n, int64_t m, double sigma, int kernel, cons
   if (bad_kernel(kernel)) return kInvalidArgument;
   typename Op::Params P;
   if (precision == kFP32Compensated) {
-    P.f = make_frame(origin, sigma, kernel, true);
+    P.f = make_frame(origin, sigma, kernel);
     fill(P);
     return run_pairs_k<Op, F2, TPB32, RT32>(P, n, m, ws, wsb, st);
   } else if (precision == kFP64) {
-    P.f = make_frame(origin, sigma, kernel, false);
+    P.f = make_frame(origin, sigma, kernel);
     fill(P);
     return run_pairs_k<Op, double, kTpb64, kRt64>(P, n, m, ws, wsb, st);
   }
@@ -87,6 +87,7 @@ size_t kernel_sums_ws_bytes(int64_t n, int64_t m, int precision) {
     upd(symx_ws_bytes<OpKSym, kTpbKSym, kRtKSym>(n));
     upd(sym_ws_bytes<OpKSymD, kTpbLight, kRtKSymL, Laplacian>(n));
   }
+  if (precision == kFP64 && n == m) upd(sym64_ws_bytes_upto<OpKSymD>(n));
   return b;
 }
 
@@ -103,10 +104,16 @@ int lddmm_apply_k(const double* y, int64_t n, const double* x, const double* a, 
   // a self-sum K(x, x) a (the same point array as targets and sources): each unordered pair once
   if (LDDMM_SYM && precision == kFP32Compensated && y == x && n == m && !bad_kernel(kernel)) {
     OpK::Params P;
-    P.f = make_frame(origin, sigma, kernel, true);
+    P.f = make_frame(origin, sigma, kernel);
     P.y = y; P.x = x; P.a = a; P.out = out;
     if (kernel == kGauss) return run_pairs_symx<OpKSym, kTpbKSym, kRtKSym>(P, n, ws, wsb, (cudaStream_t)stream);
     return run_pairs_sym<OpKSymD, kTpbLight, kRtKSymL, Laplacian>(P, n, ws, wsb, (cudaStream_t)stream);
+  }
+  if (precision == kFP64 && y == x && n == m && !bad_kernel(kernel) && sym64_takes<OpKSymD>(n)) {
+    OpK::Params P;
+    P.f = make_frame(origin, sigma, kernel);
+    P.y = y; P.x = x; P.a = a; P.out = out;
+    return run_sym64<OpKSymD>(P, n, ws, wsb, (cudaStream_t)stream);
   }
   return dispatch<OpK, kTpbLight, kRtLight>(precision, n, m, sigma, kernel, origin, ws, wsb, (cudaStream_t)stream,
                                             [&](OpK::Params& P) { P.y = y; P.x = x; P.a = a; P.out = out; });

@@ -97,5 +97,15 @@ constexpr int kRtKSym = LDDMM_RT_KSYM;
 // FP64 baseline path.
 constexpr int kTpb64 = LDDMM_TPB_64;
 constexpr int kRt64 = LDDMM_RT_64;
+// FP64 symmetric sums (pairs_kernel_sym with V = double), threads per CTA x targets per thread. 64 x 4 for K a, the
+// forward step and the first-order adjoint step, 128 x 2 for the adjoint step (17 target values per thread: 4 targets
+// would leave 1 CTA per SM); 64 x 2 for small sets, whose unit triangle would otherwise have fewer units than the GPU
+// has SMs. us at n = 642 / 10,242 / 40,962, 64 x 2 | 64 x 4 | 128 x 2 | 128 x 4: K a 16.7 / 123 / 1631 | 19.8 / 113 /
+// 1486 | 19.9 / 120 / 1593 | 29.1 / 111 / 1494; adjoint step 23.0 / 297 / 4165 | 43.5 / 302 / 4218 | 35.3 / 291 / 4100
+// | 74 / 299 / 4232 (every ordered pair with exp(): K a 23.0 / 227 / 3111, adjoint step 35.3 / 463 / 6606).
+constexpr int kTpbSym64 = 64, kRtSym64 = 4;
+constexpr int kTpbSym64Adj = 128, kRtSym64Adj = 2;
+constexpr int kTpbSym64Small = 64, kRtSym64Small = 2;
+constexpr int64_t kSym64SmallN = 2048;
 
 }  // namespace lddmm

@@ -19,7 +19,7 @@
 // float64 Euler update of the state).
 // Ops whose sum needs no coordinate differences (K a, the surface energies) run pairs_kernel_x instead: the
 // squared distance expanded about the centre of each target block, three packed FMAs per pair (see there).
-// FP64 path (the faithful baseline): the same pair functors instantiated with double, exp() and FP64 sums.
+// FP64 path (the faithful baseline): the same pair functors instantiated with double, exp2_neg() and FP64 sums.
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
@@ -135,14 +135,53 @@ __device__ __forceinline__ float ex2neg(float x) {
   return y;
 }
 
+// 2^-t in FP64 for t >= 0, by Tang's table-driven scheme (P. T. P. Tang, ACM TOMS 15(2), 1989, for exp): t is rounded
+// to a multiple of 1/16, t = k/16 - f with |f| <= 1/32, and 2^-t = 2^-m T[j] (1 + f q(f)) with k = 16 m - j, T[j] =
+// 2^(j/16) and q the degree-5 Chebyshev interpolant of (2^f - 1)/f on |f| <= 1/32 (1.4e-17 relative). 10 FP64
+// instructions (exp() of the CUDA library: as long as ~25 of them, 53 against 22 clocks per warp and scheduler), the
+// exponent arithmetic on the integer pipe, one 8-byte shared-memory load: the 16 entries cover the 32 banks once, so
+// lanes on different entries never conflict. Results below 2^-1022 are zero; NaN stays NaN.
+static __constant__ double kExp2Frac[16] = {
+    1.0, 1.0442737824274138, 1.0905077326652577, 1.1387886347566916, 1.189207115002721, 1.241857812073484,
+    1.2968395546510096, 1.3542555469368927, 1.4142135623730951, 1.4768261459394993, 1.5422108254079407,
+    1.6104903319492543, 1.681792830507429, 1.7562521603732995, 1.8340080864093424, 1.9152065613971474};
+__device__ __forceinline__ double* exp2_table() {
+  __shared__ double t[16];
+  return t;
+}
+// Fills the kernel's table; a barrier must follow before the first exp2_neg.
+__device__ __forceinline__ void exp2_table_fill() {
+  if (threadIdx.x < 16) exp2_table()[threadIdx.x] = kExp2Frac[threadIdx.x];
+}
+__device__ __forceinline__ double exp2_neg(double t) {
+  constexpr double kRound = 422212465065984.0;  // 1.5 * 2^48: the low word of t + kRound is t rounded to 1/16
+  const double s = t + kRound;
+  const int k = __double2loint(s);
+  const double f = (s - kRound) - t;
+  double q = 0.00015403723980749256;
+  q = ::fma(q, f, 0.0013333781576784268);
+  q = ::fma(q, f, 0.009618129106919537);
+  q = ::fma(q, f, 0.0555041086566393);
+  q = ::fma(q, f, 0.24022650695910075);
+  q = ::fma(q, f, 0.6931471805599457);
+  const double tj = exp2_table()[-k & 15];
+  const double ts = __hiloint2double(__double2hiint(tj) - (((k + 15) >> 4) << 20), __double2loint(tj));
+  const double e = ::fma(ts, q * f, ts);
+  // t in [1022, inf]: zero (high words 0x408ff000 .. 0x7ff00000; a NaN's is above)
+  const bool zero = (unsigned)__double2hiint(t) - 0x408ff000u <= 0x7ff00000u - 0x408ff000u;
+  return zero ? 0.0 : e;
+}
+
+// sqrt(log2(e) / 2): exp(-r^2/(2 sigma^2)) == 2^-(s r)^2 with s = kScale / sigma.
+constexpr double kScale = 0.84932180028801904272;
+
 // Value-type traits: V = F2 (two FP32 targets per lane group) or double (one FP64 target).
 template <typename V> struct VT;
 template <> struct VT<F2> {
   using Scalar = float;
   static constexpr int kLanes = 2;
-  // sqrt(log2(e) / 2): exp(-r^2/(2 sigma^2)) == 2^-(s r)^2 with s = kScale / sigma.
-  static constexpr double kScale = 0.84932180028801904272;
   using Partial = float2;  // (hi, lo) of the compensated chunk sum
+  static __device__ __forceinline__ void setup() {}
   static __device__ __forceinline__ F2 zero() { return f2(0.f, 0.f); }
   static __device__ __forceinline__ F2 dup(double a) { return f2((float)a, (float)a); }
   static __device__ __forceinline__ F2 pack(double a, double b) { return f2((float)a, (float)b); }
@@ -150,6 +189,13 @@ template <> struct VT<F2> {
     float a, b;
     split(r2, a, b);
     return f2(ex2neg(a), ex2neg(b));
+  }
+  // a scalar as the first lane of a value, and the sum of a value's lanes
+  static __device__ __forceinline__ F2 first(float a) { return f2(a, 0.f); }
+  static __device__ __forceinline__ float hsum(F2 v) {
+    float a, b;
+    split(v, a, b);
+    return a + b;
   }
   static __device__ __forceinline__ double lane(F2 v, int k) {
     float a, b;
@@ -160,12 +206,15 @@ template <> struct VT<F2> {
 template <> struct VT<double> {
   using Scalar = double;
   static constexpr int kLanes = 1;
-  static constexpr double kScale = 0.70710678118654752440;  // sqrt(1/2): exp(-(s r)^2)
   using Partial = double;
+  static __device__ __forceinline__ void setup() { exp2_table_fill(); }  // a barrier must follow before expneg
   static __device__ __forceinline__ double zero() { return 0.0; }
   static __device__ __forceinline__ double dup(double a) { return a; }
   static __device__ __forceinline__ double pack(double a, double) { return a; }
-  static __device__ __forceinline__ double expneg(double r2) { return exp(-r2); }
+  static __device__ __forceinline__ double expneg(double r2) { return exp2_neg(r2); }
+  // a scalar as the first lane of a value, and the sum of a value's lanes
+  static __device__ __forceinline__ double first(double a) { return a; }
+  static __device__ __forceinline__ double hsum(double v) { return v; }
   static __device__ __forceinline__ double lane(double v, int) { return v; }
 };
 
@@ -221,12 +270,12 @@ enum KernelFamily : int { kGauss = 0, kLaplacian0 = 16, kLaplacianMax = 20 };
 // Geometry shared by every op: centred, pre-scaled coordinates, and the radial profile of the kernel.
 struct Frame {
   double o0, o1, o2;  // origin subtracted before scaling
-  double s;           // coordinate scale (Gaussian: kScale / sigma; Laplacian: 1/sigma, times log2(e) in FP32)
+  double s;           // coordinate scale (Gaussian: kScale / sigma; Laplacian: log2(e) / sigma)
   double kappa;       // 1 / (s sigma^2): turns a scaled difference into (y - x) / sigma^2
   double inv_s2;      // 1 / sigma^2
   int family;         // KernelFamily
   // Laplacian profile in the scaled radius u' = |d|: K0 = P0(u') E, K1 = P1(u') E, K2 = P2(u') E with
-  // E = exp(-u') (FP64) or 2^-u' (FP32, coefficients rescaled). grad_y K = -K1 kappa d, Hessian = kappa^2 K2 d d^T
+  // E = 2^-u' (coefficients rescaled). grad_y K = -K1 kappa d, Hessian = kappa^2 K2 d d^T
   // - K1/sigma^2 I. Row r holds the coefficients of P_r in increasing degree (zeros past the order).
   float lc[3][5];
   double dc[3][5];
@@ -246,7 +295,7 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 }
 
 // kCullR2<V>: a scaled squared distance beyond which every radial factor is exactly zero in the arithmetic of V
-// (FP32: ex2.approx.ftz of an argument below -126 flushes to +0; FP64: exp below -745.2 underflows to 0), with a
+// (FP32: ex2.approx.ftz of an argument below -126 flushes to +0; FP64: exp2_neg is zero from 1022 on), with a
 // margin for the FP32 rounding of the box test that uses it.
 struct Gauss {
   template <typename V>
@@ -255,14 +304,14 @@ struct Gauss {
     return {e, e, e};
   }
   template <typename V>
-  static constexpr float kCullR2 = VT<V>::kLanes == 2 ? 127.0f : 746.0f;
+  static constexpr float kCullR2 = VT<V>::kLanes == 2 ? 127.0f : 1024.0f;
 };
 
 struct Laplacian {
   template <typename V>
   static __device__ __forceinline__ KV<V> eval(const Frame& f, V r2);
   template <typename V>
-  static constexpr float kCullR2 = VT<V>::kLanes == 2 ? 127.0f * 127.0f : 746.0f * 746.0f;  // the radius u = |d|
+  static constexpr float kCullR2 = VT<V>::kLanes == 2 ? 127.0f * 127.0f : 1024.0f * 1024.0f;  // the radius u = |d|
 };
 
 // Axis-aligned box of the scaled coordinates held by a block of threads: per-thread (lo, hi), reduced over the
@@ -332,7 +381,7 @@ __device__ __forceinline__ KV<F2> Laplacian::eval<F2>(const Frame& f, F2 r2) {
 }
 template <>
 __device__ __forceinline__ KV<double> Laplacian::eval<double>(const Frame& f, double r2) {
-  const double u = sqrt(r2), e = exp(-u);
+  const double u = sqrt(r2), e = exp2_neg(u);
   return {e * horner5(f.dc[0], u), e * horner5(f.dc[1], u), e * horner5(f.dc[2], u)};
 }
 
@@ -495,6 +544,7 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
   constexpr float kZeroR2 = Fam::template kCullR2<V>;
   const int gx = (n + TPB * RT - 1) / (TPB * RT);
   __shared__ float tbox[6];  // the segment's target box, in shared memory (re-read per tile, not held in registers)
+  VT<V>::setup();
 
   const long long u_end = sk_start(blockIdx.x + 1, W, C);
   long long u = sk_start(blockIdx.x, W, C);
@@ -952,8 +1002,8 @@ inline size_t pairs_ws_bytes_any(int64_t n, int64_t m) {
 
 inline bool bad_kernel(int kernel) { return !(kernel == kGauss || (kernel >= kLaplacian0 && kernel <= kLaplacianMax)); }
 
-// Frame of one kernel width. `fp32` selects the FP32 scaling (exp2-based) or the FP64 one (exp-based).
-inline Frame make_frame(const double* origin, double sigma, int kernel, bool fp32) {
+// Frame of one kernel width. Coordinates are scaled so that the kernel's exponential is a power of two.
+inline Frame make_frame(const double* origin, double sigma, int kernel) {
   Frame f = {};
   f.family = kernel;
   f.o0 = origin ? origin[0] : 0.0;
@@ -961,7 +1011,7 @@ inline Frame make_frame(const double* origin, double sigma, int kernel, bool fp3
   f.o2 = origin ? origin[2] : 0.0;
   constexpr double kLog2e = 1.44269504088896340736;
   if (kernel == kGauss) {
-    f.s = (fp32 ? VT<F2>::kScale : VT<double>::kScale) / sigma;
+    f.s = kScale / sigma;
   } else {
     // P0 = lapPol of the order (Matern polynomial); P1 = (P0 - P0') / u and P2 = (P1 - P1') / u when the division
     // is exact (the constant terms cancel), else zero -- the reference's derivative tables for orders 0 and 1.
@@ -979,15 +1029,14 @@ inline Frame make_frame(const double* origin, double sigma, int kernel, bool fp3
       if (d[0] > -1e-12 && d[0] < 1e-12)  // exact in rationals; rounding leaves ~1e-17
         for (int k = 0; k < 4; ++k) c[r][k] = d[k + 1];
     }
-    const double unit = fp32 ? kLog2e : 1.0;  // FP32 works in u' = log2(e) u so that E = 2^-u'
-    f.s = unit / sigma;
+    f.s = kLog2e / sigma;  // u' = log2(e) u, E = 2^-u'
     double pw = 1.0;
     for (int k = 0; k < 5; ++k) {
       for (int r = 0; r < 3; ++r) {
         f.dc[r][k] = c[r][k] * pw;
         f.lc[r][k] = (float)(c[r][k] * pw);
       }
-      pw /= unit;
+      pw /= kLog2e;
     }
   }
   f.kappa = 1.0 / (f.s * sigma * sigma);

@@ -1,4 +1,4 @@
-// Symmetric all-pairs kernel for self-interaction sums (targets and sources are the same n points), FP32 only.
+// Symmetric all-pairs kernel for self-interaction sums (targets and sources are the same n points).
 //
 // A sum out_k = sum_l f(k, l) over the same point set evaluates every unordered pair twice in pairs_kernel. When
 // f(l, k) follows from the quantities of f(k, l) (the kernel value, the dot products and the difference vector, up to
@@ -28,12 +28,17 @@
 // Op interface (besides Params, finalize_sym):
 //   NSS                                  source fields staged per source (scaled coordinates 0-2 first)
 //   NR, NC                               row and column accumulators per point
-//   SymTgt                               per-lane-group (two targets) register state
-//   load_target_sym(P, i0, i1, v0, v1, SymTgt&)     targets i0, i1 (< n); v0 / v1 false = padding (zero payload)
+//   SymTgt<V>                            per-lane-group register state (V = F2: two targets, V = double: one)
+//   load_target_sym<V>(P, i0, i1, v0, v1, SymTgt<V>&)  targets i0, i1 (< n); v0 / v1 false = padding (zero payload)
 //   source_fields_sym(P, l, double* f)   NSS fields of source l (FP64)
-//   pair_sym<COL>(const Frame&, const SymTgt&, const F2* s, F2* row, F2* col)
+//   pair_sym<COL, Fam, V>(const Frame&, const SymTgt<V>&, const V* s, V* row, V* col)
 //   finalize_sym(P, i, const double* row, const double* col)
+//
+// FP64 (V = double): one target per lane group, sources staged as doubles, row sums, column sums and column partials
+// in FP64; the rotating accumulator costs two shuffles per field. What it saves is the exponential (about a third of
+// an FP64 pair) and the shared products, on a pipe of half the FP32 rate.
 #pragma once
+#include "launch_config.cuh"
 #include "lddmm_common.cuh"
 
 #ifndef LDDMM_SYM
@@ -62,8 +67,28 @@ constexpr int kSymxUnroll = LDDMM_SYMX_UNROLL;
 // sources at every step (no broadcast), so the record size is what the loads cost: compact records hold each field
 // once in FP32 (float4 groups) and the packed (f, f) operands are formed in registers; the duplicated layout of
 // pairs_kernel (Unit<F2>: one 16-byte load gives two packed operands) reads twice the bytes.
+template <int NF, int TPB, typename V>
+struct SymStage;
 template <int NF, int TPB>
-struct SymStage {
+struct SymStage<NF, TPB, double> {
+  static constexpr int NQ = (NF + 1) / 2;  // 16-byte units of two fields
+  using T = double2;
+  static __device__ __forceinline__ void store(T (*sm)[TPB], int t, const double* fl) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) sm[q][t] = make_double2(fl[2 * q], fl[2 * q + 1]);
+  }
+  static __device__ __forceinline__ void load(const T (*sm)[TPB], int src, double* sv) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const double2 w = sm[q][src];
+      sv[2 * q] = w.x;
+      sv[2 * q + 1] = w.y;
+    }
+  }
+  static constexpr int kFields = 2 * NQ;
+};
+template <int NF, int TPB>
+struct SymStage<NF, TPB, F2> {
 #if LDDMM_SYM_COMPACT
   static constexpr int NQ = (NF + 3) / 4;  // float4 groups
   using T = float4;
@@ -127,8 +152,9 @@ struct SymPlan {
   size_t col_off = 0, ws_bytes = 0;
 };
 
+// row_bytes, col_bytes: size of one row / column partial
 template <int TPB, int RT>
-inline SymPlan make_sym_plan(int64_t n, int nr, int nc, int ctas_per_sm) {
+inline SymPlan make_sym_plan(int64_t n, int nr, int nc, int ctas_per_sm, size_t row_bytes, size_t col_bytes) {
   SymPlan p;
   if (n <= 0) return p;
   constexpr int64_t B = (int64_t)TPB * RT;
@@ -144,44 +170,43 @@ inline SymPlan make_sym_plan(int64_t n, int nr, int nc, int ctas_per_sm) {
     if (c1 - c0 + 1 > smax) smax = c1 - c0 + 1;
   }
   p.S = smax;
-  p.col_off = ((size_t)p.S * (size_t)nr * (size_t)n * sizeof(float2) + 255) & ~(size_t)255;
-  p.ws_bytes = p.col_off + (size_t)sym_tri(p.nblk) * (size_t)nc * (size_t)B * sizeof(float);
+  p.col_off = ((size_t)p.S * (size_t)nr * (size_t)n * row_bytes + 255) & ~(size_t)255;
+  p.ws_bytes = p.col_off + (size_t)sym_tri(p.nblk) * (size_t)nc * (size_t)B * col_bytes;
   return p;
 }
 
-template <class Op, int TPB, int RT, bool COL, class Fam>
-__device__ __forceinline__ void sym_tile(const Frame& f, const typename Op::SymTgt (&tgt)[RT / 2],
-                                         const typename SymStage<Op::NSS, TPB>::T (*sm)[TPB], float (*colacc)[TPB],
-                                         F2 (&acc)[RT / 2][Op::NR]) {
-  using St = SymStage<Op::NSS, TPB>;
-  constexpr int G = RT / 2, W = TPB / 32;
+template <class Op, int TPB, int RT, bool COL, class Fam, typename V>
+__device__ __forceinline__ void sym_tile(const Frame& f,
+                                         const typename Op::template SymTgt<V> (&tgt)[RT / VT<V>::kLanes],
+                                         const typename SymStage<Op::NSS, TPB, V>::T (*sm)[TPB],
+                                         typename VT<V>::Scalar (*colacc)[TPB],
+                                         V (&acc)[RT / VT<V>::kLanes][Op::NR]) {
+  using St = SymStage<Op::NSS, TPB, V>;
+  using S = typename VT<V>::Scalar;
+  constexpr int G = RT / VT<V>::kLanes, W = TPB / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll 1
   for (int ph = 0; ph < W; ++ph) {
     const int chunk = (warp + ph) % W;
-    float cs[Op::NC];
+    S cs[Op::NC];
 #pragma unroll
-    for (int c = 0; c < Op::NC; ++c) cs[c] = 0.f;
+    for (int c = 0; c < Op::NC; ++c) cs[c] = S(0);
 #pragma unroll kSymUnroll
     for (int s = 0; s < 32; ++s) {
       const int src = chunk * 32 + ((lane + s) & 31);
-      F2 sv[St::kFields];
+      V sv[St::kFields];
       St::load(sm, src, sv);
       if constexpr (COL) {
-        F2 col[Op::NC];
+        V col[Op::NC];
 #pragma unroll
-        for (int c = 0; c < Op::NC; ++c) col[c] = f2(cs[c], 0.f);
+        for (int c = 0; c < Op::NC; ++c) col[c] = VT<V>::first(cs[c]);
 #pragma unroll
-        for (int g = 0; g < G; ++g) Op::template pair_sym<true, Fam>(f, tgt[g], sv, acc[g], col);
+        for (int g = 0; g < G; ++g) Op::template pair_sym<true, Fam, V>(f, tgt[g], sv, acc[g], col);
 #pragma unroll
-        for (int c = 0; c < Op::NC; ++c) {
-          float lo, hi;
-          split(col[c], lo, hi);
-          cs[c] = __shfl_sync(0xffffffffu, lo + hi, (lane + 1) & 31);
-        }
+        for (int c = 0; c < Op::NC; ++c) cs[c] = __shfl_sync(0xffffffffu, VT<V>::hsum(col[c]), (lane + 1) & 31);
       } else {
 #pragma unroll
-        for (int g = 0; g < G; ++g) Op::template pair_sym<false, Fam>(f, tgt[g], sv, acc[g], nullptr);
+        for (int g = 0; g < G; ++g) Op::template pair_sym<false, Fam, V>(f, tgt[g], sv, acc[g], nullptr);
       }
     }
     if constexpr (COL) {
@@ -192,21 +217,26 @@ __device__ __forceinline__ void sym_tile(const Frame& f, const typename Op::SymT
   }
 }
 
-template <class Op, int TPB, int RT, class Fam = Gauss>
-__global__ void __launch_bounds__(TPB, Op::kSymMinCtas)
+// minimum resident CTAs per SM: the op's for FP32; no register cap in FP64
+template <class Op, typename V>
+constexpr int kSymCtas = std::is_same<V, F2>::value ? Op::kSymMinCtas : 1;
+
+template <class Op, int TPB, int RT, class Fam, typename V>
+__global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
     pairs_kernel_sym(const typename Op::Params P, int n, int nblk, int TT, long long U, int C,
-                     float2* __restrict__ row_ws, float* __restrict__ col_ws) {
-  using St = SymStage<Op::NSS, TPB>;
-  constexpr int L = 2, G = RT / L, NR = Op::NR, NC = Op::NC;
+                     typename VT<V>::Partial* __restrict__ row_ws, typename VT<V>::Scalar* __restrict__ col_ws) {
+  using St = SymStage<Op::NSS, TPB, V>;
+  constexpr int L = VT<V>::kLanes, G = RT / L, NR = Op::NR, NC = Op::NC;
   constexpr int B = TPB * RT;
   static_assert(TPB % 32 == 0 && RT % L == 0, "launch shape");
   __shared__ typename St::T sm[St::NQ][TPB];
-  __shared__ float colacc[NC][TPB];
-  // compensated row sums of the segment, one private column per thread (G * NR * 2 rows of TPB): dynamic shared
+  __shared__ typename VT<V>::Scalar colacc[NC][TPB];
+  // compensated row sums of the segment, one private column per thread (G * NR * Comp<V>::kWords rows of TPB): dynamic shared
   // memory, so that 8 targets per thread may take more than the 48 KiB of static shared memory
   extern __shared__ __align__(16) unsigned char sym_dyn_smem[];
-  F2 (*cs)[TPB] = reinterpret_cast<F2 (*)[TPB]>(sym_dyn_smem);
+  V (*cs)[TPB] = reinterpret_cast<V (*)[TPB]>(sym_dyn_smem);
   const Frame& f = P.f;
+  VT<V>::setup();  // the staging barrier of the first tile follows
 
   const long long u_end = sk_start(blockIdx.x + 1, U, C);
   long long u = sk_start(blockIdx.x, U, C);
@@ -219,12 +249,12 @@ __global__ void __launch_bounds__(TPB, Op::kSymMinCtas)
     const int slot = (int)blockIdx.x - sk_cta_of(off, U, C);
     const int base = i * B + threadIdx.x;
 
-    typename Op::SymTgt tgt[G];
+    typename Op::template SymTgt<V> tgt[G];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-      const int i0 = base + (g * L) * TPB, i1 = base + (g * L + 1) * TPB;
-      Op::load_target_sym(P, i0 < n ? i0 : n - 1, i1 < n ? i1 : n - 1, i0 < n, i1 < n, tgt[g]);
-      Comp<F2> z;
+      const int i0 = base + (g * L) * TPB, i1 = base + (g * L + L - 1) * TPB;
+      Op::template load_target_sym<V>(P, i0 < n ? i0 : n - 1, i1 < n ? i1 : n - 1, i0 < n, i1 < n, tgt[g]);
+      Comp<V> z;
       z.zero();
 #pragma unroll
       for (int c = 0; c < NR; ++c) z.template store<TPB>(cs, g * NR + c, threadIdx.x);
@@ -241,23 +271,23 @@ __global__ void __launch_bounds__(TPB, Op::kSymMinCtas)
         if (l < n) Op::source_fields_sym(P, l, fl);
         St::store(sm, threadIdx.x, fl);
 #pragma unroll
-        for (int c = 0; c < NC; ++c) colacc[c][threadIdx.x] = 0.f;
+        for (int c = 0; c < NC; ++c) colacc[c][threadIdx.x] = 0;
       }
       __syncthreads();
-      F2 acc[G][NR];
+      V acc[G][NR];
 #pragma unroll
       for (int g = 0; g < G; ++g)
 #pragma unroll
-        for (int c = 0; c < NR; ++c) acc[g][c] = VT<F2>::zero();
+        for (int c = 0; c < NR; ++c) acc[g][c] = VT<V>::zero();
       if (diag)
-        sym_tile<Op, TPB, RT, false, Fam>(f, tgt, sm, colacc, acc);
+        sym_tile<Op, TPB, RT, false, Fam, V>(f, tgt, sm, colacc, acc);
       else
-        sym_tile<Op, TPB, RT, true, Fam>(f, tgt, sm, colacc, acc);
+        sym_tile<Op, TPB, RT, true, Fam, V>(f, tgt, sm, colacc, acc);
 #pragma unroll
       for (int g = 0; g < G; ++g)
 #pragma unroll
         for (int c = 0; c < NR; ++c) {
-          Comp<F2> m;
+          Comp<V> m;
           m.template load<TPB>(cs, g * NR + c, threadIdx.x);
           m.merge(acc[g][c]);
           m.template store<TPB>(cs, g * NR + c, threadIdx.x);
@@ -280,7 +310,7 @@ __global__ void __launch_bounds__(TPB, Op::kSymMinCtas)
         if (idx < n) {
 #pragma unroll
           for (int c = 0; c < NR; ++c) {
-            Comp<F2> m;
+            Comp<V> m;
             m.template load<TPB>(cs, g * NR + c, threadIdx.x);
             row_ws[((size_t)slot * NR + c) * (size_t)n + idx] = m.partial(k);
           }
@@ -300,10 +330,11 @@ __global__ void __launch_bounds__(TPB, Op::kSymMinCtas)
 // of dependent loads (at 2,562 points: 11 CTAs, ~11 us, latency-bound); several threads shorten the chain and
 // spread the points over more CTAs.
 constexpr int kFinThreads = 256;
-template <class Op, int TPB, int RT>
+template <class Op, int TPB, int RT, typename V>
 __global__ void __launch_bounds__(kFinThreads)
     finalize_sym_kernel(const typename Op::Params P, int n, int nblk, int TT, long long U, int C,
-                        const float2* __restrict__ row_ws, const float* __restrict__ col_ws, int tpp) {
+                        const typename VT<V>::Partial* __restrict__ row_ws,
+                        const typename VT<V>::Scalar* __restrict__ col_ws, int tpp) {
   constexpr int B = TPB * RT, NV = Op::NR + Op::NC;
   __shared__ double red[kFinThreads][NV];
   const int np = kFinThreads / tpp;
@@ -352,14 +383,14 @@ inline int sym_finalize_grid(int64_t n, int tpp, int threads) {
 }
 
 // Dynamic shared memory of pairs_kernel_sym (its compensated row sums).
-template <class Op, int TPB, int RT>
+template <class Op, int TPB, int RT, typename V>
 constexpr size_t sym_dyn_smem_bytes() {
-  return (size_t)(RT / 2) * Op::NR * 2 * TPB * sizeof(F2);
+  return (size_t)(RT / VT<V>::kLanes) * Op::NR * Comp<V>::kWords * TPB * sizeof(V);
 }
 
 // Declare the kernel's dynamic shared memory, once per device (the attribute belongs to the device's context):
 // without it static + dynamic shared memory may not exceed 48 KiB. Returns false when the device refuses.
-template <class Op, int TPB, int RT, class Fam = Gauss>
+template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2>
 inline bool sym_prepare() {
   static signed char state[64] = {};
   int dev = 0;
@@ -369,51 +400,120 @@ inline bool sym_prepare() {
   }
   if (dev < 0 || dev >= 64) return false;
   if (state[dev] == 0) {
-    const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&pairs_kernel_sym<Op, TPB, RT, Fam>),
+    const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&pairs_kernel_sym<Op, TPB, RT, Fam, V>),
                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)sym_dyn_smem_bytes<Op, TPB, RT>());
+                                               (int)sym_dyn_smem_bytes<Op, TPB, RT, V>());
     if (e != cudaSuccess) cudaGetLastError();
     state[dev] = e == cudaSuccess ? 1 : -1;
   }
   return state[dev] > 0;
 }
 
-template <class Op, int TPB, int RT, class Fam = Gauss>
+template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2>
 inline int sym_ctas_per_sm() {
   static int cached = 0;
   if (cached == 0) {
-    sym_prepare<Op, TPB, RT, Fam>();
-    int c = resident_ctas(reinterpret_cast<const void*>(&pairs_kernel_sym<Op, TPB, RT, Fam>), TPB,
-                          sym_dyn_smem_bytes<Op, TPB, RT>());
+    sym_prepare<Op, TPB, RT, Fam, V>();
+    int c = resident_ctas(reinterpret_cast<const void*>(&pairs_kernel_sym<Op, TPB, RT, Fam, V>), TPB,
+                          sym_dyn_smem_bytes<Op, TPB, RT, V>());
     cached = c > 0 ? c : 2;
   }
   return cached;
 }
 
-template <class Op, int TPB, int RT, class Fam = Gauss>
-inline size_t sym_ws_bytes(int64_t n) {
-  return make_sym_plan<TPB, RT>(n, Op::NR, Op::NC, sym_ctas_per_sm<Op, TPB, RT, Fam>()).ws_bytes;
+template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2>
+inline SymPlan sym_plan(int64_t n) {
+  return make_sym_plan<TPB, RT>(n, Op::NR, Op::NC, sym_ctas_per_sm<Op, TPB, RT, Fam, V>(),
+                                sizeof(typename VT<V>::Partial), sizeof(typename VT<V>::Scalar));
 }
 
-template <class Op, int TPB, int RT, class Fam = Gauss>
+template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2>
+inline size_t sym_ws_bytes(int64_t n) {
+  return sym_plan<Op, TPB, RT, Fam, V>(n).ws_bytes;
+}
+
+template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2>
 inline int run_pairs_sym(const typename Op::Params& P, int64_t n, void* ws, size_t ws_bytes, cudaStream_t stream) {
   if (n <= 0) return kOk;
   if (n > INT32_MAX / 4) return kInvalidArgument;
-  const SymPlan plan = make_sym_plan<TPB, RT>(n, Op::NR, Op::NC, sym_ctas_per_sm<Op, TPB, RT, Fam>());
+  const SymPlan plan = sym_plan<Op, TPB, RT, Fam, V>(n);
   if (plan.ws_bytes > ws_bytes) return kWorkspaceTooSmall;
   if (ws == nullptr) return kInvalidArgument;
-  if (!sym_prepare<Op, TPB, RT, Fam>()) return kLaunchFailure;
-  auto* row_ws = reinterpret_cast<float2*>(ws);
-  auto* col_ws = reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + plan.col_off);
-  pairs_kernel_sym<Op, TPB, RT, Fam><<<plan.C, TPB, sym_dyn_smem_bytes<Op, TPB, RT>(), stream>>>(
+  if (!sym_prepare<Op, TPB, RT, Fam, V>()) return kLaunchFailure;
+  auto* row_ws = reinterpret_cast<typename VT<V>::Partial*>(ws);
+  auto* col_ws = reinterpret_cast<typename VT<V>::Scalar*>(reinterpret_cast<char*>(ws) + plan.col_off);
+  pairs_kernel_sym<Op, TPB, RT, Fam, V><<<plan.C, TPB, sym_dyn_smem_bytes<Op, TPB, RT, V>(), stream>>>(
       P, (int)n, plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws);
   const int fb = kFinThreads, tpp = sym_finalize_tpp(plan);
-  finalize_sym_kernel<Op, TPB, RT><<<sym_finalize_grid(n, tpp, fb), fb, 0, stream>>>(P, (int)n, plan.nblk, plan.TT,
-                                                                                      plan.U, plan.C, row_ws, col_ws,
-                                                                                      tpp);
+  finalize_sym_kernel<Op, TPB, RT, V><<<sym_finalize_grid(n, tpp, fb), fb, 0, stream>>>(
+      P, (int)n, plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws, tpp);
   return cudaPeekAtLastError() == cudaSuccess ? kOk : kLaunchFailure;
 }
 
+
+// FP64 launch shape of a symmetric op (the adjoint step declares kSym64Adjoint).
+template <class Op, class = void>
+struct Sym64Shape {
+  static constexpr int kTpb = kTpbSym64, kRt = kRtSym64;
+};
+template <class Op>
+struct Sym64Shape<Op, std::void_t<decltype(Op::kSym64Adjoint)>> {
+  static constexpr int kTpb = kTpbSym64Adj, kRt = kRtSym64Adj;
+};
+
+// Whether an FP64 self-sum takes the symmetric kernel. Its column partials are bounded at 2 GiB (150,000 points for
+// the six-field steps): they grow with n^2, and larger sets keep the ordered-pair kernel, whose scratch does not.
+constexpr int64_t kSym64MaxColBytes = int64_t(2) << 30;
+template <class Op>
+inline int64_t sym64_max_n() {
+  constexpr int64_t B = Sym64Shape<Op>::kTpb * Sym64Shape<Op>::kRt;
+  constexpr int64_t tri = kSym64MaxColBytes / (int64_t)(Op::NC * B * sizeof(double));  // blocks: tri(nblk) <= this
+  static const int64_t nblk = [] {
+    int64_t k = 1;
+    while (sym_tri(k + 1) <= tri) ++k;
+    return k;
+  }();
+  return nblk * B;
+}
+template <class Op>
+inline bool sym64_takes(int64_t n) {
+  return LDDMM_SYM != 0 && n > 0 && n <= sym64_max_n<Op>();
+}
+
+template <class Op, class Fam>
+inline size_t sym64_ws_bytes_fam(int64_t n) {
+  if (n <= kSym64SmallN) return sym_ws_bytes<Op, kTpbSym64Small, kRtSym64Small, Fam, double>(n);
+  return sym_ws_bytes<Op, Sym64Shape<Op>::kTpb, Sym64Shape<Op>::kRt, Fam, double>(n);
+}
+template <class Op>
+inline size_t sym64_ws_bytes(int64_t n, int family) {
+  return family == kGauss ? sym64_ws_bytes_fam<Op, Gauss>(n) : sym64_ws_bytes_fam<Op, Laplacian>(n);
+}
+
+// Scratch for every point count up to n.
+template <class Op>
+inline size_t sym64_ws_bytes_upto(int64_t n) {
+  if (LDDMM_SYM == 0) return 0;
+  size_t b = 0;
+  for (const int64_t k : {n < kSym64SmallN ? n : kSym64SmallN, n < sym64_max_n<Op>() ? n : sym64_max_n<Op>()})
+    for (const int family : {(int)kGauss, (int)kLaplacian0}) {
+      const size_t v = k > 0 ? sym64_ws_bytes<Op>(k, family) : 0;
+      b = v > b ? v : b;
+    }
+  return b;
+}
+
+template <class Op, class Fam>
+inline int run_sym64_fam(const typename Op::Params& P, int64_t n, void* ws, size_t wsb, cudaStream_t st) {
+  if (n <= kSym64SmallN) return run_pairs_sym<Op, kTpbSym64Small, kRtSym64Small, Fam, double>(P, n, ws, wsb, st);
+  return run_pairs_sym<Op, Sym64Shape<Op>::kTpb, Sym64Shape<Op>::kRt, Fam, double>(P, n, ws, wsb, st);
+}
+// The FP64 launch of a symmetric op, for the kernel family of its frame.
+template <class Op>
+inline int run_sym64(const typename Op::Params& P, int64_t n, void* ws, size_t wsb, cudaStream_t st) {
+  if (P.f.family == kGauss) return run_sym64_fam<Op, Gauss>(P, n, ws, wsb, st);
+  return run_sym64_fam<Op, Laplacian>(P, n, ws, wsb, st);
+}
 
 // ---------------------------------------------------------------------------------------------------------
 // Expanded-distance form of the symmetric kernel, for sums whose pair term is the kernel value times a payload of
@@ -434,9 +534,9 @@ inline int run_pairs_sym(const typename Op::Params& P, int64_t n, void* ws, size
 // ---------------------------------------------------------------------------------------------------------
 template <class Op, int TPB, int RT, bool COL, bool X>
 __device__ __forceinline__ void symx_tile(const F2 (&yt)[RT / 2][3], const F2 (&tp)[RT / 2][Op::NP],
-                                          const typename SymStage<4 + Op::NP, TPB>::T (*sm)[TPB],
+                                          const typename SymStage<4 + Op::NP, TPB, F2>::T (*sm)[TPB],
                                           float (*colacc)[TPB], F2 (&acc)[RT / 2][Op::NP]) {
-  using St = SymStage<4 + Op::NP, TPB>;
+  using St = SymStage<4 + Op::NP, TPB, F2>;
   constexpr int G = RT / 2, NP = Op::NP, W = TPB / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll 1
@@ -504,7 +604,7 @@ template <class Op, int TPB, int RT>
 __global__ void __launch_bounds__(TPB, Op::kSymMinCtas)
     pairs_kernel_symx(const typename Op::Params P, int n, int nblk, int TT, long long U, int C,
                       float2* __restrict__ row_ws, float* __restrict__ col_ws) {
-  using St = SymStage<4 + Op::NP, TPB>;
+  using St = SymStage<4 + Op::NP, TPB, F2>;
   constexpr int L = 2, G = RT / L, NP = Op::NP;
   constexpr int B = TPB * RT;
   static_assert(TPB % 32 == 0 && RT % L == 0, "launch shape");
@@ -707,14 +807,14 @@ inline int symx_ctas_per_sm() {
 
 template <class Op, int TPB, int RT>
 inline size_t symx_ws_bytes(int64_t n) {
-  return make_sym_plan<TPB, RT>(n, Op::NP, Op::NP, symx_ctas_per_sm<Op, TPB, RT>()).ws_bytes;
+  return make_sym_plan<TPB, RT>(n, Op::NP, Op::NP, symx_ctas_per_sm<Op, TPB, RT>(), sizeof(float2), sizeof(float)).ws_bytes;
 }
 
 template <class Op, int TPB, int RT>
 inline int run_pairs_symx(const typename Op::Params& P, int64_t n, void* ws, size_t ws_bytes, cudaStream_t stream) {
   if (n <= 0) return kOk;
   if (n > INT32_MAX / 4) return kInvalidArgument;
-  const SymPlan plan = make_sym_plan<TPB, RT>(n, Op::NP, Op::NP, symx_ctas_per_sm<Op, TPB, RT>());
+  const SymPlan plan = make_sym_plan<TPB, RT>(n, Op::NP, Op::NP, symx_ctas_per_sm<Op, TPB, RT>(), sizeof(float2), sizeof(float));
   if (plan.ws_bytes > ws_bytes) return kWorkspaceTooSmall;
   if (ws == nullptr) return kInvalidArgument;
   if (!symx_prepare<Op, TPB, RT>()) return kLaunchFailure;
@@ -723,9 +823,8 @@ inline int run_pairs_symx(const typename Op::Params& P, int64_t n, void* ws, siz
   pairs_kernel_symx<Op, TPB, RT><<<plan.C, TPB, symx_dyn_smem_bytes<Op, TPB, RT>(), stream>>>(
       P, (int)n, plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws);
   const int fb = kFinThreads, tpp = sym_finalize_tpp(plan);
-  finalize_sym_kernel<Op, TPB, RT><<<sym_finalize_grid(n, tpp, fb), fb, 0, stream>>>(P, (int)n, plan.nblk, plan.TT,
-                                                                                      plan.U, plan.C, row_ws, col_ws,
-                                                                                      tpp);
+  finalize_sym_kernel<Op, TPB, RT, F2><<<sym_finalize_grid(n, tpp, fb), fb, 0, stream>>>(
+      P, (int)n, plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws, tpp);
   return cudaPeekAtLastError() == cudaSuccess ? kOk : kLaunchFailure;
 }
 

@@ -214,26 +214,27 @@ struct OpSOFwdSym {
   using Params = OpSOFwd::Params;
   static constexpr int NSS = 6, NR = 6, NC = 6;
   static constexpr int kSymMinCtas = LDDMM_SOFWD_SYM_MIN_CTAS;
-  struct SymTgt { F2 y0, y1, y2, a0, a1, a2; };
+  template <typename V> struct SymTgt { V y0, y1, y2, a0, a1, a2; };
+  template <typename V>
   static __device__ __forceinline__ void load_target_sym(const Params& P, int i0, int i1, bool v0, bool v1,
-                                                         SymTgt& t) {
-    t.y0 = tgt_coord<F2>(P.x, i0, i1, 0, P.f.o0, P.f.s);
-    t.y1 = tgt_coord<F2>(P.x, i0, i1, 1, P.f.o1, P.f.s);
-    t.y2 = tgt_coord<F2>(P.x, i0, i1, 2, P.f.o2, P.f.s);
-    t.a0 = VT<F2>::pack(v0 ? P.a[3 * i0] : 0.0, v1 ? P.a[3 * i1] : 0.0);
-    t.a1 = VT<F2>::pack(v0 ? P.a[3 * i0 + 1] : 0.0, v1 ? P.a[3 * i1 + 1] : 0.0);
-    t.a2 = VT<F2>::pack(v0 ? P.a[3 * i0 + 2] : 0.0, v1 ? P.a[3 * i1 + 2] : 0.0);
+                                                         SymTgt<V>& t) {
+    t.y0 = tgt_coord<V>(P.x, i0, i1, 0, P.f.o0, P.f.s);
+    t.y1 = tgt_coord<V>(P.x, i0, i1, 1, P.f.o1, P.f.s);
+    t.y2 = tgt_coord<V>(P.x, i0, i1, 2, P.f.o2, P.f.s);
+    t.a0 = VT<V>::pack(v0 ? P.a[3 * i0] : 0.0, v1 ? P.a[3 * i1] : 0.0);
+    t.a1 = VT<V>::pack(v0 ? P.a[3 * i0 + 1] : 0.0, v1 ? P.a[3 * i1 + 1] : 0.0);
+    t.a2 = VT<V>::pack(v0 ? P.a[3 * i0 + 2] : 0.0, v1 ? P.a[3 * i1 + 2] : 0.0);
   }
   // fields: x' (0-2), a (3-5)
   static __device__ __forceinline__ void source_fields_sym(const Params& P, int l, double* f) {
     OpSOFwd::source_fields(P, l, f);
   }
   // Fam: the radial factors k0 (K a) and k1 (the momentum term); both are e for the Gaussian
-  template <bool COL, class Fam>
-  static __device__ __forceinline__ void pair_sym(const Frame& f, const SymTgt& t, const F2* s, F2* row, F2* col) {
-    const F2 d0 = t.y0 - s[0], d1 = t.y1 - s[1], d2 = t.y2 - s[2];
-    const KV<F2> k = Fam::template eval<F2>(f, sqdist(d0, d1, d2));
-    const F2 ec = k.k1 * dot3(t.a0, t.a1, t.a2, s[3], s[4], s[5]);
+  template <bool COL, class Fam, typename V>
+  static __device__ __forceinline__ void pair_sym(const Frame& f, const SymTgt<V>& t, const V* s, V* row, V* col) {
+    const V d0 = t.y0 - s[0], d1 = t.y1 - s[1], d2 = t.y2 - s[2];
+    const KV<V> k = Fam::template eval<V>(f, sqdist(d0, d1, d2));
+    const V ec = k.k1 * dot3(t.a0, t.a1, t.a2, s[3], s[4], s[5]);
     row[0] = fma(k.k0, s[3], row[0]);
     row[1] = fma(k.k0, s[4], row[1]);
     row[2] = fma(k.k0, s[5], row[2]);
@@ -270,23 +271,25 @@ struct OpSOFwdSym {
 struct OpSOBwdSym {
   using Params = OpSOBwd::Params;
   static constexpr int NSS = 12, NR = 6, NC = 6;
+  static constexpr bool kSym64Adjoint = true;
   static constexpr int kSymMinCtas = LDDMM_SOBWD_SYM_MIN_CTAS;
-  struct SymTgt { F2 y0, y1, y2, a0, a1, a2, b0, b1, b2, p0, p1, p2, q0, q1, q2, cd, k2; };
+  template <typename V> struct SymTgt { V y0, y1, y2, a0, a1, a2, b0, b1, b2, p0, p1, p2, q0, q1, q2, cd, k2; };
+  template <typename V>
   static __device__ __forceinline__ void load_target_sym(const Params& P, int i0, int i1, bool v0, bool v1,
-                                                         SymTgt& t) {
+                                                         SymTgt<V>& t) {
     const double k = P.f.kappa;
     auto fld = [&](const double* a, int c, double sc) {
-      return VT<F2>::pack(v0 ? sc * a[3 * i0 + c] : 0.0, v1 ? sc * a[3 * i1 + c] : 0.0);
+      return VT<V>::pack(v0 ? sc * a[3 * i0 + c] : 0.0, v1 ? sc * a[3 * i1 + c] : 0.0);
     };
-    t.y0 = tgt_coord<F2>(P.x, i0, i1, 0, P.f.o0, P.f.s);
-    t.y1 = tgt_coord<F2>(P.x, i0, i1, 1, P.f.o1, P.f.s);
-    t.y2 = tgt_coord<F2>(P.x, i0, i1, 2, P.f.o2, P.f.s);
+    t.y0 = tgt_coord<V>(P.x, i0, i1, 0, P.f.o0, P.f.s);
+    t.y1 = tgt_coord<V>(P.x, i0, i1, 1, P.f.o1, P.f.s);
+    t.y2 = tgt_coord<V>(P.x, i0, i1, 2, P.f.o2, P.f.s);
     t.a0 = fld(P.a, 0, 1.0); t.a1 = fld(P.a, 1, 1.0); t.a2 = fld(P.a, 2, 1.0);
     t.b0 = fld(P.a, 0, -k * k); t.b1 = fld(P.a, 1, -k * k); t.b2 = fld(P.a, 2, -k * k);
     t.p0 = fld(P.px, 0, -k); t.p1 = fld(P.px, 1, -k); t.p2 = fld(P.px, 2, -k);
     t.q0 = fld(P.pa, 0, 1.0); t.q1 = fld(P.pa, 1, 1.0); t.q2 = fld(P.pa, 2, 1.0);
-    t.cd = VT<F2>::dup(-P.f.inv_s2 / (k * k));
-    t.k2 = VT<F2>::dup(-k * k);
+    t.cd = VT<V>::dup(-P.f.inv_s2 / (k * k));
+    t.k2 = VT<V>::dup(-k * k);
   }
   // fields: x' (0-2), a (3-5), pa (6-8), px' = -kappa px (9-11)
   static __device__ __forceinline__ void source_fields_sym(const Params& P, int l, double* f) {
@@ -294,23 +297,23 @@ struct OpSOBwdSym {
   }
   // Fam: the radial factors k0 (the px'-sum), k1 (first-derivative terms) and k2 (the second-derivative term
   // c2 dq d); all three are e for the Gaussian, where k1 c2 and k2 c2 are one product
-  template <bool COL, class Fam>
-  static __device__ __forceinline__ void pair_sym(const Frame& f, const SymTgt& t, const F2* s, F2* row, F2* col) {
-    const F2 d0 = t.y0 - s[0], d1 = t.y1 - s[1], d2 = t.y2 - s[2];
-    const KV<F2> k = Fam::template eval<F2>(f, sqdist(d0, d1, d2));
-    const F2 w0 = t.q0 - s[6], w1 = t.q1 - s[7], w2 = t.q2 - s[8];
-    const F2 dq = dot3(d0, d1, d2, w0, w1, w2);
-    const F2 c1 = fma(t.a2, s[11], fma(t.a1, s[10], fma(t.a0, s[9], dot3(t.p0, t.p1, t.p2, s[3], s[4], s[5]))));
-    const F2 c2 = dot3(t.b0, t.b1, t.b2, s[3], s[4], s[5]);
-    const F2 ec2 = k.k1 * c2;
-    const F2 eg = fma(k.k2 * c2, dq, k.k1 * c1);
-    const F2 tw = ec2 * t.cd;
-    const F2 v0 = fma(tw, w0, eg * d0), v1 = fma(tw, w1, eg * d1), v2 = fma(tw, w2, eg * d2);
+  template <bool COL, class Fam, typename V>
+  static __device__ __forceinline__ void pair_sym(const Frame& f, const SymTgt<V>& t, const V* s, V* row, V* col) {
+    const V d0 = t.y0 - s[0], d1 = t.y1 - s[1], d2 = t.y2 - s[2];
+    const KV<V> k = Fam::template eval<V>(f, sqdist(d0, d1, d2));
+    const V w0 = t.q0 - s[6], w1 = t.q1 - s[7], w2 = t.q2 - s[8];
+    const V dq = dot3(d0, d1, d2, w0, w1, w2);
+    const V c1 = fma(t.a2, s[11], fma(t.a1, s[10], fma(t.a0, s[9], dot3(t.p0, t.p1, t.p2, s[3], s[4], s[5]))));
+    const V c2 = dot3(t.b0, t.b1, t.b2, s[3], s[4], s[5]);
+    const V ec2 = k.k1 * c2;
+    const V eg = fma(k.k2 * c2, dq, k.k1 * c1);
+    const V tw = ec2 * t.cd;
+    const V v0 = fma(tw, w0, eg * d0), v1 = fma(tw, w1, eg * d1), v2 = fma(tw, w2, eg * d2);
     row[0] += v0;
     row[1] += v1;
     row[2] += v2;
-    const F2 edq = k.k1 * dq;
-    const F2 edqk = edq * t.k2;
+    const V edq = k.k1 * dq;
+    const V edqk = edq * t.k2;
     row[3] = fma(edqk, s[3], fma(k.k0, s[9], row[3]));
     row[4] = fma(edqk, s[4], fma(k.k0, s[10], row[4]));
     row[5] = fma(edqk, s[5], fma(k.k0, s[11], row[5]));
@@ -402,19 +405,20 @@ struct OpFOBwdSym {
   using Params = OpFOBwd::Params;
   static constexpr int NSS = 9, NR = 6, NC = 6;
   static constexpr int kSymMinCtas = LDDMM_FOBWD_SYM_MIN_CTAS;
-  struct SymTgt { F2 y0, y1, y2, p0, p1, p2, a0, a1, a2, q0, q1, q2; };
+  template <typename V> struct SymTgt { V y0, y1, y2, p0, p1, p2, a0, a1, a2, q0, q1, q2; };
+  template <typename V>
   static __device__ __forceinline__ void load_target_sym(const Params& P, int i0, int i1, bool v0, bool v1,
-                                                         SymTgt& t) {
+                                                         SymTgt<V>& t) {
     auto fld = [&](const double* a, int c) {
-      return VT<F2>::pack(v0 ? a[3 * i0 + c] : 0.0, v1 ? a[3 * i1 + c] : 0.0);
+      return VT<V>::pack(v0 ? a[3 * i0 + c] : 0.0, v1 ? a[3 * i1 + c] : 0.0);
     };
     auto qf = [&](int c) {
-      return VT<F2>::pack(v0 ? P.p[3 * i0 + c] - 2.0 * P.w * P.a[3 * i0 + c] : 0.0,
+      return VT<V>::pack(v0 ? P.p[3 * i0 + c] - 2.0 * P.w * P.a[3 * i0 + c] : 0.0,
                           v1 ? P.p[3 * i1 + c] - 2.0 * P.w * P.a[3 * i1 + c] : 0.0);
     };
-    t.y0 = tgt_coord<F2>(P.x, i0, i1, 0, P.f.o0, P.f.s);
-    t.y1 = tgt_coord<F2>(P.x, i0, i1, 1, P.f.o1, P.f.s);
-    t.y2 = tgt_coord<F2>(P.x, i0, i1, 2, P.f.o2, P.f.s);
+    t.y0 = tgt_coord<V>(P.x, i0, i1, 0, P.f.o0, P.f.s);
+    t.y1 = tgt_coord<V>(P.x, i0, i1, 1, P.f.o1, P.f.s);
+    t.y2 = tgt_coord<V>(P.x, i0, i1, 2, P.f.o2, P.f.s);
     t.p0 = fld(P.p, 0); t.p1 = fld(P.p, 1); t.p2 = fld(P.p, 2);
     t.a0 = fld(P.a, 0); t.a1 = fld(P.a, 1); t.a2 = fld(P.a, 2);
     t.q0 = qf(0); t.q1 = qf(1); t.q2 = qf(2);
@@ -424,12 +428,12 @@ struct OpFOBwdSym {
     OpFOBwd::source_fields(P, l, f);
   }
   // Fam: k1 for the adjoint term, k0 for the Q sum (both e for the Gaussian)
-  template <bool COL, class Fam>
-  static __device__ __forceinline__ void pair_sym(const Frame& f, const SymTgt& t, const F2* s, F2* row, F2* col) {
-    const F2 d0 = t.y0 - s[0], d1 = t.y1 - s[1], d2 = t.y2 - s[2];
-    const KV<F2> k = Fam::template eval<F2>(f, sqdist(d0, d1, d2));
-    const F2 c = fma(t.a2, s[8], fma(t.a1, s[7], fma(t.a0, s[6], dot3(t.p0, t.p1, t.p2, s[3], s[4], s[5]))));
-    const F2 ec = k.k1 * c;
+  template <bool COL, class Fam, typename V>
+  static __device__ __forceinline__ void pair_sym(const Frame& f, const SymTgt<V>& t, const V* s, V* row, V* col) {
+    const V d0 = t.y0 - s[0], d1 = t.y1 - s[1], d2 = t.y2 - s[2];
+    const KV<V> k = Fam::template eval<V>(f, sqdist(d0, d1, d2));
+    const V c = fma(t.a2, s[8], fma(t.a1, s[7], fma(t.a0, s[6], dot3(t.p0, t.p1, t.p2, s[3], s[4], s[5]))));
+    const V ec = k.k1 * c;
     row[0] = fma(ec, d0, row[0]);
     row[1] = fma(ec, d1, row[1]);
     row[2] = fma(ec, d2, row[2]);
@@ -475,6 +479,10 @@ size_t shooting_ws_bytes(int64_t n, int precision) {
     upd(pairs_ws_bytes_any<OpFOBwd, F2, kTpbLight, kRtLight>(n, n));
     upd(pairs_ws_bytes_any<OpK, F2, kTpbLight, kRtLight>(n, n));
   } else {
+    upd(sym64_ws_bytes_upto<OpSOFwdSym>(n));
+    upd(sym64_ws_bytes_upto<OpSOBwdSym>(n));
+    upd(sym64_ws_bytes_upto<OpFOBwdSym>(n));
+    upd(sym64_ws_bytes_upto<OpKSymD>(n));
     upd(pairs_ws_bytes_any<OpSOFwd, double, kTpb64, kRt64>(n, n));
     upd(pairs_ws_bytes_any<OpSOBwd, double, kTpb64, kRt64>(n, n));
     upd(pairs_ws_bytes_any<OpFOBwd, double, kTpb64, kRt64>(n, n));
@@ -499,7 +507,7 @@ template <> struct Shape<double> {
 
 template <typename V>
 inline Frame frame(const double* origin, double sigma, int kernel) {
-  return make_frame(origin, sigma, kernel, VT<V>::kLanes == 2);
+  return make_frame(origin, sigma, kernel);
 }
 
 inline double* dots_region(void* ws, size_t pair_bytes) {
@@ -516,11 +524,12 @@ int k_energy_and_update(const double* x, const double* a, int64_t n, const Frame
   OpK::Params P;
   P.y = x; P.x = x; P.a = a; P.out = out; P.f = f;
   P.base = base; P.base_sign = base_sign; P.scale = scale;
-  // K(x) a is a self-sum: FP32 sums evaluate each unordered pair once (pairs_kernel_symx for the Gaussian,
-  // pairs_kernel_sym in the difference form for the Laplacian)
-  constexpr bool kSymOk = std::is_same<V, F2>::value && LDDMM_SYM != 0;
-  const bool gauss = f.family == kGauss;
-  const size_t pb = !kSymOk ? pairs_ws_bytes_any<OpK, V, TPB, RT>(n, n)
+  // K(x) a is a self-sum: each unordered pair once (pairs_kernel_symx for the FP32 Gaussian, pairs_kernel_sym in the
+  // difference form otherwise)
+  constexpr bool kF32 = std::is_same<V, F2>::value;
+  const bool sym = kF32 ? LDDMM_SYM != 0 : sym64_takes<OpKSymD>(n), gauss = f.family == kGauss;
+  const size_t pb = !sym    ? pairs_ws_bytes_any<OpK, V, TPB, RT>(n, n)
+                    : !kF32 ? sym64_ws_bytes<OpKSymD>(n, f.family)
                     : gauss ? symx_ws_bytes<OpKSym, kTpbKSym, kRtKSym>(n)
                             : sym_ws_bytes<OpKSymD, kTpbLight, kRtKSymL, Laplacian>(n);
   if (energy) {
@@ -529,11 +538,13 @@ int k_energy_and_update(const double* x, const double* a, int64_t n, const Frame
     P.dots = dots_region(ws, pb);
   }
   int rc;
-  if constexpr (kSymOk) {
+  if (!sym) {
+    rc = run_pairs_k<OpK, V, TPB, RT>(P, n, n, ws, wsb, st);
+  } else if constexpr (kF32) {
     rc = gauss ? run_pairs_symx<OpKSym, kTpbKSym, kRtKSym>(P, n, ws, wsb, st)
                : run_pairs_sym<OpKSymD, kTpbLight, kRtKSymL, Laplacian>(P, n, ws, wsb, st);
   } else {
-    rc = run_pairs_k<OpK, V, TPB, RT>(P, n, n, ws, wsb, st);
+    rc = run_sym64<OpKSymD>(P, n, ws, wsb, st);
   }
   if (rc != kOk) return rc;
   if (energy) {
@@ -556,6 +567,9 @@ int so_step(const double* x, const double* a, int64_t n, const Frame& f, double 
       return run_pairs_sym<OpSOFwdSym, kTpbLight, kRtSymFwdL, Laplacian>(P, n, ws, wsb, st);
     }
   }
+  if constexpr (!std::is_same<V, F2>::value) {
+    if (row0 == 0 && rows == n && sym64_takes<OpSOFwdSym>(n)) return run_sym64<OpSOFwdSym>(P, n, ws, wsb, st);
+  }
   return run_pairs_k<OpSOFwd, V, Shape<V>::kTpb, Shape<V>::kRt>(P, rows, n, ws, wsb, st);
 }
 
@@ -572,6 +586,9 @@ int so_adjoint_step(const double* x, const double* a, const double* px, const do
       if (f.family == kGauss) return run_pairs_sym<OpSOBwdSym, kTpbHeavy, kRtAdjoint>(P, n, ws, wsb, st);
       return run_pairs_sym<OpSOBwdSym, kTpbHeavy, kRtAdjointSymL, Laplacian>(P, n, ws, wsb, st);
     }
+  }
+  if constexpr (!std::is_same<V, F2>::value) {
+    if (row0 == 0 && rows == n && sym64_takes<OpSOBwdSym>(n)) return run_sym64<OpSOBwdSym>(P, n, ws, wsb, st);
   }
   if (f.family == kGauss) return run_pairs<OpSOBwd, V, Shape<V>::kTpbH, Shape<V>::kRtH, Gauss>(P, rows, n, ws, wsb, st);
   return run_pairs<OpSOBwd, V, Shape<V>::kTpbH, Shape<V>::kRtHL, Laplacian>(P, rows, n, ws, wsb, st);
@@ -643,7 +660,9 @@ int fo_gradient(const double* xt, const double* at, int64_t n, int64_t T, const 
       rc = f.family == kGauss ? run_pairs_sym<OpFOBwdSym, kTpbLight, kRtFoSym>(P, n, ws, wsb, st)
                               : run_pairs_sym<OpFOBwdSym, kTpbLight, kRtFoSymL, Laplacian>(P, n, ws, wsb, st);
     } else {
-      rc = run_pairs_k<OpFOBwd, V, Shape<V>::kTpb, Shape<V>::kRt>(P, n, n, ws, wsb, st);
+      rc = !std::is_same<V, F2>::value && sym64_takes<OpFOBwdSym>(n)
+               ? run_sym64<OpFOBwdSym>(P, n, ws, wsb, st)
+               : run_pairs_k<OpFOBwd, V, Shape<V>::kTpb, Shape<V>::kRt>(P, n, n, ws, wsb, st);
     }
     if (rc != kOk) return rc;
   }

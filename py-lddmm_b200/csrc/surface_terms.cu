@@ -445,9 +445,9 @@ int surf_energy_dispatch(int precision, const FaceRec* def, int nf, const FaceRe
                          double sigma, int with_norm0, double* energy, double* dots, void* pairs, size_t pb,
                          cudaStream_t st) {
   if (precision == kFP32Compensated)
-    return surf_energy<F2, kTpbLight, kRtLight, KIND>(def, nf, tgt, nf1, make_frame(origin, sigma, kGauss, true),
+    return surf_energy<F2, kTpbLight, kRtLight, KIND>(def, nf, tgt, nf1, make_frame(origin, sigma, kGauss),
                                                       with_norm0, energy, dots, pairs, pb, st);
-  return surf_energy<double, kTpb64, kRt64, KIND>(def, nf, tgt, nf1, make_frame(origin, sigma, kGauss, false),
+  return surf_energy<double, kTpb64, kRt64, KIND>(def, nf, tgt, nf1, make_frame(origin, sigma, kGauss),
                                                   with_norm0, energy, dots, pairs, pb, st);
 }
 
@@ -455,9 +455,9 @@ template <int KIND>
 int surf_grad_dispatch(int precision, const FaceRec* def, int nf, const FaceRec* tgt, int nf1, const double* origin,
                        double sigma, FaceGrad* grads, void* pairs, size_t pb, cudaStream_t st) {
   if (precision == kFP32Compensated)
-    return surf_grad<F2, kTpbLight, kRtLight, KIND>(def, nf, tgt, nf1, make_frame(origin, sigma, kGauss, true),
+    return surf_grad<F2, kTpbLight, kRtLight, KIND>(def, nf, tgt, nf1, make_frame(origin, sigma, kGauss),
                                                     grads, pairs, pb, st);
-  return surf_grad<double, kTpb64, kRt64, KIND>(def, nf, tgt, nf1, make_frame(origin, sigma, kGauss, false),
+  return surf_grad<double, kTpb64, kRt64, KIND>(def, nf, tgt, nf1, make_frame(origin, sigma, kGauss),
                                                 grads, pairs, pb, st);
 }
 
