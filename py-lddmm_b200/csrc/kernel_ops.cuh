@@ -6,6 +6,7 @@
 // figures used for the roofline; a packed instruction counts as two lane-ops).
 #pragma once
 #include "lddmm_common.cuh"
+#include "pairs_sym.cuh"
 
 namespace lddmm {
 
@@ -110,6 +111,7 @@ struct OpKSymD {
   using Params = OpK::Params;
   static constexpr int NSS = 6, NR = 3, NC = 3;
   static constexpr int kSymMinCtas = LDDMM_KSYM_MIN_CTAS;
+  using Shape = SymRule<kSplit2N, kSplit4N, kSplit8N, kSplit8N, kRtKSym, kRtKSymL, kTpbSym64, kRtSym64>;
   template <typename V> struct SymTgt { V y0, y1, y2, a0, a1, a2; };
   template <typename V>
   static __device__ __forceinline__ void load_target_sym(const Params& P, int i0, int i1, bool v0, bool v1,

@@ -33,6 +33,7 @@ __global__ void ordered_sum_kernel(const double* __restrict__ v, int count, doub
                                    int accumulate) {
   __shared__ double red[1024];
   double s = 0.0;
+  chain_wait();
   for (int i = threadIdx.x; i < count; i += blockDim.x) s += v[i];
   red[threadIdx.x] = s;
   __syncthreads();
@@ -83,11 +84,9 @@ size_t kernel_sums_ws_bytes(int64_t n, int64_t m, int precision) {
   upd(op_ws<OpDiffK1and2, kTpbLight, kRtLight>(n, m, precision));
   upd(op_ws<OpDiv, kTpbLight, kRtLight>(n, m, precision));
   upd(op_ws<OpKTensor, kTpbLight, kRtLight>(n, m, precision));
-  if (LDDMM_SYM && precision == kFP32Compensated && n == m) {
-    upd(symx_ws_bytes<OpKSym, kTpbKSym, kRtKSym>(n));
-    upd(sym_ws_bytes<OpKSymD, kTpbLight, kRtKSymL, Laplacian>(n));
-  }
-  if (precision == kFP64 && n == m) upd(sym64_ws_bytes_upto<OpKSymD>(n));
+  if (n == m)
+    upd(precision == kFP32Compensated ? ksym_scratch_upto<OpKSym, OpKSymD, F2>(n)
+                                      : ksym_scratch_upto<OpKSym, OpKSymD, double>(n));
   return b;
 }
 
@@ -102,18 +101,15 @@ int lddmm_apply_k(const double* y, int64_t n, const double* x, const double* a, 
   if (n < 0 || m < 0 || bad_sigma(sigma) || bad_ptr(y, n) || bad_ptr(out, n) || bad_ptr(x, m) || bad_ptr(a, m))
     return kInvalidArgument;
   // a self-sum K(x, x) a (the same point array as targets and sources): each unordered pair once
-  if (LDDMM_SYM && precision == kFP32Compensated && y == x && n == m && !bad_kernel(kernel)) {
-    OpK::Params P;
-    P.f = make_frame(origin, sigma, kernel);
-    P.y = y; P.x = x; P.a = a; P.out = out;
-    if (kernel == kGauss) return run_pairs_symx<OpKSym, kTpbKSym, kRtKSym>(P, n, ws, wsb, (cudaStream_t)stream);
-    return run_pairs_sym<OpKSymD, kTpbLight, kRtKSymL, Laplacian>(P, n, ws, wsb, (cudaStream_t)stream);
-  }
-  if (precision == kFP64 && y == x && n == m && !bad_kernel(kernel) && sym64_takes<OpKSymD>(n)) {
-    OpK::Params P;
-    P.f = make_frame(origin, sigma, kernel);
-    P.y = y; P.x = x; P.a = a; P.out = out;
-    return run_sym64<OpKSymD>(P, n, ws, wsb, (cudaStream_t)stream);
+  if (y == x && n == m && !bad_kernel(kernel) && (precision == kFP32Compensated || precision == kFP64)) {
+    const bool f32 = precision == kFP32Compensated;
+    if (f32 ? sym_takes<OpKSymD, F2>(n) : sym_takes<OpKSymD, double>(n)) {
+      OpK::Params P;
+      P.f = make_frame(origin, sigma, kernel);
+      P.y = y; P.x = x; P.a = a; P.out = out;
+      return f32 ? run_ksym<OpKSym, OpKSymD, F2>(P, n, ws, wsb, (cudaStream_t)stream)
+                 : run_ksym<OpKSym, OpKSymD, double>(P, n, ws, wsb, (cudaStream_t)stream);
+    }
   }
   return dispatch<OpK, kTpbLight, kRtLight>(precision, n, m, sigma, kernel, origin, ws, wsb, (cudaStream_t)stream,
                                             [&](OpK::Params& P) { P.y = y; P.x = x; P.a = a; P.out = out; });

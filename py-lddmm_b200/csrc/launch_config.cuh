@@ -24,15 +24,6 @@
 #ifndef LDDMM_RT_FO_SYM
 #define LDDMM_RT_FO_SYM 4
 #endif
-#ifndef LDDMM_RT_SYM_SMALL
-#define LDDMM_RT_SYM_SMALL 2
-#endif
-#ifndef LDDMM_SYM_FWD_SMALL_N
-#define LDDMM_SYM_FWD_SMALL_N 16384
-#endif
-#ifndef LDDMM_SYM_ADJ_SMALL_N
-#define LDDMM_SYM_ADJ_SMALL_N 6144
-#endif
 #ifndef LDDMM_RT_SYM_FWD_L
 #define LDDMM_RT_SYM_FWD_L 4
 #endif
@@ -75,14 +66,25 @@ constexpr int kRtAdjoint = LDDMM_RT_ADJOINT;
 // thread (134 registers, 3 CTAs per SM): the per-step source loads and the column shuffles are shared by twice
 // as many pairs, and four independent lane groups hide the latency of the ex2 chain.
 constexpr int kRtSymFwd = LDDMM_RT_SYM_FWD;
-// Small point sets (the coarse levels of a coarse-to-fine registration): row blocks of 256 points instead of 1,024
-// (forward) or 512 (adjoint), so that the unit triangle gives the GPU ~10x more units. At level 4 (2,562 points)
-// 1,024-point blocks leave 39 units for 444 resident CTAs and a step is latency-bound (39.5 us forward, 39.4 us
-// adjoint, with the epilogue); 2 targets per thread: 27.2 and 31.2 us. At level 5 (10,242) the forward step
-// still gains (123.5 -> 95.7 us) and the adjoint step loses (134.4 -> 146.6 us); at level 6 both lose 30-40%.
-constexpr int kRtSymSmall = LDDMM_RT_SYM_SMALL;
-constexpr int64_t kSymFwdSmallN = LDDMM_SYM_FWD_SMALL_N;  // Gaussian forward step: 2 targets per thread up to here
-constexpr int64_t kSymAdjSmallN = LDDMM_SYM_ADJ_SMALL_N;  // Gaussian adjoint step: 2 targets per thread up to here
+// Small and middle point sets: the split symmetric kernel (pairs_kernel_sym with SPLIT: the four warps of a CTA share
+// 32 RT targets and take a quarter of every tile each), with more targets per thread as the set grows. A small RT gives
+// more units, a large one fewer loads, shuffles and partials per pair. Each line lies where the next shape starts to
+// win; us per step, launches overlapped (2 | 4 | 8 targets split; "-": the shape that was used up to here):
+//   forward step   n = 1,500: 11.5 | 11.1 | 14.4 (- 14.7)   2,562: 16.4 | 14.7 | 15.3 (- 15.5)   4,000: 23.2 | 20.9 |
+//                  20.5 (- 20.9)   7,000: 50.9 | 40.2 | 41.0 (- 56.7)   10,242: 89 | 74.5 | 67.9 (- 80.3)
+//                  16,000: 190 | 152 | 138 (- 174)   20,000: 301 | 236 | 221, without the split 223
+//   adjoint step   642: 11.1 | 14.1 (- 18.7)   2,000: 14.9 | 15.0 (- 19.7)   3,200: 29.0 | 26.1 (- 30.0)   7,000: 77.0 |
+//                  70.9 (- 83.4)   10,242: 139 | 129, without the split 120
+//   K a            642: 8.1 | 9.0 | 10.1 (- 16.3)   2,562: 12.0 | 11.9 | 12.0 (- 20.1)   4,000: 17.1 | 15.3 | 14.9 (-
+//                  20.1)   10,242: 55 | 45.5 | 41.0 (- 48.9)   16,000: 114 | 91 | 79.7 (- 79.9)
+//   first-order    642: 9.5 | 11.8 (- 19.4)   2,562: 17.3 | 16.1 (- 20.6)   7,000: 55.5 | 44.6 (- 43.6)   8,000: 63 |
+//   adjoint step   56 (- 74.8)   10,242: 97.7 | 83.0, without the split 74.6
+// and for the Laplacian (2 | 4 split): forward 2,562: 18.3 | 16.7 (- 23.8), 6,000: 45.1 | 42.9 (- 46.7), 10,242: 110 |
+// 98, without 91; adjoint 6,000: 75.9 | 63.7 (- 87.7); K a 10,242: 67 | 58.1 (- 63.6).
+constexpr int64_t kSplit2N = 1280, kSplit2NAdj = 2048;  // 2 targets per thread up to here
+constexpr int64_t kSplit4N = 3600;                      // 4 up to here, then 8 (forward step and K a, Gaussian)
+constexpr int64_t kSplit4NLast = 8192;                  // 4 up to here, then no split (adjoint steps, Laplacian)
+constexpr int64_t kSplit8N = 16384;                     // 8 up to here, then no split
 // The symmetric K(x, x) a (pairs_kernel_symx): 8 targets per thread.
 // The symmetric first-order adjoint step (pairs_kernel_sym): 4 targets per thread.
 constexpr int kRtFoSym = LDDMM_RT_FO_SYM;
@@ -99,13 +101,14 @@ constexpr int kTpb64 = LDDMM_TPB_64;
 constexpr int kRt64 = LDDMM_RT_64;
 // FP64 symmetric sums (pairs_kernel_sym with V = double), threads per CTA x targets per thread. 64 x 4 for K a, the
 // forward step and the first-order adjoint step, 128 x 2 for the adjoint step (17 target values per thread: 4 targets
-// would leave 1 CTA per SM); 64 x 2 for small sets, whose unit triangle would otherwise have fewer units than the GPU
-// has SMs. us at n = 642 / 10,242 / 40,962, 64 x 2 | 64 x 4 | 128 x 2 | 128 x 4: K a 16.7 / 123 / 1631 | 19.8 / 113 /
-// 1486 | 19.9 / 120 / 1593 | 29.1 / 111 / 1494; adjoint step 23.0 / 297 / 4165 | 43.5 / 302 / 4218 | 35.3 / 291 / 4100
-// | 74 / 299 / 4232 (every ordered pair with exp(): K a 23.0 / 227 / 3111, adjoint step 35.3 / 463 / 6606).
+// would leave 1 CTA per SM). us at n = 10,242 / 40,962, 64 x 4 | 128 x 2 | 128 x 4: K a 113 / 1486 | 120 / 1593 | 111 /
+// 1494; adjoint step 302 / 4218 | 291 / 4100 | 299 / 4232 (every ordered pair with exp(): K a 227 / 3111, adjoint step
+// 463 / 6606).
 constexpr int kTpbSym64 = 64, kRtSym64 = 4;
 constexpr int kTpbSym64Adj = 128, kRtSym64Adj = 2;
-constexpr int kTpbSym64Small = 64, kRtSym64Small = 2;
-constexpr int64_t kSym64SmallN = 2048;
+// Small sets split: 128 x 1, then 128 x 2 (us per step with 1 | 2 targets split, then the shape above: forward 642:
+// 10.8 | 11.6 | 20, 1,500: 16.1 | 15.4 | 21, 2,562: 28.4 | 24.6 | 22.7; the Laplacian's 2,562: 36.4 | 34.6 | 48.7,
+// 4,000: 62.8 | 55.3 | 55.6).
+constexpr int64_t kSplit1N64 = 1280, kSplit2N64 = 2304, kSplit2N64Lap = 4096;
 
 }  // namespace lddmm

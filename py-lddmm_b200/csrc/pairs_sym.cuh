@@ -131,20 +131,36 @@ struct SymStage<NF, TPB, F2> {
   static constexpr int kFields = 4 * ((NF + 3) / 4);  // size of the FP64 field buffer and of the operand array
 };
 
-// first unit of row i (rows: target blocks; row i holds the tiles RT i .. TT - 1)
-__host__ __device__ __forceinline__ long long sym_row_off(long long i, long long TT, long long RT) {
-  return i * TT - RT * (i * (i - 1) / 2);
-}
 __host__ __device__ __forceinline__ long long sym_tri(long long j) { return j * (j - 1) / 2; }
 
-__device__ __forceinline__ int sym_row_of(long long u, int nblk, long long TT, long long RT) {
-  int lo = 0, hi = nblk - 1;  // largest i with off(i) <= u
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (sym_row_off(mid, TT, RT) <= u) lo = mid; else hi = mid - 1;
+// The unit triangle for row blocks of B points and tiles of TPB: B a multiple of TPB (a row block spans kSpan tiles)
+// or a divisor of it (a tile holds kShare row blocks). Row i takes the tiles from its own first one on; the tiles that
+// overlap its own superblock of K = max(B, TPB) points are diagonal (rows only).
+template <int TPB, int B>
+struct SymGeom {
+  static_assert(B % TPB == 0 || TPB % B == 0, "row blocks and tiles must nest");
+  static constexpr int kSpan = B >= TPB ? B / TPB : 1, kShare = B < TPB ? TPB / B : 1;
+  static constexpr int K = B >= TPB ? B : TPB;
+  static __host__ __device__ __forceinline__ int first_tile(int i) { return B >= TPB ? i * kSpan : i / kShare; }
+  // first unit of row i: the sum of TT - first_tile over the rows before it
+  static __host__ __device__ __forceinline__ long long row_off(long long i, long long TT) {
+    if (B >= TPB) return i * TT - kSpan * sym_tri(i);
+    const long long q = i / kShare, r = i - q * kShare;
+    return i * TT - (kShare * sym_tri(q) + q * r);
   }
-  return lo;
-}
+  // column partials: superblock J receives one per row block before it (kShare J of them), K points each; offset of
+  // the first one (in units of K points)
+  static __host__ __device__ __forceinline__ long long col_first(long long J) { return kShare * sym_tri(J); }
+
+  static __device__ __forceinline__ int row_of(long long u, int nblk, long long TT) {
+    int lo = 0, hi = nblk - 1;  // largest i with row_off(i) <= u
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (row_off(mid, TT) <= u) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+  }
+};
 
 struct SymPlan {
   int nblk = 0, TT = 0, C = 0, S = 0;
@@ -153,26 +169,61 @@ struct SymPlan {
 };
 
 // row_bytes, col_bytes: size of one row / column partial
-template <int TPB, int RT>
+template <int TPB, int B>
 inline SymPlan make_sym_plan(int64_t n, int nr, int nc, int ctas_per_sm, size_t row_bytes, size_t col_bytes) {
+  using Geo = SymGeom<TPB, B>;
   SymPlan p;
   if (n <= 0) return p;
-  constexpr int64_t B = (int64_t)TPB * RT;
   p.nblk = (int)((n + B - 1) / B);
   p.TT = (int)((n + TPB - 1) / TPB);
-  p.U = sym_row_off(p.nblk, p.TT, RT);
+  p.U = Geo::row_off(p.nblk, p.TT);
   const long long wave = (long long)device_sm_count() * (ctas_per_sm > 0 ? ctas_per_sm : 1);
-  p.C = (int)(p.U < wave ? p.U : wave);
+  // one resident wave of CTAs; up to half a wave more units run as one CTA each, so that no CTA takes two units while
+  // others take one (forward step at 6,000 points, 576 units, 444 resident CTAs: 41.4 -> 31.7 us)
+  p.C = (int)(2 * p.U < 3 * wave ? p.U : wave);
   int smax = 1;
   for (int i = 0; i < p.nblk; ++i) {
-    const int c0 = sk_cta_of(sym_row_off(i, p.TT, RT), p.U, p.C);
-    const int c1 = sk_cta_of(sym_row_off(i + 1, p.TT, RT) - 1, p.U, p.C);
+    const int c0 = sk_cta_of(Geo::row_off(i, p.TT), p.U, p.C);
+    const int c1 = sk_cta_of(Geo::row_off(i + 1, p.TT) - 1, p.U, p.C);
     if (c1 - c0 + 1 > smax) smax = c1 - c0 + 1;
   }
   p.S = smax;
   p.col_off = ((size_t)p.S * (size_t)nr * (size_t)n * row_bytes + 255) & ~(size_t)255;
-  p.ws_bytes = p.col_off + (size_t)sym_tri(p.nblk) * (size_t)nc * (size_t)B * col_bytes;
+  p.ws_bytes =
+      p.col_off + (size_t)Geo::col_first((n + Geo::K - 1) / Geo::K) * (size_t)nc * (size_t)Geo::K * col_bytes;
   return p;
+}
+
+// One chunk of 32 sources against the warp's targets; lane λ returns the warp's column sums of source λ in cs.
+template <class Op, int TPB, int RT, bool COL, class Fam, typename V>
+__device__ __forceinline__ void sym_chunk(const Frame& f,
+                                          const typename Op::template SymTgt<V> (&tgt)[RT / VT<V>::kLanes],
+                                          const typename SymStage<Op::NSS, TPB, V>::T (*sm)[TPB], int chunk,
+                                          V (&acc)[RT / VT<V>::kLanes][Op::NR],
+                                          typename VT<V>::Scalar (&cs)[Op::NC]) {
+  using St = SymStage<Op::NSS, TPB, V>;
+  constexpr int G = RT / VT<V>::kLanes;
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int c = 0; c < Op::NC; ++c) cs[c] = 0;
+#pragma unroll kSymUnroll
+  for (int s = 0; s < 32; ++s) {
+    const int src = chunk * 32 + ((lane + s) & 31);
+    V sv[St::kFields];
+    St::load(sm, src, sv);
+    if constexpr (COL) {
+      V col[Op::NC];
+#pragma unroll
+      for (int c = 0; c < Op::NC; ++c) col[c] = VT<V>::first(cs[c]);
+#pragma unroll
+      for (int g = 0; g < G; ++g) Op::template pair_sym<true, Fam, V>(f, tgt[g], sv, acc[g], col);
+#pragma unroll
+      for (int c = 0; c < Op::NC; ++c) cs[c] = __shfl_sync(0xffffffffu, VT<V>::hsum(col[c]), (lane + 1) & 31);
+    } else {
+#pragma unroll
+      for (int g = 0; g < G; ++g) Op::template pair_sym<false, Fam, V>(f, tgt[g], sv, acc[g], nullptr);
+    }
+  }
 }
 
 template <class Op, int TPB, int RT, bool COL, class Fam, typename V>
@@ -181,34 +232,13 @@ __device__ __forceinline__ void sym_tile(const Frame& f,
                                          const typename SymStage<Op::NSS, TPB, V>::T (*sm)[TPB],
                                          typename VT<V>::Scalar (*colacc)[TPB],
                                          V (&acc)[RT / VT<V>::kLanes][Op::NR]) {
-  using St = SymStage<Op::NSS, TPB, V>;
-  using S = typename VT<V>::Scalar;
-  constexpr int G = RT / VT<V>::kLanes, W = TPB / 32;
+  constexpr int W = TPB / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll 1
   for (int ph = 0; ph < W; ++ph) {
     const int chunk = (warp + ph) % W;
-    S cs[Op::NC];
-#pragma unroll
-    for (int c = 0; c < Op::NC; ++c) cs[c] = S(0);
-#pragma unroll kSymUnroll
-    for (int s = 0; s < 32; ++s) {
-      const int src = chunk * 32 + ((lane + s) & 31);
-      V sv[St::kFields];
-      St::load(sm, src, sv);
-      if constexpr (COL) {
-        V col[Op::NC];
-#pragma unroll
-        for (int c = 0; c < Op::NC; ++c) col[c] = VT<V>::first(cs[c]);
-#pragma unroll
-        for (int g = 0; g < G; ++g) Op::template pair_sym<true, Fam, V>(f, tgt[g], sv, acc[g], col);
-#pragma unroll
-        for (int c = 0; c < Op::NC; ++c) cs[c] = __shfl_sync(0xffffffffu, VT<V>::hsum(col[c]), (lane + 1) & 31);
-      } else {
-#pragma unroll
-        for (int g = 0; g < G; ++g) Op::template pair_sym<false, Fam, V>(f, tgt[g], sv, acc[g], nullptr);
-      }
-    }
+    typename VT<V>::Scalar cs[Op::NC];
+    sym_chunk<Op, TPB, RT, COL, Fam, V>(f, tgt, sm, chunk, acc, cs);
     if constexpr (COL) {
 #pragma unroll
       for (int c = 0; c < Op::NC; ++c) colacc[c][chunk * 32 + lane] += cs[c];
@@ -221,38 +251,48 @@ __device__ __forceinline__ void sym_tile(const Frame& f,
 template <class Op, typename V>
 constexpr int kSymCtas = std::is_same<V, F2>::value ? Op::kSymMinCtas : 1;
 
-template <class Op, int TPB, int RT, class Fam, typename V>
+// SPLIT (small point sets): the warps of a CTA share its 32 RT targets and take one chunk of every tile each, instead
+// of TPB RT targets and all chunks in turn. A unit is TPB / 32 times shorter and the triangle has that many times more
+// units, which is what a set too small to fill the GPU needs: at 2,562 points a forward step's longest chain falls
+// from 128 pair evaluations to 32 and its 462 units occupy every SM. The warps' row sums meet in shared memory at the
+// end of a segment; a chunk's column sums are one warp's and go straight to the column partial.
+template <class Op, int TPB, int RT, class Fam, typename V, bool SPLIT>
 __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
     pairs_kernel_sym(const typename Op::Params P, int n, int nblk, int TT, long long U, int C,
                      typename VT<V>::Partial* __restrict__ row_ws, typename VT<V>::Scalar* __restrict__ col_ws) {
   using St = SymStage<Op::NSS, TPB, V>;
-  constexpr int L = VT<V>::kLanes, G = RT / L, NR = Op::NR, NC = Op::NC;
-  constexpr int B = TPB * RT;
+  constexpr int L = VT<V>::kLanes, G = RT / L, NR = Op::NR, NC = Op::NC, W = TPB / 32;
+  constexpr int TW = SPLIT ? 32 : TPB;  // targets a lane-group index apart
+  constexpr int B = TW * RT;
+  using Geo = SymGeom<TPB, B>;
+  constexpr int K = Geo::K;
   static_assert(TPB % 32 == 0 && RT % L == 0, "launch shape");
   __shared__ typename St::T sm[St::NQ][TPB];
-  __shared__ typename VT<V>::Scalar colacc[NC][TPB];
-  // compensated row sums of the segment, one private column per thread (G * NR * Comp<V>::kWords rows of TPB): dynamic shared
-  // memory, so that 8 targets per thread may take more than the 48 KiB of static shared memory
+  __shared__ typename VT<V>::Scalar colacc[SPLIT ? 1 : NC][TPB];
+  // compensated row sums of the segment, one private column per thread (G * NR * Comp<V>::kWords rows of TPB): dynamic
+  // shared memory, so that 8 targets per thread may take more than the 48 KiB of static shared memory
   extern __shared__ __align__(16) unsigned char sym_dyn_smem[];
   V (*cs)[TPB] = reinterpret_cast<V (*)[TPB]>(sym_dyn_smem);
   const Frame& f = P.f;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   VT<V>::setup();  // the staging barrier of the first tile follows
+  chain_wait();
 
   const long long u_end = sk_start(blockIdx.x + 1, U, C);
   long long u = sk_start(blockIdx.x, U, C);
-  int i = u < u_end ? sym_row_of(u, nblk, TT, RT) : 0;
+  int i = u < u_end ? Geo::row_of(u, nblk, TT) : 0;
   while (u < u_end) {
-    const long long off = sym_row_off(i, TT, RT);
-    const int cnt = TT - RT * i;
+    const long long off = Geo::row_off(i, TT);
+    const int first = Geo::first_tile(i), cnt = TT - first;
     const int t0 = (int)(u - off);
     const int t1 = (int)((u_end - off) < cnt ? (u_end - off) : cnt);
     const int slot = (int)blockIdx.x - sk_cta_of(off, U, C);
-    const int base = i * B + threadIdx.x;
+    const int base = i * B + (SPLIT ? lane : (int)threadIdx.x);
 
     typename Op::template SymTgt<V> tgt[G];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-      const int i0 = base + (g * L) * TPB, i1 = base + (g * L + L - 1) * TPB;
+      const int i0 = base + (g * L) * TW, i1 = base + (g * L + L - 1) * TW;
       Op::template load_target_sym<V>(P, i0 < n ? i0 : n - 1, i1 < n ? i1 : n - 1, i0 < n, i1 < n, tgt[g]);
       Comp<V> z;
       z.zero();
@@ -261,8 +301,8 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
     }
 
     for (int tt = t0; tt < t1; ++tt) {
-      const int t = RT * i + tt;  // absolute source tile
-      const bool diag = tt < RT;  // tile of block i itself: rows only
+      const int t = first + tt;                // absolute source tile
+      const bool diag = tt < Geo::kSpan;       // tile of the block's own superblock: rows only
       {
         const int l = t * TPB + threadIdx.x;
         double fl[St::kFields];
@@ -270,8 +310,10 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
         for (int q = 0; q < St::kFields; ++q) fl[q] = 0.0;
         if (l < n) Op::source_fields_sym(P, l, fl);
         St::store(sm, threadIdx.x, fl);
+        if constexpr (!SPLIT) {
 #pragma unroll
-        for (int c = 0; c < NC; ++c) colacc[c][threadIdx.x] = 0;
+          for (int c = 0; c < NC; ++c) colacc[c][threadIdx.x] = 0;
+        }
       }
       __syncthreads();
       V acc[G][NR];
@@ -279,10 +321,23 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
       for (int g = 0; g < G; ++g)
 #pragma unroll
         for (int c = 0; c < NR; ++c) acc[g][c] = VT<V>::zero();
-      if (diag)
+      const int J = (int)(t * (long long)TPB / K);
+      const size_t cb = (size_t)(Geo::col_first(J) + i) * NC * K + (size_t)(t * (long long)TPB - (long long)K * J) +
+                        threadIdx.x;  // column partial of (row block i, tile t), field stride K
+      if constexpr (SPLIT) {
+        typename VT<V>::Scalar col[NC];
+        if (diag) {
+          sym_chunk<Op, TPB, RT, false, Fam, V>(f, tgt, sm, warp, acc, col);
+        } else {
+          sym_chunk<Op, TPB, RT, true, Fam, V>(f, tgt, sm, warp, acc, col);
+#pragma unroll
+          for (int c = 0; c < NC; ++c) col_ws[cb + (size_t)c * K] = col[c];
+        }
+      } else if (diag) {
         sym_tile<Op, TPB, RT, false, Fam, V>(f, tgt, sm, colacc, acc);
-      else
+      } else {
         sym_tile<Op, TPB, RT, true, Fam, V>(f, tgt, sm, colacc, acc);
+      }
 #pragma unroll
       for (int g = 0; g < G; ++g)
 #pragma unroll
@@ -292,30 +347,53 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
           m.merge(acc[g][c]);
           m.template store<TPB>(cs, g * NR + c, threadIdx.x);
         }
-      if (!diag) {
-        // column partial of unit (block i, tile t): block j of the tile, from row block i (< j)
-        const int j = t / RT;
-        const size_t cb = (size_t)(sym_tri(j) + i) * NC * B + (size_t)(t - RT * j) * TPB + threadIdx.x;
+      if constexpr (SPLIT) {
+        __syncthreads();  // every warp has read the tile and left its row sums
+      } else if (!diag) {
 #pragma unroll
-        for (int c = 0; c < NC; ++c) col_ws[cb + (size_t)c * B] = colacc[c][threadIdx.x];
+        for (int c = 0; c < NC; ++c) col_ws[cb + (size_t)c * K] = colacc[c][threadIdx.x];
       }
-      // the last phase barrier of sym_tile orders every read of sm and colacc before the next tile's staging
+      // (not SPLIT) the last phase barrier of sym_tile orders every read of sm and colacc before the next staging
     }
 
+    if constexpr (SPLIT) {
+      // the block's row sums: field c of the lanes' targets by warp c mod W, over the W warps in order
 #pragma unroll
-    for (int g = 0; g < G; ++g)
+      for (int g = 0; g < G; ++g)
+        for (int c = warp; c < NR; c += W) {
+          double sum[L];
 #pragma unroll
-      for (int k = 0; k < L; ++k) {
-        const int idx = base + (g * L + k) * TPB;
-        if (idx < n) {
+          for (int k = 0; k < L; ++k) sum[k] = 0.0;
 #pragma unroll
-          for (int c = 0; c < NR; ++c) {
+          for (int w = 0; w < W; ++w) {
             Comp<V> m;
-            m.template load<TPB>(cs, g * NR + c, threadIdx.x);
-            row_ws[((size_t)slot * NR + c) * (size_t)n + idx] = m.partial(k);
+            m.template load<TPB>(cs, g * NR + c, w * 32 + lane);
+#pragma unroll
+            for (int k = 0; k < L; ++k) sum[k] += partial_value(m.partial(k));
+          }
+#pragma unroll
+          for (int k = 0; k < L; ++k) {
+            const int idx = base + (g * L + k) * TW;
+            if (idx < n) row_ws[((size_t)slot * NR + c) * (size_t)n + idx] = VT<V>::to_partial(sum[k]);
           }
         }
-      }
+      __syncthreads();  // the next segment clears the sums
+    } else {
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int k = 0; k < L; ++k) {
+          const int idx = base + (g * L + k) * TW;
+          if (idx < n) {
+#pragma unroll
+            for (int c = 0; c < NR; ++c) {
+              Comp<V> m;
+              m.template load<TPB>(cs, g * NR + c, threadIdx.x);
+              row_ws[((size_t)slot * NR + c) * (size_t)n + idx] = m.partial(k);
+            }
+          }
+        }
+    }
     u += t1 - t0;
     ++i;
   }
@@ -330,30 +408,32 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
 // of dependent loads (at 2,562 points: 11 CTAs, ~11 us, latency-bound); several threads shorten the chain and
 // spread the points over more CTAs.
 constexpr int kFinThreads = 256;
-template <class Op, int TPB, int RT, typename V>
+template <class Op, int TPB, int B, typename V>
 __global__ void __launch_bounds__(kFinThreads)
     finalize_sym_kernel(const typename Op::Params P, int n, int nblk, int TT, long long U, int C,
                         const typename VT<V>::Partial* __restrict__ row_ws,
                         const typename VT<V>::Scalar* __restrict__ col_ws, int tpp) {
-  constexpr int B = TPB * RT, NV = Op::NR + Op::NC;
+  using Geo = SymGeom<TPB, B>;
+  constexpr int NV = Op::NR + Op::NC, K = Geo::K;
   __shared__ double red[kFinThreads][NV];
   const int np = kFinThreads / tpp;
   const int p = threadIdx.x % np, j = threadIdx.x / np;
   const int idx = blockIdx.x * np + p;
   const bool live = idx < n;
+  chain_wait();
   double v[NV];
 #pragma unroll
   for (int c = 0; c < NV; ++c) v[c] = 0.0;
-  const int b = live ? idx / B : 0, r = live ? idx - b * B : 0;
+  const int b = live ? idx / B : 0, J = live ? idx / K : 0, r = live ? idx - J * K : 0;
   if (live) {
-    const int nslot = sk_cta_of(sym_row_off(b + 1, TT, RT) - 1, U, C) - sk_cta_of(sym_row_off(b, TT, RT), U, C) + 1;
+    const int nslot = sk_cta_of(Geo::row_off(b + 1, TT) - 1, U, C) - sk_cta_of(Geo::row_off(b, TT), U, C) + 1;
     for (int s = j; s < nslot; s += tpp)
 #pragma unroll
       for (int c = 0; c < Op::NR; ++c) v[c] += partial_value(row_ws[((size_t)s * Op::NR + c) * (size_t)n + idx]);
-    for (int q = j; q < b; q += tpp) {
-      const size_t cb = (size_t)(sym_tri(b) + q) * Op::NC * B + r;
+    for (int q = j; q < J * Geo::kShare; q += tpp) {
+      const size_t cb = (size_t)(Geo::col_first(J) + q) * Op::NC * K + r;
 #pragma unroll
-      for (int c = 0; c < Op::NC; ++c) v[Op::NR + c] += (double)col_ws[cb + (size_t)c * B];
+      for (int c = 0; c < Op::NC; ++c) v[Op::NR + c] += (double)col_ws[cb + (size_t)c * K];
     }
   }
   if (tpp > 1) {
@@ -390,7 +470,7 @@ constexpr size_t sym_dyn_smem_bytes() {
 
 // Declare the kernel's dynamic shared memory, once per device (the attribute belongs to the device's context):
 // without it static + dynamic shared memory may not exceed 48 KiB. Returns false when the device refuses.
-template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2>
+template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2, bool SPLIT = false>
 inline bool sym_prepare() {
   static signed char state[64] = {};
   int dev = 0;
@@ -400,7 +480,7 @@ inline bool sym_prepare() {
   }
   if (dev < 0 || dev >= 64) return false;
   if (state[dev] == 0) {
-    const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&pairs_kernel_sym<Op, TPB, RT, Fam, V>),
+    const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&pairs_kernel_sym<Op, TPB, RT, Fam, V, SPLIT>),
                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)sym_dyn_smem_bytes<Op, TPB, RT, V>());
     if (e != cudaSuccess) cudaGetLastError();
@@ -409,64 +489,89 @@ inline bool sym_prepare() {
   return state[dev] > 0;
 }
 
-template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2>
+template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2, bool SPLIT = false>
 inline int sym_ctas_per_sm() {
   static int cached = 0;
   if (cached == 0) {
-    sym_prepare<Op, TPB, RT, Fam, V>();
-    int c = resident_ctas(reinterpret_cast<const void*>(&pairs_kernel_sym<Op, TPB, RT, Fam, V>), TPB,
+    sym_prepare<Op, TPB, RT, Fam, V, SPLIT>();
+    int c = resident_ctas(reinterpret_cast<const void*>(&pairs_kernel_sym<Op, TPB, RT, Fam, V, SPLIT>), TPB,
                           sym_dyn_smem_bytes<Op, TPB, RT, V>());
     cached = c > 0 ? c : 2;
   }
   return cached;
 }
 
-template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2>
+template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2, bool SPLIT = false>
 inline SymPlan sym_plan(int64_t n) {
-  return make_sym_plan<TPB, RT>(n, Op::NR, Op::NC, sym_ctas_per_sm<Op, TPB, RT, Fam, V>(),
+  return make_sym_plan<TPB, (SPLIT ? 32 : TPB) * RT>(n, Op::NR, Op::NC, sym_ctas_per_sm<Op, TPB, RT, Fam, V, SPLIT>(),
                                 sizeof(typename VT<V>::Partial), sizeof(typename VT<V>::Scalar));
 }
 
-template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2>
+template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2, bool SPLIT = false>
 inline size_t sym_ws_bytes(int64_t n) {
-  return sym_plan<Op, TPB, RT, Fam, V>(n).ws_bytes;
+  return sym_plan<Op, TPB, RT, Fam, V, SPLIT>(n).ws_bytes;
 }
 
-template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2>
+template <class Op, int TPB, int RT, class Fam = Gauss, typename V = F2, bool SPLIT = false>
 inline int run_pairs_sym(const typename Op::Params& P, int64_t n, void* ws, size_t ws_bytes, cudaStream_t stream) {
   if (n <= 0) return kOk;
   if (n > INT32_MAX / 4) return kInvalidArgument;
-  const SymPlan plan = sym_plan<Op, TPB, RT, Fam, V>(n);
+  const SymPlan plan = sym_plan<Op, TPB, RT, Fam, V, SPLIT>(n);
   if (plan.ws_bytes > ws_bytes) return kWorkspaceTooSmall;
   if (ws == nullptr) return kInvalidArgument;
-  if (!sym_prepare<Op, TPB, RT, Fam, V>()) return kLaunchFailure;
+  if (!sym_prepare<Op, TPB, RT, Fam, V, SPLIT>()) return kLaunchFailure;
   auto* row_ws = reinterpret_cast<typename VT<V>::Partial*>(ws);
   auto* col_ws = reinterpret_cast<typename VT<V>::Scalar*>(reinterpret_cast<char*>(ws) + plan.col_off);
-  pairs_kernel_sym<Op, TPB, RT, Fam, V><<<plan.C, TPB, sym_dyn_smem_bytes<Op, TPB, RT, V>(), stream>>>(
-      P, (int)n, plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws);
+  launch_chained(pairs_kernel_sym<Op, TPB, RT, Fam, V, SPLIT>, plan.C, TPB, sym_dyn_smem_bytes<Op, TPB, RT, V>(),
+                 stream, P, (int)n, plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws);
   const int fb = kFinThreads, tpp = sym_finalize_tpp(plan);
-  finalize_sym_kernel<Op, TPB, RT, V><<<sym_finalize_grid(n, tpp, fb), fb, 0, stream>>>(
-      P, (int)n, plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws, tpp);
+  launch_chained(finalize_sym_kernel<Op, TPB, (SPLIT ? 32 : TPB) * RT, V>, sym_finalize_grid(n, tpp, fb), fb, 0,
+                 stream, P, (int)n, plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws, tpp);
   return cudaPeekAtLastError() == cudaSuccess ? kOk : kLaunchFailure;
 }
 
 
-// FP64 launch shape of a symmetric op (the adjoint step declares kSym64Adjoint).
-template <class Op, class = void>
-struct Sym64Shape {
-  static constexpr int kTpb = kTpbSym64, kRt = kRtSym64;
+// Launch shapes. Each symmetric op names its rule (Op::Shape): the FP32 lines between 2, 4 and 8 targets per thread
+// with the split and the shape without it, and the FP64 shape (launch_config.cuh has the measurements).
+template <int SPLIT2_N, int SPLIT4_N, int SPLIT8_N, int SPLIT4_N_LAP, int RT, int RT_LAP, int TPB64, int RT64>
+struct SymRule {
+  static constexpr int64_t kSplit2 = SPLIT2_N, kSplit4 = SPLIT4_N, kSplit8 = SPLIT8_N, kSplit4Lap = SPLIT4_N_LAP;
+  static constexpr int kRt = RT, kRtLap = RT_LAP, kTpb64 = TPB64, kRt64 = RT64;
 };
-template <class Op>
-struct Sym64Shape<Op, std::void_t<decltype(Op::kSym64Adjoint)>> {
-  static constexpr int kTpb = kTpbSym64Adj, kRt = kRtSym64Adj;
+template <int TPB, int RT, bool SPLIT>
+struct SymShape {
+  static constexpr int kTpb = TPB, kRt = RT;
+  static constexpr bool kSplit = SPLIT;
 };
 
-// Whether an FP64 self-sum takes the symmetric kernel. Its column partials are bounded at 2 GiB (150,000 points for
-// the six-field steps): they grow with n^2, and larger sets keep the ordered-pair kernel, whose scratch does not.
+// fn(SymShape{}) with the shape of n points.
+template <class Op, typename V, class Fam, class Fn>
+inline auto sym_shape(int64_t n, Fn fn) {
+  using R = typename Op::Shape;
+  constexpr bool kG = std::is_same<Fam, Gauss>::value;
+  if constexpr (std::is_same<V, double>::value) {
+    if (n <= kSplit1N64) return fn(SymShape<128, 1, true>{});
+    if (n <= (kG ? kSplit2N64 : kSplit2N64Lap)) return fn(SymShape<128, 2, true>{});
+    return fn(SymShape<R::kTpb64, R::kRt64, false>{});
+  } else {
+    if (n <= R::kSplit2) return fn(SymShape<128, 2, true>{});
+    if (n <= (kG ? R::kSplit4 : R::kSplit4Lap)) return fn(SymShape<128, 4, true>{});
+    if constexpr (kG && R::kSplit8 > R::kSplit4) {
+      if (n <= R::kSplit8) return fn(SymShape<128, 8, true>{});
+    }
+    return fn(SymShape<128, kG ? R::kRt : R::kRtLap, false>{});
+  }
+}
+
+// Whether a self-sum takes the symmetric kernel: always in FP32. In FP64 the column partials of the unsplit shape are
+// bounded at 2 GiB (150,000 points for the six-field steps): they grow with n^2, and larger sets keep the ordered-pair
+// kernel, whose scratch does not.
 constexpr int64_t kSym64MaxColBytes = int64_t(2) << 30;
-template <class Op>
-inline int64_t sym64_max_n() {
-  constexpr int64_t B = Sym64Shape<Op>::kTpb * Sym64Shape<Op>::kRt;
+template <class Op, typename V>
+inline int64_t sym_max_n() {
+  if (LDDMM_SYM == 0) return 0;
+  if (std::is_same<V, F2>::value) return INT32_MAX / 4;
+  constexpr int64_t B = Op::Shape::kTpb64 * Op::Shape::kRt64;
   constexpr int64_t tri = kSym64MaxColBytes / (int64_t)(Op::NC * B * sizeof(double));  // blocks: tri(nblk) <= this
   static const int64_t nblk = [] {
     int64_t k = 1;
@@ -475,44 +580,49 @@ inline int64_t sym64_max_n() {
   }();
   return nblk * B;
 }
-template <class Op>
-inline bool sym64_takes(int64_t n) {
-  return LDDMM_SYM != 0 && n > 0 && n <= sym64_max_n<Op>();
+template <class Op, typename V>
+inline bool sym_takes(int64_t n) {
+  return n > 0 && n <= sym_max_n<Op, V>();
 }
 
-template <class Op, class Fam>
-inline size_t sym64_ws_bytes_fam(int64_t n) {
-  if (n <= kSym64SmallN) return sym_ws_bytes<Op, kTpbSym64Small, kRtSym64Small, Fam, double>(n);
-  return sym_ws_bytes<Op, Sym64Shape<Op>::kTpb, Sym64Shape<Op>::kRt, Fam, double>(n);
+template <class Op, typename V, class Fam>
+inline size_t sym_scratch_fam(int64_t n) {
+  return sym_shape<Op, V, Fam>(n, [&](auto sh) {
+    return sym_ws_bytes<Op, decltype(sh)::kTpb, decltype(sh)::kRt, Fam, V, decltype(sh)::kSplit>(n);
+  });
 }
-template <class Op>
-inline size_t sym64_ws_bytes(int64_t n, int family) {
-  return family == kGauss ? sym64_ws_bytes_fam<Op, Gauss>(n) : sym64_ws_bytes_fam<Op, Laplacian>(n);
+// Scratch of one launch.
+template <class Op, typename V>
+inline size_t sym_scratch(int64_t n, int family) {
+  return family == kGauss ? sym_scratch_fam<Op, V, Gauss>(n) : sym_scratch_fam<Op, V, Laplacian>(n);
 }
-
-// Scratch for every point count up to n.
-template <class Op>
-inline size_t sym64_ws_bytes_upto(int64_t n) {
-  if (LDDMM_SYM == 0) return 0;
+// Scratch for every point count up to n: the largest of each shape's range.
+template <class Op, typename V>
+inline size_t sym_scratch_upto(int64_t n) {
+  using R = typename Op::Shape;
   size_t b = 0;
-  for (const int64_t k : {n < kSym64SmallN ? n : kSym64SmallN, n < sym64_max_n<Op>() ? n : sym64_max_n<Op>()})
+  for (const int64_t k : {R::kSplit2, R::kSplit4, R::kSplit8, R::kSplit4Lap, kSplit1N64, kSplit2N64, kSplit2N64Lap,
+                          sym_max_n<Op, V>(), n}) {
+    if (k > n || !sym_takes<Op, V>(k)) continue;
     for (const int family : {(int)kGauss, (int)kLaplacian0}) {
-      const size_t v = k > 0 ? sym64_ws_bytes<Op>(k, family) : 0;
+      const size_t v = sym_scratch<Op, V>(k, family);
       b = v > b ? v : b;
     }
+  }
   return b;
 }
 
-template <class Op, class Fam>
-inline int run_sym64_fam(const typename Op::Params& P, int64_t n, void* ws, size_t wsb, cudaStream_t st) {
-  if (n <= kSym64SmallN) return run_pairs_sym<Op, kTpbSym64Small, kRtSym64Small, Fam, double>(P, n, ws, wsb, st);
-  return run_pairs_sym<Op, Sym64Shape<Op>::kTpb, Sym64Shape<Op>::kRt, Fam, double>(P, n, ws, wsb, st);
+template <class Op, typename V, class Fam>
+inline int run_sym_fam(const typename Op::Params& P, int64_t n, void* ws, size_t wsb, cudaStream_t st) {
+  return sym_shape<Op, V, Fam>(n, [&](auto sh) {
+    return run_pairs_sym<Op, decltype(sh)::kTpb, decltype(sh)::kRt, Fam, V, decltype(sh)::kSplit>(P, n, ws, wsb, st);
+  });
 }
-// The FP64 launch of a symmetric op, for the kernel family of its frame.
-template <class Op>
-inline int run_sym64(const typename Op::Params& P, int64_t n, void* ws, size_t wsb, cudaStream_t st) {
-  if (P.f.family == kGauss) return run_sym64_fam<Op, Gauss>(P, n, ws, wsb, st);
-  return run_sym64_fam<Op, Laplacian>(P, n, ws, wsb, st);
+// Launch of a symmetric op, for the kernel family of its frame.
+template <class Op, typename V>
+inline int run_sym(const typename Op::Params& P, int64_t n, void* ws, size_t wsb, cudaStream_t st) {
+  if (P.f.family == kGauss) return run_sym_fam<Op, V, Gauss>(P, n, ws, wsb, st);
+  return run_sym_fam<Op, V, Laplacian>(P, n, ws, wsb, st);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -607,6 +717,7 @@ __global__ void __launch_bounds__(TPB, Op::kSymMinCtas)
   using St = SymStage<4 + Op::NP, TPB, F2>;
   constexpr int L = 2, G = RT / L, NP = Op::NP;
   constexpr int B = TPB * RT;
+  using Geo = SymGeom<TPB, B>;
   static_assert(TPB % 32 == 0 && RT % L == 0, "launch shape");
   __shared__ typename St::T sm[St::NQ][TPB];
   __shared__ float colacc[NP][TPB];
@@ -615,12 +726,13 @@ __global__ void __launch_bounds__(TPB, Op::kSymMinCtas)
   F2 (*cs)[TPB] = reinterpret_cast<F2 (*)[TPB]>(sym_dyn_smem);  // compensated row sums, G * NP * 2 rows
   const Frame& f = P.f;
   const double fo[3] = {f.o0, f.o1, f.o2};
+  chain_wait();
 
   const long long u_end = sk_start(blockIdx.x + 1, U, C);
   long long u = sk_start(blockIdx.x, U, C);
-  int i = u < u_end ? sym_row_of(u, nblk, TT, RT) : 0;
+  int i = u < u_end ? Geo::row_of(u, nblk, TT) : 0;
   while (u < u_end) {
-    const long long off = sym_row_off(i, TT, RT);
+    const long long off = Geo::row_off(i, TT);
     const int cnt = TT - RT * i;
     const int t0 = (int)(u - off);
     const int t1 = (int)((u_end - off) < cnt ? (u_end - off) : cnt);
@@ -733,7 +845,7 @@ __global__ void __launch_bounds__(TPB, Op::kSymMinCtas)
         }
       if (!diag) {
         const int j = t / RT;
-        const size_t cb = (size_t)(sym_tri(j) + i) * NP * B + (size_t)(t - RT * j) * TPB + threadIdx.x;
+        const size_t cb = (size_t)(Geo::col_first(j) + i) * NP * B + (size_t)(t - RT * j) * TPB + threadIdx.x;
 #pragma unroll
         for (int c = 0; c < NP; ++c) col_ws[cb + (size_t)c * B] = colacc[c][threadIdx.x];
       }
@@ -807,25 +919,45 @@ inline int symx_ctas_per_sm() {
 
 template <class Op, int TPB, int RT>
 inline size_t symx_ws_bytes(int64_t n) {
-  return make_sym_plan<TPB, RT>(n, Op::NP, Op::NP, symx_ctas_per_sm<Op, TPB, RT>(), sizeof(float2), sizeof(float)).ws_bytes;
+  return make_sym_plan<TPB, TPB * RT>(n, Op::NP, Op::NP, symx_ctas_per_sm<Op, TPB, RT>(), sizeof(float2), sizeof(float)).ws_bytes;
 }
 
 template <class Op, int TPB, int RT>
 inline int run_pairs_symx(const typename Op::Params& P, int64_t n, void* ws, size_t ws_bytes, cudaStream_t stream) {
   if (n <= 0) return kOk;
   if (n > INT32_MAX / 4) return kInvalidArgument;
-  const SymPlan plan = make_sym_plan<TPB, RT>(n, Op::NP, Op::NP, symx_ctas_per_sm<Op, TPB, RT>(), sizeof(float2), sizeof(float));
+  const SymPlan plan = make_sym_plan<TPB, TPB * RT>(n, Op::NP, Op::NP, symx_ctas_per_sm<Op, TPB, RT>(), sizeof(float2), sizeof(float));
   if (plan.ws_bytes > ws_bytes) return kWorkspaceTooSmall;
   if (ws == nullptr) return kInvalidArgument;
   if (!symx_prepare<Op, TPB, RT>()) return kLaunchFailure;
   auto* row_ws = reinterpret_cast<float2*>(ws);
   auto* col_ws = reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + plan.col_off);
-  pairs_kernel_symx<Op, TPB, RT><<<plan.C, TPB, symx_dyn_smem_bytes<Op, TPB, RT>(), stream>>>(
-      P, (int)n, plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws);
+  launch_chained(pairs_kernel_symx<Op, TPB, RT>, plan.C, TPB, symx_dyn_smem_bytes<Op, TPB, RT>(), stream, P, (int)n,
+                 plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws);
   const int fb = kFinThreads, tpp = sym_finalize_tpp(plan);
-  finalize_sym_kernel<Op, TPB, RT, F2><<<sym_finalize_grid(n, tpp, fb), fb, 0, stream>>>(
-      P, (int)n, plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws, tpp);
+  launch_chained(finalize_sym_kernel<Op, TPB, TPB * RT, F2>, sym_finalize_grid(n, tpp, fb), fb, 0, stream, P, (int)n,
+                 plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws, tpp);
   return cudaPeekAtLastError() == cudaSuccess ? kOk : kLaunchFailure;
+}
+
+// K(x, x) a: the FP32 Gaussian sum of a set beyond the split shapes runs the expanded form (OpX), everything else the
+// difference form (OpD).
+template <class OpX, class OpD, typename V>
+inline int run_ksym(const typename OpD::Params& P, int64_t n, void* ws, size_t wsb, cudaStream_t st) {
+  if (std::is_same<V, F2>::value && P.f.family == kGauss && n > OpD::Shape::kSplit8)
+    return run_pairs_symx<OpX, kTpbKSym, kRtKSym>(P, n, ws, wsb, st);
+  return run_sym<OpD, V>(P, n, ws, wsb, st);
+}
+template <class OpX, class OpD, typename V>
+inline size_t ksym_scratch(int64_t n, int family) {
+  if (std::is_same<V, F2>::value && family == kGauss && n > OpD::Shape::kSplit8)
+    return symx_ws_bytes<OpX, kTpbKSym, kRtKSym>(n);
+  return sym_scratch<OpD, V>(n, family);
+}
+template <class OpX, class OpD, typename V>
+inline size_t ksym_scratch_upto(int64_t n) {
+  const size_t b = sym_scratch_upto<OpD, V>(n), x = ksym_scratch<OpX, OpD, V>(n, kGauss);
+  return sym_takes<OpD, V>(n) && x > b ? x : b;
 }
 
 }  // namespace lddmm

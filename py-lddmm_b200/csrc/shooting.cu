@@ -214,6 +214,7 @@ struct OpSOFwdSym {
   using Params = OpSOFwd::Params;
   static constexpr int NSS = 6, NR = 6, NC = 6;
   static constexpr int kSymMinCtas = LDDMM_SOFWD_SYM_MIN_CTAS;
+  using Shape = SymRule<kSplit2N, kSplit4N, kSplit8N, kSplit4NLast, kRtSymFwd, kRtSymFwdL, kTpbSym64, kRtSym64>;
   template <typename V> struct SymTgt { V y0, y1, y2, a0, a1, a2; };
   template <typename V>
   static __device__ __forceinline__ void load_target_sym(const Params& P, int i0, int i1, bool v0, bool v1,
@@ -271,8 +272,9 @@ struct OpSOFwdSym {
 struct OpSOBwdSym {
   using Params = OpSOBwd::Params;
   static constexpr int NSS = 12, NR = 6, NC = 6;
-  static constexpr bool kSym64Adjoint = true;
   static constexpr int kSymMinCtas = LDDMM_SOBWD_SYM_MIN_CTAS;
+  using Shape = SymRule<kSplit2NAdj, kSplit4NLast, 0, kSplit4NLast, kRtAdjoint, kRtAdjointSymL, kTpbSym64Adj,
+                        kRtSym64Adj>;
   template <typename V> struct SymTgt { V y0, y1, y2, a0, a1, a2, b0, b1, b2, p0, p1, p2, q0, q1, q2, cd, k2; };
   template <typename V>
   static __device__ __forceinline__ void load_target_sym(const Params& P, int i0, int i1, bool v0, bool v1,
@@ -405,6 +407,7 @@ struct OpFOBwdSym {
   using Params = OpFOBwd::Params;
   static constexpr int NSS = 9, NR = 6, NC = 6;
   static constexpr int kSymMinCtas = LDDMM_FOBWD_SYM_MIN_CTAS;
+  using Shape = SymRule<kSplit2N, kSplit4NLast, 0, kSplit4NLast, kRtFoSym, kRtFoSymL, kTpbSym64, kRtSym64>;
   template <typename V> struct SymTgt { V y0, y1, y2, p0, p1, p2, a0, a1, a2, q0, q1, q2; };
   template <typename V>
   static __device__ __forceinline__ void load_target_sym(const Params& P, int i0, int i1, bool v0, bool v1,
@@ -460,29 +463,22 @@ struct OpFOBwdSym {
 size_t shooting_ws_bytes(int64_t n, int precision) {
   size_t b = 0;
   auto upd = [&](size_t v) { b = v > b ? v : b; };
+  auto sym = [&](auto v) {
+    using V = decltype(v);
+    upd(sym_scratch_upto<OpSOFwdSym, V>(n));
+    upd(sym_scratch_upto<OpSOBwdSym, V>(n));
+    upd(sym_scratch_upto<OpFOBwdSym, V>(n));
+    upd(ksym_scratch_upto<OpKSym, OpKSymD, V>(n));
+  };
   if (precision == kFP32Compensated) {
-    if (LDDMM_SYM) {
-      upd(sym_ws_bytes<OpSOBwdSym, kTpbHeavy, kRtAdjoint>(n));
-      upd(sym_ws_bytes<OpSOFwdSym, kTpbLight, kRtSymFwd>(n));
-      if (n <= kSymAdjSmallN) upd(sym_ws_bytes<OpSOBwdSym, kTpbHeavy, kRtSymSmall>(n));
-      if (n <= kSymFwdSmallN) upd(sym_ws_bytes<OpSOFwdSym, kTpbLight, kRtSymSmall>(n));
-      upd(sym_ws_bytes<OpFOBwdSym, kTpbLight, kRtFoSym>(n));
-      upd(sym_ws_bytes<OpSOBwdSym, kTpbHeavy, kRtAdjointSymL, Laplacian>(n));
-      upd(sym_ws_bytes<OpSOFwdSym, kTpbLight, kRtSymFwdL, Laplacian>(n));
-      upd(sym_ws_bytes<OpFOBwdSym, kTpbLight, kRtFoSymL, Laplacian>(n));
-      upd(symx_ws_bytes<OpKSym, kTpbKSym, kRtKSym>(n));
-      upd(sym_ws_bytes<OpKSymD, kTpbLight, kRtKSymL, Laplacian>(n));
-    }
+    sym(F2{});
     upd(pairs_ws_bytes_any<OpSOFwd, F2, kTpbLight, kRtLight>(n, n));
     upd(pairs_ws_bytes<OpSOBwd, F2, kTpbHeavy, kRtAdjoint, Gauss>(n, n));
     upd(pairs_ws_bytes<OpSOBwd, F2, kTpbHeavy, kRtHeavy, Laplacian>(n, n));
     upd(pairs_ws_bytes_any<OpFOBwd, F2, kTpbLight, kRtLight>(n, n));
     upd(pairs_ws_bytes_any<OpK, F2, kTpbLight, kRtLight>(n, n));
   } else {
-    upd(sym64_ws_bytes_upto<OpSOFwdSym>(n));
-    upd(sym64_ws_bytes_upto<OpSOBwdSym>(n));
-    upd(sym64_ws_bytes_upto<OpFOBwdSym>(n));
-    upd(sym64_ws_bytes_upto<OpKSymD>(n));
+    sym(0.0);
     upd(pairs_ws_bytes_any<OpSOFwd, double, kTpb64, kRt64>(n, n));
     upd(pairs_ws_bytes_any<OpSOBwd, double, kTpb64, kRt64>(n, n));
     upd(pairs_ws_bytes_any<OpFOBwd, double, kTpb64, kRt64>(n, n));
@@ -495,13 +491,13 @@ size_t shooting_ws_bytes(int64_t n, int precision) {
 namespace {
 
 // Launch shapes per precision: light (forward / first-order) ops and the second-order adjoint step.
-template <typename V> struct Shape;
-template <> struct Shape<F2> {
+template <typename V> struct StepShape;
+template <> struct StepShape<F2> {
   // the adjoint step: 4 targets per thread for the Gaussian, 2 for the Laplacian (whose radial profile needs the
   // registers: 4 would spill)
   static constexpr int kTpb = kTpbLight, kRt = kRtLight, kTpbH = kTpbHeavy, kRtH = kRtAdjoint, kRtHL = kRtHeavy;
 };
-template <> struct Shape<double> {
+template <> struct StepShape<double> {
   static constexpr int kTpb = kTpb64, kRt = kRt64, kTpbH = kTpb64, kRtH = kRt64, kRtHL = kRt64;
 };
 
@@ -520,35 +516,23 @@ template <typename V>
 int k_energy_and_update(const double* x, const double* a, int64_t n, const Frame& f, const double* base,
                         double base_sign, double scale, double* out, const double* dotw, double* energy,
                         double escale, int accumulate, void* ws, size_t wsb, cudaStream_t st) {
-  constexpr int TPB = Shape<V>::kTpb, RT = Shape<V>::kRt;
+  constexpr int TPB = StepShape<V>::kTpb, RT = StepShape<V>::kRt;
   OpK::Params P;
   P.y = x; P.x = x; P.a = a; P.out = out; P.f = f;
   P.base = base; P.base_sign = base_sign; P.scale = scale;
-  // K(x) a is a self-sum: each unordered pair once (pairs_kernel_symx for the FP32 Gaussian, pairs_kernel_sym in the
-  // difference form otherwise)
-  constexpr bool kF32 = std::is_same<V, F2>::value;
-  const bool sym = kF32 ? LDDMM_SYM != 0 : sym64_takes<OpKSymD>(n), gauss = f.family == kGauss;
-  const size_t pb = !sym    ? pairs_ws_bytes_any<OpK, V, TPB, RT>(n, n)
-                    : !kF32 ? sym64_ws_bytes<OpKSymD>(n, f.family)
-                    : gauss ? symx_ws_bytes<OpKSym, kTpbKSym, kRtKSym>(n)
-                            : sym_ws_bytes<OpKSymD, kTpbLight, kRtKSymL, Laplacian>(n);
+  // K(x) a is a self-sum: each unordered pair once
+  const bool sym = sym_takes<OpKSymD, V>(n);
+  const size_t pb = sym ? ksym_scratch<OpKSym, OpKSymD, V>(n, f.family) : pairs_ws_bytes_any<OpK, V, TPB, RT>(n, n);
   if (energy) {
     if (((pb + 255) & ~(size_t)255) + (size_t)n * sizeof(double) > wsb) return kWorkspaceTooSmall;
     P.dotw = dotw;
     P.dots = dots_region(ws, pb);
   }
-  int rc;
-  if (!sym) {
-    rc = run_pairs_k<OpK, V, TPB, RT>(P, n, n, ws, wsb, st);
-  } else if constexpr (kF32) {
-    rc = gauss ? run_pairs_symx<OpKSym, kTpbKSym, kRtKSym>(P, n, ws, wsb, st)
-               : run_pairs_sym<OpKSymD, kTpbLight, kRtKSymL, Laplacian>(P, n, ws, wsb, st);
-  } else {
-    rc = run_sym64<OpKSymD>(P, n, ws, wsb, st);
-  }
+  const int rc = sym ? run_ksym<OpKSym, OpKSymD, V>(P, n, ws, wsb, st)
+                     : run_pairs_k<OpK, V, TPB, RT>(P, n, n, ws, wsb, st);
   if (rc != kOk) return rc;
   if (energy) {
-    ordered_sum_kernel<<<1, 1024, 0, st>>>(P.dots, (int)n, escale, energy, accumulate);
+    launch_chained(ordered_sum_kernel, 1, 1024, 0, st, P.dots, (int)n, escale, energy, accumulate);
     if (cudaPeekAtLastError() != cudaSuccess) return kLaunchFailure;
   }
   return kOk;
@@ -559,18 +543,8 @@ int so_step(const double* x, const double* a, int64_t n, const Frame& f, double 
             size_t wsb, cudaStream_t st, int64_t row0 = 0, int64_t nrows = -1) {
   OpSOFwd::Params P{x, a, x1, a1, f, dt, (int)row0};
   const int64_t rows = nrows < 0 ? n : nrows;
-  if constexpr (std::is_same<V, F2>::value && LDDMM_SYM != 0) {
-    if (row0 == 0 && rows == n) {
-      if (f.family == kGauss && n <= kSymFwdSmallN)
-        return run_pairs_sym<OpSOFwdSym, kTpbLight, kRtSymSmall>(P, n, ws, wsb, st);
-      if (f.family == kGauss) return run_pairs_sym<OpSOFwdSym, kTpbLight, kRtSymFwd>(P, n, ws, wsb, st);
-      return run_pairs_sym<OpSOFwdSym, kTpbLight, kRtSymFwdL, Laplacian>(P, n, ws, wsb, st);
-    }
-  }
-  if constexpr (!std::is_same<V, F2>::value) {
-    if (row0 == 0 && rows == n && sym64_takes<OpSOFwdSym>(n)) return run_sym64<OpSOFwdSym>(P, n, ws, wsb, st);
-  }
-  return run_pairs_k<OpSOFwd, V, Shape<V>::kTpb, Shape<V>::kRt>(P, rows, n, ws, wsb, st);
+  if (row0 == 0 && rows == n && sym_takes<OpSOFwdSym, V>(n)) return run_sym<OpSOFwdSym, V>(P, n, ws, wsb, st);
+  return run_pairs_k<OpSOFwd, V, StepShape<V>::kTpb, StepShape<V>::kRt>(P, rows, n, ws, wsb, st);
 }
 
 template <typename V>
@@ -579,19 +553,9 @@ int so_adjoint_step(const double* x, const double* a, const double* px, const do
                     int64_t row0 = 0, int64_t nrows = -1) {
   OpSOBwd::Params P{x, a, px, pa, px_prev, pa_prev, f, dt, (int)row0};
   const int64_t rows = nrows < 0 ? n : nrows;
-  if constexpr (std::is_same<V, F2>::value && LDDMM_SYM != 0) {
-    if (row0 == 0 && rows == n) {
-      if (f.family == kGauss && n <= kSymAdjSmallN)
-        return run_pairs_sym<OpSOBwdSym, kTpbHeavy, kRtSymSmall>(P, n, ws, wsb, st);
-      if (f.family == kGauss) return run_pairs_sym<OpSOBwdSym, kTpbHeavy, kRtAdjoint>(P, n, ws, wsb, st);
-      return run_pairs_sym<OpSOBwdSym, kTpbHeavy, kRtAdjointSymL, Laplacian>(P, n, ws, wsb, st);
-    }
-  }
-  if constexpr (!std::is_same<V, F2>::value) {
-    if (row0 == 0 && rows == n && sym64_takes<OpSOBwdSym>(n)) return run_sym64<OpSOBwdSym>(P, n, ws, wsb, st);
-  }
-  if (f.family == kGauss) return run_pairs<OpSOBwd, V, Shape<V>::kTpbH, Shape<V>::kRtH, Gauss>(P, rows, n, ws, wsb, st);
-  return run_pairs<OpSOBwd, V, Shape<V>::kTpbH, Shape<V>::kRtHL, Laplacian>(P, rows, n, ws, wsb, st);
+  if (row0 == 0 && rows == n && sym_takes<OpSOBwdSym, V>(n)) return run_sym<OpSOBwdSym, V>(P, n, ws, wsb, st);
+  if (f.family == kGauss) return run_pairs<OpSOBwd, V, StepShape<V>::kTpbH, StepShape<V>::kRtH, Gauss>(P, rows, n, ws, wsb, st);
+  return run_pairs<OpSOBwd, V, StepShape<V>::kTpbH, StepShape<V>::kRtHL, Laplacian>(P, rows, n, ws, wsb, st);
 }
 
 template <typename V>
@@ -655,15 +619,9 @@ int fo_gradient(const double* xt, const double* at, int64_t n, int64_t T, const 
   for (int64_t t = T - 1; t >= 0; --t) {
     OpFOBwd::Params P{xt + t * stride, at + t * stride, pxt + (t + 1) * stride, pxt + t * stride, dat + t * stride,
                       f, dt, regweight, euclidean};
-    int rc;
-    if constexpr (std::is_same<V, F2>::value && LDDMM_SYM != 0) {
-      rc = f.family == kGauss ? run_pairs_sym<OpFOBwdSym, kTpbLight, kRtFoSym>(P, n, ws, wsb, st)
-                              : run_pairs_sym<OpFOBwdSym, kTpbLight, kRtFoSymL, Laplacian>(P, n, ws, wsb, st);
-    } else {
-      rc = !std::is_same<V, F2>::value && sym64_takes<OpFOBwdSym>(n)
-               ? run_sym64<OpFOBwdSym>(P, n, ws, wsb, st)
-               : run_pairs_k<OpFOBwd, V, Shape<V>::kTpb, Shape<V>::kRt>(P, n, n, ws, wsb, st);
-    }
+    const int rc = sym_takes<OpFOBwdSym, V>(n)
+                       ? run_sym<OpFOBwdSym, V>(P, n, ws, wsb, st)
+                       : run_pairs_k<OpFOBwd, V, StepShape<V>::kTpb, StepShape<V>::kRt>(P, n, n, ws, wsb, st);
     if (rc != kOk) return rc;
   }
   return kOk;

@@ -18,6 +18,7 @@ struct FaceRec {
 __global__ void face_geometry_kernel(const double* __restrict__ v, const int64_t* __restrict__ faces,
                                      const double* __restrict__ w, int nf, FaceRec* __restrict__ out) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  chain_wait();
   if (f >= nf) return;
   const int64_t i0 = faces[3 * f], i1 = faces[3 * f + 1], i2 = faces[3 * f + 2];
   double p0[3], p1[3], p2[3];
@@ -352,6 +353,7 @@ __global__ void vertex_gather_kernel(const double* __restrict__ v, const int64_t
                                      const int32_t* __restrict__ items, int nv, double* __restrict__ px,
                                      double* __restrict__ pxw) {
   const int vi = blockIdx.x * blockDim.x + threadIdx.x;
+  chain_wait();
   if (vi >= nv) return;
   double acc[3] = {0.0, 0.0, 0.0}, accw = 0.0;
   for (int it = off[vi]; it < off[vi + 1]; ++it) {
@@ -419,13 +421,13 @@ int surf_energy(const FaceRec* def, int nf, const FaceRec* tgt, int nf1, const F
   P.T = def; P.S = FaceSources{def, nf, tgt, -2.0}; P.dots = dots; P.f = f;
   int rc = run_pairs<Op, V, TPB, RT>(P, nf, (int64_t)nf + nf1, pairs, pairs_bytes, st);
   if (rc != kOk) return rc;
-  if (nf > 0) ordered_sum_kernel<<<1, 1024, 0, st>>>(dots, nf, 1.0, energy, 0);
+  if (nf > 0) launch_chained(ordered_sum_kernel, 1, 1024, 0, st, dots, nf, 1.0, energy, 0);
   else if (cudaMemsetAsync(energy, 0, sizeof(double), st) != cudaSuccess) return kCudaError;
   if (with_norm0) {
     P.T = tgt; P.S = FaceSources{tgt, nf1, nullptr, 0.0};
     rc = run_pairs<Op, V, TPB, RT>(P, nf1, nf1, pairs, pairs_bytes, st);
     if (rc != kOk) return rc;
-    if (nf1 > 0) ordered_sum_kernel<<<1, 1024, 0, st>>>(dots, nf1, 1.0, energy + 1, 0);
+    if (nf1 > 0) launch_chained(ordered_sum_kernel, 1, 1024, 0, st, dots, nf1, 1.0, energy + 1, 0);
     else if (cudaMemsetAsync(energy + 1, 0, sizeof(double), st) != cudaSuccess) return kCudaError;
   }
   return cudaPeekAtLastError() == cudaSuccess ? kOk : kLaunchFailure;
@@ -466,9 +468,10 @@ bool bad(const void* p, int64_t n) { return n > 0 && p == nullptr; }
 int prep_faces(const double* xdef, const int64_t* faces, int64_t nf, const double* weights, const double* x1,
                const int64_t* faces1, int64_t nf1, const double* weights1, FaceRec* recs, cudaStream_t st) {
   const int b = 256;
-  if (nf > 0) face_geometry_kernel<<<(int)((nf + b - 1) / b), b, 0, st>>>(xdef, faces, weights, (int)nf, recs);
+  if (nf > 0)
+    launch_chained(face_geometry_kernel, (int)((nf + b - 1) / b), b, 0, st, xdef, faces, weights, (int)nf, recs);
   if (nf1 > 0)
-    face_geometry_kernel<<<(int)((nf1 + b - 1) / b), b, 0, st>>>(x1, faces1, weights1, (int)nf1, recs + nf);
+    launch_chained(face_geometry_kernel, (int)((nf1 + b - 1) / b), b, 0, st, x1, faces1, weights1, (int)nf1, recs + nf);
   return cudaPeekAtLastError() == cudaSuccess ? kOk : kLaunchFailure;
 }
 
@@ -552,8 +555,8 @@ int lddmm_surface_gradient(int kind, const double* xdef, int64_t nv, const int64
                                                 pairs, pb, st);
   if (rc != kOk) return rc;
   const int b = 256;
-  vertex_gather_kernel<<<(int)((nv + b - 1) / b), b, 0, st>>>(xdef, faces, grads, vf_offsets, vf_items, (int)nv, px,
-                                                              pxw);
+  launch_chained(vertex_gather_kernel, (int)((nv + b - 1) / b), b, 0, st, xdef, faces, grads, vf_offsets, vf_items,
+                 (int)nv, px, pxw);
   return cudaPeekAtLastError() == cudaSuccess ? kOk : kLaunchFailure;
 }
 
