@@ -460,26 +460,26 @@ __host__ __device__ __forceinline__ int sk_cta_of(long long u, long long W, long
 
 int device_sm_count();
 
+// Most CTAs that a window of `len` consecutive units of W meets when C CTAs divide them evenly (each takes at least
+// floor(W / C) units): the partial slots of a target block.
+inline int sk_max_slots(long long len, long long W, long long C) {
+  const long long q = W / C;
+  return (int)((len - 1 + q - 1) / q + 1);
+}
+
 // `boxes`: reserve the coordinate boxes of exact culling (ops with Culled<Op>); other ops never read them, so their
 // scratch is the partial slots alone (at most (C / gx + 2) * na * n partials, whatever m is).
-template <int TPB, int RT>
+template <int TPB, int B>
 inline SKPlan make_plan(int64_t n, int64_t m, int na, size_t partial_bytes, int ctas_per_sm, bool boxes = true) {
   SKPlan p;
   if (n <= 0) return p;
-  const int64_t tb_targets = (int64_t)TPB * RT;
-  p.gx = (int)((n + tb_targets - 1) / tb_targets);
+  p.gx = (int)((n + B - 1) / B);
   if (m <= 0) return p;
   p.TT = (int)((m + TPB - 1) / TPB);
   p.W = (long long)p.gx * p.TT;
   const long long wave = (long long)device_sm_count() * (ctas_per_sm > 0 ? ctas_per_sm : 1);
   p.C = (int)(p.W < wave ? p.W : wave);
-  int smax = 1;
-  for (int tb = 0; tb < p.gx; ++tb) {
-    const int c0 = sk_cta_of((long long)tb * p.TT, p.W, p.C);
-    const int c1 = sk_cta_of((long long)(tb + 1) * p.TT - 1, p.W, p.C);
-    if (c1 - c0 + 1 > smax) smax = c1 - c0 + 1;
-  }
-  p.S = smax;
+  p.S = sk_max_slots(p.TT, p.W, p.C);
   p.box_off = ((size_t)p.S * (size_t)na * (size_t)n * partial_bytes + 255) & ~(size_t)255;
   p.ws_bytes = p.box_off + (boxes ? (size_t)(p.gx + p.TT) * 6 * sizeof(float) : 0);
   return p;
@@ -556,7 +556,9 @@ struct NAXOf<Op, std::void_t<decltype(Op::NAX)>> : std::integral_constant<int, O
 template <class Op, typename V, int RT, class Fam>
 constexpr int kRunRT = (kUseExpanded<Op, V, Fam> && RtXOf<Op>::value > 0) ? RtXOf<Op>::value : RT;
 
-template <class Op, typename V, int TPB, int RT, class Fam = Gauss>
+// SPLIT (problems too small to fill the GPU): the warps of a CTA share its 32 RT targets and take a quarter of every
+// source tile each, instead of TPB RT targets and whole tiles; their sums meet in shared memory when a segment ends.
+template <class Op, typename V, int TPB, int RT, class Fam, bool SPLIT>
 __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
     pairs_kernel(const typename Op::Params P, int n, int m, int TT, long long W, int C,
                  typename VT<V>::Partial* __restrict__ ws, const float* __restrict__ boxes) {
@@ -569,12 +571,14 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
   // The segment's compensated sums live in shared memory (one private column per thread: no barrier needed) unless
   // the op keeps them in registers; shared memory frees 2-4 registers per accumulator for more resident warps.
   constexpr bool kSm = LDDMM_COMP_SMEM && !CompInRegisters<Op>::value;
-  __shared__ V cs[kSm ? G * Op::NA * Comp<V>::kWords : 1][TPB];
+  __shared__ V cs[kSm || SPLIT ? G * Op::NA * Comp<V>::kWords : 1][TPB];
+  constexpr int TW = SPLIT ? 32 : TPB;  // targets a lane-group index apart
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // Exact culling (ops with Culled<Op>): a (target block, source tile) unit whose coordinate boxes (box_kernel) are
   // farther apart than the distance at which the kernel's radial factors are exactly zero in this arithmetic
   // contributes exactly nothing, and is skipped by the whole CTA.
   constexpr float kZeroR2 = Fam::template kCullR2<V>;
-  const int gx = (n + TPB * RT - 1) / (TPB * RT);
+  const int gx = (n + TW * RT - 1) / (TW * RT);
   __shared__ float tbox[6];  // the segment's target box, in shared memory (re-read per tile, not held in registers)
   VT<V>::setup();
   chain_wait();
@@ -589,11 +593,11 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
 
     typename Op::template Tgt<V> tgt[G];
     Comp<V> cmp[G][Op::NA];   // used when !kSm
-    // target of (group g, lane k): base + (g * L + k) * TPB
-    const int base = tb * (TPB * RT) + threadIdx.x;
+    // target of (group g, lane k): base + (g * L + k) * TW
+    const int base = tb * (TW * RT) + (SPLIT ? lane : (int)threadIdx.x);
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-      int i0 = base + (g * L) * TPB, i1 = base + (g * L + L - 1) * TPB;
+      int i0 = base + (g * L) * TW, i1 = base + (g * L + L - 1) * TW;
       i0 = i0 < n ? i0 : n - 1;
       i1 = i1 < n ? i1 : n - 1;
       Op::template load_target<V>(P, i0, i1, tgt[g]);
@@ -635,11 +639,11 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
 #pragma unroll
         for (int c = 0; c < Op::NA; ++c) acc[g][c] = VT<V>::zero();
 #pragma unroll kUnroll
-      for (int jj = 0; jj < TPB; ++jj) {
+      for (int jj = 0; jj < TW; ++jj) {
         V s[2 * NU];
 #pragma unroll
         for (int q = 0; q < NU; ++q) {
-          const Unit<V> w = sm[q][jj];
+          const Unit<V> w = sm[q][SPLIT ? warp * 32 + jj : jj];
           s[2 * q] = w.a;
           s[2 * q + 1] = w.b;
         }
@@ -657,19 +661,50 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
       __syncthreads();
     }
 
+    if constexpr (SPLIT) {
+      if constexpr (!kSm) {
 #pragma unroll
-    for (int g = 0; g < G; ++g)
+        for (int g = 0; g < G; ++g)
 #pragma unroll
-      for (int k = 0; k < L; ++k) {
-        const int i = base + (g * L + k) * TPB;
-        if (i < n) {
+          for (int c = 0; c < Op::NA; ++c) cmp[g][c].template store<TPB>(cs, g * Op::NA + c, threadIdx.x);
+      }
+      __syncthreads();
+      // sum c of the lanes' targets by warp c mod W, over the W warps in order
 #pragma unroll
-          for (int c = 0; c < Op::NA; ++c) {
-            if constexpr (kSm) cmp[g][c].template load<TPB>(cs, g * Op::NA + c, threadIdx.x);
-            ws[((size_t)slot * Op::NA + c) * (size_t)n + i] = cmp[g][c].partial(k);
+      for (int g = 0; g < G; ++g)
+        for (int c = warp; c < Op::NA; c += TPB / 32) {
+          double sum[L];
+#pragma unroll
+          for (int k = 0; k < L; ++k) sum[k] = 0.0;
+#pragma unroll
+          for (int w = 0; w < TPB / 32; ++w) {
+            Comp<V> m;
+            m.template load<TPB>(cs, g * Op::NA + c, w * 32 + lane);
+#pragma unroll
+            for (int k = 0; k < L; ++k) sum[k] += partial_value(m.partial(k));
+          }
+#pragma unroll
+          for (int k = 0; k < L; ++k) {
+            const int i = base + (g * L + k) * TW;
+            if (i < n) ws[((size_t)slot * Op::NA + c) * (size_t)n + i] = VT<V>::to_partial(sum[k]);
           }
         }
-      }
+      __syncthreads();  // the next segment clears the sums
+    } else {
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int k = 0; k < L; ++k) {
+          const int i = base + (g * L + k) * TW;
+          if (i < n) {
+#pragma unroll
+            for (int c = 0; c < Op::NA; ++c) {
+              if constexpr (kSm) cmp[g][c].template load<TPB>(cs, g * Op::NA + c, threadIdx.x);
+              ws[((size_t)slot * Op::NA + c) * (size_t)n + i] = cmp[g][c].partial(k);
+            }
+          }
+        }
+    }
     u += j1 - j0;
   }
 }
@@ -706,7 +741,7 @@ struct HasXPartial : std::false_type {};
 template <class Op>
 struct HasXPartial<Op, std::void_t<decltype(&Op::x_partial)>> : std::true_type {};
 
-template <class Op, int TPB, int RT>
+template <class Op, int TPB, int RT, bool SPLIT>
 __global__ void __launch_bounds__(TPB, MinCtas<Op, F2>::value)
     pairs_kernel_x(const typename Op::Params P, int n, int m, int TT, long long W, int C,
                    float2* __restrict__ ws, const float* __restrict__ boxes) {
@@ -714,16 +749,18 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, F2>::value)
   constexpr int G = RT / L;
   constexpr int NF = 4 + Op::NP;  // staged fields: X or x (3), q (1), payload (NP)
   constexpr int NU = (NF + 1) / 2;
+  constexpr int TW = SPLIT ? 32 : TPB;   // targets a lane-group index apart (SPLIT: as in pairs_kernel)
   constexpr int NAX = NAXOf<Op>::value;  // accumulators of the expanded form
   constexpr int kUnroll = UnrollOf<Op>::value;
   static_assert(RT % L == 0, "targets per thread must be a multiple of the lane count");
   __shared__ Unit<F2> sm[NU][TPB];
   __shared__ float red[6][TPB / 32];
-  constexpr bool kSm = LDDMM_X_COMP_SMEM != 0;
+  constexpr bool kSm = SPLIT || LDDMM_X_COMP_SMEM != 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __shared__ F2 cs[kSm ? G * NAX * 2 : 1][TPB];
   const Frame& f = P.f;
   const double fo[3] = {f.o0, f.o1, f.o2};
-  const int gx = (n + TPB * RT - 1) / (TPB * RT);
+  const int gx = (n + TW * RT - 1) / (TW * RT);
   chain_wait();
 
   const long long u_end = sk_start(blockIdx.x + 1, W, C);
@@ -733,13 +770,13 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, F2>::value)
     const int j0 = (int)(u - (long long)tb * TT);
     const int j1 = (int)((u_end - (long long)tb * TT) < TT ? (u_end - (long long)tb * TT) : TT);
     const int slot = (int)blockIdx.x - sk_cta_of((long long)tb * TT, W, C);
-    const int base = tb * (TPB * RT) + threadIdx.x;
+    const int base = tb * (TW * RT) + (SPLIT ? lane : (int)threadIdx.x);
 
     // the block's box and centre (every CTA working on block tb derives the same ones)
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
     for (int t = 0; t < RT; ++t) {
-      int i = base + t * TPB;
+      int i = base + t * TW;
       i = i < n ? i : n - 1;
       double y[3];
       Op::target_point(P, i, y);
@@ -765,7 +802,7 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, F2>::value)
     Comp<F2> cmp[G][NAX];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-      int i0 = base + (g * L) * TPB, i1 = base + (g * L + 1) * TPB;
+      int i0 = base + (g * L) * TW, i1 = base + (g * L + 1) * TW;
       i0 = i0 < n ? i0 : n - 1;
       i1 = i1 < n ? i1 : n - 1;
       double y0[3], y1[3];
@@ -821,11 +858,11 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, F2>::value)
         for (int c = 0; c < NAX; ++c) acc[g][c] = VT<F2>::zero();
       if (expand) {
 #pragma unroll kUnroll
-        for (int jj = 0; jj < TPB; ++jj) {
+        for (int jj = 0; jj < TW; ++jj) {
           F2 s[2 * NU];
 #pragma unroll
           for (int q = 0; q < NU; ++q) {
-            const Unit<F2> w = sm[q][jj];
+            const Unit<F2> w = sm[q][SPLIT ? warp * 32 + jj : jj];
             s[2 * q] = w.a;
             s[2 * q + 1] = w.b;
           }
@@ -839,11 +876,11 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, F2>::value)
         }
       } else {
 #pragma unroll kUnroll
-        for (int jj = 0; jj < TPB; ++jj) {
+        for (int jj = 0; jj < TW; ++jj) {
           F2 s[2 * NU];
 #pragma unroll
           for (int q = 0; q < NU; ++q) {
-            const Unit<F2> w = sm[q][jj];
+            const Unit<F2> w = sm[q][SPLIT ? warp * 32 + jj : jj];
             s[2 * q] = w.a;
             s[2 * q + 1] = w.b;
           }
@@ -865,12 +902,14 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, F2>::value)
       __syncthreads();
     }
 
+    if constexpr (SPLIT) __syncthreads();  // every warp's sums are in shared memory (also when no tile was evaluated)
 #pragma unroll
     for (int g = 0; g < G; ++g)
 #pragma unroll
       for (int k = 0; k < L; ++k) {
-        const int i = base + (g * L + k) * TPB;
-        if (i < n) {
+        const int i = base + (g * L + k) * TW;
+        // SPLIT: target g L + k of the lanes by warp (g L + k) mod W, over the W warps in order
+        if (i < n && (!SPLIT || (g * L + k) % (TPB / 32) == warp)) {
           double yr[3], y2 = 0.0;
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
@@ -881,9 +920,18 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, F2>::value)
           double v[NAX], o[Op::NA];
 #pragma unroll
           for (int c = 0; c < NAX; ++c) {
-            if constexpr (kSm) cmp[g][c].template load<TPB>(cs, g * NAX + c, threadIdx.x);
-            const float2 p = cmp[g][c].partial(k);
-            v[c] = (double)p.x + (double)p.y;
+            if constexpr (SPLIT) {
+              v[c] = 0.0;
+#pragma unroll
+              for (int w = 0; w < TPB / 32; ++w) {
+                Comp<F2> m;
+                m.template load<TPB>(cs, g * NAX + c, w * 32 + lane);
+                v[c] += partial_value(m.partial(k));
+              }
+            } else {
+              if constexpr (kSm) cmp[g][c].template load<TPB>(cs, g * NAX + c, threadIdx.x);
+              v[c] = partial_value(cmp[g][c].partial(k));
+            }
           }
           if constexpr (HasXPartial<Op>::value) {
             Op::x_partial(expand, yr, v, o);
@@ -893,33 +941,33 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, F2>::value)
           }
 #pragma unroll
           for (int c = 0; c < Op::NA; ++c) {
-            const double w = o[c] * fac;
-            const float h = (float)w;
-            ws[((size_t)slot * Op::NA + c) * (size_t)n + i] = make_float2(h, (float)(w - (double)h));
+            ws[((size_t)slot * Op::NA + c) * (size_t)n + i] = VT<F2>::to_partial(o[c] * fac);
           }
         }
       }
+    if constexpr (SPLIT) __syncthreads();  // the next segment clears the sums
     u += j1 - j0;
   }
 }
 
 // Coordinate boxes for exact culling, from the same scaled coordinates the pair kernel uses: block b < gx covers
 // target block b (its TPB * RT targets), block gx + j source tile j. boxes[6 b ..] = (lo xyz, hi xyz).
-template <class Op, typename V, int TPB, int RT>
+template <class Op, typename V, int TPB, int RT, bool SPLIT>
 __global__ void __launch_bounds__(TPB) box_kernel(const typename Op::Params P, int n, int m, int gx,
                                                   float* __restrict__ boxes) {
   constexpr int L = VT<V>::kLanes;
   constexpr int G = RT / L;
   constexpr int NU = (Op::NS + 1) / 2;
+  constexpr int TW = SPLIT ? 32 : TPB;
   __shared__ float red[6][TPB / 32];
   float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
   const int b = blockIdx.x;
   chain_wait();
   if (b < gx) {
-    const int base = b * (TPB * RT) + threadIdx.x;
+    const int base = b * (TW * RT) + (int)threadIdx.x % TW;
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-      int i0 = base + (g * L) * TPB, i1 = base + (g * L + L - 1) * TPB;
+      int i0 = base + (g * L) * TW, i1 = base + (g * L + L - 1) * TW;
       i0 = i0 < n ? i0 : n - 1;
       i1 = i1 < n ? i1 : n - 1;
       typename Op::template Tgt<V> t;
@@ -953,24 +1001,51 @@ __global__ void __launch_bounds__(TPB) box_kernel(const typename Op::Params P, i
   }
 }
 
-// Epilogue: reduce the partial slots of target i (its block's CTAs, in CTA order) in FP64, then Op::finalize.
+// Epilogue: reduce the partial slots of target i (its block's CTAs) in FP64, then Op::finalize. `tpp` threads per
+// target (a power of two <= 32): thread j sums the slots j, j + tpp, ... and the tpp sums are added in the order j = 0,
+// 1, ... from shared memory, so the order of every addition is fixed. With one thread per target its slots are one
+// serial chain (surface gradient of 2,990 against 3,534 faces: 41 us for 47 slots of 8 sums).
+constexpr int kFinThreads = 256;
 template <class Op, typename V>
-__global__ void finalize_kernel(const typename Op::Params P, int n, int tb_targets, int TT, long long W, int C,
-                                const typename VT<V>::Partial* __restrict__ ws) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kFinThreads)
+    finalize_kernel(const typename Op::Params P, int n, int tb_targets, int TT, long long W, int C,
+                    const typename VT<V>::Partial* __restrict__ ws, int tpp) {
+  __shared__ double red[kFinThreads][Op::NA];
+  const int np = kFinThreads / tpp;
+  const int p = threadIdx.x % np, j = threadIdx.x / np;
+  const int i = blockIdx.x * np + p;
   chain_wait();
-  if (i >= n) return;
   double acc[Op::NA];
 #pragma unroll
   for (int c = 0; c < Op::NA; ++c) acc[c] = 0.0;
-  if (W > 0) {
+  if (i < n && W > 0) {
     const int tb = i / tb_targets;
     const int nslot = sk_cta_of((long long)(tb + 1) * TT - 1, W, C) - sk_cta_of((long long)tb * TT, W, C) + 1;
-    for (int s = 0; s < nslot; ++s)
+    for (int s = j; s < nslot; s += tpp)
 #pragma unroll
       for (int c = 0; c < Op::NA; ++c) acc[c] += partial_value(ws[((size_t)s * Op::NA + c) * (size_t)n + i]);
   }
-  Op::finalize(P, i, acc);
+  if (tpp > 1) {
+#pragma unroll
+    for (int c = 0; c < Op::NA; ++c) red[threadIdx.x][c] = acc[c];
+    __syncthreads();
+    if (j == 0)
+      for (int k = 1; k < tpp; ++k)
+#pragma unroll
+        for (int c = 0; c < Op::NA; ++c) acc[c] += red[k * np + p][c];
+  }
+  if (i < n && j == 0) Op::finalize(P, i, acc);
+}
+
+// Threads per point of an epilogue: enough to split a chain of slots into pieces of about four, at most 8.
+inline int finalize_tpp(int chain) {
+  int t = 1;
+  while (t < 8 && chain > 4 * t) t <<= 1;
+  return t;
+}
+inline int finalize_grid(int64_t n, int tpp) {
+  const int64_t np = kFinThreads / tpp;
+  return (int)((n + np - 1) / np);
 }
 
 // Deterministic single-block sum of `count` doubles: out[0] = (accumulate ? out[0] : 0) + scale * sum(v).
@@ -978,19 +1053,72 @@ __global__ void ordered_sum_kernel(const double* __restrict__ v, int count, doub
 
 int resident_ctas(const void* kernel, int threads, size_t dynamic_smem = 0);
 
-template <class Op, typename V, int TPB, int RT, class Fam = Gauss>
+template <class Op, typename V, int TPB, int RT, class Fam, bool SPLIT>
 inline int ctas_per_sm() {
   static int cached = 0;
   if (cached == 0) {
     const void* k;
     if constexpr (kUseExpanded<Op, V, Fam>)
-      k = reinterpret_cast<const void*>(&pairs_kernel_x<Op, TPB, kRunRT<Op, V, RT, Fam>>);
+      k = reinterpret_cast<const void*>(&pairs_kernel_x<Op, TPB, kRunRT<Op, V, RT, Fam>, SPLIT>);
     else
-      k = reinterpret_cast<const void*>(&pairs_kernel<Op, V, TPB, RT, Fam>);
+      k = reinterpret_cast<const void*>(&pairs_kernel<Op, V, TPB, RT, Fam, SPLIT>);
     int c = resident_ctas(k, TPB);
     cached = c > 0 ? c : 4;
   }
   return cached;
+}
+
+// Ops that never split declare `static constexpr bool kNoSplit = true;`.
+template <class Op, class = void>
+struct CanSplit : std::true_type {};
+template <class Op>
+struct CanSplit<Op, std::void_t<decltype(Op::kNoSplit)>> : std::bool_constant<!Op::kNoSplit> {};
+
+template <class Op, typename V, int TPB, int RT, class Fam, bool SPLIT>
+inline SKPlan pairs_plan(int64_t n, int64_t m) {
+  return make_plan<TPB, (SPLIT ? 32 : TPB) * kRunRT<Op, V, RT, Fam>>(
+      n, m, Op::NA, sizeof(typename VT<V>::Partial), ctas_per_sm<Op, V, TPB, RT, Fam, SPLIT>(), Culled<Op>::value);
+}
+
+// Whether a problem splits: its whole-tile units would fill less than a third of one resident wave (FP32), or less than
+// two and a half waves (FP64, whose units are several times longer). us, unsplit | split, n = m: FP32 K a 162: 12.7 |
+// 8.5, 1,500: 15.8 | 10.6, 2,562 (0.14 waves): 16.0 | 12.8, 6,000 (0.64): 23.3 | 27.6; applyDiffKT 2,562 (0.21): 13.6 |
+// 13.1, 6,000 (0.95): 32.3 | 35.5; DDK 1,500 (0.16): 11.7 | 10.3, 2,562 (0.5): 16.0 | 19.0; varifold gradient 1,280
+// faces: 33.6 | 30.4, 5,120 (1.8): 79.3 | 81.4. FP64 K a 642: 13.6 | 8.0, applyDiffKT 2,562 (0.4): 25.8 | 22.7, 6,000
+// (1.9): 93 | 82, varifold gradient 5,120 (2.7): 159 | 162, K a 20,000 (21): 577 | 597.
+template <class Op, typename V, int TPB, int RT, class Fam>
+inline bool pairs_split(int64_t n, int64_t m) {
+  constexpr int64_t B = (int64_t)TPB * kRunRT<Op, V, RT, Fam>;
+  const int64_t units = ((n + B - 1) / B) * ((m + TPB - 1) / TPB);
+  const int64_t wave = (int64_t)device_sm_count() * ctas_per_sm<Op, V, TPB, RT, Fam, false>();
+  return std::is_same<V, F2>::value ? 3 * units < wave : 2 * units < 5 * wave;
+}
+
+template <class Op, typename V, int TPB, int RT, class Fam, bool SPLIT>
+inline int launch_pairs(const typename Op::Params& P, int64_t n, int64_t m, void* ws, size_t ws_bytes,
+                        cudaStream_t stream) {
+  constexpr int R = kRunRT<Op, V, RT, Fam>;
+  const SKPlan plan = pairs_plan<Op, V, TPB, RT, Fam, SPLIT>(n, m);
+  if (plan.ws_bytes > ws_bytes) return kWorkspaceTooSmall;
+  if (plan.ws_bytes > 0 && ws == nullptr) return kInvalidArgument;
+  auto* part = reinterpret_cast<typename VT<V>::Partial*>(ws);
+  if (plan.W > 0) {
+    float* boxes = Culled<Op>::value ? reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + plan.box_off) : nullptr;
+    if (Culled<Op>::value)
+      launch_chained(box_kernel<Op, V, TPB, R, SPLIT>, plan.gx + plan.TT, TPB, 0, stream, P, (int)n, (int)m, plan.gx,
+                     boxes);
+    if constexpr (kUseExpanded<Op, V, Fam>) {
+      launch_chained(pairs_kernel_x<Op, TPB, R, SPLIT>, plan.C, TPB, 0, stream, P, (int)n, (int)m, plan.TT, plan.W,
+                     plan.C, part, boxes);
+    } else {
+      launch_chained(pairs_kernel<Op, V, TPB, RT, Fam, SPLIT>, plan.C, TPB, 0, stream, P, (int)n, (int)m, plan.TT,
+                     plan.W, plan.C, part, boxes);
+    }
+  }
+  const int tpp = finalize_tpp(plan.S);
+  launch_chained(finalize_kernel<Op, V>, finalize_grid(n, tpp), kFinThreads, 0, stream, P, (int)n,
+                 (SPLIT ? 32 : TPB) * R, plan.TT, plan.W, plan.C, part, tpp);
+  return cudaPeekAtLastError() == cudaSuccess ? kOk : kLaunchFailure;
 }
 
 template <class Op, typename V, int TPB, int RT, class Fam = Gauss>
@@ -998,35 +1126,22 @@ inline int run_pairs(const typename Op::Params& P, int64_t n, int64_t m, void* w
                      cudaStream_t stream) {
   if (n <= 0) return kOk;
   if (n > INT32_MAX / 4 || m > INT32_MAX / 4) return kInvalidArgument;
-  constexpr int R = kRunRT<Op, V, RT, Fam>;
-  SKPlan plan = make_plan<TPB, R>(n, m, Op::NA, sizeof(typename VT<V>::Partial),
-                                  ctas_per_sm<Op, V, TPB, RT, Fam>(), Culled<Op>::value);
-  if (plan.ws_bytes > ws_bytes) return kWorkspaceTooSmall;
-  if (plan.ws_bytes > 0 && ws == nullptr) return kInvalidArgument;
-  auto* part = reinterpret_cast<typename VT<V>::Partial*>(ws);
-  if (plan.W > 0) {
-    float* boxes = Culled<Op>::value ? reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + plan.box_off) : nullptr;
-    if (Culled<Op>::value)
-      launch_chained(box_kernel<Op, V, TPB, R>, plan.gx + plan.TT, TPB, 0, stream, P, (int)n, (int)m, plan.gx, boxes);
-    if constexpr (kUseExpanded<Op, V, Fam>) {
-      launch_chained(pairs_kernel_x<Op, TPB, R>, plan.C, TPB, 0, stream, P, (int)n, (int)m, plan.TT, plan.W, plan.C,
-                     part, boxes);
-    } else {
-      launch_chained(pairs_kernel<Op, V, TPB, RT, Fam>, plan.C, TPB, 0, stream, P, (int)n, (int)m, plan.TT, plan.W,
-                     plan.C, part, boxes);
-    }
+  if constexpr (CanSplit<Op>::value) {
+    if (pairs_split<Op, V, TPB, RT, Fam>(n, m))
+      return launch_pairs<Op, V, TPB, RT, Fam, true>(P, n, m, ws, ws_bytes, stream);
   }
-  const int fb = 256;
-  launch_chained(finalize_kernel<Op, V>, (int)((n + fb - 1) / fb), fb, 0, stream, P, (int)n, TPB * R, plan.TT, plan.W,
-                 plan.C, part);
-  return cudaPeekAtLastError() == cudaSuccess ? kOk : kLaunchFailure;
+  return launch_pairs<Op, V, TPB, RT, Fam, false>(P, n, m, ws, ws_bytes, stream);
 }
 
+// Scratch of either launch (a smaller problem in the same workspace may split).
 template <class Op, typename V, int TPB, int RT, class Fam = Gauss>
 inline size_t pairs_ws_bytes(int64_t n, int64_t m) {
-  return make_plan<TPB, kRunRT<Op, V, RT, Fam>>(n, m, Op::NA, sizeof(typename VT<V>::Partial),
-                                                ctas_per_sm<Op, V, TPB, RT, Fam>(), Culled<Op>::value)
-      .ws_bytes;
+  size_t b = pairs_plan<Op, V, TPB, RT, Fam, false>(n, m).ws_bytes;
+  if constexpr (CanSplit<Op>::value) {
+    const size_t s = pairs_plan<Op, V, TPB, RT, Fam, true>(n, m).ws_bytes;
+    b = s > b ? s : b;
+  }
+  return b;
 }
 
 // Workspace of an op for every kernel family (the larger of the Gaussian and Laplacian plans).

@@ -181,13 +181,7 @@ inline SymPlan make_sym_plan(int64_t n, int nr, int nc, int ctas_per_sm, size_t 
   // one resident wave of CTAs; up to half a wave more units run as one CTA each, so that no CTA takes two units while
   // others take one (forward step at 6,000 points, 576 units, 444 resident CTAs: 41.4 -> 31.7 us)
   p.C = (int)(2 * p.U < 3 * wave ? p.U : wave);
-  int smax = 1;
-  for (int i = 0; i < p.nblk; ++i) {
-    const int c0 = sk_cta_of(Geo::row_off(i, p.TT), p.U, p.C);
-    const int c1 = sk_cta_of(Geo::row_off(i + 1, p.TT) - 1, p.U, p.C);
-    if (c1 - c0 + 1 > smax) smax = c1 - c0 + 1;
-  }
-  p.S = smax;
+  p.S = sk_max_slots(p.TT, p.U, p.C);  // the longest row has TT units
   p.col_off = ((size_t)p.S * (size_t)nr * (size_t)n * row_bytes + 255) & ~(size_t)255;
   p.ws_bytes =
       p.col_off + (size_t)Geo::col_first((n + Geo::K - 1) / Geo::K) * (size_t)nc * (size_t)Geo::K * col_bytes;
@@ -407,7 +401,6 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
 // TPP): deterministic. With one thread per point, a point's slots and partials are one serial chain of up to tens
 // of dependent loads (at 2,562 points: 11 CTAs, ~11 us, latency-bound); several threads shorten the chain and
 // spread the points over more CTAs.
-constexpr int kFinThreads = 256;
 template <class Op, int TPB, int B, typename V>
 __global__ void __launch_bounds__(kFinThreads)
     finalize_sym_kernel(const typename Op::Params P, int n, int nblk, int TT, long long U, int C,
@@ -448,19 +441,8 @@ __global__ void __launch_bounds__(kFinThreads)
   if (live && j == 0) Op::finalize_sym(P, idx, v, v + Op::NR);
 }
 
-// Threads per point of finalize_sym_kernel: enough to split the longest chain of slots and column partials (a row
-// block's slots plus the blocks below it) into pieces of about four, at most 8.
-inline int sym_finalize_tpp(const SymPlan& p) {
-  const int chain = p.S + p.nblk;
-  int t = 1;
-  while (t < 8 && chain > 4 * t) t <<= 1;
-  return t;
-}
-
-inline int sym_finalize_grid(int64_t n, int tpp, int threads) {
-  const int64_t np = threads / tpp;
-  return (int)((n + np - 1) / np);
-}
+// The chain a point's epilogue sums: its block's slots and the column partials of the blocks before it.
+inline int sym_finalize_tpp(const SymPlan& p) { return finalize_tpp(p.S + p.nblk); }
 
 // Dynamic shared memory of pairs_kernel_sym (its compensated row sums).
 template <class Op, int TPB, int RT, typename V>
@@ -524,8 +506,8 @@ inline int run_pairs_sym(const typename Op::Params& P, int64_t n, void* ws, size
   auto* col_ws = reinterpret_cast<typename VT<V>::Scalar*>(reinterpret_cast<char*>(ws) + plan.col_off);
   launch_chained(pairs_kernel_sym<Op, TPB, RT, Fam, V, SPLIT>, plan.C, TPB, sym_dyn_smem_bytes<Op, TPB, RT, V>(),
                  stream, P, (int)n, plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws);
-  const int fb = kFinThreads, tpp = sym_finalize_tpp(plan);
-  launch_chained(finalize_sym_kernel<Op, TPB, (SPLIT ? 32 : TPB) * RT, V>, sym_finalize_grid(n, tpp, fb), fb, 0,
+  const int tpp = sym_finalize_tpp(plan);
+  launch_chained(finalize_sym_kernel<Op, TPB, (SPLIT ? 32 : TPB) * RT, V>, finalize_grid(n, tpp), kFinThreads, 0,
                  stream, P, (int)n, plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws, tpp);
   return cudaPeekAtLastError() == cudaSuccess ? kOk : kLaunchFailure;
 }
@@ -934,8 +916,8 @@ inline int run_pairs_symx(const typename Op::Params& P, int64_t n, void* ws, siz
   auto* col_ws = reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + plan.col_off);
   launch_chained(pairs_kernel_symx<Op, TPB, RT>, plan.C, TPB, symx_dyn_smem_bytes<Op, TPB, RT>(), stream, P, (int)n,
                  plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws);
-  const int fb = kFinThreads, tpp = sym_finalize_tpp(plan);
-  launch_chained(finalize_sym_kernel<Op, TPB, TPB * RT, F2>, sym_finalize_grid(n, tpp, fb), fb, 0, stream, P, (int)n,
+  const int tpp = sym_finalize_tpp(plan);
+  launch_chained(finalize_sym_kernel<Op, TPB, TPB * RT, F2>, finalize_grid(n, tpp), kFinThreads, 0, stream, P, (int)n,
                  plan.nblk, plan.TT, plan.U, plan.C, row_ws, col_ws, tpp);
   return cudaPeekAtLastError() == cudaSuccess ? kOk : kLaunchFailure;
 }

@@ -126,6 +126,7 @@ struct OpSOFwd {
 // outputs px_prev, pa_prev are indexed by the local target index.
 struct OpSOBwd {
   static constexpr int NS = 12, NA = 12;
+  static constexpr bool kNoSplit = true;  // its sums would take 48 KiB of shared memory
   static constexpr int kMinCtas = LDDMM_SOBWD_MIN_CTAS;
   static constexpr bool kCompInRegisters = true;  // with 4 targets per thread: measured faster than shared memory
   static constexpr int kUnroll = 8;  // measured 1.4% faster than 4 (level 6)

@@ -41,3 +41,31 @@ def test_fp32_self_sums_against_fp64_ordered(n, name):
     f1, f0 = evol.first_order_gradient(torch.stack([X, X]), A[None].contiguous(), PX, K, 0.5, euclidean=True, origin=o)
     assert close(f1[0] - PX, K64.applyDiffKT(X, PX, A, firstVar=Y, regweight=0.5, lddmm=True), 30.0)
     assert close(f0[0], K64.applyK(X, A - PX, firstVar=Y), 10.0)
+
+
+@pytest.mark.parametrize('dtype,tol', [('float32', 2e-5), ('float64', 1e-12)])
+@pytest.mark.parametrize('n,m', [(1, 1), (1, 700), (31, 33), (63, 128), (64, 129), (129, 1), (256, 127), (257, 511),
+                                 (1025, 2000), (3000, 1500), (5000, 5000)])
+def test_ordered_sums_split_and_whole(n, m, dtype, tol):
+    """The ordered-pair operators at the edges of the split shapes' blocks (32 RT targets), on both sides of the rule
+    that chooses them, against the oracle; tolerances of the operator tests."""
+    import oracle as O
+    from base.kernelFunctions import Kernel
+    rng = np.random.default_rng(1000 * n + m)
+    y, x = rng.normal(size=(n, 3)), rng.normal(size=(m, 3))
+    a, p = rng.normal(size=(m, 3)), rng.normal(size=(n, 3))
+    K = Kernel(name='gauss', sigma=0.7)
+    K.pk_dtype = dtype
+
+    def close(got, ref):
+        return np.linalg.norm(got - ref) <= tol * np.linalg.norm(ref) + 0.05 * tol * np.sqrt(ref.size)
+
+    assert close(K.applyK(x, a, firstVar=y), O.apply_k(y, x, a, 0.7))
+    assert close(K.applyDiffKT(x, p, a, firstVar=y), O.apply_diff_kt(y, x, p, a, 0.7))
+    assert close(K.applyDivergence(x, a, firstVar=y).ravel(), np.ravel(O.apply_divergence(y, x, a, 0.7)))
+    ay, ax = rng.normal(size=n), rng.normal(size=m)
+    kt = O.apply_k_tensor(y, x, ay, ax, p, a, 0.7)
+    assert close(K.applyKTensor(x, ay, ax, p, a, firstVar=y).ravel(), np.ravel(kt))
+    q = rng.normal(size=(n, 3))
+    assert close(K.applyDDiffK11and12(y, p, q, p), O.apply_ddiff_k11and12(y, p, q, p, 0.7))
+    assert close(K.applyDiffK1and2(y, p, q), O.apply_diff_k1and2(y, p, q, 0.7))
