@@ -460,6 +460,91 @@ __host__ __device__ __forceinline__ int sk_cta_of(long long u, long long W, long
 
 int device_sm_count();
 
+__host__ __device__ __forceinline__ long long sym_tri(long long j) { return j * (j - 1) / 2; }
+
+// The unit triangle for row blocks of B points and tiles of TPB: B a multiple of TPB (a row block spans kSpan tiles)
+// or a divisor of it (a tile holds kShare row blocks). Row i takes the tiles from its own first one on; the tiles that
+// overlap its own superblock of K = max(B, TPB) points are diagonal (rows only).
+template <int TPB, int B>
+struct SymGeom {
+  static_assert(B % TPB == 0 || TPB % B == 0, "row blocks and tiles must nest");
+  static constexpr int kSpan = B >= TPB ? B / TPB : 1, kShare = B < TPB ? TPB / B : 1;
+  static constexpr int K = B >= TPB ? B : TPB;
+  static __host__ __device__ __forceinline__ int first_tile(int i) { return B >= TPB ? i * kSpan : i / kShare; }
+  // first unit of row i: the sum of TT - first_tile over the rows before it
+  static __host__ __device__ __forceinline__ long long row_off(long long i, long long TT) {
+    if (B >= TPB) return i * TT - kSpan * sym_tri(i);
+    const long long q = i / kShare, r = i - q * kShare;
+    return i * TT - (kShare * sym_tri(q) + q * r);
+  }
+  // column partials: superblock J receives one per row block before it (kShare J of them), K points each; offset of
+  // the first one (in units of K points)
+  static __host__ __device__ __forceinline__ long long col_first(long long J) { return kShare * sym_tri(J); }
+
+  static __device__ __forceinline__ int row_of(long long u, int nblk, long long TT) {
+    int lo = 0, hi = nblk - 1;  // largest i with row_off(i) <= u
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (row_off(mid, TT) <= u) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+  }
+};
+
+// Ops whose sum over all targets is all that is used (the energies) declare `static constexpr bool kTriangle = true;`.
+// Their sources begin with the targets themselves (Op::self_count(P) of them, padded to whole tiles), and a term of
+// that part is symmetric in the pair: target block i takes the self tiles from its own first one on, with weight 1 on
+// its own superblock and 2 beyond it (Op::weigh), and every other source. A quarter of the pairs of an energy |S|^2 -
+// 2 <S, S1> between surfaces of like size goes, half of those of a norm.
+template <class Op, class = void>
+struct Triangle : std::false_type {};
+template <class Op>
+struct Triangle<Op, std::void_t<decltype(Op::kTriangle)>> : std::bool_constant<Op::kTriangle> {};
+
+// The units of an ordered sum: target blocks of B, source tiles of TPB, row-major; a triangle op's rows begin at their
+// own first tile.
+template <class Op, int TPB, int B>
+struct Units {
+  static constexpr bool kTri = Triangle<Op>::value;
+  using Geo = SymGeom<TPB, B>;
+  static __host__ __device__ __forceinline__ long long row_off(long long i, long long TT) {
+    return kTri ? Geo::row_off(i, TT) : i * TT;
+  }
+  static __device__ __forceinline__ int row_of(long long u, int gx, long long TT) {
+    return kTri ? Geo::row_of(u, gx, TT) : (int)(u / TT);
+  }
+  static __device__ __forceinline__ int first_tile(int i) { return kTri ? Geo::first_tile(i) : 0; }
+  // source of thread `tid` in tile j (whether there is one in `live`), and its weight for target block i
+  static __device__ __forceinline__ int source(const typename Op::Params& P, int i, int j, int m, bool& live,
+                                               double& weight) {
+    weight = 1.0;
+    if constexpr (kTri) {
+      const int self = Op::self_count(P), ts = (self + TPB - 1) / TPB;
+      if (j < ts) {
+        const int l = j * TPB + (int)threadIdx.x;
+        live = l < self;
+        if (j >= Geo::first_tile(i) + Geo::kSpan) weight = 2.0;
+        return l;
+      }
+      const int l = self + (j - ts) * TPB + (int)threadIdx.x;
+      live = l < m;
+      return l;
+    } else {
+      const int l = j * TPB + (int)threadIdx.x;
+      live = l < m;
+      return l;
+    }
+  }
+  static inline int64_t tiles(const typename Op::Params& P, int64_t m) {
+    if constexpr (kTri) {
+      const int64_t self = Op::self_count(P);
+      return (self + TPB - 1) / TPB + (m - self + TPB - 1) / TPB;
+    } else {
+      return (m + TPB - 1) / TPB;
+    }
+  }
+};
+
 // Most CTAs that a window of `len` consecutive units of W meets when C CTAs divide them evenly (each takes at least
 // floor(W / C) units): the partial slots of a target block.
 inline int sk_max_slots(long long len, long long W, long long C) {
@@ -469,14 +554,14 @@ inline int sk_max_slots(long long len, long long W, long long C) {
 
 // `boxes`: reserve the coordinate boxes of exact culling (ops with Culled<Op>); other ops never read them, so their
 // scratch is the partial slots alone (at most (C / gx + 2) * na * n partials, whatever m is).
-template <int TPB, int B>
-inline SKPlan make_plan(int64_t n, int64_t m, int na, size_t partial_bytes, int ctas_per_sm, bool boxes = true) {
+template <class Op, int TPB, int B>
+inline SKPlan make_plan(int64_t n, int64_t tiles, int na, size_t partial_bytes, int ctas_per_sm, bool boxes = true) {
   SKPlan p;
   if (n <= 0) return p;
   p.gx = (int)((n + B - 1) / B);
-  if (m <= 0) return p;
-  p.TT = (int)((m + TPB - 1) / TPB);
-  p.W = (long long)p.gx * p.TT;
+  if (tiles <= 0) return p;
+  p.TT = (int)tiles;
+  p.W = Units<Op, TPB, B>::row_off(p.gx, p.TT);
   const long long wave = (long long)device_sm_count() * (ctas_per_sm > 0 ? ctas_per_sm : 1);
   p.C = (int)(p.W < wave ? p.W : wave);
   p.S = sk_max_slots(p.TT, p.W, p.C);
@@ -578,6 +663,7 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
   // farther apart than the distance at which the kernel's radial factors are exactly zero in this arithmetic
   // contributes exactly nothing, and is skipped by the whole CTA.
   constexpr float kZeroR2 = Fam::template kCullR2<V>;
+  using Un = Units<Op, TPB, TW * RT>;
   const int gx = (n + TW * RT - 1) / (TW * RT);
   __shared__ float tbox[6];  // the segment's target box, in shared memory (re-read per tile, not held in registers)
   VT<V>::setup();
@@ -585,11 +671,13 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
 
   const long long u_end = sk_start(blockIdx.x + 1, W, C);
   long long u = sk_start(blockIdx.x, W, C);
+  int tb = u < u_end ? Un::row_of(u, gx, TT) : 0;
   while (u < u_end) {
-    const int tb = (int)(u / TT);
-    const int j0 = (int)(u - (long long)tb * TT);
-    const int j1 = (int)((u_end - (long long)tb * TT) < TT ? (u_end - (long long)tb * TT) : TT);
-    const int slot = (int)blockIdx.x - sk_cta_of((long long)tb * TT, W, C);
+    const long long off = Un::row_off(tb, TT);
+    const int first = Un::first_tile(tb);
+    const int j0 = first + (int)(u - off);
+    const int j1 = first + (int)((u_end - off) < TT - first ? (u_end - off) : TT - first);
+    const int slot = (int)blockIdx.x - sk_cta_of(off, W, C);
 
     typename Op::template Tgt<V> tgt[G];
     Comp<V> cmp[G][Op::NA];   // used when !kSm
@@ -618,12 +706,15 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
         const float* sbox = boxes + 6 * (gx + j);
         if (box_gap2(tbox, tbox + 3, sbox, sbox + 3) > kZeroR2) continue;  // uniform over the CTA
       }
-      const int l = j * TPB + threadIdx.x;
       {
+        bool live;
+        double weight;
+        const int l = Un::source(P, tb, j, m, live, weight);
         double f[2 * NU];
 #pragma unroll
         for (int q = 0; q < 2 * NU; ++q) f[q] = 0.0;
-        if (l < m) Op::source_fields(P, l, f);
+        if (live) Op::source_fields(P, l, f);
+        if constexpr (Un::kTri) Op::weigh(f + 3, weight);
 #pragma unroll
         for (int q = 0; q < NU; ++q) {
           Unit<V> w;
@@ -706,6 +797,7 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
         }
     }
     u += j1 - j0;
+    ++tb;
   }
 }
 
@@ -760,16 +852,19 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, F2>::value)
   __shared__ F2 cs[kSm ? G * NAX * 2 : 1][TPB];
   const Frame& f = P.f;
   const double fo[3] = {f.o0, f.o1, f.o2};
+  using Un = Units<Op, TPB, TW * RT>;
   const int gx = (n + TW * RT - 1) / (TW * RT);
   chain_wait();
 
   const long long u_end = sk_start(blockIdx.x + 1, W, C);
   long long u = sk_start(blockIdx.x, W, C);
+  int tb = u < u_end ? Un::row_of(u, gx, TT) : 0;
   while (u < u_end) {
-    const int tb = (int)(u / TT);
-    const int j0 = (int)(u - (long long)tb * TT);
-    const int j1 = (int)((u_end - (long long)tb * TT) < TT ? (u_end - (long long)tb * TT) : TT);
-    const int slot = (int)blockIdx.x - sk_cta_of((long long)tb * TT, W, C);
+    const long long off = Un::row_off(tb, TT);
+    const int first = Un::first_tile(tb);
+    const int j0 = first + (int)(u - off);
+    const int j1 = first + (int)((u_end - off) < TT - first ? (u_end - off) : TT - first);
+    const int slot = (int)blockIdx.x - sk_cta_of(off, W, C);
     const int base = tb * (TW * RT) + (SPLIT ? lane : (int)threadIdx.x);
 
     // the block's box and centre (every CTA working on block tb derives the same ones)
@@ -826,14 +921,17 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, F2>::value)
         const float* sbox = boxes + 6 * (gx + j);
         if (box_gap2(lo, hi, sbox, sbox + 3) > Gauss::kCullR2<F2>) continue;  // uniform over the CTA
       }
-      const int l = j * TPB + threadIdx.x;
       {
+        bool live;
+        double weight;
+        const int l = Un::source(P, tb, j, m, live, weight);
         double fl[2 * NU];
 #pragma unroll
         for (int q = 0; q < 2 * NU; ++q) fl[q] = 0.0;
-        if (l < m) {
+        if (live) {
           double xr[3], r2 = 0.0;
           Op::source_point(P, l, xr, fl + 4);
+          if constexpr (Un::kTri) Op::weigh_x(fl + 4, weight);
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             const float xc = (float)((xr[c] - fo[c]) * f.s - (double)ob[c]);
@@ -947,6 +1045,7 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, F2>::value)
       }
     if constexpr (SPLIT) __syncthreads();  // the next segment clears the sums
     u += j1 - j0;
+    ++tb;
   }
 }
 
@@ -983,8 +1082,10 @@ __global__ void __launch_bounds__(TPB) box_kernel(const typename Op::Params P, i
       }
     }
   } else {
-    const int l = (b - gx) * TPB + threadIdx.x;
-    if (l < m) {
+    bool live;
+    double weight;
+    const int l = Units<Op, TPB, TW * RT>::source(P, 0, b - gx, m, live, weight);
+    if (live) {
       double f[2 * NU];
       Op::source_fields(P, l, f);
 #pragma unroll
@@ -1006,9 +1107,9 @@ __global__ void __launch_bounds__(TPB) box_kernel(const typename Op::Params P, i
 // 1, ... from shared memory, so the order of every addition is fixed. With one thread per target its slots are one
 // serial chain (surface gradient of 2,990 against 3,534 faces: 41 us for 47 slots of 8 sums).
 constexpr int kFinThreads = 256;
-template <class Op, typename V>
+template <class Op, typename V, int TPB, int B>
 __global__ void __launch_bounds__(kFinThreads)
-    finalize_kernel(const typename Op::Params P, int n, int tb_targets, int TT, long long W, int C,
+    finalize_kernel(const typename Op::Params P, int n, int TT, long long W, int C,
                     const typename VT<V>::Partial* __restrict__ ws, int tpp) {
   __shared__ double red[kFinThreads][Op::NA];
   const int np = kFinThreads / tpp;
@@ -1019,8 +1120,9 @@ __global__ void __launch_bounds__(kFinThreads)
 #pragma unroll
   for (int c = 0; c < Op::NA; ++c) acc[c] = 0.0;
   if (i < n && W > 0) {
-    const int tb = i / tb_targets;
-    const int nslot = sk_cta_of((long long)(tb + 1) * TT - 1, W, C) - sk_cta_of((long long)tb * TT, W, C) + 1;
+    using Un = Units<Op, TPB, B>;
+    const int tb = i / B;
+    const int nslot = sk_cta_of(Un::row_off(tb + 1, TT) - 1, W, C) - sk_cta_of(Un::row_off(tb, TT), W, C) + 1;
     for (int s = j; s < nslot; s += tpp)
 #pragma unroll
       for (int c = 0; c < Op::NA; ++c) acc[c] += partial_value(ws[((size_t)s * Op::NA + c) * (size_t)n + i]);
@@ -1075,9 +1177,9 @@ template <class Op>
 struct CanSplit<Op, std::void_t<decltype(Op::kNoSplit)>> : std::bool_constant<!Op::kNoSplit> {};
 
 template <class Op, typename V, int TPB, int RT, class Fam, bool SPLIT>
-inline SKPlan pairs_plan(int64_t n, int64_t m) {
-  return make_plan<TPB, (SPLIT ? 32 : TPB) * kRunRT<Op, V, RT, Fam>>(
-      n, m, Op::NA, sizeof(typename VT<V>::Partial), ctas_per_sm<Op, V, TPB, RT, Fam, SPLIT>(), Culled<Op>::value);
+inline SKPlan pairs_plan(int64_t n, int64_t tiles) {
+  return make_plan<Op, TPB, (SPLIT ? 32 : TPB) * kRunRT<Op, V, RT, Fam>>(
+      n, tiles, Op::NA, sizeof(typename VT<V>::Partial), ctas_per_sm<Op, V, TPB, RT, Fam, SPLIT>(), Culled<Op>::value);
 }
 
 // Whether a problem splits: its whole-tile units would fill less than a third of one resident wave (FP32), or less than
@@ -1087,9 +1189,9 @@ inline SKPlan pairs_plan(int64_t n, int64_t m) {
 // faces: 33.6 | 30.4, 5,120 (1.8): 79.3 | 81.4. FP64 K a 642: 13.6 | 8.0, applyDiffKT 2,562 (0.4): 25.8 | 22.7, 6,000
 // (1.9): 93 | 82, varifold gradient 5,120 (2.7): 159 | 162, K a 20,000 (21): 577 | 597.
 template <class Op, typename V, int TPB, int RT, class Fam>
-inline bool pairs_split(int64_t n, int64_t m) {
+inline bool pairs_split(int64_t n, int64_t tiles) {
   constexpr int64_t B = (int64_t)TPB * kRunRT<Op, V, RT, Fam>;
-  const int64_t units = ((n + B - 1) / B) * ((m + TPB - 1) / TPB);
+  const int64_t units = ((n + B - 1) / B) * tiles;
   const int64_t wave = (int64_t)device_sm_count() * ctas_per_sm<Op, V, TPB, RT, Fam, false>();
   return std::is_same<V, F2>::value ? 3 * units < wave : 2 * units < 5 * wave;
 }
@@ -1098,7 +1200,7 @@ template <class Op, typename V, int TPB, int RT, class Fam, bool SPLIT>
 inline int launch_pairs(const typename Op::Params& P, int64_t n, int64_t m, void* ws, size_t ws_bytes,
                         cudaStream_t stream) {
   constexpr int R = kRunRT<Op, V, RT, Fam>;
-  const SKPlan plan = pairs_plan<Op, V, TPB, RT, Fam, SPLIT>(n, m);
+  const SKPlan plan = pairs_plan<Op, V, TPB, RT, Fam, SPLIT>(n, Units<Op, TPB, TPB>::tiles(P, m));
   if (plan.ws_bytes > ws_bytes) return kWorkspaceTooSmall;
   if (plan.ws_bytes > 0 && ws == nullptr) return kInvalidArgument;
   auto* part = reinterpret_cast<typename VT<V>::Partial*>(ws);
@@ -1116,8 +1218,8 @@ inline int launch_pairs(const typename Op::Params& P, int64_t n, int64_t m, void
     }
   }
   const int tpp = finalize_tpp(plan.S);
-  launch_chained(finalize_kernel<Op, V>, finalize_grid(n, tpp), kFinThreads, 0, stream, P, (int)n,
-                 (SPLIT ? 32 : TPB) * R, plan.TT, plan.W, plan.C, part, tpp);
+  launch_chained(finalize_kernel<Op, V, TPB, (SPLIT ? 32 : TPB) * R>, finalize_grid(n, tpp), kFinThreads, 0, stream, P,
+                 (int)n, plan.TT, plan.W, plan.C, part, tpp);
   return cudaPeekAtLastError() == cudaSuccess ? kOk : kLaunchFailure;
 }
 
@@ -1127,18 +1229,20 @@ inline int run_pairs(const typename Op::Params& P, int64_t n, int64_t m, void* w
   if (n <= 0) return kOk;
   if (n > INT32_MAX / 4 || m > INT32_MAX / 4) return kInvalidArgument;
   if constexpr (CanSplit<Op>::value) {
-    if (pairs_split<Op, V, TPB, RT, Fam>(n, m))
+    if (pairs_split<Op, V, TPB, RT, Fam>(n, Units<Op, TPB, TPB>::tiles(P, m)))
       return launch_pairs<Op, V, TPB, RT, Fam, true>(P, n, m, ws, ws_bytes, stream);
   }
   return launch_pairs<Op, V, TPB, RT, Fam, false>(P, n, m, ws, ws_bytes, stream);
 }
 
-// Scratch of either launch (a smaller problem in the same workspace may split).
+// Scratch of either launch (a smaller problem in the same workspace may split). A triangle op's sources are n targets
+// and m - n others, each padded to whole tiles.
 template <class Op, typename V, int TPB, int RT, class Fam = Gauss>
 inline size_t pairs_ws_bytes(int64_t n, int64_t m) {
-  size_t b = pairs_plan<Op, V, TPB, RT, Fam, false>(n, m).ws_bytes;
+  const int64_t tiles = Triangle<Op>::value ? (n + TPB - 1) / TPB + (m - n + TPB - 1) / TPB : (m + TPB - 1) / TPB;
+  size_t b = pairs_plan<Op, V, TPB, RT, Fam, false>(n, tiles).ws_bytes;
   if constexpr (CanSplit<Op>::value) {
-    const size_t s = pairs_plan<Op, V, TPB, RT, Fam, true>(n, m).ws_bytes;
+    const size_t s = pairs_plan<Op, V, TPB, RT, Fam, true>(n, tiles).ws_bytes;
     b = s > b ? s : b;
   }
   return b;

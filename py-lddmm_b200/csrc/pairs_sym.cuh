@@ -131,37 +131,6 @@ struct SymStage<NF, TPB, F2> {
   static constexpr int kFields = 4 * ((NF + 3) / 4);  // size of the FP64 field buffer and of the operand array
 };
 
-__host__ __device__ __forceinline__ long long sym_tri(long long j) { return j * (j - 1) / 2; }
-
-// The unit triangle for row blocks of B points and tiles of TPB: B a multiple of TPB (a row block spans kSpan tiles)
-// or a divisor of it (a tile holds kShare row blocks). Row i takes the tiles from its own first one on; the tiles that
-// overlap its own superblock of K = max(B, TPB) points are diagonal (rows only).
-template <int TPB, int B>
-struct SymGeom {
-  static_assert(B % TPB == 0 || TPB % B == 0, "row blocks and tiles must nest");
-  static constexpr int kSpan = B >= TPB ? B / TPB : 1, kShare = B < TPB ? TPB / B : 1;
-  static constexpr int K = B >= TPB ? B : TPB;
-  static __host__ __device__ __forceinline__ int first_tile(int i) { return B >= TPB ? i * kSpan : i / kShare; }
-  // first unit of row i: the sum of TT - first_tile over the rows before it
-  static __host__ __device__ __forceinline__ long long row_off(long long i, long long TT) {
-    if (B >= TPB) return i * TT - kSpan * sym_tri(i);
-    const long long q = i / kShare, r = i - q * kShare;
-    return i * TT - (kShare * sym_tri(q) + q * r);
-  }
-  // column partials: superblock J receives one per row block before it (kShare J of them), K points each; offset of
-  // the first one (in units of K points)
-  static __host__ __device__ __forceinline__ long long col_first(long long J) { return kShare * sym_tri(J); }
-
-  static __device__ __forceinline__ int row_of(long long u, int nblk, long long TT) {
-    int lo = 0, hi = nblk - 1;  // largest i with row_off(i) <= u
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (row_off(mid, TT) <= u) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-  }
-};
-
 struct SymPlan {
   int nblk = 0, TT = 0, C = 0, S = 0;
   long long U = 0;

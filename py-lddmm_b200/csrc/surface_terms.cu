@@ -95,7 +95,7 @@ __device__ __forceinline__ void load_face_target(const FaceRec* T, const Frame& 
   }
 }
 
-// ---- energies: dots[k] = weight_k * sum_l e_kl payload_kl. Varifold 13 FP32 + 1 SFU per pair. ----
+// ---- energies: dots[k] = weight_k * sum_l e_kl payload_kl; only their sum is used. Varifold 13 FP32 + 1 SFU per pair. ----
 template <int KIND>
 struct OpSurfEnergy {
   static constexpr int NS = 7, NA = (KIND == LDDMM_DATA_CURRENT) ? 3 : 1;
@@ -107,6 +107,18 @@ struct OpSurfEnergy {
     double* dots;
     Frame f;
   };
+  static constexpr bool kTriangle = true;  // the sum over the targets is what is used; sources begin with them
+  static __host__ __device__ __forceinline__ int self_count(const Params& P) { return P.S.mA; }
+  // weight of a source: on the staged fields after the coordinates, and on the payload of the expanded form
+  static __device__ __forceinline__ void weigh(double* f, double w) {
+    if (KIND == LDDMM_DATA_CURRENT)
+      for (int c = 1; c < 4; ++c) f[c] *= w;
+    else
+      f[0] *= w;
+  }
+  static __device__ __forceinline__ void weigh_x(double* f, double w) {
+    for (int c = 0; c < (KIND == LDDMM_DATA_CURRENT ? 3 : 1); ++c) f[c] *= w;
+  }
   template <typename V> using Tgt = FaceTgt<V>;
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {

@@ -69,3 +69,28 @@ def test_ordered_sums_split_and_whole(n, m, dtype, tol):
     q = rng.normal(size=(n, 3))
     assert close(K.applyDDiffK11and12(y, p, q, p), O.apply_ddiff_k11and12(y, p, q, p, 0.7))
     assert close(K.applyDiffK1and2(y, p, q), O.apply_diff_k1and2(y, p, q, 0.7))
+
+
+@pytest.mark.parametrize('nf,nf1', [(1, 1), (127, 1), (128, 129), (129, 640), (257, 255), (1025, 3000), (3000, 700),
+                                    (5120, 5119)])
+def test_energies_once_per_unordered_self_pair(nf, nf1):
+    """Varifold, current and measure energies and norms of meshes whose face counts end inside a tile, a row block and
+    the self part of the sources, against the oracle. Tolerances of the surface tests: 1e-6 of the energy's two norms
+    in FP32, 1e-11 in FP64."""
+    import oracle as O
+    from base.kernelFunctions import Kernel
+    from base.surfaceDistances import SurfaceDataTerm
+    from base.syntheticShapes import bumpy_ellipsoid, icosphere
+    v, f = icosphere(4)
+    x, x1 = bumpy_ellipsoid(v, seed=3), bumpy_ellipsoid(v, seed=4)
+    f0, f1 = f[:nf], f[::-1][:nf1].copy()
+    for kind in ('varifold', 'current', 'measure'):
+        norm0 = {'varifold': O.varifold_norm0, 'current': O.current_norm0, 'measure': O.measure_norm0}[kind]
+        ndef = {'varifold': O.varifold_norm_def, 'current': O.current_norm_def, 'measure': O.measure_norm_def}[kind]
+        ref, ref0 = ndef(x, f0, x1, f1, 0.3), norm0(x1, f1, 0.3)
+        size = abs(ref0) + norm0(x, f0, 0.3)
+        for dtype, tol in (('float32', 1e-6), ('float64', 1e-11)):
+            Kd = Kernel(name='gauss', sigma=0.3)
+            Kd.pk_dtype = dtype
+            e = SurfaceDataTerm(f0, x1, f1, Kd, kind=kind, nv=x.shape[0]).energy(x, with_norm0=True).tolist()
+            assert abs(e[0] - ref) <= tol * size and abs(e[1] - ref0) <= tol * size, (kind, dtype)
