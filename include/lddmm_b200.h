@@ -241,6 +241,29 @@ int lddmm_mse_grad(const float* y, int64_t M, int64_t N, const float* target, in
 int lddmm_adam_step(float* param, const float* grad, float* m1, float* m2, void* param_bf16, int64_t count, float lr,
                     float beta1, float beta2, float eps, int64_t step, float weight_decay, lddmm_stream_t stream);
 
+/* lddmm_adam_step on several tensors in one launch; the arguments of lddmm_adam_step as HOST arrays of `tensors`
+ * entries (param_bf16[k] may be NULL). */
+#define LDDMM_ADAM_MAX_TENSORS 32
+int lddmm_adam_steps(int tensors, float* const* param, const float* const* grad, float* const* m1, float* const* m2,
+                     void* const* param_bf16, const int64_t* count, float lr, float beta1, float beta2, float eps,
+                     int64_t step, float weight_decay, lddmm_stream_t stream);
+
+/* The network's layers in one call: h_0 = x (M, dims[0]) bf16, h_{i+1} = relu(h_i W_i + b_i) bf16 into acts[i], and
+ * y (M, dims[layers]) f32 = h W + b of the last layer. W_i (dims[i], dims[i+1]) bf16, b_i f32; `dims`, W, b and acts
+ * are HOST arrays (layers + 1, layers, layers and layers - 1 entries). M and all dims multiples of 64. */
+#define LDDMM_MLP_MAX_LAYERS 8
+int lddmm_mlp_forward(const int64_t* dims, int layers, const void* x, int64_t M, const void* const* W,
+                      const float* const* b, void* const* acts, float* y, lddmm_stream_t stream);
+
+/* Forward and backward pass: loss[0] = w * sum of the squared errors of the first nout outputs of rows < valid against
+ * target (M, nout) f32, dW_i and db_i (f32) its gradients with BF16 activations and deltas (lddmm_mse_grad,
+ * lddmm_bf16_gemm). Fixed reduction order. workspace: lddmm_mlp_workspace_bytes(dims, layers, M). */
+size_t lddmm_mlp_workspace_bytes(const int64_t* dims, int layers, int64_t M);
+int lddmm_mlp_gradients(const int64_t* dims, int layers, const void* x, int64_t M, const void* const* W,
+                        const float* const* b, const float* target, int64_t nout, int64_t valid, float w,
+                        float* const* dW, float* const* db, float* loss, void* workspace, size_t workspace_bytes,
+                        lddmm_stream_t stream);
+
 /* disp(n,3) = tgt[argmin_l |src_k - tgt_l|] - src_k: nearest-target displacement of every source point. */
 int lddmm_nearest_displacement(const double* src, int64_t n, const double* tgt, int64_t m, double* disp,
                                lddmm_stream_t stream);

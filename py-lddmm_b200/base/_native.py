@@ -63,11 +63,18 @@ SIGNATURES = {
     'lddmm_mse_grad': [_dp, _i64, _i64, _dp, _i64, _i64, ctypes.c_float, _dp, _dp, _vp],
     'lddmm_adam_step': [_dp, _dp, _dp, _dp, _dp, _i64, ctypes.c_float, ctypes.c_float, ctypes.c_float,
                         ctypes.c_float, _i64, ctypes.c_float, _vp],
+    'lddmm_adam_steps': [_int, _vp, _vp, _vp, _vp, _vp, _vp, ctypes.c_float, ctypes.c_float, ctypes.c_float,
+                         ctypes.c_float, _i64, ctypes.c_float, _vp],
+    'lddmm_mlp_forward': [_vp, _int, _dp, _i64, _vp, _vp, _vp, _dp, _vp],
+    'lddmm_mlp_workspace_bytes': [_vp, _int, _i64],
+    'lddmm_mlp_gradients': [_vp, _int, _dp, _i64, _vp, _vp, _dp, _i64, _i64, ctypes.c_float, _vp, _vp, _dp, _vp, _sz,
+                            _vp],
     'lddmm_nearest_displacement': [_dp, _i64, _dp, _i64, _dp, _vp],
     'lddmm_lbfgs_direction': [_vp, _vp, _int, _dp, _i64, _dp, _vp],
 }
 LBFGS_MAX_PAIRS = 64        # LDDMM_LBFGS_MAX_PAIRS of the header
 _RESTYPES = {'lddmm_version': ctypes.c_char_p, 'lddmm_status_string': ctypes.c_char_p,
+             'lddmm_mlp_workspace_bytes': ctypes.c_size_t,
              'lddmm_workspace_bytes': ctypes.c_size_t, 'lddmm_surface_workspace_bytes': ctypes.c_size_t}
 
 _lib = None
@@ -125,6 +132,11 @@ def stream_ptr():
 
 def ptr(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None else ctypes.c_void_p(0)
+
+
+def ptrs(tensors):
+    """Host array of the tensors' device pointers (None: NULL)."""
+    return (ctypes.c_void_p * max(len(tensors), 1))(*[0 if t is None else t.data_ptr() for t in tensors])
 
 
 def origin_arg(origin):

@@ -28,6 +28,7 @@ registration meets); each is rescaled to an initial speed drawn in [vmin, vmax].
 Coarse to fine (multilevel_warm_start): the proposal is made on a coarse triangulation of the source, refined there
 by the plain optimiser, and its momentum density carried to the full-resolution source (prolong_momentum).
 """
+import ctypes
 import math
 
 import numpy as np
@@ -54,8 +55,6 @@ MOMENTUM_LAW_SHAPES = ('a = (w1 q + w2 b + w3 K_0.4 z) n: q = x^T M x (M symmetr
                        'white noise, weights U[0,1], each field scaled to max 1; rescaled to a maximum initial speed '
                        'U[0.05, 0.35]; shot with sigma 0.5, T = 10')
 SCALAR_WIDTHS = (0.1, 0.2, 0.35, 0.7)
-# rows per split of the weight-gradient GEMMs (act^T dy, K = the batch's rows): split-K keeps the whole GPU busy
-SPLIT_ROWS = 512
 ROW_PAD = 64
 
 
@@ -158,65 +157,45 @@ class MomentumProposal:
         self.step = 0
 
     # ------------------------------------------------------------------ kernels
-    @staticmethod
-    def _gemm(ta, tb, epi, A, B, C, M, N, K, bias=None, mask=None, splits=1, split_ws=None):
-        sw, swb = (split_ws, split_ws.numel() * 4) if split_ws is not None else (None, 0)
-        nat.check(nat.lib().lddmm_bf16_gemm(ta, tb, epi, M, N, K, nat.ptr(A), nat.ptr(B), nat.ptr(bias),
-                                            nat.ptr(mask), nat.ptr(C), splits, nat.ptr(sw), swb, nat.stream_ptr()),
-                  'bf16_gemm')
+    def _dims(self):
+        return (ctypes.c_int64 * len(self.dims))(*self.dims)
 
     def forward(self, F, keep=False):
         """F (M, IN_DIM) bf16, M a multiple of 64 -> (M, 64) f32 outputs (and the activations when keep)."""
         M = F.shape[0]
-        acts = [F]
-        h = F
-        for i in range(3):
-            out = torch.empty((M, self.dims[i + 1]), dtype=torch.bfloat16, device=F.device)
-            self._gemm(0, 0, 2, h, self.Wb[i], out, M, self.dims[i + 1], self.dims[i], bias=self.b[i])
-            acts.append(out)
-            h = out
+        acts = [torch.empty((M, d), dtype=torch.bfloat16, device=F.device) for d in self.dims[1:-1]]
         y = torch.empty((M, OUT_DIM), dtype=torch.float32, device=F.device)
-        self._gemm(0, 0, 1, h, self.Wb[3], y, M, OUT_DIM, HIDDEN, bias=self.b[3])
-        return (y, acts) if keep else y
+        nat.check(nat.lib().lddmm_mlp_forward(self._dims(), len(self.W), nat.ptr(F), M, nat.ptrs(self.Wb),
+                                              nat.ptrs(self.b), nat.ptrs(acts), nat.ptr(y), nat.stream_ptr()),
+                  'mlp_forward')
+        return (y, [F] + acts) if keep else y
 
     def gradients(self, F, target, valid, weight=None):
         """Loss (device scalar) and FP32 gradients [dW0..dW3, db0..db3] of the mean squared error on the first 3
         outputs of rows < valid (target (M,3) f32)."""
         M = F.shape[0]
-        y, acts = self.forward(F, keep=True)
         w = (1.0 / max(valid, 1)) if weight is None else weight
-        dy = torch.empty((M, OUT_DIM), dtype=torch.bfloat16, device=F.device)
-        row_loss = torch.empty(M, dtype=torch.float32, device=F.device)
-        nat.check(nat.lib().lddmm_mse_grad(nat.ptr(y), M, OUT_DIM, nat.ptr(target), N_OUT, int(valid), float(w),
-                                           nat.ptr(dy), nat.ptr(row_loss), nat.stream_ptr()), 'mse_grad')
-        splits = max(1, min(64, M // SPLIT_ROWS))
-        split_ws = torch.empty(splits * HIDDEN * HIDDEN, dtype=torch.float32, device=F.device) if splits > 1 else None
-        col_ws = torch.empty(((M + 255) // 256) * max(self.dims), dtype=torch.float32, device=F.device)
-        dW, db = [None] * 4, [None] * 4
-        for i in range(3, -1, -1):
-            fi, fo = self.dims[i], self.dims[i + 1]
-            gw = torch.empty((fi, fo), dtype=torch.float32, device=F.device)
-            sp = splits if split_ws is not None and fi * fo <= HIDDEN * HIDDEN else 1
-            self._gemm(1, 0, 0, acts[i], dy, gw, fi, fo, M, splits=sp, split_ws=split_ws if sp > 1 else None)
-            gb = torch.empty(fo, dtype=torch.float32, device=F.device)
-            nat.check(nat.lib().lddmm_bf16_colsum(nat.ptr(dy), M, fo, nat.ptr(gb), nat.ptr(col_ws), col_ws.numel() * 4,
-                                                  nat.stream_ptr()), 'colsum')
-            dW[i], db[i] = gw, gb
-            if i > 0:
-                dx = torch.empty((M, fi), dtype=torch.bfloat16, device=F.device)
-                self._gemm(0, 1, 4, dy, self.Wb[i], dx, M, fi, fo, mask=acts[i])
-                dy = dx
-        loss = row_loss.sum() * w
-        return loss, dW + db
+        sizes = [p.numel() for p in self.W + self.b]
+        flat = torch.empty(sum(sizes) + 1, dtype=torch.float32, device=F.device)
+        out = flat.split(sizes + [1])
+        grads = [g.view(p.shape) for g, p in zip(out, self.W + self.b)]
+        dims, n = self._dims(), len(self.W)
+        nb = nat.lib().lddmm_mlp_workspace_bytes(dims, n, M)
+        ws = torch.empty(max(nb, 1), dtype=torch.uint8, device=F.device)
+        nat.check(nat.lib().lddmm_mlp_gradients(dims, n, nat.ptr(F), M, nat.ptrs(self.Wb), nat.ptrs(self.b),
+                                                nat.ptr(target), N_OUT, int(valid), float(w), nat.ptrs(grads[:n]),
+                                                nat.ptrs(grads[n:]), nat.ptr(out[-1]), nat.ptr(ws), nb,
+                                                nat.stream_ptr()), 'mlp_gradients')
+        return out[-1].view(()), grads
 
     def adam(self, grads, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0):
         self.step += 1
         params = self.W + self.b
-        for k, (p, g) in enumerate(zip(params, grads)):
-            pb = self.Wb[k] if k < 4 else None
-            nat.check(nat.lib().lddmm_adam_step(nat.ptr(p), nat.ptr(g), nat.ptr(self.m[k]), nat.ptr(self.v[k]),
-                                                nat.ptr(pb), p.numel(), lr, beta1, beta2, eps, self.step,
-                                                weight_decay, nat.stream_ptr()), 'adam_step')
+        n = len(params)
+        counts = (ctypes.c_int64 * n)(*[p.numel() for p in params])
+        nat.check(nat.lib().lddmm_adam_steps(n, nat.ptrs(params), nat.ptrs(grads), nat.ptrs(self.m), nat.ptrs(self.v),
+                                             nat.ptrs(list(self.Wb) + [None] * (n - len(self.Wb))), counts, lr, beta1,
+                                             beta2, eps, self.step, weight_decay, nat.stream_ptr()), 'adam_steps')
 
     # ------------------------------------------------------------------ inference
     def predict_density(self, X0, faces_t, X1, normals=None):

@@ -103,13 +103,13 @@ constexpr int kSourceUnroll = LDDMM_SOURCE_UNROLL;
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <class... KArgs, class... Args>
-inline void launch_chained(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t stream,
+inline void launch_chained(void (*kernel)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t stream,
                            Args... args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
