@@ -7,10 +7,12 @@
  *    (T+1, N, 3), faces are int64 (F, 3). Outputs are written, never accumulated into, and never alias inputs.
  *  - One kernel width `sigma` per call (Gaussian, or the Laplacian family where an entry point takes `kernel`),
  *    with the reference's default `ms_exponent = -1` weighting; multi-scale kernels are one call per width.
- *  - `origin` (host pointer to 3 doubles, may be NULL = 0): coordinates are centred on it before the FP32
- *    conversion. Results are translation invariant; pass the centroid of the points for best FP32 accuracy.
- *    The Gaussian FP32 kernels of lddmm_apply_k, the second-order forward step, the surface energies and the
- *    varifold / measure gradients centre every target block on its own in FP64 and do not depend on it.
+ *  - `origin` (host pointer to 3 doubles, may be NULL): coordinates are taken relative to it before the conversion to
+ *    the arithmetic of the sum. Results are translation invariant; pass the centroid of the points for best accuracy.
+ *    With NULL it is 0, except that in the self-sums and shooting steps of small sets (at least up to
+ *    LDDMM_OWN_ORIGIN_POINTS of the precision) every block of targets takes an origin of its own, the median of three
+ *    of its points, which is as accurate and needs no centroid. The Gaussian FP32 expanded-distance kernels (ordered
+ *    K a, large K(x,x)a, surface terms) centre every target block on its own in either case.
  *  - `precision`: LDDMM_FP32C = FP32 pair arithmetic with compensated (two-sum) accumulation across tiles and
  *    FP64 epilogues; LDDMM_FP64 = the same kernels in FP64 (the faithful baseline).
  *  - `workspace` / `workspace_bytes`: caller-provided device scratch of at least
@@ -42,6 +44,7 @@ enum {
 };
 
 enum { LDDMM_FP32C = 0, LDDMM_FP64 = 1 };
+#define LDDMM_OWN_ORIGIN_POINTS(precision) ((precision) == LDDMM_FP64 ? 2304 : 8192)
 
 /* Kernel family (`kernel` argument): the Gaussian exp(-r^2 / (2 sigma^2)) (KernelSpec name 'gauss'), or the
  * reference's 'laplacian' kernel of order q = 0..4, P_q(r / sigma) exp(-r / sigma) with the polynomials lapPol /

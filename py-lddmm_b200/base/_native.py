@@ -72,6 +72,7 @@ SIGNATURES = {
     'lddmm_nearest_displacement': [_dp, _i64, _dp, _i64, _dp, _vp],
     'lddmm_lbfgs_direction': [_vp, _vp, _int, _dp, _i64, _dp, _vp],
 }
+OWN_ORIGIN_POINTS = {FP32C: 8192, FP64: 2304}       # LDDMM_OWN_ORIGIN_POINTS of the header
 LBFGS_MAX_PAIRS = 64        # LDDMM_LBFGS_MAX_PAIRS of the header
 _RESTYPES = {'lddmm_version': ctypes.c_char_p, 'lddmm_status_string': ctypes.c_char_p,
              'lddmm_mlp_workspace_bytes': ctypes.c_size_t,
@@ -127,7 +128,8 @@ def check(status, what=''):
 
 
 def stream_ptr():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current CUDA stream's handle (the raw one: torch.cuda.current_stream() builds an object, 15 us a call)."""
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def ptr(t):
@@ -156,9 +158,10 @@ class Workspace:
         self._retired = {}
 
     def get(self, nbytes, device=None):
-        dev = torch.device('cuda', torch.cuda.current_device() if device is None else device)
-        buf = self._bufs.get(dev.index)
+        index = torch.cuda.current_device() if device is None else device
+        buf = self._bufs.get(index)
         if buf is None or buf.numel() < nbytes:
+            dev = torch.device('cuda', index)
             size = max(int(nbytes), 1 << 20)
             size = 1 << (size - 1).bit_length()
             if buf is not None:
@@ -220,6 +223,12 @@ def to_host(t):
     h.copy_(t, non_blocking=True)
     torch.cuda.current_stream().synchronize()
     return h.numpy()
+
+
+def self_origin(t, precision):
+    """Origin argument of a self-sum or shooting step at points t: none for sets whose blocks take their own (reading
+    a centroid back would synchronise a call that lasts tens of microseconds), else the centroid."""
+    return None if t.shape[0] <= OWN_ORIGIN_POINTS[precision] else centroid(t)
 
 
 def centroid(t):

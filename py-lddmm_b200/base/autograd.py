@@ -52,7 +52,7 @@ class GeodesicShooting(torch.autograd.Function):
         T = int(np.round(1.0 / timeStep))
         k = max(1, int(checkpoint_every))
         x0, a0 = x0.detach().contiguous(), a0.detach().contiguous()
-        origin_list = nat.centroid(x0)
+        origin_list = nat.self_origin(x0, K.precision)
         origin = nat.origin_arg(origin_list)
         ws = nat.workspace(x0.shape[0], x0.shape[0], K.precision)
         checkpoints = [(x0, a0)]

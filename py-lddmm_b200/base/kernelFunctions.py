@@ -30,9 +30,6 @@ def _is_np(v):
     return not isinstance(v, torch.Tensor)
 
 
-_NO_ORIGIN = object()   # marks calls whose kernel needs no coordinate origin
-
-
 def _out(t, like_numpy):
     return nat.to_host(t) if like_numpy else t
 
@@ -129,28 +126,28 @@ class Kernel(KernelSpec):
         squeeze = A.dim() == 1
         if squeeze:
             A = A[:, None]
-        # The Gaussian sums run the expanded-distance kernel (FP32) or FP64 arithmetic, both of which take coordinates
-        # relative to each target block's own centre in FP64: no origin is needed, and the host pass that computes one
-        # is skipped. The Laplacian FP32 kernel evaluates differences of origin-centred FP32 coordinates.
-        origin = _NO_ORIGIN if self.code == nat.KERNEL_GAUSS else nat.centroid(x)
         if A.shape[1] != 3:
-            r = self._multi(lambda s: self._k_generic(Y, X, A, s, origin))
+            r = self._multi(lambda s: self._k_generic(Y, X, A, s))
         else:
-            r = self._multi(lambda s: self._apply_k(Y, X, A, s, origin))
+            r = self._multi(lambda s: self._apply_k(Y, X, A, s))
         if squeeze:
             r = r[:, 0]
         return _out(r, like_np)
 
     def _apply_k(self, Y, X, A, sigma, origin=None):
+        # The Gaussian sums run expanded-distance kernels (FP32) or FP64 arithmetic on the coordinates as they are: no
+        # origin. The Laplacian FP32 kernels evaluate differences of origin-centred FP32 coordinates.
+        if origin is None and self.code != nat.KERNEL_GAUSS:
+            origin = nat.self_origin(X, self.precision) if Y is X else nat.centroid(X)
         n, m = Y.shape[0], X.shape[0]
         out = torch.empty((n, 3), dtype=torch.float64, device=Y.device)
         ws, wsb = nat.workspace(n, m, self.precision)
-        o = None if origin is _NO_ORIGIN else nat.origin_arg(origin if origin is not None else nat.centroid(X))
+        o = nat.origin_arg(origin)
         nat.check(nat.lib().lddmm_apply_k(nat.ptr(Y), n, nat.ptr(X), nat.ptr(A), m, float(sigma), self.code, o,
                                           nat.ptr(out), self.precision, ws, wsb, nat.stream_ptr()), 'applyK')
         return out
 
-    def _k_generic(self, Y, X, A, sigma, origin=None):
+    def _k_generic(self, Y, X, A, sigma):
         """K a for momenta of any width d: columns in groups of 3 (zero padded)."""
         d = A.shape[1]
         cols = []
@@ -158,7 +155,7 @@ class Kernel(KernelSpec):
             blk = A[:, c0:c0 + 3]
             if blk.shape[1] < 3:
                 blk = torch.cat([blk, blk.new_zeros(blk.shape[0], 3 - blk.shape[1])], dim=1)
-            cols.append(self._apply_k(Y, X, blk.contiguous(), sigma, origin))
+            cols.append(self._apply_k(Y, X, blk.contiguous(), sigma))
         return torch.cat(cols, dim=1)[:, :d].contiguous()
 
     def _k_mat(self, Y, X, U, sigma):

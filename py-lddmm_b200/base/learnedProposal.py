@@ -282,7 +282,7 @@ def generate_pairs(x0, faces, n_pairs, seed=0, sigma_def=0.5, sigma_smooth=0.4, 
     feats = torch.zeros((n_pairs, Mp, IN_DIM), dtype=torch.bfloat16, device='cuda')
     labels = torch.zeros((n_pairs, Mp, N_OUT), dtype=torch.float32, device='cuda')
     momenta = torch.zeros((n_pairs, n, 3), dtype=torch.float64, device='cuda')
-    origin = nat.centroid(X0)
+    origin = nat.self_origin(X0, Kdef.precision)       # not inside the capture: a centroid is read back
     mass = kernel_mass(Kdef, X0)
     if law not in ('noise', 'shapes'):
         raise ValueError(f'unknown momentum law {law!r}')

@@ -48,7 +48,7 @@ def shoot_first_order(X0, AT, K, regweight=1.0, energy=None, origin=None):
             energy.copy_(e)
         return xt
     ws, wsb = nat.workspace(N, N, K.precision)
-    o = nat.origin_arg(origin if origin is not None else nat.centroid(X0))
+    o = nat.origin_arg(origin if origin is not None else nat.self_origin(X0, K.precision))
     nat.check(nat.lib().lddmm_first_order_shoot(nat.ptr(X0), nat.ptr(AT), N, T, sig, K.code, float(regweight), o,
                                                 nat.ptr(xt), nat.ptr(energy), K.precision, ws, wsb, nat.stream_ptr()),
               'first_order_shoot')
@@ -70,7 +70,7 @@ def first_order_gradient(XT, AT, PX1, K, regweight, euclidean=False, origin=None
             dat[t] = K.applyK(XT[t], g) if euclidean else g
         return pxt, dat
     ws, wsb = nat.workspace(N, N, K.precision)
-    o = nat.origin_arg(origin if origin is not None else nat.centroid(XT[0]))
+    o = nat.origin_arg(origin if origin is not None else nat.self_origin(XT[0], K.precision))
     nat.check(nat.lib().lddmm_first_order_gradient(nat.ptr(XT), nat.ptr(AT), N, T, sig, K.code, float(regweight),
                                                    nat.ptr(PX1.contiguous()), int(bool(euclidean)), o, nat.ptr(pxt),
                                                    nat.ptr(dat), K.precision, ws, wsb, nat.stream_ptr()),
@@ -92,7 +92,7 @@ def shoot_second_order(X0, A0, K, timeStep, origin=None):
             at[k + 1] = at[k] - timeStep * K.applyDiffKT(xt[k], at[k], at[k])
         return xt, at
     ws, wsb = nat.workspace(N, N, K.precision)
-    o = nat.origin_arg(origin if origin is not None else nat.centroid(X0))
+    o = nat.origin_arg(origin if origin is not None else nat.self_origin(X0, K.precision))
     nat.check(nat.lib().lddmm_second_order_shoot(nat.ptr(X0), nat.ptr(A0), N, T, sig, K.code, float(timeStep), o,
                                                  nat.ptr(xt), nat.ptr(at), K.precision, ws, wsb, nat.stream_ptr()),
               'second_order_shoot')
@@ -119,7 +119,7 @@ def second_order_adjoint(XT, AT, PX1, PA1, K, timeStep, origin=None, with_da0=Tr
             da0.copy_(K.applyK(XT[0], AT[0]) - pat[0])
         return pxt, pat, da0
     ws, wsb = nat.workspace(N, N, K.precision)
-    o = nat.origin_arg(origin if origin is not None else nat.centroid(XT[0]))
+    o = nat.origin_arg(origin if origin is not None else nat.self_origin(XT[0], K.precision))
     nat.check(nat.lib().lddmm_second_order_gradient(nat.ptr(XT), nat.ptr(AT), N, T, sig, K.code, float(timeStep),
                                                     nat.ptr(PX1.contiguous()), nat.ptr(PA1.contiguous()), o,
                                                     nat.ptr(pxt), nat.ptr(pat), nat.ptr(da0), K.precision, ws, wsb,

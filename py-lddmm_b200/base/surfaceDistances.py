@@ -8,8 +8,6 @@ varifoldNormDef, varifoldNormGradient, currentNorm*, measureNorm*) wrap it; they
 
 Only the default varifold weight f0(u) = 1 + u^2 (`fun=None`) is implemented.
 """
-import hashlib
-
 import numpy as np
 import torch
 
@@ -17,26 +15,18 @@ from . import _native as nat
 
 KINDS = {'varifold': nat.DATA_VARIFOLD, 'current': nat.DATA_CURRENT, 'measure': nat.DATA_MEASURE}
 
-_TABLES = {}
-
 
 def vertex_face_table(faces_np, nv):
-    """(offsets (nv+1) int32, items (3F) int32) on the device, cached per topology."""
+    """(offsets (nv+1) int32, items (3F) int32) on the device, built on the host in one pass over the faces."""
     faces_np = np.ascontiguousarray(faces_np, dtype=np.int64)
-    key = (hashlib.sha1(faces_np.tobytes()).hexdigest(), int(nv), torch.cuda.current_device())
-    hit = _TABLES.get(key)
-    if hit is not None:
-        return hit
-    off = np.zeros(nv + 1, dtype=np.int32)
-    items = np.zeros(max(3 * faces_np.shape[0], 1), dtype=np.int32)
-    rc = nat.lib().lddmm_vertex_face_table(faces_np.ctypes.data, faces_np.shape[0], int(nv), off.ctypes.data,
-                                           items.ctypes.data)
+    n = max(3 * faces_np.shape[0], 1)
+    table = torch.empty(nv + 1 + n, dtype=torch.int32, pin_memory=True)
+    off, items = table[:nv + 1], table[nv + 1:]
+    rc = nat.lib().lddmm_vertex_face_table(faces_np.ctypes.data, faces_np.shape[0], int(nv), off.data_ptr(),
+                                           items.data_ptr())
     nat.check(rc, 'vertex_face_table')
-    val = (torch.from_numpy(off).cuda(), torch.from_numpy(items).cuda())
-    if len(_TABLES) > 32:
-        _TABLES.clear()
-    _TABLES[key] = val
-    return val
+    table = table.to('cuda')
+    return table[:nv + 1], table[nv + 1:]
 
 
 def _kernel_widths(KparDist):
@@ -52,6 +42,7 @@ def _kernel_widths(KparDist):
 
 class SurfaceDataTerm:
     """Device-resident data term |S_def|^2 - 2<S_def, S_1> (+ |S_1|^2) for a fixed topology and target."""
+    _with_gradient = True       # build the vertex -> face table
 
     def __init__(self, faces, target_vertices, target_faces, KparDist, kind='varifold', weights=None,
                  target_weights=None, precision=None, nv=None):
@@ -72,8 +63,11 @@ class SurfaceDataTerm:
         self.nf1 = self.faces1.shape[0]
         self.w = None if weights is None else nat.as_device(weights)
         self.w1 = None if target_weights is None else nat.as_device(target_weights)
-        self.vf_off, self.vf_items = vertex_face_table(self.faces_np, self.nv)
-        self.origin = nat.centroid(self.x1)
+        if self._with_gradient:
+            self.vf_off, self.vf_items = vertex_face_table(self.faces_np, self.nv)
+        elif self.faces_np.size and (self.faces_np.min() < 0 or self.faces_np.max() >= self.nv):
+            raise nat.LddmmError('faces index outside the vertices')
+        self.origin = nat.centroid(target_vertices)
         self._norm0 = None
 
     def _ws(self):
@@ -84,7 +78,8 @@ class SurfaceDataTerm:
         X = None if xdef is None else nat.as_device(xdef)
         nv, nf = (0, 0) if X is None else (X.shape[0], self.nf)
         out = torch.zeros(2, dtype=torch.float64, device=self.x1.device)
-        tmp = torch.empty(2, dtype=torch.float64, device=self.x1.device)
+        one = len(self.widths) == 1 and self.widths[0][1] == 1.0      # one width: no weighting pass
+        tmp = out if one else torch.zeros_like(out)
         ws, wsb = self._ws()
         o = nat.origin_arg(self.origin)
         for s, wt in self.widths:
@@ -93,9 +88,8 @@ class SurfaceDataTerm:
                                                      nat.ptr(self.faces1), self.nf1, nat.ptr(self.w1), float(s), o,
                                                      int(bool(with_norm0)), nat.ptr(tmp), self.precision, ws, wsb,
                                                      nat.stream_ptr()), 'surface_energy')
-            if not with_norm0:
-                tmp[1] = 0.0
-            out += wt * tmp
+            if not one:
+                out += wt * tmp
         return out
 
     def norm0(self):
@@ -107,10 +101,12 @@ class SurfaceDataTerm:
     def gradient(self, xdef, with_weights=False):
         """Vertex gradient of xNormDef, (nv,3) FP64 device tensor (and (nv,) weight gradient if requested)."""
         X = nat.as_device(xdef)
-        px = torch.zeros((X.shape[0], 3), dtype=torch.float64, device=X.device)
-        pxw = torch.zeros(X.shape[0], dtype=torch.float64, device=X.device) if with_weights else None
-        tmp = torch.empty_like(px)
-        tmpw = torch.empty_like(pxw) if with_weights else None
+        one = len(self.widths) == 1 and self.widths[0][1] == 1.0      # one width: no weighting pass
+        make = torch.empty if one else torch.zeros
+        px = make((X.shape[0], 3), dtype=torch.float64, device=X.device)
+        pxw = make(X.shape[0], dtype=torch.float64, device=X.device) if with_weights else None
+        tmp = px if one else torch.empty_like(px)
+        tmpw = pxw if one or not with_weights else torch.empty_like(pxw)
         ws, wsb = self._ws()
         o = nat.origin_arg(self.origin)
         for s, wt in self.widths:
@@ -120,9 +116,10 @@ class SurfaceDataTerm:
                                                        nat.ptr(self.faces1), self.nf1, nat.ptr(self.w1), float(s), o,
                                                        nat.ptr(tmp), nat.ptr(tmpw), self.precision, ws, wsb,
                                                        nat.stream_ptr()), 'surface_gradient')
-            px += wt * tmp
-            if with_weights:
-                pxw += wt * tmpw
+            if not one:
+                px += wt * tmp
+                if with_weights:
+                    pxw += wt * tmpw
         return (px, pxw) if with_weights else px
 
 
@@ -134,14 +131,19 @@ def _weights(fv):
     return None if np.all(w == 1.0) else w
 
 
-def _term(fvDef, fv1, KparDist, kind):
-    return SurfaceDataTerm(fvDef.faces, fv1.vertices, fv1.faces, KparDist, kind=kind, weights=_weights(fvDef),
-                           target_weights=_weights(fv1), nv=fvDef.vertices.shape[0])
+class _Energy(SurfaceDataTerm):
+    """A data term that is only evaluated, never differentiated."""
+    _with_gradient = False
+
+
+def _term(fvDef, fv1, KparDist, kind, cls=SurfaceDataTerm):
+    return cls(fvDef.faces, fv1.vertices, fv1.faces, KparDist, kind=kind, weights=_weights(fvDef),
+               target_weights=_weights(fv1), nv=fvDef.vertices.shape[0])
 
 
 def _self_term(fv1, KparDist, kind):
-    return SurfaceDataTerm(fv1.faces, fv1.vertices, fv1.faces, KparDist, kind=kind, weights=_weights(fv1),
-                           target_weights=_weights(fv1), nv=fv1.vertices.shape[0])
+    return _Energy(fv1.faces, fv1.vertices, fv1.faces, KparDist, kind=kind, weights=_weights(fv1),
+                   target_weights=_weights(fv1), nv=fv1.vertices.shape[0])
 
 
 def _check_fun(fun):
@@ -157,7 +159,7 @@ def varifoldNorm0(fv1, KparDist, fun=None, cpu=False, dtype='float64'):
 
 def varifoldNormDef(fvDef, fv1, KparDist, fun=None, cpu=False, dtype='float64'):
     _check_fun(fun)
-    return float(_term(fvDef, fv1, KparDist, 'varifold').energy(fvDef.vertices)[0])
+    return float(_term(fvDef, fv1, KparDist, 'varifold', _Energy).energy(fvDef.vertices)[0])
 
 
 def varifoldNorm(fvDef, fv1, KparDist, fun=None):
@@ -178,7 +180,7 @@ def currentNorm0(fv1, KparDist, weight=1.):
 
 
 def currentNormDef(fvDef, fv1, KparDist, weight=1.):
-    return float(_term(fvDef, fv1, KparDist, 'current').energy(fvDef.vertices)[0])
+    return float(_term(fvDef, fv1, KparDist, 'current', _Energy).energy(fvDef.vertices)[0])
 
 
 def currentNorm(fvDef, fv1, KparDist, weight=1.):
@@ -197,7 +199,7 @@ def measureNorm0(fv1, KparDist):
 
 
 def measureNormDef(fvDef, fv1, KparDist):
-    return float(_term(fvDef, fv1, KparDist, 'measure').energy(fvDef.vertices)[0])
+    return float(_term(fvDef, fv1, KparDist, 'measure', _Energy).energy(fvDef.vertices)[0])
 
 
 def measureNorm(fvDef, fv1, KparDist):

@@ -101,7 +101,7 @@ class _DeviceMatching:
                                     else w1, nv=self.fv0.vertices.shape[0])
         self.x0 = nat.as_device(self.fv0.vertices)
         self.npt = self.x0.shape[0]
-        self.origin = nat.centroid(self.x0)
+        self.origin = nat.centroid(self.fv0.vertices)
         self.Tsize = int(round(1.0 / o['timeStep']))
         self.sigma2 = o['sigmaError'] ** 2
         self.euclideanGradient = True
@@ -264,7 +264,7 @@ class _DeviceMatching:
 
     def dotProduct_euclidean(self, g1, g2):
         vals = [self.dotProduct_device(g1, gr) for gr in g2]
-        return torch.stack(vals).tolist()
+        return [vals[0].item()] if len(vals) == 1 else torch.stack(vals).tolist()
 
     dotProduct = dotProduct_euclidean
 

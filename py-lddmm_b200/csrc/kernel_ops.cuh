@@ -35,6 +35,7 @@ struct OpK {
     const double* dotw = nullptr;
     double* dots = nullptr;
   };
+  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.y; }
   template <typename V> struct Tgt { V y0, y1, y2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {
@@ -160,6 +161,7 @@ struct OpDiffKT {
     Frame f;
     double w;  // regweight (lddmm)
   };
+  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.y; }
   template <typename V> struct Tgt { V y0, y1, y2, p0, p1, p2, a0, a1, a2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {
@@ -216,6 +218,7 @@ struct OpDDiffK {
     double* out;
     Frame f;
   };
+  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.x; }
   template <typename V> struct Tgt { V y0, y1, y2, n0, n1, n2, p0, p1, p2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {
@@ -267,6 +270,7 @@ struct OpDiffK1and2 {
     double* out;
     Frame f;
   };
+  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.x; }
   template <typename V> struct Tgt { V y0, y1, y2, b0, b1, b2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {
@@ -310,6 +314,7 @@ struct OpDiv {
     double* out;
     Frame f;
   };
+  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.y; }
   template <typename V> struct Tgt { V y0, y1, y2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {
@@ -341,6 +346,7 @@ struct OpKTensor {
     double* out;
     Frame f;
   };
+  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.y; }
   template <typename V> struct Tgt { V y0, y1, y2, b0, b1, b2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {

@@ -111,4 +111,7 @@ constexpr int kTpbSym64Adj = 128, kRtSym64Adj = 2;
 // 4,000: 62.8 | 55.3 | 55.6).
 constexpr int64_t kSplit1N64 = 1280, kSplit2N64 = 2304, kSplit2N64Lap = 4096;
 
+static_assert(kSplit4NLast >= 8192 && kSplit8N >= 8192 && kSplit2N64 >= 2304,
+              "every self-sum up to LDDMM_OWN_ORIGIN_POINTS runs a split kernel");
+
 }  // namespace lddmm

@@ -302,6 +302,7 @@ enum KernelFamily : int { kGauss = 0, kLaplacian0 = 16, kLaplacianMax = 20 };
 // Geometry shared by every op: centred, pre-scaled coordinates, and the radial profile of the kernel.
 struct Frame {
   double o0, o1, o2;  // origin subtracted before scaling
+  int own;            // no origin given: the split kernels' blocks take one of their own (segment_origin)
   double s;           // coordinate scale (Gaussian: kScale / sigma; Laplacian: log2(e) / sigma)
   double kappa;       // 1 / (s sigma^2): turns a scaled difference into (y - x) / sigma^2
   double inv_s2;      // 1 / sigma^2
@@ -641,6 +642,39 @@ struct NAXOf<Op, std::void_t<decltype(Op::NAX)>> : std::integral_constant<int, O
 template <class Op, typename V, int RT, class Fam>
 constexpr int kRunRT = (kUseExpanded<Op, V, Fam> && RtXOf<Op>::value > 0) ? RtXOf<Op>::value : RT;
 
+// Origin of a target block's coordinates: the caller's, or, coordinate by coordinate, the median of the block's first,
+// middle and last point, so that a caller whose points live on the device need not read a centroid back (one
+// synchronisation per call before). Coordinates relative to their own block lose no more than about a common centroid
+// would, the median keeps one far or non-finite point of the three from moving it, and a median that is not finite
+// leaves the block in the caller's frame. The split kernels use it, whose calls are short against a synchronisation;
+// in the others the six more registers cost 1-4% (forward step at 40,962 points 783 -> 792 us, FP64 first-order
+// adjoint step 2458 -> 2569).
+__device__ __forceinline__ double median3(double a, double b, double c) {
+  return fmax(fmin(a, b), fmin(fmax(a, b), c));
+}
+__device__ __forceinline__ void segment_origin(const Frame& f, const double* __restrict__ points, int first, int last,
+                                               double (&o)[3]) {
+  o[0] = f.o0;
+  o[1] = f.o1;
+  o[2] = f.o2;
+  if (!f.own) return;
+  const int mid = first + (last - first) / 2;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double m = median3(points[3 * (size_t)first + c], points[3 * (size_t)mid + c], points[3 * (size_t)last + c]);
+    if (isfinite(m)) o[c] = m;
+  }
+}
+// The op's parameters with the segment's origin (kept in shared memory: every thread writes the same values).
+template <class Params>
+__device__ __forceinline__ Params with_origin(const Params& P, const double* org) {
+  Params q = P;
+  q.f.o0 = org[0];
+  q.f.o1 = org[1];
+  q.f.o2 = org[2];
+  return q;
+}
+
 // SPLIT (problems too small to fill the GPU): the warps of a CTA share its 32 RT targets and take a quarter of every
 // source tile each, instead of TPB RT targets and whole tiles; their sums meet in shared memory when a segment ends.
 template <class Op, typename V, int TPB, int RT, class Fam, bool SPLIT>
@@ -665,6 +699,9 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
   constexpr float kZeroR2 = Fam::template kCullR2<V>;
   using Un = Units<Op, TPB, TW * RT>;
   const int gx = (n + TW * RT - 1) / (TW * RT);
+  // (the culled ops' boxes are in the caller's frame, and so are their coordinates)
+  constexpr bool kOwn = SPLIT && !Culled<Op>::value;
+  __shared__ double org[3];
   __shared__ float tbox[6];  // the segment's target box, in shared memory (re-read per tile, not held in registers)
   VT<V>::setup();
   chain_wait();
@@ -679,6 +716,13 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
     const int j1 = first + (int)((u_end - off) < TT - first ? (u_end - off) : TT - first);
     const int slot = (int)blockIdx.x - sk_cta_of(off, W, C);
 
+    if constexpr (kOwn) {
+      const int b0 = tb * (TW * RT), b1 = b0 + TW * RT < n ? b0 + TW * RT : n;
+      double o[3];
+      segment_origin(P.f, Op::target_points(P), b0, b1 - 1, o);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) org[c] = o[c];
+    }
     typename Op::template Tgt<V> tgt[G];
     Comp<V> cmp[G][Op::NA];   // used when !kSm
     // target of (group g, lane k): base + (g * L + k) * TW
@@ -688,7 +732,10 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
       int i0 = base + (g * L) * TW, i1 = base + (g * L + L - 1) * TW;
       i0 = i0 < n ? i0 : n - 1;
       i1 = i1 < n ? i1 : n - 1;
-      Op::template load_target<V>(P, i0, i1, tgt[g]);
+      if constexpr (kOwn)
+        Op::template load_target<V>(with_origin(P, org), i0, i1, tgt[g]);
+      else
+        Op::template load_target<V>(P, i0, i1, tgt[g]);
 #pragma unroll
       for (int c = 0; c < Op::NA; ++c) {
         cmp[g][c].zero();
@@ -713,7 +760,12 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
         double f[2 * NU];
 #pragma unroll
         for (int q = 0; q < 2 * NU; ++q) f[q] = 0.0;
-        if (live) Op::source_fields(P, l, f);
+        if (live) {
+          if constexpr (kOwn)
+            Op::source_fields(with_origin(P, org), l, f);
+          else
+            Op::source_fields(P, l, f);
+        }
         if constexpr (Un::kTri) Op::weigh(f + 3, weight);
 #pragma unroll
         for (int q = 0; q < NU; ++q) {
@@ -1261,6 +1313,7 @@ inline bool bad_kernel(int kernel) { return !(kernel == kGauss || (kernel >= kLa
 inline Frame make_frame(const double* origin, double sigma, int kernel) {
   Frame f = {};
   f.family = kernel;
+  f.own = origin == nullptr;
   f.o0 = origin ? origin[0] : 0.0;
   f.o1 = origin ? origin[1] : 0.0;
   f.o2 = origin ? origin[2] : 0.0;

@@ -236,6 +236,7 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
   // shared memory, so that 8 targets per thread may take more than the 48 KiB of static shared memory
   extern __shared__ __align__(16) unsigned char sym_dyn_smem[];
   V (*cs)[TPB] = reinterpret_cast<V (*)[TPB]>(sym_dyn_smem);
+  __shared__ double org[3];
   const Frame& f = P.f;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   VT<V>::setup();  // the staging barrier of the first tile follows
@@ -252,11 +253,21 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
     const int slot = (int)blockIdx.x - sk_cta_of(off, U, C);
     const int base = i * B + (SPLIT ? lane : (int)threadIdx.x);
 
+    if constexpr (SPLIT) {
+      double o[3];
+      segment_origin(f, P.x, i * B, i * B + B < n ? i * B + B - 1 : n - 1, o);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) org[c] = o[c];
+    }
     typename Op::template SymTgt<V> tgt[G];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       const int i0 = base + (g * L) * TW, i1 = base + (g * L + L - 1) * TW;
-      Op::template load_target_sym<V>(P, i0 < n ? i0 : n - 1, i1 < n ? i1 : n - 1, i0 < n, i1 < n, tgt[g]);
+      if constexpr (SPLIT)
+        Op::template load_target_sym<V>(with_origin(P, org), i0 < n ? i0 : n - 1, i1 < n ? i1 : n - 1, i0 < n, i1 < n,
+                                        tgt[g]);
+      else
+        Op::template load_target_sym<V>(P, i0 < n ? i0 : n - 1, i1 < n ? i1 : n - 1, i0 < n, i1 < n, tgt[g]);
       Comp<V> z;
       z.zero();
 #pragma unroll
@@ -271,7 +282,12 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
         double fl[St::kFields];
 #pragma unroll
         for (int q = 0; q < St::kFields; ++q) fl[q] = 0.0;
-        if (l < n) Op::source_fields_sym(P, l, fl);
+        if (l < n) {
+          if constexpr (SPLIT)
+            Op::source_fields_sym(with_origin(P, org), l, fl);
+          else
+            Op::source_fields_sym(P, l, fl);
+        }
         St::store(sm, threadIdx.x, fl);
         if constexpr (!SPLIT) {
 #pragma unroll

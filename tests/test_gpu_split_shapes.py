@@ -94,3 +94,31 @@ def test_energies_once_per_unordered_self_pair(nf, nf1):
             Kd.pk_dtype = dtype
             e = SurfaceDataTerm(f0, x1, f1, Kd, kind=kind, nv=x.shape[0]).energy(x, with_norm0=True).tolist()
             assert abs(e[0] - ref) <= tol * size and abs(e[1] - ref0) <= tol * size, (kind, dtype)
+
+
+@pytest.mark.parametrize('name', ['gauss', 'laplacian'])
+@pytest.mark.parametrize('n', [1, 700, 3000, 9000, 17000])
+def test_sums_far_from_the_coordinate_origin(n, name):
+    """Self-sums and a shooting step without a caller's origin on points 1,000 widths from 0, one of them much further:
+    the same FP32 accuracy as at 0 (2e-5 relative, Laplacian 3e-5), against the FP64 sums of the shifted points."""
+    import torch
+    from base import pointEvolution as evol
+    from base.kernelFunctions import Kernel
+    rng = np.random.default_rng(n)
+    X = torch.from_numpy(rng.normal(size=(n, 3))).cuda()
+    A = torch.from_numpy(rng.normal(size=(n, 3))).cuda()
+    if 1 < n <= 16384:             # larger sets centre a block on its box, which one far point stretches
+        X[0, 1] = 2.0e5            # the first point of the first block
+    off = torch.tensor([800.0, -500.0, 300.0], dtype=torch.float64, device='cuda')
+    K, K64 = Kernel(name=name, sigma=0.8, order=3), Kernel(name=name, sigma=0.8, order=3)
+    K.pk_dtype, K64.pk_dtype = 'float32', 'float64'
+    tol = 2e-5 if name == 'gauss' else 3e-5
+    ka, za = K64.applyK(X, A), -K64.applyDiffKT(X, A, A)
+
+    def close(a, b):
+        return float((a - b).norm()) <= tol * float(b.norm()) + 1e-6 * n ** 0.5
+
+    assert close(K.applyK(X + off, A), ka)
+    xt, at = evol.shoot_second_order(X + off, A, K, 1.0)
+    assert close(xt[1] - xt[0], ka)
+    assert close(at[1] - A, za)
