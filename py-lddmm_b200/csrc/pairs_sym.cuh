@@ -561,7 +561,7 @@ inline size_t sym_scratch_fam(int64_t n) {
 // Scratch of one launch.
 template <class Op, typename V>
 inline size_t sym_scratch(int64_t n, int family) {
-  return family == kGauss ? sym_scratch_fam<Op, V, Gauss>(n) : sym_scratch_fam<Op, V, Laplacian>(n);
+  return by_family(family, [&](auto fam) { return sym_scratch_fam<Op, V, decltype(fam)>(n); });
 }
 // Scratch for every point count up to n: the largest of each shape's range.
 template <class Op, typename V>
@@ -571,7 +571,7 @@ inline size_t sym_scratch_upto(int64_t n) {
   for (const int64_t k : {R::kSplit2, R::kSplit4, R::kSplit8, R::kSplit4Lap, kSplit1N64, kSplit2N64, kSplit2N64Lap,
                           sym_max_n<Op, V>(), n}) {
     if (k > n || !sym_takes<Op, V>(k)) continue;
-    for (const int family : {(int)kGauss, (int)kLaplacian0}) {
+    for (const int family : {(int)kGauss, (int)kLaplacian0, (int)kLaplacianMax}) {
       const size_t v = sym_scratch<Op, V>(k, family);
       b = v > b ? v : b;
     }
@@ -588,8 +588,7 @@ inline int run_sym_fam(const typename Op::Params& P, int64_t n, void* ws, size_t
 // Launch of a symmetric op, for the kernel family of its frame.
 template <class Op, typename V>
 inline int run_sym(const typename Op::Params& P, int64_t n, void* ws, size_t wsb, cudaStream_t st) {
-  if (P.f.family == kGauss) return run_sym_fam<Op, V, Gauss>(P, n, ws, wsb, st);
-  return run_sym_fam<Op, V, Laplacian>(P, n, ws, wsb, st);
+  return by_family(P.f.family, [&](auto fam) { return run_sym_fam<Op, V, decltype(fam)>(P, n, ws, wsb, st); });
 }
 
 // ---------------------------------------------------------------------------------------------------------

@@ -478,7 +478,8 @@ size_t shooting_ws_bytes(int64_t n, int precision) {
     sym(F2{});
     upd(pairs_ws_bytes_any<OpSOFwd, F2, kTpbLight, kRtLight>(n, n));
     upd(pairs_ws_bytes<OpSOBwd, F2, kTpbHeavy, kRtAdjoint, Gauss>(n, n));
-    upd(pairs_ws_bytes<OpSOBwd, F2, kTpbHeavy, kRtHeavy, Laplacian>(n, n));
+    upd(pairs_ws_bytes<OpSOBwd, F2, kTpbHeavy, kRtHeavy, Laplacian3>(n, n));
+    upd(pairs_ws_bytes<OpSOBwd, F2, kTpbHeavy, kRtHeavy, Laplacian4>(n, n));
     upd(pairs_ws_bytes_any<OpFOBwd, F2, kTpbLight, kRtLight>(n, n));
     upd(pairs_ws_bytes_any<OpK, F2, kTpbLight, kRtLight>(n, n));
   } else {
@@ -558,8 +559,11 @@ int so_adjoint_step(const double* x, const double* a, const double* px, const do
   OpSOBwd::Params P{x, a, px, pa, px_prev, pa_prev, f, dt, (int)row0};
   const int64_t rows = nrows < 0 ? n : nrows;
   if (row0 == 0 && rows == n && sym_takes<OpSOBwdSym, V>(n)) return run_sym<OpSOBwdSym, V>(P, n, ws, wsb, st);
-  if (f.family == kGauss) return run_pairs<OpSOBwd, V, StepShape<V>::kTpbH, StepShape<V>::kRtH, Gauss>(P, rows, n, ws, wsb, st);
-  return run_pairs<OpSOBwd, V, StepShape<V>::kTpbH, StepShape<V>::kRtHL, Laplacian>(P, rows, n, ws, wsb, st);
+  return by_family(f.family, [&](auto fam) {
+    using Fam = decltype(fam);
+    constexpr int RT = std::is_same<Fam, Gauss>::value ? StepShape<V>::kRtH : StepShape<V>::kRtHL;
+    return run_pairs<OpSOBwd, V, StepShape<V>::kTpbH, RT, Fam>(P, rows, n, ws, wsb, st);
+  });
 }
 
 template <typename V>
