@@ -154,7 +154,12 @@ __device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c) {
   return r;
 }
 __device__ __forceinline__ F2& operator+=(F2& a, F2 b) { return a = a + b; }
-__device__ __forceinline__ F2 operator-(F2 a) { return f2(0.f, 0.f) - a; }
+// Lane by lane: a sign in front of an operand, not a packed operation.
+__device__ __forceinline__ F2 operator-(F2 a) {
+  float x, y;
+  split(a, x, y);
+  return f2(-x, -y);
+}
 
 __device__ __forceinline__ float ex2neg(float x) {
   float y;

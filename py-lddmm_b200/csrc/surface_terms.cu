@@ -201,8 +201,11 @@ struct FaceGrad {
   double z[3], dz[3], zw, pad;
 };
 
-// Varifold gradient pair: z += e aw_l [2g n_l + (1-g^2) n_k] (as Z = sum 2g e aw n_l and W = sum e aw (1-g^2)),
-// D = sum e aw (1+g^2) d, S = sum e aw (1+g^2): 22 FP32 + 1 SFU per pair.
+// Varifold gradient pair: z += e aw_l [2g n_l + (1-g^2) n_k], dz from f d and zw from f with f = e aw (1+g^2). The sums
+// kept are Z = sum e aw g n_l (doubled in the epilogue), W = sum e aw (1-g^2), D = sum f d and S = sum f. Both f and the
+// term of W are one fused multiply-add of e aw g (the sign costs no operation), the doubling is the epilogue's: 20 FP32
+// + 1 SFU per pair (expanded form 18; with separate products 20, 81,920 faces 9.94 -> 9.49 ms, errors equal). W taken
+// as 2 sum e aw - S is one operation less (9.19 ms) and loses the digits of 1 - g^2: twice the error, not used.
 template <int KIND>
 struct OpSurfGrad {
   static constexpr int NS = 7, NA = (KIND == LDDMM_DATA_VARIFOLD) ? 8 : (KIND == LDDMM_DATA_CURRENT ? 6 : 4);
@@ -231,13 +234,11 @@ struct OpSurfGrad {
       const V g = dot3(t.n0, t.n1, t.n2, s[4], s[5], s[6]);
       const V ea = e * s[3];
       const V eag = ea * g;
-      const V eag2 = eag * g;
-      const V t2 = eag + eag;
-      acc[0] = fma(t2, s[4], acc[0]);
-      acc[1] = fma(t2, s[5], acc[1]);
-      acc[2] = fma(t2, s[6], acc[2]);
-      acc[3] = acc[3] + (ea - eag2);
-      const V eaf = ea + eag2;
+      acc[0] = fma(eag, s[4], acc[0]);
+      acc[1] = fma(eag, s[5], acc[1]);
+      acc[2] = fma(eag, s[6], acc[2]);
+      acc[3] = acc[3] + fma(-eag, g, ea);
+      const V eaf = fma(eag, g, ea);
       acc[4] = fma(eaf, d0, acc[4]);
       acc[5] = fma(eaf, d1, acc[5]);
       acc[6] = fma(eaf, d2, acc[6]);
@@ -261,7 +262,7 @@ struct OpSurfGrad {
   // Expanded-distance form (pairs_kernel_x; varifold and measure): the centre term sum f (y - x) is written
   // y S - sum f x with S = sum f, a sum these kinds accumulate anyway (varifold: f = e aw (1 + g^2), S in slot 7;
   // measure: f = e aw, slot 0), and the staged X = -2 x gives sum f x = -E/2; no difference y - x is formed
-  // (varifold: 19 FP32 + 1 SFU per pair) and no accumulator or staged field is added. Blocks too wide for the form
+  // (varifold: 18 FP32 + 1 SFU per pair) and no accumulator or staged field is added. Blocks too wide for the form
   // sum f (y - x) directly. Radius^2 bound 32, as for the second-order forward step.
   static constexpr bool kExpand = LDDMM_SURFGRAD_EXPAND != 0 && KIND != LDDMM_DATA_CURRENT;
   static constexpr int NP = (KIND == LDDMM_DATA_VARIFOLD) ? 4 : 1, kRtX = 4;
@@ -295,13 +296,11 @@ struct OpSurfGrad {
     if constexpr (KIND == LDDMM_DATA_VARIFOLD) {
       const V g = dot3(t.n0, t.n1, t.n2, s[5], s[6], s[7]);
       const V eag = ea * g;
-      const V eag2 = eag * g;
-      const V t2 = eag + eag;
-      acc[0] = fma(t2, s[5], acc[0]);
-      acc[1] = fma(t2, s[6], acc[1]);
-      acc[2] = fma(t2, s[7], acc[2]);
-      acc[3] = acc[3] + (ea - eag2);
-      const V eaf = ea + eag2;
+      acc[0] = fma(eag, s[5], acc[0]);
+      acc[1] = fma(eag, s[6], acc[1]);
+      acc[2] = fma(eag, s[7], acc[2]);
+      acc[3] = acc[3] + fma(-eag, g, ea);
+      const V eaf = fma(eag, g, ea);
       if constexpr (X) {
         acc[4] = fma(eaf, s[0], acc[4]);
         acc[5] = fma(eaf, s[1], acc[5]);
@@ -337,7 +336,7 @@ struct OpSurfGrad {
     const double k23 = -(2.0 / 3.0) * P.f.kappa;
     if (KIND == LDDMM_DATA_VARIFOLD) {
       for (int c = 0; c < 3; ++c) {
-        g.z[c] = r.fw * (acc[c] + acc[3] * r.n[c]);
+        g.z[c] = r.fw * (2.0 * acc[c] + acc[3] * r.n[c]);
         g.dz[c] = k23 * r.aw * acc[4 + c];
       }
       g.zw = (2.0 / 3.0) * r.fw * r.a * acc[7];
