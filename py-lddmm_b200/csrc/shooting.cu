@@ -264,81 +264,82 @@ struct OpSOFwdSym {
   }
 };
 
-// The second-order adjoint step evaluated once per unordered pair (pairs_kernel_sym; Gaussian, FP32, whole steps).
-// Every per-pair quantity of OpSOBwd is symmetric in (k, l) or changes sign: e, c1 = px'_k.a_l + a_k.px'_l,
-// c2 = b_k.a_l (b = -kappa^2 a) and dq = d.(pa_k - pa_l) are symmetric, d and w = pa_k - pa_l change sign. With the
-// four sums merged pairwise (as the epilogue of OpSOBwd combines them),
-//   row px-sum of k:  v = eg d + cd ec2 w          (eg = e (c1 + c2 dq), ec2 = e c2, cd = -1/(kappa^2 sigma^2))
-//   row pa-sum of k:  e px'_l - kappa^2 edq a_l    (edq = e dq)
-// the mirrored contributions to l are -v and e px'_k + edq b_k. 51 FP32 lane-ops per unordered pair (25.5 per
-// ordered pair, against 37 for OpSOBwd), one ex2.
+// The second-order adjoint step evaluated once per unordered pair (pairs_kernel_sym; whole steps). Every per-pair
+// quantity of OpSOBwd is symmetric in (k, l) or changes sign. With A = kappa a, c = A_k.A_l, c1 = px_k.A_l + A_k.px_l,
+// w = beta (pa_l - pa_k), beta = 1/(kappa sigma)^2, and dq = d.(pa_k - pa_l) = -(d.w)/beta,
+//   row px-sum of k:  v = (e c dq + e c1) d + e c w       (zpx = -v)
+//   row pa-sum of k:  e px_l + e dq A_l                   (zpa)
+// and the mirrored contributions to l are -v and e px_k + e dq A_k: no scaled copy of a and no constant in the pair.
+// 50 FP32 lane-ops per unordered pair (25 per ordered pair, against 37 for OpSOBwd), one ex2, and 13 target values
+// where -kappa^2 a and two constants made 17: 40,962 points 1637 -> 1611 us (FP64 4098 -> 4010, Laplacian of order 3
+// 2156 -> 2070, where the profile is short of registers).
 struct OpSOBwdSym {
   using Params = OpSOBwd::Params;
   static constexpr int NSS = 12, NR = 6, NC = 6;
   static constexpr int kSymMinCtas = LDDMM_SOBWD_SYM_MIN_CTAS;
   using Shape = SymRule<kSplit2NAdj, kSplit4NLast, 0, kSplit4NLast, kRtAdjoint, kRtAdjointSymL, kTpbSym64Adj,
                         kRtSym64Adj>;
-  template <typename V> struct SymTgt { V y0, y1, y2, a0, a1, a2, b0, b1, b2, p0, p1, p2, q0, q1, q2, cd, k2; };
+  template <typename V> struct SymTgt { V y0, y1, y2, a0, a1, a2, p0, p1, p2, q0, q1, q2, ib; };
+  static __device__ __forceinline__ double beta(const Params& P) { return P.f.inv_s2 / (P.f.kappa * P.f.kappa); }
   template <typename V>
   static __device__ __forceinline__ void load_target_sym(const Params& P, int i0, int i1, bool v0, bool v1,
                                                          SymTgt<V>& t) {
-    const double k = P.f.kappa;
+    const double k = P.f.kappa, b = beta(P);
     auto fld = [&](const double* a, int c, double sc) {
       return VT<V>::pack(v0 ? sc * a[3 * i0 + c] : 0.0, v1 ? sc * a[3 * i1 + c] : 0.0);
     };
     t.y0 = tgt_coord<V>(P.x, i0, i1, 0, P.f.o0, P.f.s);
     t.y1 = tgt_coord<V>(P.x, i0, i1, 1, P.f.o1, P.f.s);
     t.y2 = tgt_coord<V>(P.x, i0, i1, 2, P.f.o2, P.f.s);
-    t.a0 = fld(P.a, 0, 1.0); t.a1 = fld(P.a, 1, 1.0); t.a2 = fld(P.a, 2, 1.0);
-    t.b0 = fld(P.a, 0, -k * k); t.b1 = fld(P.a, 1, -k * k); t.b2 = fld(P.a, 2, -k * k);
-    t.p0 = fld(P.px, 0, -k); t.p1 = fld(P.px, 1, -k); t.p2 = fld(P.px, 2, -k);
-    t.q0 = fld(P.pa, 0, 1.0); t.q1 = fld(P.pa, 1, 1.0); t.q2 = fld(P.pa, 2, 1.0);
-    t.cd = VT<V>::dup(-P.f.inv_s2 / (k * k));
-    t.k2 = VT<V>::dup(-k * k);
+    t.a0 = fld(P.a, 0, k); t.a1 = fld(P.a, 1, k); t.a2 = fld(P.a, 2, k);
+    t.p0 = fld(P.px, 0, 1.0); t.p1 = fld(P.px, 1, 1.0); t.p2 = fld(P.px, 2, 1.0);
+    t.q0 = fld(P.pa, 0, b); t.q1 = fld(P.pa, 1, b); t.q2 = fld(P.pa, 2, b);
+    t.ib = VT<V>::dup(-1.0 / b);
   }
-  // fields: x' (0-2), a (3-5), pa (6-8), px' = -kappa px (9-11)
+  // fields: x' (0-2), A = kappa a (3-5), beta pa (6-8), px (9-11)
   static __device__ __forceinline__ void source_fields_sym(const Params& P, int l, double* f) {
-    OpSOBwd::source_fields(P, l, f);
+    const double k = P.f.kappa, b = beta(P);
+    src_point(P.x, l, P.f, f);
+    for (int c = 0; c < 3; ++c) {
+      f[3 + c] = k * P.a[3 * l + c];
+      f[6 + c] = b * P.pa[3 * l + c];
+      f[9 + c] = P.px[3 * l + c];
+    }
   }
-  // Fam: the radial factors k0 (the px'-sum), k1 (first-derivative terms) and k2 (the second-derivative term
-  // c2 dq d); all three are e for the Gaussian, where k1 c2 and k2 c2 are one product
+  // Fam: the radial factors k0 (the px-sum), k1 (first-derivative terms) and k2 (the second-derivative term c dq d);
+  // all three are e for the Gaussian, where k1 c and k2 c are one product
   template <bool COL, class Fam, typename V>
   static __device__ __forceinline__ void pair_sym(const Frame& f, const SymTgt<V>& t, const V* s, V* row, V* col) {
     const V d0 = t.y0 - s[0], d1 = t.y1 - s[1], d2 = t.y2 - s[2];
     const KV<V> k = Fam::template eval<V>(f, sqdist(d0, d1, d2));
-    const V w0 = t.q0 - s[6], w1 = t.q1 - s[7], w2 = t.q2 - s[8];
-    const V dq = dot3(d0, d1, d2, w0, w1, w2);
+    const V w0 = s[6] - t.q0, w1 = s[7] - t.q1, w2 = s[8] - t.q2;
+    const V dq = dot3(d0, d1, d2, w0, w1, w2) * t.ib;
     const V c1 = fma(t.a2, s[11], fma(t.a1, s[10], fma(t.a0, s[9], dot3(t.p0, t.p1, t.p2, s[3], s[4], s[5]))));
-    const V c2 = dot3(t.b0, t.b1, t.b2, s[3], s[4], s[5]);
-    const V ec2 = k.k1 * c2;
-    const V eg = fma(k.k2 * c2, dq, k.k1 * c1);
-    const V tw = ec2 * t.cd;
-    const V v0 = fma(tw, w0, eg * d0), v1 = fma(tw, w1, eg * d1), v2 = fma(tw, w2, eg * d2);
+    const V c = dot3(t.a0, t.a1, t.a2, s[3], s[4], s[5]);
+    const V ec = k.k1 * c;
+    const V eg = fma(k.k2 * c, dq, k.k1 * c1);
+    const V v0 = fma(ec, w0, eg * d0), v1 = fma(ec, w1, eg * d1), v2 = fma(ec, w2, eg * d2);
     row[0] += v0;
     row[1] += v1;
     row[2] += v2;
     const V edq = k.k1 * dq;
-    const V edqk = edq * t.k2;
-    row[3] = fma(edqk, s[3], fma(k.k0, s[9], row[3]));
-    row[4] = fma(edqk, s[4], fma(k.k0, s[10], row[4]));
-    row[5] = fma(edqk, s[5], fma(k.k0, s[11], row[5]));
+    row[3] = fma(edq, s[3], fma(k.k0, s[9], row[3]));
+    row[4] = fma(edq, s[4], fma(k.k0, s[10], row[4]));
+    row[5] = fma(edq, s[5], fma(k.k0, s[11], row[5]));
     if constexpr (COL) {
       col[0] += v0;
       col[1] += v1;
       col[2] += v2;
-      col[3] = fma(edq, t.b0, fma(k.k0, t.p0, col[3]));
-      col[4] = fma(edq, t.b1, fma(k.k0, t.p1, col[4]));
-      col[5] = fma(edq, t.b2, fma(k.k0, t.p2, col[5]));
+      col[3] = fma(edq, t.a0, fma(k.k0, t.p0, col[3]));
+      col[4] = fma(edq, t.a1, fma(k.k0, t.p1, col[4]));
+      col[5] = fma(edq, t.a2, fma(k.k0, t.p2, col[5]));
     }
   }
-  // zpx = row - col (the mirrored px-sum changes sign), zpa = -(row + col) / kappa
+  // zpx = col - row (the mirrored px-sum changes sign), zpa = row + col
   static __device__ __forceinline__ void finalize_sym(const Params& P, int i, const double* row, const double* col) {
-    const double k = P.f.kappa;
     for (int c = 0; c < 3; ++c) {
-      const double zpx = row[c] - col[c];
-      const double zpa = -(row[3 + c] + col[3 + c]) / k;
-      P.px_prev[3 * i + c] = P.px[3 * i + c] + P.dt * zpx;
-      P.pa_prev[3 * i + c] = P.pa[3 * i + c] + P.dt * zpa;
+      P.px_prev[3 * i + c] = P.px[3 * i + c] + P.dt * (col[c] - row[c]);
+      P.pa_prev[3 * i + c] = P.pa[3 * i + c] + P.dt * (row[3 + c] + col[3 + c]);
     }
   }
 };
