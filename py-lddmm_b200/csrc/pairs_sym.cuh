@@ -300,9 +300,15 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
       for (int g = 0; g < G; ++g)
 #pragma unroll
         for (int c = 0; c < NR; ++c) acc[g][c] = VT<V>::zero();
-      const int J = (int)(t * (long long)TPB / K);
-      const size_t cb = (size_t)(Geo::col_first(J) + i) * NC * K + (size_t)(t * (long long)TPB - (long long)K * J) +
-                        threadIdx.x;  // column partial of (row block i, tile t), field stride K
+      // column partial of (row block i, tile t), field stride K. Held over the tile, except where the six sums and the
+      // order-4 profile leave no register for it (40,962 points: forward step 1216 -> 1197 us, first-order adjoint
+      // 1299 -> 1286; held elsewhere: at 20,000 points of order 3 the first-order adjoint is 309 us against 324).
+      auto column_base = [&]() {
+        const int J = (int)(t * (long long)TPB / K);
+        return (size_t)(Geo::col_first(J) + i) * NC * K + (size_t)(t * (long long)TPB - (long long)K * J) + threadIdx.x;
+      };
+      constexpr bool kHeld = SPLIT || NC < 6 || VT<V>::kLanes == 1 || !std::is_same<Fam, Laplacian4>::value;
+      const size_t cb = kHeld ? column_base() : 0;
       if constexpr (SPLIT) {
         typename VT<V>::Scalar col[NC];
         if (diag) {
@@ -330,7 +336,7 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
         __syncthreads();  // every warp has read the tile and left its row sums
       } else if (!diag) {
 #pragma unroll
-        for (int c = 0; c < NC; ++c) col_ws[cb + (size_t)c * K] = colacc[c][threadIdx.x];
+        for (int c = 0; c < NC; ++c) col_ws[(kHeld ? cb : column_base()) + (size_t)c * K] = colacc[c][threadIdx.x];
       }
       // (not SPLIT) the last phase barrier of sym_tile orders every read of sm and colacc before the next staging
     }
