@@ -96,11 +96,17 @@ constexpr int kSourceUnroll = LDDMM_SOURCE_UNROLL;
 // of the stream has completed and its writes are visible; nothing global is read or written before it, so the order is
 // that of an ordinary stream. What overlaps is the next kernel's launch with the previous one's drain: 4 us per step
 // of two kernels at every size (second-order forward step at 300 / 2,562 / 10,242 points: 18.9 -> 13.5, 19.7 -> 15.5,
-// 85.1 -> 80.5 us). No kernel triggers its dependents early: their blocks would take slots while the previous grid is
-// still being placed, and a grid of one block per SM then lands on half of the SMs (adjoint step at 2,562 points: 24.4
-// us without the attribute, 33.5 with a trigger at the start of every kernel, 20.2 with the implicit one at its end).
+// 85.1 -> 80.5 us). A CTA of a split kernel releases its epilogue (chain_go()) when its last tile is done, so that the
+// epilogue's blocks are resident when the last partial is written: 0.3-0.4 us per step (2,562 points, forward / adjoint
+// / first-order adjoint step: 13.2 -> 12.8, 18.2 -> 17.8, 14.0 -> 13.6 us). The unsplit kernels, whose calls are long
+// against that, do not (forward step at 40,962 points 777 -> 810 us with it: the register allocation of the loop).
+// No kernel releases its dependents earlier, and an epilogue not at all: the blocks of the next pair kernel would take
+// slots while others are still held, and a grid of one or two blocks per SM then lands on half of the SMs (adjoint step
+// at 2,562 points: 24.4 us without the attribute, 33.5 with a release at the start of every kernel; forward step 14.8
+// -> 16.3 with one in the epilogue).
 // ---------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class... KArgs, class... Args>
 inline void launch_chained(void (*kernel)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t stream,
@@ -485,13 +491,21 @@ struct SKPlan {
   size_t ws_bytes = 0;
 };
 
-__host__ __device__ __forceinline__ long long sk_start(long long c, long long W, long long C) { return c * W / C; }
+// a / b of non-negative values, in 32 bits where both fit (all but the largest problems): every CTA and every target of
+// an epilogue divides before its first load, and a 64-bit division is some hundred dependent instructions. With one
+// quotient per index instead of up to five of 64 bits: a step's two kernels 14.8 -> 13.2 us (forward, 2,562 points),
+// 11.2 -> 10.1 (adjoint, 642 points).
+__host__ __device__ __forceinline__ long long sk_quot(long long a, long long b) {
+  if (((a | b) >> 32) == 0) return (unsigned)a / (unsigned)b;
+  return a / b;
+}
 
+// CTA c takes the units [sk_start(c), sk_start(c + 1)); unit u belongs to the last c with c W / C < u + 1.
+__host__ __device__ __forceinline__ long long sk_start(long long c, long long W, long long C) {
+  return sk_quot(c * W, C);
+}
 __host__ __device__ __forceinline__ int sk_cta_of(long long u, long long W, long long C) {
-  long long c = ((u + 1) * C - 1) / W;
-  while (c + 1 < C && sk_start(c + 1, W, C) <= u) ++c;
-  while (c > 0 && sk_start(c, W, C) > u) --c;
-  return (int)c;
+  return (int)sk_quot((u + 1) * C - 1, W);
 }
 
 int device_sm_count();
@@ -547,7 +561,7 @@ struct Units {
     return kTri ? Geo::row_off(i, TT) : i * TT;
   }
   static __device__ __forceinline__ int row_of(long long u, int gx, long long TT) {
-    return kTri ? Geo::row_of(u, gx, TT) : (int)(u / TT);
+    return kTri ? Geo::row_of(u, gx, TT) : (int)sk_quot(u, TT);
   }
   static __device__ __forceinline__ int first_tile(int i) { return kTri ? Geo::first_tile(i) : 0; }
   // source of thread `tid` in tile j (whether there is one in `live`), and its weight for target block i
@@ -839,6 +853,7 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
       __syncthreads();
     }
 
+    if (SPLIT && u + (j1 - j0) >= u_end) chain_go();
     if constexpr (SPLIT) {
       if constexpr (!kSm) {
 #pragma unroll
@@ -1087,6 +1102,7 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, F2>::value)
       __syncthreads();
     }
 
+    if (SPLIT && u + (j1 - j0) >= u_end) chain_go();
     if constexpr (SPLIT) __syncthreads();  // every warp's sums are in shared memory (also when no tile was evaluated)
 #pragma unroll
     for (int g = 0; g < G; ++g)
@@ -1194,35 +1210,46 @@ __global__ void __launch_bounds__(TPB) box_kernel(const typename Op::Params P, i
 // 1, ... from shared memory, so the order of every addition is fixed. With one thread per target its slots are one
 // serial chain (surface gradient of 2,990 against 3,534 faces: 41 us for 47 slots of 8 sums).
 constexpr int kFinThreads = 256;
+
+// The NV sums of point p over its tpp threads (thread j of np * tpp holds v), in the order j = 0, 1, ...: field c by
+// thread c mod tpp, returned to thread 0.
+template <int NV>
+__device__ __forceinline__ void finalize_meet(double (*red)[kFinThreads], int np, int tpp, int p, int j, double* v) {
+  if (tpp == 1) return;
+#pragma unroll
+  for (int c = 0; c < NV; ++c) red[c][threadIdx.x] = v[c];
+  __syncthreads();
+  for (int c = j; c < NV; c += tpp) {
+    double sum = red[c][p];
+    for (int k = 1; k < tpp; ++k) sum += red[c][k * np + p];
+    red[c][p] = sum;
+  }
+  __syncthreads();
+  if (j == 0)
+#pragma unroll
+    for (int c = 0; c < NV; ++c) v[c] = red[c][p];
+}
+
 template <class Op, typename V, int TPB, int B>
 __global__ void __launch_bounds__(kFinThreads)
     finalize_kernel(const typename Op::Params P, int n, int TT, long long W, int C,
                     const typename VT<V>::Partial* __restrict__ ws, int tpp) {
-  __shared__ double red[kFinThreads][Op::NA];
+  __shared__ double red[Op::NA][kFinThreads];
   const int np = kFinThreads / tpp;
   const int p = threadIdx.x % np, j = threadIdx.x / np;
   const int i = blockIdx.x * np + p;
+  using Un = Units<Op, TPB, B>;
+  const int tb = i / B;
+  const int nslot =
+      i < n && W > 0 ? sk_cta_of(Un::row_off(tb + 1, TT) - 1, W, C) - sk_cta_of(Un::row_off(tb, TT), W, C) + 1 : 0;
   chain_wait();
   double acc[Op::NA];
 #pragma unroll
   for (int c = 0; c < Op::NA; ++c) acc[c] = 0.0;
-  if (i < n && W > 0) {
-    using Un = Units<Op, TPB, B>;
-    const int tb = i / B;
-    const int nslot = sk_cta_of(Un::row_off(tb + 1, TT) - 1, W, C) - sk_cta_of(Un::row_off(tb, TT), W, C) + 1;
-    for (int s = j; s < nslot; s += tpp)
+  for (int s = j; s < nslot; s += tpp)
 #pragma unroll
-      for (int c = 0; c < Op::NA; ++c) acc[c] += partial_value(ws[((size_t)s * Op::NA + c) * (size_t)n + i]);
-  }
-  if (tpp > 1) {
-#pragma unroll
-    for (int c = 0; c < Op::NA; ++c) red[threadIdx.x][c] = acc[c];
-    __syncthreads();
-    if (j == 0)
-      for (int k = 1; k < tpp; ++k)
-#pragma unroll
-        for (int c = 0; c < Op::NA; ++c) acc[c] += red[k * np + p][c];
-  }
+    for (int c = 0; c < Op::NA; ++c) acc[c] += partial_value(ws[((size_t)s * Op::NA + c) * (size_t)n + i]);
+  finalize_meet<Op::NA>(red, np, tpp, p, j, acc);
   if (i < n && j == 0) Op::finalize(P, i, acc);
 }
 

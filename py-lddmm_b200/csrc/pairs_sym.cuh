@@ -341,6 +341,7 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
       // (not SPLIT) the last phase barrier of sym_tile orders every read of sm and colacc before the next staging
     }
 
+    if (SPLIT && u + (t1 - t0) >= u_end) chain_go();
     if constexpr (SPLIT) {
       // the block's row sums: field c of the lanes' targets by warp c mod W, over the W warps in order
 #pragma unroll
@@ -399,36 +400,27 @@ __global__ void __launch_bounds__(kFinThreads)
                         const typename VT<V>::Scalar* __restrict__ col_ws, int tpp) {
   using Geo = SymGeom<TPB, B>;
   constexpr int NV = Op::NR + Op::NC, K = Geo::K;
-  __shared__ double red[kFinThreads][NV];
+  __shared__ double red[NV][kFinThreads];
   const int np = kFinThreads / tpp;
   const int p = threadIdx.x % np, j = threadIdx.x / np;
   const int idx = blockIdx.x * np + p;
   const bool live = idx < n;
+  const int b = live ? idx / B : 0, J = live ? idx / K : 0, r = live ? idx - J * K : 0;
+  const int nslot =
+      live ? sk_cta_of(Geo::row_off(b + 1, TT) - 1, U, C) - sk_cta_of(Geo::row_off(b, TT), U, C) + 1 : 0;
+  const int ncol = live ? J * Geo::kShare : 0;
+  const size_t cfirst = (size_t)Geo::col_first(J) * Op::NC * K + r;
   chain_wait();
   double v[NV];
 #pragma unroll
   for (int c = 0; c < NV; ++c) v[c] = 0.0;
-  const int b = live ? idx / B : 0, J = live ? idx / K : 0, r = live ? idx - J * K : 0;
-  if (live) {
-    const int nslot = sk_cta_of(Geo::row_off(b + 1, TT) - 1, U, C) - sk_cta_of(Geo::row_off(b, TT), U, C) + 1;
-    for (int s = j; s < nslot; s += tpp)
+  for (int s = j; s < nslot; s += tpp)
 #pragma unroll
-      for (int c = 0; c < Op::NR; ++c) v[c] += partial_value(row_ws[((size_t)s * Op::NR + c) * (size_t)n + idx]);
-    for (int q = j; q < J * Geo::kShare; q += tpp) {
-      const size_t cb = (size_t)(Geo::col_first(J) + q) * Op::NC * K + r;
+    for (int c = 0; c < Op::NR; ++c) v[c] += partial_value(row_ws[((size_t)s * Op::NR + c) * (size_t)n + idx]);
+  for (int q = j; q < ncol; q += tpp)
 #pragma unroll
-      for (int c = 0; c < Op::NC; ++c) v[Op::NR + c] += (double)col_ws[cb + (size_t)c * K];
-    }
-  }
-  if (tpp > 1) {
-#pragma unroll
-    for (int c = 0; c < NV; ++c) red[threadIdx.x][c] = v[c];
-    __syncthreads();
-    if (j == 0)
-      for (int k = 1; k < tpp; ++k)
-#pragma unroll
-        for (int c = 0; c < NV; ++c) v[c] += red[k * np + p][c];
-  }
+    for (int c = 0; c < Op::NC; ++c) v[Op::NR + c] += (double)col_ws[cfirst + ((size_t)q * Op::NC + c) * K];
+  finalize_meet<NV>(red, np, tpp, p, j, v);
   if (live && j == 0) Op::finalize_sym(P, idx, v, v + Op::NR);
 }
 
