@@ -211,20 +211,37 @@ __global__ void __launch_bounds__(THREADS) gemm_kernel(int M, int N, int K, int 
       }
   if constexpr (!kF32) {
     __syncthreads();
+    auto masked = [](bf16 v, bf16 m) { return __bfloat162float(m) > 0.f ? v : __float2bfloat16_rn(0.f); };
+    // C and the mask need no more than the alignment of a column pair: 16 bytes at a time where both have it (rows are
+    // multiples of 128 bytes)
+    const uintptr_t at = reinterpret_cast<uintptr_t>(C) | (EPI == kEpiMaskBf16 ? reinterpret_cast<uintptr_t>(mask) : 0);
+    if (at % 16 == 0) {
 #pragma unroll
-    for (int it = threadIdx.x; it < (BM * BN) / 8; it += THREADS) {
-      const int r = it / (BN / 8), c = (it % (BN / 8)) * 8;
-      uint4 v = *reinterpret_cast<const uint4*>(&tile[r][c]);
-      const size_t o = (size_t)(m0 + r) * N + n0 + c;
-      if (EPI == kEpiMaskBf16) {
-        const uint4 mk = *reinterpret_cast<const uint4*>(&mask[o]);
-        const bf16* mv = reinterpret_cast<const bf16*>(&mk);
-        bf16* vv = reinterpret_cast<bf16*>(&v);
+      for (int it = threadIdx.x; it < (BM * BN) / 8; it += THREADS) {
+        const int r = it / (BN / 8), c = (it % (BN / 8)) * 8;
+        uint4 v = *reinterpret_cast<const uint4*>(&tile[r][c]);
+        const size_t o = (size_t)(m0 + r) * N + n0 + c;
+        if (EPI == kEpiMaskBf16) {
+          const uint4 mk = *reinterpret_cast<const uint4*>(&mask[o]);
+          const bf16* mv = reinterpret_cast<const bf16*>(&mk);
+          bf16* vv = reinterpret_cast<bf16*>(&v);
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (!(__bfloat162float(mv[q]) > 0.f)) vv[q] = __float2bfloat16_rn(0.f);
+          for (int q = 0; q < 8; ++q) vv[q] = masked(vv[q], mv[q]);
+        }
+        *reinterpret_cast<uint4*>(&reinterpret_cast<bf16*>(C)[o]) = v;
       }
-      *reinterpret_cast<uint4*>(&reinterpret_cast<bf16*>(C)[o]) = v;
+    } else {
+      for (int it = threadIdx.x; it < (BM * BN) / 2; it += THREADS) {
+        const int r = it / (BN / 2), c = (it % (BN / 2)) * 2;
+        __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&tile[r][c]);
+        const size_t o = (size_t)(m0 + r) * N + n0 + c;
+        if (EPI == kEpiMaskBf16) {
+          const __nv_bfloat162 mk = *reinterpret_cast<const __nv_bfloat162*>(&mask[o]);
+          v.x = masked(v.x, mk.x);
+          v.y = masked(v.y, mk.y);
+        }
+        *reinterpret_cast<__nv_bfloat162*>(&reinterpret_cast<bf16*>(C)[o]) = v;
+      }
     }
   }
 }

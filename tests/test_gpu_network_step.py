@@ -62,3 +62,27 @@ def test_adam_steps_match_the_formula():
         assert np.allclose(p.cpu().numpy(), r.cpu().numpy(), rtol=2e-5, atol=2e-6)
     for wb, w in zip(model.Wb, model.W):
         assert torch.equal(wb, w.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize('offset', [0, 2, 4, 6])
+@pytest.mark.parametrize('epi', [2, 3, 4])
+def test_bf16_outputs_and_mask_aligned_to_a_column_pair(offset, epi):
+    """C and the mask of a BF16 epilogue at any 4-byte boundary: the same bits as at a 16-byte one, and nothing beside
+    them is written."""
+    import torch
+    import base._native as nat
+    M, N, K = 128, 128, 64
+    g = torch.Generator(device='cuda').manual_seed(3)
+    A, B = (torch.randn(s, generator=g, device='cuda').to(torch.bfloat16) for s in ((M, K), (K, N)))
+    bias, mask = torch.randn(N, generator=g, device='cuda'), torch.randn((M, N), generator=g, device='cuda')
+    outs = []
+    for off in (0, offset):
+        buf = torch.full((M * N + 16,), 7.0, dtype=torch.bfloat16, device='cuda')
+        mb = torch.zeros(M * N + 16, dtype=torch.bfloat16, device='cuda')
+        C, mk = buf[off:off + M * N], mb[off:off + M * N]
+        mk.copy_(mask.reshape(-1))
+        nat.check(nat.lib().lddmm_bf16_gemm(0, 0, epi, M, N, K, nat.ptr(A), nat.ptr(B), nat.ptr(bias), nat.ptr(mk),
+                                            nat.ptr(C), 1, None, 0, nat.stream_ptr()), 'gemm')
+        assert torch.all(buf[:off] == 7.0) and torch.all(buf[off + M * N:] == 7.0)
+        outs.append(C.clone())
+    assert torch.equal(*outs)
