@@ -86,3 +86,16 @@ def test_bf16_outputs_and_mask_aligned_to_a_column_pair(offset, epi):
         assert torch.all(buf[:off] == 7.0) and torch.all(buf[off + M * N:] == 7.0)
         outs.append(C.clone())
     assert torch.equal(*outs)
+
+
+def test_adam_with_fewer_gradients_than_tensors():
+    """The weights alone: the tensors without a gradient stay as they are."""
+    import torch
+    from base.learnedProposal import MomentumProposal
+    model = MomentumProposal(seed=1)
+    before = [p.clone() for p in model.W + model.b]
+    model.adam([torch.ones_like(w) for w in model.W], lr=1e-2)
+    assert all(not torch.equal(p, q) for p, q in zip(model.W, before))
+    assert all(torch.equal(p, q) for p, q in zip(model.b, before[len(model.W):]))
+    model.adam([])
+    assert model.step == 2
