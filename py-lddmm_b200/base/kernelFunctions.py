@@ -126,19 +126,28 @@ class Kernel(KernelSpec):
         squeeze = A.dim() == 1
         if squeeze:
             A = A[:, None]
+        origin = self._origin(Y, X, x)        # of every width and column group
         if A.shape[1] != 3:
-            r = self._multi(lambda s: self._k_generic(Y, X, A, s))
+            r = self._multi(lambda s: self._k_generic(Y, X, A, s, origin))
         else:
-            r = self._multi(lambda s: self._apply_k(Y, X, A, s))
+            r = self._multi(lambda s: self._apply_k(Y, X, A, s, origin))
         if squeeze:
             r = r[:, 0]
         return _out(r, like_np)
 
+    def _origin(self, Y, X, points=None):
+        # Origin of K(Y, X) a; `points`: X as the caller gave it (a host array is averaged on the host). The Gaussian
+        # sums run expanded-distance kernels (FP32) or FP64 arithmetic on the coordinates as they are: no origin. The
+        # Laplacian FP32 kernels evaluate differences of origin-centred FP32 coordinates.
+        if self.code == nat.KERNEL_GAUSS:
+            return None
+        if Y is X and X.shape[0] <= nat.OWN_ORIGIN_POINTS[self.precision]:
+            return None                                 # blocks take their own (nat.self_origin)
+        return nat.centroid(X if points is None or isinstance(points, torch.Tensor) else points)
+
     def _apply_k(self, Y, X, A, sigma, origin=None):
-        # The Gaussian sums run expanded-distance kernels (FP32) or FP64 arithmetic on the coordinates as they are: no
-        # origin. The Laplacian FP32 kernels evaluate differences of origin-centred FP32 coordinates.
-        if origin is None and self.code != nat.KERNEL_GAUSS:
-            origin = nat.self_origin(X, self.precision) if Y is X else nat.centroid(X)
+        if origin is None:
+            origin = self._origin(Y, X)
         n, m = Y.shape[0], X.shape[0]
         out = torch.empty((n, 3), dtype=torch.float64, device=Y.device)
         ws, wsb = nat.workspace(n, m, self.precision)
@@ -147,7 +156,7 @@ class Kernel(KernelSpec):
                                           nat.ptr(out), self.precision, ws, wsb, nat.stream_ptr()), 'applyK')
         return out
 
-    def _k_generic(self, Y, X, A, sigma):
+    def _k_generic(self, Y, X, A, sigma, origin):
         """K a for momenta of any width d: columns in groups of 3 (zero padded)."""
         d = A.shape[1]
         cols = []
@@ -155,7 +164,7 @@ class Kernel(KernelSpec):
             blk = A[:, c0:c0 + 3]
             if blk.shape[1] < 3:
                 blk = torch.cat([blk, blk.new_zeros(blk.shape[0], 3 - blk.shape[1])], dim=1)
-            cols.append(self._apply_k(Y, X, blk.contiguous(), sigma))
+            cols.append(self._apply_k(Y, X, blk.contiguous(), sigma, origin))
         return torch.cat(cols, dim=1)[:, :d].contiguous()
 
     def _k_mat(self, Y, X, U, sigma):

@@ -67,7 +67,8 @@ class SurfaceDataTerm:
             self.vf_off, self.vf_items = vertex_face_table(self.faces_np, self.nv)
         elif self.faces_np.size and (self.faces_np.min() < 0 or self.faces_np.max() >= self.nv):
             raise nat.LddmmError('faces index outside the vertices')
-        self.origin = nat.centroid(target_vertices)
+        # host vertices: averaged there, no read-back
+        self.origin = nat.centroid(self.x1 if isinstance(target_vertices, torch.Tensor) else target_vertices)
         self._norm0 = None
 
     def _ws(self):
