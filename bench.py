@@ -61,10 +61,10 @@ sys.path.insert(0, REPO)
 
 LEVEL = 6
 SIGMAS = (0.25, 0.5)
-# The self-sum K(x,x)a runs the symmetric expanded-distance kernel (pairs_kernel_symx<OpKSym, 128, 8>): rows in
-# blocks of 128 x 8 points; an unordered pair of different blocks costs 9 FP32 lane-ops and one ex2 (row term,
+# The self-sum K(x,x)a runs the symmetric expanded-distance kernel (pairs_kernel_symx<OpKSym, 128, 6>): rows in
+# blocks of 128 x 6 points; an unordered pair of different blocks costs 9 FP32 lane-ops and one ex2 (row term,
 # column term, the expanded squared distance), an ordered pair inside a block 6 and one ex2 (row term only).
-KSYM_BLOCK = 1024
+KSYM_BLOCK = 768
 OPS_FP32_OFFDIAG, OPS_FP32_DIAG, OPS_SFU_PER_PAIR = 9, 6, 1
 METRIC = 'Gauss kernel pairs/s'
 # Coarse-to-fine warm start of the registrations: the coarse levels (icosphere levels of the source) per fine level,
@@ -661,10 +661,10 @@ def run_level4_fp64():
 # take the difference form: 9, 16, 12 and 22)
 OP_COUNTS = {'applyK': (6, 1), 'applyDiffKT_lddmm': (16, 1), 'applyDDiffK11and12': (23, 1), 'applyDiffK1and2': (16, 1),
              'so_step': (14, 1), 'so_adjoint_step': (37, 1), 'fo_adjoint_step': (19, 1), 'varifold_energy': (9, 1),
-             'varifold_gradient': (19, 1)}
+             'varifold_gradient': (18, 1)}
 # Self-sums that run a symmetric kernel (FP32, Gaussian): (row block size, FP32 lane-ops per ordered pair inside a
 # block (row terms only), FP32 lane-ops per unordered pair between blocks (row and column terms)); one ex2 each.
-SYM_COUNTS = {'applyK': (1024, 6, 9), 'so_step': (1024, 16, 22), 'so_adjoint_step': (512, 42, 51),
+SYM_COUNTS = {'applyK': (768, 6, 9), 'so_step': (768, 16, 22), 'so_adjoint_step': (512, 41, 50),
               'fo_adjoint_step': (512, 19, 25)}
 
 
@@ -1061,7 +1061,7 @@ def run_b200(args, rank, world, local_rank):
         'roofline': {'bound': 'fp32', 'achieved': achieved, 'peak': peak_fp32, 'unit': 'T FP32 lane-ops/s',
                      'frac': achieved / peak_fp32, 'sfu_frac': sfu_frac, 'traffic': traffic,
                      'traffic_source': traffic_source, 'algorithmic_bytes': 2 * n * 3 * 8 + n * 3 * 8,
-                     'kernel': 'pairs_kernel_symx<OpKSym, 128, 8> + finalize_sym_kernel (timed together per call)',
+                     'kernel': 'pairs_kernel_symx<OpKSym, 128, 6> + finalize_sym_kernel (timed together per call)',
                      'pairs_evaluated_per_launch': {'ordered_in_block': diag, 'unordered_between_blocks': off},
                      'ops_per_pair': {'fp32_between_blocks': OPS_FP32_OFFDIAG, 'fp32_in_block': OPS_FP32_DIAG,
                                       'sfu': OPS_SFU_PER_PAIR},

@@ -111,8 +111,9 @@ struct OpKSym {
 struct OpKSymD {
   using Params = OpK::Params;
   static constexpr int NSS = 6, NR = 3, NC = 3;
-  static constexpr int kSymMinCtas = LDDMM_KSYM_MIN_CTAS;
-  using Shape = SymRule<kSplit2N, kSplit4N, kSplit8N, kSplit8N, kRtKSym, kRtKSymL, kTpbSym64, kRtSym64>;
+  static constexpr int kSymMinCtas = 3;
+  static constexpr int kSymUnrollG = 8;  // 13,000 points, 8 targets split: 51.9 us, 4: 53.3
+  using Shape = SymRule<kSplit4N, kSplit4N, 0, kRtKSymL, kTpbSym64, kRtSym64>;  // whole tiles, Gaussian: OpKSym
   template <typename V> struct SymTgt { V y0, y1, y2, a0, a1, a2; };
   template <typename V>
   static __device__ __forceinline__ void load_target_sym(const Params& P, int i0, int i1, bool v0, bool v1,

@@ -19,7 +19,7 @@
 #define LDDMM_RT_ADJOINT 4
 #endif
 #ifndef LDDMM_RT_SYM_FWD
-#define LDDMM_RT_SYM_FWD 8
+#define LDDMM_RT_SYM_FWD 6
 #endif
 #ifndef LDDMM_RT_FO_SYM
 #define LDDMM_RT_FO_SYM 4
@@ -28,7 +28,7 @@
 #define LDDMM_RT_SYM_FWD_L 4
 #endif
 #ifndef LDDMM_RT_ADJOINT_SYM_L
-#define LDDMM_RT_ADJOINT_SYM_L 2
+#define LDDMM_RT_ADJOINT_SYM_L 4
 #endif
 #ifndef LDDMM_RT_FO_SYM_L
 #define LDDMM_RT_FO_SYM_L 4
@@ -40,7 +40,7 @@
 #define LDDMM_TPB_KSYM 128
 #endif
 #ifndef LDDMM_RT_KSYM
-#define LDDMM_RT_KSYM 8
+#define LDDMM_RT_KSYM 6
 #endif
 #ifndef LDDMM_TPB_64
 #define LDDMM_TPB_64 128
@@ -61,39 +61,47 @@ constexpr int kRtHeavy = LDDMM_RT_HEAVY;
 // 2 CTAs per SM) measured 4% faster than 2 targets per thread at 4 CTAs per SM (half the shared-memory reads per
 // pair, two independent lane groups per source).
 constexpr int kRtAdjoint = LDDMM_RT_ADJOINT;
-// The symmetric second-order forward step (pairs_kernel_sym): 8 targets per thread (168 registers, 3 CTAs per SM,
-// its compensated row sums in 48 KiB of dynamic shared memory) measured 15% faster at level 6 than 4 targets per
-// thread (134 registers, 3 CTAs per SM): the per-step source loads and the column shuffles are shared by twice
-// as many pairs, and four independent lane groups hide the latency of the ex2 chain.
+// Symmetric sums, FP32, whole tiles: targets per thread. More of them share a source's loads and column shuffles; each
+// takes two registers per value (both lanes of a packed operand are the target). us at 40,962 points, Gaussian, threads
+// of 128 (the kernels with two targets to a packed value, at their best shape: forward 775, adjoint 1609, first-order
+// adjoint 955, K a 381; Laplacian of order 3: 1114, 2047, 1215, 627):
+//   forward step 4 | 6: 786 | 744          adjoint step 4 | 5: 1498 | 1525     first-order adjoint 4 | 5 | 6 at the
+//   K a (expanded form) 4 | 6 | 8 | 10: 393 | 373 | 365 | 354                  better of two unroll depths: 845 | 826 | 842
+//   Laplacian: forward step 4 | 6: 1051 | 1008, adjoint 4 | 5: 1830 | 1948, first-order adjoint 4 | 5 | 6: 1103 | 1105 |
+//   1135, K a 4 | 6 | 8: 601 | 594 | 579
+// A column sum is a chain of RT additions per step, and its rounding grows with RT: the shapes taken are the fastest
+// whose errors against FP64 are not above those of the kernels before (K a of 30,001 points, sigma 0.3: 6.8e-8 before,
+// with 6 | 8 | 10 targets 6.6e-8 | 7.3e-8 | 8.2e-8; the Laplacian's K a of 20,000 points with 4 | 6 | 8: 0.97 | 1.06 | 1.13
+// of it, its forward step with 4 | 5 | 6: 0.97 | 1.02 | 1.05).
 constexpr int kRtSymFwd = LDDMM_RT_SYM_FWD;
-// Small and middle point sets: the split symmetric kernel (pairs_kernel_sym with SPLIT: the four warps of a CTA share
-// 32 RT targets and take a quarter of every tile each), with more targets per thread as the set grows. A small RT gives
-// more units, a large one fewer loads, shuffles and partials per pair. Each line lies where the next shape starts to
-// win; us per step, launches overlapped (2 | 4 | 8 targets split; "-": the shape that was used up to here):
-//   forward step   n = 1,500: 11.5 | 11.1 | 14.4 (- 14.7)   2,562: 16.4 | 14.7 | 15.3 (- 15.5)   4,000: 23.2 | 20.9 |
-//                  20.5 (- 20.9)   7,000: 50.9 | 40.2 | 41.0 (- 56.7)   10,242: 89 | 74.5 | 67.9 (- 80.3)
-//                  16,000: 190 | 152 | 138 (- 174)   20,000: 301 | 236 | 221, without the split 223
-//   adjoint step   642: 11.1 | 14.1 (- 18.7)   2,000: 14.9 | 15.0 (- 19.7)   3,200: 29.0 | 26.1 (- 30.0)   7,000: 77.0 |
-//                  70.9 (- 83.4)   10,242: 139 | 129, without the split 120
-//   K a            642: 8.1 | 9.0 | 10.1 (- 16.3)   2,562: 12.0 | 11.9 | 12.0 (- 20.1)   4,000: 17.1 | 15.3 | 14.9 (-
-//                  20.1)   10,242: 55 | 45.5 | 41.0 (- 48.9)   16,000: 114 | 91 | 79.7 (- 79.9)
-//   first-order    642: 9.5 | 11.8 (- 19.4)   2,562: 17.3 | 16.1 (- 20.6)   7,000: 55.5 | 44.6 (- 43.6)   8,000: 63 |
-//   adjoint step   56 (- 74.8)   10,242: 97.7 | 83.0, without the split 74.6
-// and for the Laplacian (2 | 4 split): forward 2,562: 18.3 | 16.7 (- 23.8), 6,000: 45.1 | 42.9 (- 46.7), 10,242: 110 |
-// 98, without 91; adjoint 6,000: 75.9 | 63.7 (- 87.7); K a 10,242: 67 | 58.1 (- 63.6).
-constexpr int64_t kSplit2N = 1280, kSplit2NAdj = 2048;  // 2 targets per thread up to here
-constexpr int64_t kSplit4N = 3600;                      // 4 up to here, then 8 (forward step and K a, Gaussian)
-constexpr int64_t kSplit4NLast = 8192;                  // 4 up to here, then no split (adjoint steps, Laplacian)
-constexpr int64_t kSplit8N = 16384;                     // 8 up to here, then no split
-// The symmetric K(x, x) a (pairs_kernel_symx): 8 targets per thread.
-// The symmetric first-order adjoint step (pairs_kernel_sym): 4 targets per thread.
 constexpr int kRtFoSym = LDDMM_RT_FO_SYM;
-// The symmetric steps with the Laplacian family (its radial profile -- a square root and the polynomial -- takes
-// registers that the Gaussian shapes spend on more targets per thread).
 constexpr int kRtSymFwdL = LDDMM_RT_SYM_FWD_L;
 constexpr int kRtAdjointSymL = LDDMM_RT_ADJOINT_SYM_L;
 constexpr int kRtFoSymL = LDDMM_RT_FO_SYM_L;
 constexpr int kRtKSymL = LDDMM_RT_KSYM_L;
+// Small and middle point sets: the split symmetric kernel (pairs_kernel_sym with SPLIT: the four warps of a CTA share
+// 32 RT targets and take a quarter of every tile each), with more targets per thread as the set grows. A small RT gives
+// more units, a large one fewer loads, shuffles and partials per pair. us, launches overlapped (2 | 4 | 8 targets split
+// / whole tiles; "-": the split kernel with two targets to a packed value at its best shape):
+//   forward step     n = 1,300: 7.8 | 8.6 | 11.9 (- 8.8)   2,562: 13.3 | 11.8 | 12.8 (- 12.2)   6,000: 33.0 | 27.4 | 27.9
+//                    (- 30.5)   10,242: 72.4 | 65.8 | 62.9 / 57.2 (- 67)   13,000: 110 | 95.8 | 88.9 / 106 (- 95.6)
+//                    16,000: 161 | 140 | 132 / 130   20,000: 250 | 215 | 203 / 194
+//   adjoint step     1,300: 9.0 | 11.6 (- 9.3)   2,562: 18.0 | 16.7 (- 17.2)   8,000: 79 | 72.3 / 74.9 (- 76.5)
+//                    10,242: 122 | 115 / 109 (- 116)   13,000: 190 | 171 / 175 (- 188)   20,000: 437 | 388 / 377
+//   first-order      1,300: 7.9 | 9.1 (- 9.5)   2,562: 14.1 | 12.5 (- 13.2)   6,000: 36.0 | 30.1 (- 33.9)   10,242: 80 |
+//   adjoint step     72 / 66.4 (- 71.4)   13,000: 122 | 105 / 105 (- 115)   20,000: 278 | 235 / 224
+//   K a              2,562: 9.5 | 8.7 | 8.8 (- 9.1)   6,000: 20.5 | 19.0 | 18.0 (- 18.9)   10,242: 46.5 | 39.7 | 36.9 /
+//                    45.6 (- 38.4)   13,000: 67 | 56 | 52 / 53 (- 54)   16,000: 98 | 81 | 79 / 70 (- 78)
+// and for the Laplacian of order 3: forward 10,242: 91 | 83 | 86 / 76 (- 82), 13,000: 139 | 123 | 122 / 141 (- 132);
+// adjoint 13,000: 227 | 208 / 230 (- 239), 16,000: 335 | 308 / 319; K a 10,242: 56 | 51 | 48 / 59 (- 53).
+// 2 targets up to kSplit2N: there the units of 64 points still have an SM each. Whole tiles are faster per pair and
+// their units four times longer, so between kWholeN and kSplitN they are taken where their units fill the resident CTAs
+// (10,242 and 16,000 points above, not 13,000), beyond kSplitN always. K a of the Gaussian keeps the split up to
+// kSplitN: its whole tiles centre a block on its box, the split on a point, which one far point does not move.
+constexpr int64_t kSplit2N = 1408;
+constexpr int64_t kSplit4N = 3600;   // 4 targets up to here in K a, then 8
+constexpr int64_t kWholeN = 8192;    // (4 targets up to here in the Gaussian's forward step, then 8)
+constexpr int64_t kSplitN = 16384;
 constexpr int kTpbKSym = LDDMM_TPB_KSYM;
 constexpr int kRtKSym = LDDMM_RT_KSYM;
 // FP64 baseline path.
@@ -111,7 +119,7 @@ constexpr int kTpbSym64Adj = 128, kRtSym64Adj = 2;
 // 4,000: 62.8 | 55.3 | 55.6).
 constexpr int64_t kSplit1N64 = 1280, kSplit2N64 = 2304, kSplit2N64Lap = 4096;
 
-static_assert(kSplit4NLast >= 8192 && kSplit8N >= 8192 && kSplit2N64 >= 2304,
+static_assert(kWholeN >= 8192 && kSplitN >= kWholeN && kSplit2N64 >= 2304,
               "every self-sum up to LDDMM_OWN_ORIGIN_POINTS runs a split kernel");
 
 }  // namespace lddmm

@@ -41,11 +41,10 @@
 #define LDDMM_SOBWD_SYM_MIN_CTAS 2  // the symmetric adjoint step (pairs_kernel_sym)
 #endif
 #ifndef LDDMM_SOFWD_SYM_MIN_CTAS
-#define LDDMM_SOFWD_SYM_MIN_CTAS 3  // the symmetric forward step (pairs_kernel_sym): caps it at 168 registers
+#define LDDMM_SOFWD_SYM_MIN_CTAS 3  // the symmetric forward step (pairs_kernel_sym) up to 4 targets per thread
 #endif
 #ifndef LDDMM_KSYM_MIN_CTAS
-#define LDDMM_KSYM_MIN_CTAS 3  // the symmetric K(x, x) a (pairs_kernel_symx): 164 registers, 3 CTAs per SM (3% faster
-                               // than 4 CTAs at 128 registers, which spill)
+#define LDDMM_KSYM_MIN_CTAS 2  // the symmetric K(x, x) a (pairs_kernel_symx)
 #endif
 #ifndef LDDMM_FOBWD_SYM_MIN_CTAS
 #define LDDMM_FOBWD_SYM_MIN_CTAS 2  // the symmetric first-order adjoint step (pairs_kernel_sym)

@@ -9,13 +9,13 @@
 //    j >= i: the upper triangle in blocks. Units with j == i ("diagonal") evaluate their ordered pairs for the rows
 //    only, like pairs_kernel; units with j > i evaluate each pair once and credit the row k (registers, as in
 //    pairs_kernel) and the column l.
-//  * Column credit without atomics: inside a tile, warp w of the CTA takes chunk (w + phase) mod W of 32 sources in
-//    phase `phase` (one barrier per phase), and lane λ processes source (λ + s) mod 32 of the chunk at step s: the 32
-//    lanes read 32 different sources (conflict-free 16-byte loads of the shared tile). The lane's column sum for its
-//    source (its RT targets) is added to a rotating accumulator that moves one lane down after every step (one
-//    shuffle per accumulator), so it follows its source around the warp; after 32 steps lane λ holds the warp's
-//    column sum of source λ of the chunk and adds it to the tile's column accumulators in shared memory. At the end
-//    of the unit those hold the unit's column sums (TPB sources x NC), written as one partial per (block i, source).
+//  * Column credit without atomics: the warps of a CTA take the chunks of a tile in turn (one barrier per phase), and
+//    lane λ processes record (λ + s) mod 32 of its chunk at step s: the 32 lanes read 32 different records. A record
+//    is two sources in FP32, one in FP64 (SymStage). The record's column sums (over the lane's RT targets) are added to
+//    an accumulator that moves one lane down after every step, so it follows its record around the warp; after 32
+//    steps lane λ holds the warp's column sums of record λ of the chunk and adds them to the tile's column accumulators
+//    in shared memory. At the end of the unit those hold the unit's column sums (TPB sources x NC), written as one
+//    partial per (block i, source).
 //  * Stream-K over the units in row-major order (as pairs_kernel over its units): a CTA's run of units of one row i
 //    is a segment with compensated row sums (one partial slot, as in pairs_kernel). Point l of block b then has the
 //    row slots of block b and b column partials (one from each block i < b); the epilogue sums both in a fixed order
@@ -28,13 +28,14 @@
 // Op interface (besides Params, finalize_sym):
 //   NSS                                  source fields staged per source (scaled coordinates 0-2 first)
 //   NR, NC                               row and column accumulators per point
-//   SymTgt<V>                            per-lane-group register state (V = F2: two targets, V = double: one)
-//   load_target_sym<V>(P, i0, i1, v0, v1, SymTgt<V>&)  targets i0, i1 (< n); v0 / v1 false = padding (zero payload)
+//   SymTgt<V>                            register state of one target (V = F2: in both lanes)
+//   load_target_sym<V>(P, i0, i1, v0, v1, SymTgt<V>&)  lanes from points i0, i1 (< n; the same here); v0 / v1 false =
+//                                        padding (zero payload)
 //   source_fields_sym(P, l, double* f)   NSS fields of source l (FP64)
 //   pair_sym<COL, Fam, V>(const Frame&, const SymTgt<V>&, const V* s, V* row, V* col)
 //   finalize_sym(P, i, const double* row, const double* col)
 //
-// FP64 (V = double): one target per lane group, sources staged as doubles, row sums, column sums and column partials
+// FP64 (V = double): one source to a record, staged as doubles, row sums, column sums and column partials
 // in FP64; the rotating accumulator costs two shuffles per field. What it saves is the exponential (about a third of
 // an FP64 pair) and the shared products, on a pipe of half the FP32 rate.
 #pragma once
@@ -43,13 +44,6 @@
 
 #ifndef LDDMM_SYM
 #define LDDMM_SYM 1  // 0: self-interaction sums evaluate every ordered pair (pairs_kernel)
-#endif
-#ifndef LDDMM_SYM_COMPACT
-#define LDDMM_SYM_COMPACT 1  // 0: the symmetric kernels stage sources in pairs_kernel's duplicated layout (measured
-                             // 3-6% slower at level 6: twice the bytes per unshared load)
-#endif
-#ifndef LDDMM_SYMX_COL_SPLIT
-#define LDDMM_SYMX_COL_SPLIT 0  // 1: pairs_kernel_symx accumulates the column terms of even and odd lane groups apart
 #endif
 #ifndef LDDMM_SYMX_UNROLL
 #define LDDMM_SYMX_UNROLL 8  // unroll depth of pairs_kernel_symx's source loop (8: 1% faster than 4 at level 6)
@@ -63,77 +57,127 @@ namespace lddmm {
 constexpr int kSymUnroll = LDDMM_SYM_UNROLL;
 constexpr int kSymxUnroll = LDDMM_SYMX_UNROLL;
 
-// Shared-memory record of a staged source tile. In the symmetric kernels the 32 lanes of a warp read 32 different
-// sources at every step (no broadcast), so the record size is what the loads cost: compact records hold each field
-// once in FP32 (float4 groups) and the packed (f, f) operands are formed in registers; the duplicated layout of
-// pairs_kernel (Unit<F2>: one 16-byte load gives two packed operands) reads twice the bytes.
-template <int NF, int TPB, typename V>
+// Shared-memory record of a staged source tile, and the column sums that ride around the warp while a chunk of sources
+// is evaluated. In the symmetric kernels the lanes of a warp read different sources at every step (no broadcast), so
+// what a load costs is its record.
+//  * FP64: a record is one source; its column sums go around R = 32 lanes in 32 steps.
+//  * FP32: the lanes of a packed value are two sources (r and r + R of a chunk of 2 R), and a 16-byte unit is two fields
+//    of both, so an operand is used as it is loaded and a column sum moves as it is. With two targets to a value every
+//    field is duplicated after its load, and every column sum is made a packed operand and its lanes added, at every
+//    step: some 30 instructions per 4 targets that the pair does not need (40,962 points: forward / adjoint /
+//    first-order adjoint step 772 / 1602 / 951 us, with two sources to a value 735 / 1478 / 840). The targets are the
+//    duplicated side, once per segment, at the price of their registers.
+//    R = 32 where a CTA's warps take all chunks of a tile in turn. R = 16 where each takes one chunk of 32 (SPLIT): the
+//    column sums go around each half of the warp, and the halves, which hold different targets, meet at the end (whole
+//    tiles with R = 16: 750 / 1503 / 862 us).
+template <typename V, bool SPLIT>
+constexpr int kSymRing = std::is_same<V, F2>::value && SPLIT ? 16 : 32;
+template <int NF, int TPB, typename V, int R>
 struct SymStage;
-template <int NF, int TPB>
-struct SymStage<NF, TPB, double> {
-  static constexpr int NQ = (NF + 1) / 2;  // 16-byte units of two fields
+template <int NF, int TPB, int R>
+struct SymStage<NF, TPB, double, R> {
+  static constexpr int NQ = (NF + 1) / 2;  // 16-byte units
+  static constexpr int kSlots = TPB;       // records of a tile
+  static constexpr int kFields = 2 * NQ;   // size of the FP64 field buffer and of the operand array
   using T = double2;
-  static __device__ __forceinline__ void store(T (*sm)[TPB], int t, const double* fl) {
+  static __device__ __forceinline__ void store(T (*sm)[kSlots], int t, const double* fl) {
 #pragma unroll
     for (int q = 0; q < NQ; ++q) sm[q][t] = make_double2(fl[2 * q], fl[2 * q + 1]);
   }
-  static __device__ __forceinline__ void load(const T (*sm)[TPB], int src, double* sv) {
+  static __device__ __forceinline__ void load(const T (*sm)[kSlots], int rec, double* sv) {
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
-      const double2 w = sm[q][src];
+      const double2 w = sm[q][rec];
       sv[2 * q] = w.x;
       sv[2 * q + 1] = w.y;
     }
   }
-  static constexpr int kFields = 2 * NQ;
 };
-template <int NF, int TPB>
-struct SymStage<NF, TPB, F2> {
-#if LDDMM_SYM_COMPACT
-  static constexpr int NQ = (NF + 3) / 4;  // float4 groups
+template <int NF, int TPB, int R>
+struct SymStage<NF, TPB, F2, R> {
+  static_assert(TPB % (2 * R) == 0, "tiles of whole chunks");
+  static constexpr int NQ = (NF + 1) / 2;
+  static constexpr int kSlots = TPB / 2;
+  static constexpr int kFields = 2 * NQ;
   using T = float4;
-  static __device__ __forceinline__ void store(T (*sm)[TPB], int t, const double* fl) {
-#pragma unroll
-    for (int q = 0; q < NQ; ++q)
-      sm[q][t] = make_float4((float)fl[4 * q], (float)fl[4 * q + 1], (float)fl[4 * q + 2], (float)fl[4 * q + 3]);
-  }
-  static __device__ __forceinline__ void load(const T (*sm)[TPB], int src, F2* sv) {
+  static __device__ __forceinline__ void store(T (*sm)[kSlots], int t, const double* fl) {
+    const int rec = t / (2 * R) * R + t % R, half = t / R & 1;
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
-      const float4 w = sm[q][src];
-      sv[4 * q] = f2(w.x, w.x);
-      sv[4 * q + 1] = f2(w.y, w.y);
-      sv[4 * q + 2] = f2(w.z, w.z);
-      sv[4 * q + 3] = f2(w.w, w.w);
+      float* w = reinterpret_cast<float*>(&sm[q][rec]) + half;
+      w[0] = (float)fl[2 * q];
+      w[2] = (float)fl[2 * q + 1];
     }
   }
-#else
-  static constexpr int NQ = (NF + 1) / 2;  // 16-byte units of two duplicated fields
-  using T = Unit<F2>;
-  static __device__ __forceinline__ void store(T (*sm)[TPB], int t, const double* fl) {
+  static __device__ __forceinline__ void load(const T (*sm)[kSlots], int rec, F2* sv) {
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
-      Unit<F2> w;
-      w.a = VT<F2>::dup(fl[2 * q]);
-      w.b = VT<F2>::dup(fl[2 * q + 1]);
-      sm[q][t] = w;
+      const float4 w = sm[q][rec];
+      sv[2 * q] = f2(w.x, w.y);
+      sv[2 * q + 1] = f2(w.z, w.w);
     }
   }
-  static __device__ __forceinline__ void load(const T (*sm)[TPB], int src, F2* sv) {
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      const Unit<F2> w = sm[q][src];
-      sv[2 * q] = w.a;
-      sv[2 * q + 1] = w.b;
-    }
+};
+// one step of the ring: `from` is the next lane of the R
+template <int R>
+__device__ __forceinline__ int ring_next(int lane) {
+  return ((lane + 1) & (R - 1)) | (lane & ~(R - 1));
+}
+__device__ __forceinline__ double ring_move(double v, int from) { return __shfl_sync(0xffffffffu, v, from); }
+__device__ __forceinline__ F2 ring_move(F2 v, int from) {
+  float a, b;
+  split(v, a, b);
+  return f2(__shfl_sync(0xffffffffu, a, from), __shfl_sync(0xffffffffu, b, from));
+}
+// SPLIT, after the last step: the warp's column sum of source `lane` of its chunk of 32
+__device__ __forceinline__ double ring_total(double v, int) { return v; }
+__device__ __forceinline__ float ring_total(F2 v, int lane) {
+  float a, b;
+  split(v, a, b);
+  const bool low = lane < 16;
+  return (low ? a : b) + __shfl_xor_sync(0xffffffffu, low ? b : a, 16);
+}
+// whole tiles, after the last step: the sums added to the accumulators of chunk `chunk`
+template <int TPB>
+__device__ __forceinline__ void ring_add(double (&acc)[TPB], double v, int chunk, int lane) {
+  acc[chunk * 32 + lane] += v;
+}
+template <int TPB>
+__device__ __forceinline__ void ring_add(float (&acc)[TPB], F2 v, int chunk, int lane) {
+  float a, b;
+  split(v, a, b);
+  acc[chunk * 64 + lane] += a;
+  acc[chunk * 64 + 32 + lane] += b;
+}
+// Column accumulators of a CTA of whole tiles: warps that take the same chunk at the same time have their own.
+template <typename V, int TPB>
+struct SymChunks {
+  static constexpr int kCount = TPB / (32 * VT<V>::kLanes);  // chunks of a tile
+  static constexpr int kCopies = (TPB / 32) / kCount;
+};
+
+// Row sums of a tile as the compensated values hold them: FP32 two targets to a value (the lanes of each added), FP64
+// one.
+template <typename V, int RT>
+struct SymRows;
+template <int RT>
+struct SymRows<double, RT> {
+  static constexpr int kValues = RT;
+  template <int NR>
+  static __device__ __forceinline__ double value(const double (&acc)[RT][NR], int h, int c) { return acc[h][c]; }
+};
+template <int RT>
+struct SymRows<F2, RT> {
+  static constexpr int kValues = (RT + 1) / 2;
+  template <int NR>
+  static __device__ __forceinline__ F2 value(const F2 (&acc)[RT][NR], int h, int c) {
+    return f2(VT<F2>::hsum(acc[2 * h][c]), 2 * h + 1 < RT ? VT<F2>::hsum(acc[2 * h + 1 < RT ? 2 * h + 1 : 0][c]) : 0.f);
   }
-#endif
-  static constexpr int kFields = 4 * ((NF + 3) / 4);  // size of the FP64 field buffer and of the operand array
 };
 
 struct SymPlan {
   int nblk = 0, TT = 0, C = 0, S = 0;
-  long long U = 0;
+  long long U = 0, wave = 1;  // units, resident CTAs
   size_t col_off = 0, ws_bytes = 0;
 };
 
@@ -146,7 +190,7 @@ inline SymPlan make_sym_plan(int64_t n, int nr, int nc, int ctas_per_sm, size_t 
   p.nblk = (int)((n + B - 1) / B);
   p.TT = (int)((n + TPB - 1) / TPB);
   p.U = Geo::row_off(p.nblk, p.TT);
-  const long long wave = (long long)device_sm_count() * (ctas_per_sm > 0 ? ctas_per_sm : 1);
+  const long long wave = p.wave = (long long)device_sm_count() * (ctas_per_sm > 0 ? ctas_per_sm : 1);
   // one resident wave of CTAs; up to half a wave more units run as one CTA each, so that no CTA takes two units while
   // others take one (forward step at 6,000 points, 576 units, 444 resident CTAs: 41.4 -> 31.7 us)
   p.C = (int)(2 * p.U < 3 * wave ? p.U : wave);
@@ -157,62 +201,81 @@ inline SymPlan make_sym_plan(int64_t n, int nr, int nc, int ctas_per_sm, size_t 
   return p;
 }
 
-// One chunk of 32 sources against the warp's targets; lane λ returns the warp's column sums of source λ in cs.
-template <class Op, int TPB, int RT, bool COL, class Fam, typename V>
-__device__ __forceinline__ void sym_chunk(const Frame& f,
-                                          const typename Op::template SymTgt<V> (&tgt)[RT / VT<V>::kLanes],
-                                          const typename SymStage<Op::NSS, TPB, V>::T (*sm)[TPB], int chunk,
-                                          V (&acc)[RT / VT<V>::kLanes][Op::NR],
-                                          typename VT<V>::Scalar (&cs)[Op::NC]) {
-  using St = SymStage<Op::NSS, TPB, V>;
-  constexpr int G = RT / VT<V>::kLanes;
-  const int lane = threadIdx.x & 31;
+// Unroll depth of the source loop: the op's for the Gaussian in FP32, where it has one.
+template <class Op, class = void>
+struct SymUnrollOf : std::integral_constant<int, kSymUnroll> {};
+template <class Op>
+struct SymUnrollOf<Op, std::void_t<decltype(Op::kSymUnrollG)>> : std::integral_constant<int, Op::kSymUnrollG> {};
+template <class Op, class Fam, typename V>
+constexpr int kSymSteps =
+    std::is_same<V, F2>::value && std::is_same<Fam, Gauss>::value ? SymUnrollOf<Op>::value : kSymUnroll;
+
+// Ops whose column terms of a step are added up before they join the ring (Laplacian, whole tiles): a column sum of 4
+// targets is a chain of 128 additions without that, and the second-order adjoint's error grew with it (pa-increment at
+// 40,962 points 1.06 of what 2 targets to a packed value gave with 3 targets per thread, 0.75 with this and 4; 1917 and
+// 1922 us).
+template <class Op, class = void>
+struct SymFresh : std::false_type {};
+template <class Op>
+struct SymFresh<Op, std::void_t<decltype(Op::kSymFresh)>> : std::bool_constant<Op::kSymFresh> {};
+
+// One chunk of sources against the warp's targets; the column sums are back where they started in col.
+template <class Op, int TPB, int RT, int R, bool COL, class Fam, typename V>
+__device__ __forceinline__ void sym_chunk(const Frame& f, const typename Op::template SymTgt<V> (&tgt)[RT],
+                                          const typename SymStage<Op::NSS, TPB, V, R>::T (*sm)[SymStage<Op::NSS, TPB, V, R>::kSlots],
+                                          int chunk, V (&acc)[RT][Op::NR], V (&col)[Op::NC]) {
+  using St = SymStage<Op::NSS, TPB, V, R>;
+  constexpr bool FRESH = SymFresh<Op>::value && std::is_same<V, F2>::value && R == 32 && !std::is_same<Fam, Gauss>::value;
+  constexpr int kUnroll = kSymSteps<Op, Fam, V>;
+  const int lane = threadIdx.x & 31, from = ring_next<R>(lane);
 #pragma unroll
-  for (int c = 0; c < Op::NC; ++c) cs[c] = 0;
-#pragma unroll kSymUnroll
-  for (int s = 0; s < 32; ++s) {
-    const int src = chunk * 32 + ((lane + s) & 31);
+  for (int c = 0; c < Op::NC; ++c) col[c] = VT<V>::zero();
+#pragma unroll kUnroll
+  for (int s = 0; s < R; ++s) {
     V sv[St::kFields];
-    St::load(sm, src, sv);
-    if constexpr (COL) {
-      V col[Op::NC];
+    St::load(sm, chunk * R + ((lane + s) & (R - 1)), sv);
+    if constexpr (COL && FRESH) {
+      V step[Op::NC];
 #pragma unroll
-      for (int c = 0; c < Op::NC; ++c) col[c] = VT<V>::first(cs[c]);
+      for (int c = 0; c < Op::NC; ++c) step[c] = VT<V>::zero();
 #pragma unroll
-      for (int g = 0; g < G; ++g) Op::template pair_sym<true, Fam, V>(f, tgt[g], sv, acc[g], col);
+      for (int g = 0; g < RT; ++g) Op::template pair_sym<COL, Fam, V>(f, tgt[g], sv, acc[g], step);
 #pragma unroll
-      for (int c = 0; c < Op::NC; ++c) cs[c] = __shfl_sync(0xffffffffu, VT<V>::hsum(col[c]), (lane + 1) & 31);
+      for (int c = 0; c < Op::NC; ++c) col[c] = ring_move(col[c] + step[c], from);
     } else {
 #pragma unroll
-      for (int g = 0; g < G; ++g) Op::template pair_sym<false, Fam, V>(f, tgt[g], sv, acc[g], nullptr);
+      for (int g = 0; g < RT; ++g) Op::template pair_sym<COL, Fam, V>(f, tgt[g], sv, acc[g], col);
+      if constexpr (COL) {
+#pragma unroll
+        for (int c = 0; c < Op::NC; ++c) col[c] = ring_move(col[c], from);
+      }
     }
   }
 }
 
 template <class Op, int TPB, int RT, bool COL, class Fam, typename V>
-__device__ __forceinline__ void sym_tile(const Frame& f,
-                                         const typename Op::template SymTgt<V> (&tgt)[RT / VT<V>::kLanes],
-                                         const typename SymStage<Op::NSS, TPB, V>::T (*sm)[TPB],
-                                         typename VT<V>::Scalar (*colacc)[TPB],
-                                         V (&acc)[RT / VT<V>::kLanes][Op::NR]) {
-  constexpr int W = TPB / 32;
+__device__ __forceinline__ void sym_tile(const Frame& f, const typename Op::template SymTgt<V> (&tgt)[RT],
+                                         const typename SymStage<Op::NSS, TPB, V, 32>::T (*sm)[SymStage<Op::NSS, TPB, V, 32>::kSlots],
+                                         typename VT<V>::Scalar (*colacc)[Op::NC][TPB], V (&acc)[RT][Op::NR]) {
+  using Ch = SymChunks<V, TPB>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll 1
-  for (int ph = 0; ph < W; ++ph) {
-    const int chunk = (warp + ph) % W;
-    typename VT<V>::Scalar cs[Op::NC];
-    sym_chunk<Op, TPB, RT, COL, Fam, V>(f, tgt, sm, chunk, acc, cs);
+  for (int ph = 0; ph < Ch::kCount; ++ph) {
+    const int chunk = (warp + ph) % Ch::kCount;
+    V col[Op::NC];
+    sym_chunk<Op, TPB, RT, 32, COL, Fam, V>(f, tgt, sm, chunk, acc, col);
     if constexpr (COL) {
 #pragma unroll
-      for (int c = 0; c < Op::NC; ++c) colacc[c][chunk * 32 + lane] += cs[c];
+      for (int c = 0; c < Op::NC; ++c) ring_add<TPB>(colacc[warp / Ch::kCount][c], col[c], chunk, lane);
     }
     __syncthreads();  // the next phase hands this chunk (and its column accumulators) to another warp
   }
 }
 
-// minimum resident CTAs per SM: the op's for FP32; no register cap in FP64
-template <class Op, typename V>
-constexpr int kSymCtas = std::is_same<V, F2>::value ? Op::kSymMinCtas : 1;
+// minimum resident CTAs per SM: the op's for FP32, 2 (255 registers) from 6 targets per thread on; no register cap in
+// FP64
+template <class Op, typename V, int RT>
+constexpr int kSymCtas = !std::is_same<V, F2>::value ? 1 : RT >= 6 ? 2 : Op::kSymMinCtas;
 
 // SPLIT (small point sets): the warps of a CTA share its 32 RT targets and take one chunk of every tile each, instead
 // of TPB RT targets and all chunks in turn. A unit is TPB / 32 times shorter and the triangle has that many times more
@@ -220,19 +283,22 @@ constexpr int kSymCtas = std::is_same<V, F2>::value ? Op::kSymMinCtas : 1;
 // from 128 pair evaluations to 32 and its 462 units occupy every SM. The warps' row sums meet in shared memory at the
 // end of a segment; a chunk's column sums are one warp's and go straight to the column partial.
 template <class Op, int TPB, int RT, class Fam, typename V, bool SPLIT>
-__global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
+__global__ void __launch_bounds__(TPB, kSymCtas<Op, V, RT>)
     pairs_kernel_sym(const typename Op::Params P, int n, int nblk, int TT, long long U, int C,
                      typename VT<V>::Partial* __restrict__ row_ws, typename VT<V>::Scalar* __restrict__ col_ws) {
-  using St = SymStage<Op::NSS, TPB, V>;
-  constexpr int L = VT<V>::kLanes, G = RT / L, NR = Op::NR, NC = Op::NC, W = TPB / 32;
+  constexpr int R = kSymRing<V, SPLIT>;
+  using St = SymStage<Op::NSS, TPB, V, R>;
+  using Rows = SymRows<V, RT>;
+  constexpr int NR = Op::NR, NC = Op::NC, W = TPB / 32, H = Rows::kValues, L = VT<V>::kLanes;
   constexpr int TW = SPLIT ? 32 : TPB;  // targets a lane-group index apart
   constexpr int B = TW * RT;
   using Geo = SymGeom<TPB, B>;
   constexpr int K = Geo::K;
-  static_assert(TPB % 32 == 0 && RT % L == 0, "launch shape");
-  __shared__ typename St::T sm[St::NQ][TPB];
-  __shared__ typename VT<V>::Scalar colacc[SPLIT ? 1 : NC][TPB];
-  // compensated row sums of the segment, one private column per thread (G * NR * Comp<V>::kWords rows of TPB): dynamic
+  static_assert(TPB % 32 == 0, "launch shape");
+  __shared__ typename St::T sm[St::NQ][St::kSlots];
+  constexpr int kCopies = SymChunks<V, TPB>::kCopies;
+  __shared__ typename VT<V>::Scalar colacc[SPLIT ? 1 : kCopies][NC][SPLIT ? 1 : TPB];
+  // compensated row sums of the segment, one private column per thread (H * NR * Comp<V>::kWords rows of TPB): dynamic
   // shared memory, so that 8 targets per thread may take more than the 48 KiB of static shared memory
   extern __shared__ __align__(16) unsigned char sym_dyn_smem[];
   V (*cs)[TPB] = reinterpret_cast<V (*)[TPB]>(sym_dyn_smem);
@@ -259,19 +325,20 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
 #pragma unroll
       for (int c = 0; c < 3; ++c) org[c] = o[c];
     }
-    typename Op::template SymTgt<V> tgt[G];
+    typename Op::template SymTgt<V> tgt[RT];
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      const int i0 = base + (g * L) * TW, i1 = base + (g * L + L - 1) * TW;
+    for (int g = 0; g < RT; ++g) {
+      const int k = base + g * TW, kc = k < n ? k : n - 1;
       if constexpr (SPLIT)
-        Op::template load_target_sym<V>(with_origin(P, org), i0 < n ? i0 : n - 1, i1 < n ? i1 : n - 1, i0 < n, i1 < n,
-                                        tgt[g]);
+        Op::template load_target_sym<V>(with_origin(P, org), kc, kc, k < n, k < n, tgt[g]);
       else
-        Op::template load_target_sym<V>(P, i0 < n ? i0 : n - 1, i1 < n ? i1 : n - 1, i0 < n, i1 < n, tgt[g]);
+        Op::template load_target_sym<V>(P, kc, kc, k < n, k < n, tgt[g]);
+    }
+#pragma unroll
+    for (int c = 0; c < H * NR; ++c) {
       Comp<V> z;
       z.zero();
-#pragma unroll
-      for (int c = 0; c < NR; ++c) z.template store<TPB>(cs, g * NR + c, threadIdx.x);
+      z.template store<TPB>(cs, c, threadIdx.x);
     }
 
     for (int tt = t0; tt < t1; ++tt) {
@@ -291,13 +358,15 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
         St::store(sm, threadIdx.x, fl);
         if constexpr (!SPLIT) {
 #pragma unroll
-          for (int c = 0; c < NC; ++c) colacc[c][threadIdx.x] = 0;
+          for (int w = 0; w < kCopies; ++w)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) colacc[w][c][threadIdx.x] = 0;
         }
       }
       __syncthreads();
-      V acc[G][NR];
+      V acc[RT][NR];
 #pragma unroll
-      for (int g = 0; g < G; ++g)
+      for (int g = 0; g < RT; ++g)
 #pragma unroll
         for (int c = 0; c < NR; ++c) acc[g][c] = VT<V>::zero();
       // column partial of (row block i, tile t), field stride K. Held over the tile, except where the six sums and the
@@ -310,13 +379,13 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
       constexpr bool kHeld = SPLIT || NC < 6 || VT<V>::kLanes == 1 || !std::is_same<Fam, Laplacian4>::value;
       const size_t cb = kHeld ? column_base() : 0;
       if constexpr (SPLIT) {
-        typename VT<V>::Scalar col[NC];
+        V col[NC];
         if (diag) {
-          sym_chunk<Op, TPB, RT, false, Fam, V>(f, tgt, sm, warp, acc, col);
+          sym_chunk<Op, TPB, RT, R, false, Fam, V>(f, tgt, sm, warp, acc, col);
         } else {
-          sym_chunk<Op, TPB, RT, true, Fam, V>(f, tgt, sm, warp, acc, col);
+          sym_chunk<Op, TPB, RT, R, true, Fam, V>(f, tgt, sm, warp, acc, col);
 #pragma unroll
-          for (int c = 0; c < NC; ++c) col_ws[cb + (size_t)c * K] = col[c];
+          for (int c = 0; c < NC; ++c) col_ws[cb + (size_t)c * K] = ring_total(col[c], lane);
         }
       } else if (diag) {
         sym_tile<Op, TPB, RT, false, Fam, V>(f, tgt, sm, colacc, acc);
@@ -324,19 +393,24 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
         sym_tile<Op, TPB, RT, true, Fam, V>(f, tgt, sm, colacc, acc);
       }
 #pragma unroll
-      for (int g = 0; g < G; ++g)
+      for (int h = 0; h < H; ++h)
 #pragma unroll
         for (int c = 0; c < NR; ++c) {
           Comp<V> m;
-          m.template load<TPB>(cs, g * NR + c, threadIdx.x);
-          m.merge(acc[g][c]);
-          m.template store<TPB>(cs, g * NR + c, threadIdx.x);
+          m.template load<TPB>(cs, h * NR + c, threadIdx.x);
+          m.merge(Rows::value(acc, h, c));
+          m.template store<TPB>(cs, h * NR + c, threadIdx.x);
         }
       if constexpr (SPLIT) {
         __syncthreads();  // every warp has read the tile and left its row sums
       } else if (!diag) {
 #pragma unroll
-        for (int c = 0; c < NC; ++c) col_ws[(kHeld ? cb : column_base()) + (size_t)c * K] = colacc[c][threadIdx.x];
+        for (int c = 0; c < NC; ++c) {
+          typename VT<V>::Scalar v = colacc[0][c][threadIdx.x];
+#pragma unroll
+          for (int w = 1; w < kCopies; ++w) v += colacc[w][c][threadIdx.x];
+          col_ws[(kHeld ? cb : column_base()) + (size_t)c * K] = v;
+        }
       }
       // (not SPLIT) the last phase barrier of sym_tile orders every read of sm and colacc before the next staging
     }
@@ -345,7 +419,7 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
     if constexpr (SPLIT) {
       // the block's row sums: field c of the lanes' targets by warp c mod W, over the W warps in order
 #pragma unroll
-      for (int g = 0; g < G; ++g)
+      for (int h = 0; h < H; ++h)
         for (int c = warp; c < NR; c += W) {
           double sum[L];
 #pragma unroll
@@ -353,28 +427,29 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V>)
 #pragma unroll
           for (int w = 0; w < W; ++w) {
             Comp<V> m;
-            m.template load<TPB>(cs, g * NR + c, w * 32 + lane);
+            m.template load<TPB>(cs, h * NR + c, w * 32 + lane);
 #pragma unroll
             for (int k = 0; k < L; ++k) sum[k] += partial_value(m.partial(k));
           }
 #pragma unroll
           for (int k = 0; k < L; ++k) {
-            const int idx = base + (g * L + k) * TW;
-            if (idx < n) row_ws[((size_t)slot * NR + c) * (size_t)n + idx] = VT<V>::to_partial(sum[k]);
+            const int idx = base + (h * L + k) * TW;
+            if (h * L + k < RT && idx < n)
+              row_ws[((size_t)slot * NR + c) * (size_t)n + idx] = VT<V>::to_partial(sum[k]);
           }
         }
       __syncthreads();  // the next segment clears the sums
     } else {
 #pragma unroll
-      for (int g = 0; g < G; ++g)
+      for (int h = 0; h < H; ++h)
 #pragma unroll
         for (int k = 0; k < L; ++k) {
-          const int idx = base + (g * L + k) * TW;
-          if (idx < n) {
+          const int idx = base + (h * L + k) * TW;
+          if (h * L + k < RT && idx < n) {
 #pragma unroll
             for (int c = 0; c < NR; ++c) {
               Comp<V> m;
-              m.template load<TPB>(cs, g * NR + c, threadIdx.x);
+              m.template load<TPB>(cs, h * NR + c, threadIdx.x);
               row_ws[((size_t)slot * NR + c) * (size_t)n + idx] = m.partial(k);
             }
           }
@@ -430,7 +505,7 @@ inline int sym_finalize_tpp(const SymPlan& p) { return finalize_tpp(p.S + p.nblk
 // Dynamic shared memory of pairs_kernel_sym (its compensated row sums).
 template <class Op, int TPB, int RT, typename V>
 constexpr size_t sym_dyn_smem_bytes() {
-  return (size_t)(RT / VT<V>::kLanes) * Op::NR * Comp<V>::kWords * TPB * sizeof(V);
+  return (size_t)SymRows<V, RT>::kValues * Op::NR * Comp<V>::kWords * TPB * sizeof(V);
 }
 
 // Declare the kernel's dynamic shared memory, once per device (the attribute belongs to the device's context):
@@ -496,11 +571,12 @@ inline int run_pairs_sym(const typename Op::Params& P, int64_t n, void* ws, size
 }
 
 
-// Launch shapes. Each symmetric op names its rule (Op::Shape): the FP32 lines between 2, 4 and 8 targets per thread
-// with the split and the shape without it, and the FP64 shape (launch_config.cuh has the measurements).
-template <int SPLIT2_N, int SPLIT4_N, int SPLIT8_N, int SPLIT4_N_LAP, int RT, int RT_LAP, int TPB64, int RT64>
+// Launch shapes. Each symmetric op names its rule (Op::Shape): up to where 4 targets per thread with the split are used
+// in FP32 (8 follow), the targets per thread of whole tiles (0: another kernel has them), each for the Gaussian and the
+// Laplacian, and the FP64 shape of whole tiles (launch_config.cuh has the measurements).
+template <int SPLIT4_N, int SPLIT4_N_LAP, int RT, int RT_LAP, int TPB64, int RT64>
 struct SymRule {
-  static constexpr int64_t kSplit2 = SPLIT2_N, kSplit4 = SPLIT4_N, kSplit8 = SPLIT8_N, kSplit4Lap = SPLIT4_N_LAP;
+  static constexpr int64_t kSplit4 = SPLIT4_N, kSplit4Lap = SPLIT4_N_LAP;
   static constexpr int kRt = RT, kRtLap = RT_LAP, kTpb64 = TPB64, kRt64 = RT64;
 };
 template <int TPB, int RT, bool SPLIT>
@@ -508,6 +584,17 @@ struct SymShape {
   static constexpr int kTpb = TPB, kRt = RT;
   static constexpr bool kSplit = SPLIT;
 };
+
+// Whether the units of a plan fill its resident CTAs: at least 95% of the rounds that they take.
+inline bool sym_full(const SymPlan& p) {
+  const long long rounds = (p.U + p.wave - 1) / p.wave;
+  return 20 * p.U >= 19 * rounds * p.wave;
+}
+// Whole tiles or the split, in FP32: see kSplitN.
+template <class PlanFn>
+inline bool sym_whole(int64_t n, PlanFn plan) {
+  return n > kSplitN || (n > kWholeN && sym_full(plan()));
+}
 
 // fn(SymShape{}) with the shape of n points.
 template <class Op, typename V, class Fam, class Fn>
@@ -519,12 +606,17 @@ inline auto sym_shape(int64_t n, Fn fn) {
     if (n <= (kG ? kSplit2N64 : kSplit2N64Lap)) return fn(SymShape<128, 2, true>{});
     return fn(SymShape<R::kTpb64, R::kRt64, false>{});
   } else {
-    if (n <= R::kSplit2) return fn(SymShape<128, 2, true>{});
-    if (n <= (kG ? R::kSplit4 : R::kSplit4Lap)) return fn(SymShape<128, 4, true>{});
-    if constexpr (kG && R::kSplit8 > R::kSplit4) {
-      if (n <= R::kSplit8) return fn(SymShape<128, 8, true>{});
+    constexpr int kRt = kG ? R::kRt : R::kRtLap;
+    constexpr int64_t kSplit4 = kG ? R::kSplit4 : R::kSplit4Lap;
+    if (n <= kSplit2N) return fn(SymShape<128, 2, true>{});
+    if constexpr (kRt > 0) {
+      if (sym_whole(n, [&] { return sym_plan<Op, 128, kRt, Fam, V, false>(n); }))
+        return fn(SymShape<128, kRt, false>{});
     }
-    return fn(SymShape<128, kG ? R::kRt : R::kRtLap, false>{});
+    if constexpr (kSplit4 < kSplitN) {
+      if (n > kSplit4) return fn(SymShape<128, 8, true>{});
+    }
+    return fn(SymShape<128, 4, true>{});
   }
 }
 
@@ -561,20 +653,24 @@ template <class Op, typename V>
 inline size_t sym_scratch(int64_t n, int family) {
   return by_family(family, [&](auto fam) { return sym_scratch_fam<Op, V, decltype(fam)>(n); });
 }
-// Scratch for every point count up to n: the largest of each shape's range.
-template <class Op, typename V>
-inline size_t sym_scratch_upto(int64_t n) {
-  using R = typename Op::Shape;
+// Scratch for every point count up to n: the largest of the shapes at the end of their ranges. scratch(k, family): that
+// of one launch.
+template <class Op, typename V, class Scratch>
+inline size_t sym_largest(int64_t n, Scratch scratch) {
   size_t b = 0;
-  for (const int64_t k : {R::kSplit2, R::kSplit4, R::kSplit8, R::kSplit4Lap, kSplit1N64, kSplit2N64, kSplit2N64Lap,
+  for (const int64_t k : {kSplit2N, kSplit4N, kWholeN, kSplitN, kSplit1N64, kSplit2N64, kSplit2N64Lap,
                           sym_max_n<Op, V>(), n}) {
     if (k > n || !sym_takes<Op, V>(k)) continue;
     for (const int family : {(int)kGauss, (int)kLaplacian0, (int)kLaplacianMax}) {
-      const size_t v = sym_scratch<Op, V>(k, family);
+      const size_t v = scratch(k, family);
       b = v > b ? v : b;
     }
   }
   return b;
+}
+template <class Op, typename V>
+inline size_t sym_scratch_upto(int64_t n) {
+  return sym_largest<Op, V>(n, [](int64_t k, int family) { return sym_scratch<Op, V>(k, family); });
 }
 
 template <class Op, typename V, class Fam>
@@ -607,33 +703,26 @@ inline int run_sym(const typename Op::Params& P, int64_t n, void* ws, size_t wsb
 // point i), payload(P, i, double* p), finalize_sym(P, i, row, col).
 // ---------------------------------------------------------------------------------------------------------
 template <class Op, int TPB, int RT, bool COL, bool X>
-__device__ __forceinline__ void symx_tile(const F2 (&yt)[RT / 2][3], const F2 (&tp)[RT / 2][Op::NP],
-                                          const typename SymStage<4 + Op::NP, TPB, F2>::T (*sm)[TPB],
-                                          float (*colacc)[TPB], F2 (&acc)[RT / 2][Op::NP]) {
-  using St = SymStage<4 + Op::NP, TPB, F2>;
-  constexpr int G = RT / 2, NP = Op::NP, W = TPB / 32;
+__device__ __forceinline__ void symx_tile(const F2 (&yt)[RT][3], const F2 (&tp)[RT][Op::NP],
+                                          const float4 (*sm)[TPB / 2], float (*colacc)[Op::NP][TPB],
+                                          F2 (&acc)[RT][Op::NP]) {
+  using St = SymStage<4 + Op::NP, TPB, F2, 32>;
+  using Ch = SymChunks<F2, TPB>;
+  constexpr int NP = Op::NP;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll 1
-  for (int ph = 0; ph < W; ++ph) {
-    const int chunk = (warp + ph) % W;
-    float cs[NP];
+  for (int ph = 0; ph < Ch::kCount; ++ph) {
+    const int chunk = (warp + ph) % Ch::kCount;
+    const int from = ring_next<32>(lane);
+    F2 col[NP];
 #pragma unroll
-    for (int c = 0; c < NP; ++c) cs[c] = 0.f;
+    for (int c = 0; c < NP; ++c) col[c] = VT<F2>::zero();
 #pragma unroll kSymxUnroll
     for (int s = 0; s < 32; ++s) {
-      const int src = chunk * 32 + ((lane + s) & 31);
       F2 sv[St::kFields];
-      St::load(sm, src, sv);
-      F2 col[NP], col2[NP];
-      if constexpr (COL) {
+      St::load(sm, chunk * 32 + ((lane + s) & 31), sv);
 #pragma unroll
-        for (int c = 0; c < NP; ++c) {
-          col[c] = f2(cs[c], 0.f);
-          col2[c] = VT<F2>::zero();
-        }
-      }
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
+      for (int g = 0; g < RT; ++g) {
         F2 arg;
         if constexpr (X) {
           arg = fma(yt[g][2], sv[2], sv[3]);  // |x|^2 - 2 y.x
@@ -647,28 +736,18 @@ __device__ __forceinline__ void symx_tile(const F2 (&yt)[RT / 2][3], const F2 (&
 #pragma unroll
         for (int c = 0; c < NP; ++c) acc[g][c] = fma(e, sv[4 + c], acc[g][c]);
         if constexpr (COL) {
-          if (LDDMM_SYMX_COL_SPLIT != 0 && (g & 1)) {  // resolved at compile time (the loop is unrolled)
 #pragma unroll
-            for (int c = 0; c < NP; ++c) col2[c] = fma(e, tp[g][c], col2[c]);
-          } else {
-#pragma unroll
-            for (int c = 0; c < NP; ++c) col[c] = fma(e, tp[g][c], col[c]);
-          }
+          for (int c = 0; c < NP; ++c) col[c] = fma(e, tp[g][c], col[c]);
         }
       }
       if constexpr (COL) {
 #pragma unroll
-        for (int c = 0; c < NP; ++c) {
-          if constexpr (LDDMM_SYMX_COL_SPLIT != 0) col[c] = col[c] + col2[c];
-          float lo, hi;
-          split(col[c], lo, hi);
-          cs[c] = __shfl_sync(0xffffffffu, lo + hi, (lane + 1) & 31);
-        }
+        for (int c = 0; c < NP; ++c) col[c] = ring_move(col[c], from);
       }
     }
     if constexpr (COL) {
 #pragma unroll
-      for (int c = 0; c < NP; ++c) colacc[c][chunk * 32 + lane] += cs[c];
+      for (int c = 0; c < NP; ++c) ring_add<TPB>(colacc[warp / Ch::kCount][c], col[c], chunk, lane);
     }
     __syncthreads();  // the next phase hands this chunk (and its column accumulators) to another warp
   }
@@ -678,16 +757,18 @@ template <class Op, int TPB, int RT>
 __global__ void __launch_bounds__(TPB, Op::kSymMinCtas)
     pairs_kernel_symx(const typename Op::Params P, int n, int nblk, int TT, long long U, int C,
                       float2* __restrict__ row_ws, float* __restrict__ col_ws) {
-  using St = SymStage<4 + Op::NP, TPB, F2>;
-  constexpr int L = 2, G = RT / L, NP = Op::NP;
+  using St = SymStage<4 + Op::NP, TPB, F2, 32>;
+  using Rows = SymRows<F2, RT>;
+  constexpr int NP = Op::NP, H = Rows::kValues;
   constexpr int B = TPB * RT;
   using Geo = SymGeom<TPB, B>;
-  static_assert(TPB % 32 == 0 && RT % L == 0, "launch shape");
-  __shared__ typename St::T sm[St::NQ][TPB];
-  __shared__ float colacc[NP][TPB];
+  static_assert(TPB % 32 == 0, "launch shape");
+  __shared__ float4 sm[St::NQ][TPB / 2];
+  constexpr int kCopies = SymChunks<F2, TPB>::kCopies;
+  __shared__ float colacc[kCopies][NP][TPB];
   __shared__ float red[6][TPB / 32];
   extern __shared__ __align__(16) unsigned char sym_dyn_smem[];
-  F2 (*cs)[TPB] = reinterpret_cast<F2 (*)[TPB]>(sym_dyn_smem);  // compensated row sums, G * NP * 2 rows
+  F2 (*cs)[TPB] = reinterpret_cast<F2 (*)[TPB]>(sym_dyn_smem);  // compensated row sums, H * NP * 2 rows
   const Frame& f = P.f;
   const double fo[3] = {f.o0, f.o1, f.o2};
   chain_wait();
@@ -728,33 +809,29 @@ __global__ void __launch_bounds__(TPB, Op::kSymMinCtas)
     }
     const bool expand = rb2 <= kExpandR2;  // uniform over the CTA
 
-    F2 yt[G][3], tp[G][NP];
+    F2 yt[RT][3], tp[RT][NP];
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      const int k0 = base + (g * L) * TPB, k1 = base + (g * L + 1) * TPB;
-      double y0[3], y1[3], p0[NP], p1[NP];
-      Op::point(P, k0 < n ? k0 : n - 1, y0);
-      Op::point(P, k1 < n ? k1 : n - 1, y1);
-      Op::payload(P, k0 < n ? k0 : n - 1, p0);
-      Op::payload(P, k1 < n ? k1 : n - 1, p1);
-      double q0 = 0.0, q1 = 0.0;
+    for (int g = 0; g < RT; ++g) {
+      const int k = base + g * TPB;
+      double y[3], pay[NP], q = 0.0;
+      Op::point(P, k < n ? k : n - 1, y);
+      Op::payload(P, k < n ? k : n - 1, pay);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const float r0 = (float)((y0[c] - fo[c]) * f.s - (double)ob[c]);
-        const float r1 = (float)((y1[c] - fo[c]) * f.s - (double)ob[c]);
-        yt[g][c] = f2(r0, r1);
-        q0 += (double)r0 * (double)r0;
-        q1 += (double)r1 * (double)r1;
+        const float r = (float)((y[c] - fo[c]) * f.s - (double)ob[c]);
+        yt[g][c] = f2(r, r);
+        q += (double)r * (double)r;
       }
       // column payload: f_k a_k (expanded form) or a_k; padded targets carry none
-      const double f0 = k0 < n ? (expand ? exp2(-q0) : 1.0) : 0.0;
-      const double f1 = k1 < n ? (expand ? exp2(-q1) : 1.0) : 0.0;
+      const double fk = k < n ? (expand ? exp2(-q) : 1.0) : 0.0;
 #pragma unroll
-      for (int c = 0; c < NP; ++c) tp[g][c] = f2((float)(f0 * p0[c]), (float)(f1 * p1[c]));
+      for (int c = 0; c < NP; ++c) tp[g][c] = VT<F2>::dup(fk * pay[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < H * NP; ++c) {
       Comp<F2> z;
       z.zero();
-#pragma unroll
-      for (int c = 0; c < NP; ++c) z.template store<TPB>(cs, g * NP + c, threadIdx.x);
+      z.template store<TPB>(cs, c, threadIdx.x);
     }
 
     for (int tt = t0; tt < t1; ++tt) {
@@ -779,12 +856,14 @@ __global__ void __launch_bounds__(TPB, Op::kSymMinCtas)
         }
         St::store(sm, threadIdx.x, fl);
 #pragma unroll
-        for (int c = 0; c < NP; ++c) colacc[c][threadIdx.x] = 0.f;
+        for (int w = 0; w < kCopies; ++w)
+#pragma unroll
+          for (int c = 0; c < NP; ++c) colacc[w][c][threadIdx.x] = 0.f;
       }
       __syncthreads();
-      F2 acc[G][NP];
+      F2 acc[RT][NP];
 #pragma unroll
-      for (int g = 0; g < G; ++g)
+      for (int g = 0; g < RT; ++g)
 #pragma unroll
         for (int c = 0; c < NP; ++c) acc[g][c] = VT<F2>::zero();
       if (expand) {
@@ -799,47 +878,47 @@ __global__ void __launch_bounds__(TPB, Op::kSymMinCtas)
           symx_tile<Op, TPB, RT, true, false>(yt, tp, sm, colacc, acc);
       }
 #pragma unroll
-      for (int g = 0; g < G; ++g)
+      for (int h = 0; h < H; ++h)
 #pragma unroll
         for (int c = 0; c < NP; ++c) {
           Comp<F2> m;
-          m.template load<TPB>(cs, g * NP + c, threadIdx.x);
-          m.merge(acc[g][c]);
-          m.template store<TPB>(cs, g * NP + c, threadIdx.x);
+          m.template load<TPB>(cs, h * NP + c, threadIdx.x);
+          m.merge(Rows::value(acc, h, c));
+          m.template store<TPB>(cs, h * NP + c, threadIdx.x);
         }
       if (!diag) {
         const int j = t / RT;
         const size_t cb = (size_t)(Geo::col_first(j) + i) * NP * B + (size_t)(t - RT * j) * TPB + threadIdx.x;
 #pragma unroll
-        for (int c = 0; c < NP; ++c) col_ws[cb + (size_t)c * B] = colacc[c][threadIdx.x];
+        for (int c = 0; c < NP; ++c) {
+          float v = colacc[0][c][threadIdx.x];
+#pragma unroll
+          for (int w = 1; w < kCopies; ++w) v += colacc[w][c][threadIdx.x];
+          col_ws[cb + (size_t)c * B] = v;
+        }
       }
       // the last phase barrier of symx_tile orders every read of sm and colacc before the next tile's staging
     }
 
 #pragma unroll
-    for (int g = 0; g < G; ++g)
+    for (int g = 0; g < RT; ++g) {
+      const int idx = base + g * TPB;
+      if (idx < n) {
+        double y2 = 0.0;
 #pragma unroll
-      for (int k = 0; k < L; ++k) {
-        const int idx = base + (g * L + k) * TPB;
-        if (idx < n) {
-          double y2 = 0.0;
+        for (int c = 0; c < 3; ++c) {
+          const double yr = VT<F2>::lane(yt[g][c], 0);
+          y2 += yr * yr;
+        }
+        const double fac = expand ? exp2(-y2) : 1.0;
 #pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            const double yr = VT<F2>::lane(yt[g][c], k);
-            y2 += yr * yr;
-          }
-          const double fac = expand ? exp2(-y2) : 1.0;
-#pragma unroll
-          for (int c = 0; c < NP; ++c) {
-            Comp<F2> m;
-            m.template load<TPB>(cs, g * NP + c, threadIdx.x);
-            const float2 pp = m.partial(k);
-            const double w = ((double)pp.x + (double)pp.y) * fac;
-            const float h = (float)w;
-            row_ws[((size_t)slot * NP + c) * (size_t)n + idx] = make_float2(h, (float)(w - (double)h));
-          }
+        for (int c = 0; c < NP; ++c) {
+          Comp<F2> m;
+          m.template load<TPB>(cs, (g / 2) * NP + c, threadIdx.x);
+          row_ws[((size_t)slot * NP + c) * (size_t)n + idx] = VT<F2>::to_partial(partial_value(m.partial(g & 1)) * fac);
         }
       }
+    }
     u += t1 - t0;
     ++i;
   }
@@ -847,7 +926,7 @@ __global__ void __launch_bounds__(TPB, Op::kSymMinCtas)
 
 template <class Op, int TPB, int RT>
 constexpr size_t symx_dyn_smem_bytes() {
-  return (size_t)(RT / 2) * Op::NP * 2 * TPB * sizeof(F2);
+  return (size_t)SymRows<F2, RT>::kValues * Op::NP * Comp<F2>::kWords * TPB * sizeof(F2);
 }
 
 template <class Op, int TPB, int RT>
@@ -882,15 +961,16 @@ inline int symx_ctas_per_sm() {
 }
 
 template <class Op, int TPB, int RT>
-inline size_t symx_ws_bytes(int64_t n) {
-  return make_sym_plan<TPB, TPB * RT>(n, Op::NP, Op::NP, symx_ctas_per_sm<Op, TPB, RT>(), sizeof(float2), sizeof(float)).ws_bytes;
+inline SymPlan symx_plan(int64_t n) {
+  return make_sym_plan<TPB, TPB * RT>(n, Op::NP, Op::NP, symx_ctas_per_sm<Op, TPB, RT>(), sizeof(float2),
+                                      sizeof(float));
 }
 
 template <class Op, int TPB, int RT>
 inline int run_pairs_symx(const typename Op::Params& P, int64_t n, void* ws, size_t ws_bytes, cudaStream_t stream) {
   if (n <= 0) return kOk;
   if (n > INT32_MAX / 4) return kInvalidArgument;
-  const SymPlan plan = make_sym_plan<TPB, TPB * RT>(n, Op::NP, Op::NP, symx_ctas_per_sm<Op, TPB, RT>(), sizeof(float2), sizeof(float));
+  const SymPlan plan = symx_plan<Op, TPB, RT>(n);
   if (plan.ws_bytes > ws_bytes) return kWorkspaceTooSmall;
   if (ws == nullptr) return kInvalidArgument;
   if (!symx_prepare<Op, TPB, RT>()) return kLaunchFailure;
@@ -906,22 +986,23 @@ inline int run_pairs_symx(const typename Op::Params& P, int64_t n, void* ws, siz
 
 // K(x, x) a: the FP32 Gaussian sum of a set beyond the split shapes runs the expanded form (OpX), everything else the
 // difference form (OpD).
+template <class OpX, typename V>
+inline bool ksym_expanded(int64_t n, int family) {
+  return std::is_same<V, F2>::value && family == kGauss && n > kSplitN;
+}
 template <class OpX, class OpD, typename V>
 inline int run_ksym(const typename OpD::Params& P, int64_t n, void* ws, size_t wsb, cudaStream_t st) {
-  if (std::is_same<V, F2>::value && P.f.family == kGauss && n > OpD::Shape::kSplit8)
-    return run_pairs_symx<OpX, kTpbKSym, kRtKSym>(P, n, ws, wsb, st);
+  if (ksym_expanded<OpX, V>(n, P.f.family)) return run_pairs_symx<OpX, kTpbKSym, kRtKSym>(P, n, ws, wsb, st);
   return run_sym<OpD, V>(P, n, ws, wsb, st);
 }
 template <class OpX, class OpD, typename V>
 inline size_t ksym_scratch(int64_t n, int family) {
-  if (std::is_same<V, F2>::value && family == kGauss && n > OpD::Shape::kSplit8)
-    return symx_ws_bytes<OpX, kTpbKSym, kRtKSym>(n);
+  if (ksym_expanded<OpX, V>(n, family)) return symx_plan<OpX, kTpbKSym, kRtKSym>(n).ws_bytes;
   return sym_scratch<OpD, V>(n, family);
 }
 template <class OpX, class OpD, typename V>
 inline size_t ksym_scratch_upto(int64_t n) {
-  const size_t b = sym_scratch_upto<OpD, V>(n), x = ksym_scratch<OpX, OpD, V>(n, kGauss);
-  return sym_takes<OpD, V>(n) && x > b ? x : b;
+  return sym_largest<OpD, V>(n, [](int64_t k, int family) { return ksym_scratch<OpX, OpD, V>(k, family); });
 }
 
 }  // namespace lddmm

@@ -217,7 +217,7 @@ struct OpSOFwdSym {
   using Params = OpSOFwd::Params;
   static constexpr int NSS = 6, NR = 6, NC = 6;
   static constexpr int kSymMinCtas = LDDMM_SOFWD_SYM_MIN_CTAS;
-  using Shape = SymRule<kSplit2N, kSplit4N, kSplit8N, kSplit4NLast, kRtSymFwd, kRtSymFwdL, kTpbSym64, kRtSym64>;
+  using Shape = SymRule<kWholeN, kSplitN, kRtSymFwd, kRtSymFwdL, kTpbSym64, kRtSym64>;
   template <typename V> struct SymTgt { V y0, y1, y2, a0, a1, a2; };
   template <typename V>
   static __device__ __forceinline__ void load_target_sym(const Params& P, int i0, int i1, bool v0, bool v1,
@@ -272,13 +272,13 @@ struct OpSOFwdSym {
 // and the mirrored contributions to l are -v and e px_k + e dq A_k: no scaled copy of a and no constant in the pair.
 // 50 FP32 lane-ops per unordered pair (25 per ordered pair, against 37 for OpSOBwd), one ex2, and 13 target values
 // where -kappa^2 a and two constants made 17: 40,962 points 1637 -> 1611 us (FP64 4098 -> 4010, Laplacian of order 3
-// 2156 -> 2070, where the profile is short of registers).
+// 2156 -> 2070, where the profile is short of registers; two sources to a packed operand then 1609 -> 1498, 2047 -> 1922).
 struct OpSOBwdSym {
   using Params = OpSOBwd::Params;
   static constexpr int NSS = 12, NR = 6, NC = 6;
   static constexpr int kSymMinCtas = LDDMM_SOBWD_SYM_MIN_CTAS;
-  using Shape = SymRule<kSplit2NAdj, kSplit4NLast, 0, kSplit4NLast, kRtAdjoint, kRtAdjointSymL, kTpbSym64Adj,
-                        kRtSym64Adj>;
+  static constexpr bool kSymFresh = true;
+  using Shape = SymRule<kSplitN, kSplitN, kRtAdjoint, kRtAdjointSymL, kTpbSym64Adj, kRtSym64Adj>;
   template <typename V> struct SymTgt { V y0, y1, y2, a0, a1, a2, p0, p1, p2, q0, q1, q2, ib; };
   static __device__ __forceinline__ double beta(const Params& P) { return P.f.inv_s2 / (P.f.kappa * P.f.kappa); }
   template <typename V>
@@ -412,7 +412,8 @@ struct OpFOBwdSym {
   using Params = OpFOBwd::Params;
   static constexpr int NSS = 9, NR = 6, NC = 6;
   static constexpr int kSymMinCtas = LDDMM_FOBWD_SYM_MIN_CTAS;
-  using Shape = SymRule<kSplit2N, kSplit4NLast, 0, kSplit4NLast, kRtFoSym, kRtFoSymL, kTpbSym64, kRtSym64>;
+  static constexpr int kSymUnrollG = 8;  // 40,962 points 845 us, 4: 878
+  using Shape = SymRule<kSplitN, kSplitN, kRtFoSym, kRtFoSymL, kTpbSym64, kRtSym64>;
   template <typename V> struct SymTgt { V y0, y1, y2, p0, p1, p2, a0, a1, a2, q0, q1, q2; };
   template <typename V>
   static __device__ __forceinline__ void load_target_sym(const Params& P, int i0, int i1, bool v0, bool v1,
