@@ -191,7 +191,8 @@ int lddmm_first_order_gradient(const double* xt, const double* at, int64_t n, in
  * ------------------------------------------------------------------------------------------------------- */
 enum { LDDMM_DATA_VARIFOLD = 0, LDDMM_DATA_CURRENT = 1, LDDMM_DATA_MEASURE = 2 };
 
-/* Scratch size (bytes) for lddmm_surface_energy / lddmm_surface_gradient with nf deformed and nf1 target faces. */
+/* Scratch size (bytes) for lddmm_surface_energy / lddmm_surface_gradient with nf deformed and nf1 target faces, and for
+ * the norm of the target alone (lddmm_surface_energy with no deformed face). */
 size_t lddmm_surface_workspace_bytes(int64_t nf, int64_t nf1, int precision);
 
 /* energy[0] = |def|^2 - 2 <def, tgt>  (xNormDef), energy[1] = |tgt|^2 (xNorm0); device scalars, FP64.

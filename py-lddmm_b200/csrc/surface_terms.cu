@@ -1,6 +1,7 @@
 // Surface data terms (unoriented varifold, current, measure): face geometry, fused energy (self - 2 cross in
 // one pass over the concatenated source faces), fused gradient and the deterministic faces->vertices gather.
 // Replaces base/surfaceDistances.py:22-573.
+#include <utility>
 #include <vector>
 
 #include "../../include/lddmm_b200.h"
@@ -403,8 +404,9 @@ size_t surf_pairs_bytes(int64_t nf, int64_t nf1) {
   upd(pairs_ws_bytes<OpSurfGrad<LDDMM_DATA_VARIFOLD>, V, TPB, RT>(nf, nf + nf1));
   upd(pairs_ws_bytes<OpSurfGrad<LDDMM_DATA_CURRENT>, V, TPB, RT>(nf, nf + nf1));
   upd(pairs_ws_bytes<OpSurfGrad<LDDMM_DATA_MEASURE>, V, TPB, RT>(nf, nf + nf1));
-  for (int64_t n : {nf, nf1}) {
-    const int64_t m = (n == nf) ? nf + nf1 : nf1;
+  // the energy between the surfaces and the norm of the target (also with no deformed surface at all): neither's
+  // scratch bounds the other's, a norm's triangle has half the units and a CTA of it meets more row blocks
+  for (const auto& [n, m] : {std::pair<int64_t, int64_t>{nf, nf + nf1}, {nf1, nf1}}) {
     upd(pairs_ws_bytes<OpSurfEnergy<LDDMM_DATA_VARIFOLD>, V, TPB, RT>(n, m));
     upd(pairs_ws_bytes<OpSurfEnergy<LDDMM_DATA_CURRENT>, V, TPB, RT>(n, m));
     upd(pairs_ws_bytes<OpSurfEnergy<LDDMM_DATA_MEASURE>, V, TPB, RT>(n, m));
