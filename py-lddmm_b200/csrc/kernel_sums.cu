@@ -67,8 +67,8 @@ int dispatch(int precision, int64_t n, int64_t m, double sigma, int kernel, cons
 
 template <class Op, int TPB32, int RT32>
 size_t op_ws(int64_t n, int64_t m, int precision) {
-  return precision == kFP32Compensated ? pairs_ws_bytes_any<Op, F2, TPB32, RT32>(n, m)
-                                       : pairs_ws_bytes_any<Op, double, kTpb64, kRt64>(n, m);
+  return precision == kFP32Compensated ? pairs_ws_upto_any<Op, F2, TPB32, RT32>(n, m)
+                                       : pairs_ws_upto_any<Op, double, kTpb64, kRt64>(n, m);
 }
 
 }  // namespace

@@ -594,11 +594,16 @@ struct Units {
   }
 };
 
-// Most CTAs that a window of `len` consecutive units of W meets when C CTAs divide them evenly (each takes at least
-// floor(W / C) units): the partial slots of a target block.
-inline int sk_max_slots(long long len, long long W, long long C) {
-  const long long q = W / C;
-  return (int)((len - 1 + q - 1) / q + 1);
+// Most CTAs that a window of `len` consecutive units of W meets when C CTAs divide them evenly, the partial slots of a
+// target block: sk_cta_of(u + len - 1) - sk_cta_of(u) is at most ceil((len - 1) C / W).
+inline int sk_max_slots(long long len, long long W, long long C) { return (int)(((len - 1) * C + W - 1) / W + 1); }
+
+// Slots times targets of an ordered sum, at most, over all problems of up to n targets and `tiles` source tiles (blocks
+// of B targets, `wave` resident CTAs): a problem of W <= wave units has a slot per tile and tiles x blocks <= wave; a
+// larger one has at most (wave / blocks) + 2 slots (W >= blocks x tiles).
+inline int64_t sk_slot_targets_upto(int64_t n, int64_t tiles, int64_t B, int64_t wave) {
+  const int64_t b = wave * B + 2 * n;
+  return n * tiles < b ? n * tiles : b;
 }
 
 // `boxes`: reserve the coordinate boxes of exact culling (ops with Culled<Op>); other ops never read them, so their
@@ -1348,8 +1353,8 @@ inline int run_pairs(const typename Op::Params& P, int64_t n, int64_t m, void* w
   return launch_pairs<Op, V, TPB, RT, Fam, false>(P, n, m, ws, ws_bytes, stream);
 }
 
-// Scratch of either launch (a smaller problem in the same workspace may split). A triangle op's sources are n targets
-// and m - n others, each padded to whole tiles.
+// Scratch of n targets and m sources (the larger of both shapes'). A triangle op's sources are n targets and m - n
+// others, each padded to whole tiles.
 template <class Op, typename V, int TPB, int RT, class Fam = Gauss>
 inline size_t pairs_ws_bytes(int64_t n, int64_t m) {
   const int64_t tiles = Triangle<Op>::value ? (n + TPB - 1) / TPB + (m - n + TPB - 1) / TPB : (m + TPB - 1) / TPB;
@@ -1361,16 +1366,46 @@ inline size_t pairs_ws_bytes(int64_t n, int64_t m) {
   return b;
 }
 
-// Workspace of an op for every kernel family (the largest of their plans).
-template <class Op, typename V, int TPB, int RT>
-inline size_t pairs_ws_bytes_any(int64_t n, int64_t m) {
+// Scratch that holds every problem of up to n targets and m sources: the slots of a plan are not monotone in either
+// (as many as tiles while every unit has a CTA of its own, half as many where two units go to one).
+template <class Op, typename V, int TPB, int RT, class Fam, bool SPLIT>
+inline size_t pairs_shape_ws_upto(int64_t n, int64_t m) {
+  static_assert(!Triangle<Op>::value, "an energy's scratch is asked for its own face counts");
+  if (n <= 0 || m <= 0) return 0;
+  constexpr int64_t B = (int64_t)(SPLIT ? 32 : TPB) * kRunRT<Op, V, RT, Fam>;
+  const int64_t tiles = (m + TPB - 1) / TPB;
+  const int64_t wave = (int64_t)device_sm_count() * ctas_per_sm<Op, V, TPB, RT, Fam, SPLIT>();
+  const size_t rows = (size_t)sk_slot_targets_upto(n, tiles, B, wave) * Op::NA * sizeof(typename VT<V>::Partial);
+  const size_t boxes = Culled<Op>::value ? (size_t)((n + B - 1) / B + tiles) * 6 * sizeof(float) : 0;
+  return ((rows + 255) & ~(size_t)255) + boxes;
+}
+template <class Op, typename V, int TPB, int RT, class Fam = Gauss>
+inline size_t pairs_ws_upto(int64_t n, int64_t m) {
+  size_t b = pairs_shape_ws_upto<Op, V, TPB, RT, Fam, false>(n, m);
+  if constexpr (CanSplit<Op>::value) {
+    const size_t s = pairs_shape_ws_upto<Op, V, TPB, RT, Fam, true>(n, m);
+    b = s > b ? s : b;
+  }
+  return b;
+}
+
+// The same for every kernel family (the largest of their plans).
+template <class Fn>
+inline size_t largest_by_family(Fn bytes) {
   size_t b = 0;
   for (const int family : {(int)kGauss, (int)kLaplacian0, (int)kLaplacianMax}) {
-    const size_t v =
-        by_family(family, [&](auto fam) { return pairs_ws_bytes<Op, V, TPB, RT, decltype(fam)>(n, m); });
+    const size_t v = by_family(family, bytes);
     b = v > b ? v : b;
   }
   return b;
+}
+template <class Op, typename V, int TPB, int RT>
+inline size_t pairs_ws_bytes_any(int64_t n, int64_t m) {
+  return largest_by_family([&](auto fam) { return pairs_ws_bytes<Op, V, TPB, RT, decltype(fam)>(n, m); });
+}
+template <class Op, typename V, int TPB, int RT>
+inline size_t pairs_ws_upto_any(int64_t n, int64_t m) {
+  return largest_by_family([&](auto fam) { return pairs_ws_upto<Op, V, TPB, RT, decltype(fam)>(n, m); });
 }
 
 inline bool bad_kernel(int kernel) { return !(kernel == kGauss || (kernel >= kLaplacian0 && kernel <= kLaplacianMax)); }

@@ -201,6 +201,22 @@ inline SymPlan make_sym_plan(int64_t n, int nr, int nc, int ctas_per_sm, size_t 
   return p;
 }
 
+// Scratch that holds the plans of every n in (lo, hi]. A plan's slots are not monotone in n. With U units in nblk rows
+// of at most TT (U >= nblk TT / 2) they are TT while every unit has a CTA of its own (2 U < 3 wave: slots x points <= TT
+// nblk B <= 2 U B), and at most (TT - 1) wave / U + 2 beyond (slots x points <= 2 wave B + 2 n).
+template <int TPB, int B>
+inline size_t sym_plan_upto(int64_t lo, int64_t hi, int nr, int nc, int ctas_per_sm, size_t row_bytes,
+                            size_t col_bytes) {
+  if (hi <= lo) return 0;
+  const SymPlan first = make_sym_plan<TPB, B>(lo + 1, nr, nc, ctas_per_sm, row_bytes, col_bytes);
+  const SymPlan last = make_sym_plan<TPB, B>(hi, nr, nc, ctas_per_sm, row_bytes, col_bytes);
+  int64_t points = 2 * first.wave * B + 2 * hi;
+  if (2 * first.U < 3 * first.wave && points < 3 * first.wave * B) points = 3 * first.wave * B;
+  if ((int64_t)last.TT * hi < points) points = (int64_t)last.TT * hi;
+  const size_t rows = (size_t)points * (size_t)nr * row_bytes;
+  return ((rows + 255) & ~(size_t)255) + (last.ws_bytes - last.col_off);
+}
+
 // Unroll depth of the source loop: the op's for the Gaussian in FP32, where it has one.
 template <class Op, class = void>
 struct SymUnrollOf : std::integral_constant<int, kSymUnroll> {};
@@ -653,24 +669,42 @@ template <class Op, typename V>
 inline size_t sym_scratch(int64_t n, int family) {
   return by_family(family, [&](auto fam) { return sym_scratch_fam<Op, V, decltype(fam)>(n); });
 }
-// Scratch for every point count up to n: the largest of the shapes at the end of their ranges. scratch(k, family): that
-// of one launch.
-template <class Op, typename V, class Scratch>
-inline size_t sym_largest(int64_t n, Scratch scratch) {
+// Scratch for every point count up to n: each shape over the range that it may be launched in (between kWholeN and
+// kSplitN either shape may be the one).
+template <class Op, typename V, class Fam>
+inline size_t sym_scratch_upto_fam(int64_t n) {
+  using R = typename Op::Shape;
+  constexpr bool kG = std::is_same<Fam, Gauss>::value;
+  n = n < sym_max_n<Op, V>() ? n : sym_max_n<Op, V>();
   size_t b = 0;
-  for (const int64_t k : {kSplit2N, kSplit4N, kWholeN, kSplitN, kSplit1N64, kSplit2N64, kSplit2N64Lap,
-                          sym_max_n<Op, V>(), n}) {
-    if (k > n || !sym_takes<Op, V>(k)) continue;
-    for (const int family : {(int)kGauss, (int)kLaplacian0, (int)kLaplacianMax}) {
-      const size_t v = scratch(k, family);
-      b = v > b ? v : b;
+  auto range = [&](auto sh, int64_t lo, int64_t hi) {
+    using Sh = decltype(sh);
+    const size_t v = sym_plan_upto<Sh::kTpb, (Sh::kSplit ? 32 : Sh::kTpb) * Sh::kRt>(
+        lo, n < hi ? n : hi, Op::NR, Op::NC, sym_ctas_per_sm<Op, Sh::kTpb, Sh::kRt, Fam, V, Sh::kSplit>(),
+        sizeof(typename VT<V>::Partial), sizeof(typename VT<V>::Scalar));
+    b = v > b ? v : b;
+  };
+  if constexpr (std::is_same<V, double>::value) {
+    constexpr int64_t kSplit2 = kG ? kSplit2N64 : kSplit2N64Lap;
+    range(SymShape<128, 1, true>{}, 0, kSplit1N64);
+    range(SymShape<128, 2, true>{}, kSplit1N64, kSplit2);
+    range(SymShape<R::kTpb64, R::kRt64, false>{}, kSplit2, n);
+  } else {
+    constexpr int kRt = kG ? R::kRt : R::kRtLap;
+    constexpr int64_t kSplit4 = kG ? R::kSplit4 : R::kSplit4Lap;
+    range(SymShape<128, 2, true>{}, 0, kSplit2N);
+    if constexpr (kRt > 0) {
+      range(SymShape<128, kRt, false>{}, kWholeN, kSplitN);
+      range(SymShape<128, kRt, false>{}, kSplitN, n);
     }
+    if constexpr (kSplit4 < kSplitN) range(SymShape<128, 8, true>{}, kSplit4, kSplitN);
+    range(SymShape<128, 4, true>{}, kSplit2N, kSplit4);
   }
   return b;
 }
 template <class Op, typename V>
 inline size_t sym_scratch_upto(int64_t n) {
-  return sym_largest<Op, V>(n, [](int64_t k, int family) { return sym_scratch<Op, V>(k, family); });
+  return largest_by_family([&](auto fam) { return sym_scratch_upto_fam<Op, V, decltype(fam)>(n); });
 }
 
 template <class Op, typename V, class Fam>
@@ -1002,7 +1036,14 @@ inline size_t ksym_scratch(int64_t n, int family) {
 }
 template <class OpX, class OpD, typename V>
 inline size_t ksym_scratch_upto(int64_t n) {
-  return sym_largest<OpD, V>(n, [](int64_t k, int family) { return ksym_scratch<OpX, OpD, V>(k, family); });
+  size_t b = sym_scratch_upto<OpD, V>(n);
+  if (ksym_expanded<OpX, V>(n, kGauss)) {
+    const size_t v = sym_plan_upto<kTpbKSym, kTpbKSym * kRtKSym>(kSplitN, n, OpX::NP, OpX::NP,
+                                                                 symx_ctas_per_sm<OpX, kTpbKSym, kRtKSym>(),
+                                                                 sizeof(float2), sizeof(float));
+    b = v > b ? v : b;
+  }
+  return b;
 }
 
 }  // namespace lddmm

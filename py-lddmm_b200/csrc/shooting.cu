@@ -478,18 +478,18 @@ size_t shooting_ws_bytes(int64_t n, int precision) {
   };
   if (precision == kFP32Compensated) {
     sym(F2{});
-    upd(pairs_ws_bytes_any<OpSOFwd, F2, kTpbLight, kRtLight>(n, n));
-    upd(pairs_ws_bytes<OpSOBwd, F2, kTpbHeavy, kRtAdjoint, Gauss>(n, n));
-    upd(pairs_ws_bytes<OpSOBwd, F2, kTpbHeavy, kRtHeavy, Laplacian3>(n, n));
-    upd(pairs_ws_bytes<OpSOBwd, F2, kTpbHeavy, kRtHeavy, Laplacian4>(n, n));
-    upd(pairs_ws_bytes_any<OpFOBwd, F2, kTpbLight, kRtLight>(n, n));
-    upd(pairs_ws_bytes_any<OpK, F2, kTpbLight, kRtLight>(n, n));
+    upd(pairs_ws_upto_any<OpSOFwd, F2, kTpbLight, kRtLight>(n, n));
+    upd(pairs_ws_upto<OpSOBwd, F2, kTpbHeavy, kRtAdjoint, Gauss>(n, n));
+    upd(pairs_ws_upto<OpSOBwd, F2, kTpbHeavy, kRtHeavy, Laplacian3>(n, n));
+    upd(pairs_ws_upto<OpSOBwd, F2, kTpbHeavy, kRtHeavy, Laplacian4>(n, n));
+    upd(pairs_ws_upto_any<OpFOBwd, F2, kTpbLight, kRtLight>(n, n));
+    upd(pairs_ws_upto_any<OpK, F2, kTpbLight, kRtLight>(n, n));
   } else {
     sym(0.0);
-    upd(pairs_ws_bytes_any<OpSOFwd, double, kTpb64, kRt64>(n, n));
-    upd(pairs_ws_bytes_any<OpSOBwd, double, kTpb64, kRt64>(n, n));
-    upd(pairs_ws_bytes_any<OpFOBwd, double, kTpb64, kRt64>(n, n));
-    upd(pairs_ws_bytes_any<OpK, double, kTpb64, kRt64>(n, n));
+    upd(pairs_ws_upto_any<OpSOFwd, double, kTpb64, kRt64>(n, n));
+    upd(pairs_ws_upto_any<OpSOBwd, double, kTpb64, kRt64>(n, n));
+    upd(pairs_ws_upto_any<OpFOBwd, double, kTpb64, kRt64>(n, n));
+    upd(pairs_ws_upto_any<OpK, double, kTpb64, kRt64>(n, n));
   }
   // per-point dot products for the FP64 energy reductions live after the pair partials
   return ((b + 255) & ~(size_t)255) + (size_t)(n > 0 ? n : 0) * sizeof(double);

@@ -30,6 +30,106 @@ def test_surface_scratch_covers_the_norm_alone(precision):
     assert not bad, bad[:10]
 
 
+@pytest.mark.parametrize('precision', [0, 1], ids=['fp32c', 'fp64'])
+def test_workspace_bytes_never_falls_with_the_problem(precision):
+    """A workspace for n_max targets and m_max sources serves every smaller problem, so its size may not fall as either
+    grows (through the ranges where the launch shapes alternate, and past the largest FP64 set of the symmetric kernels)."""
+    size = _lib().lddmm_workspace_bytes
+    ns = list(range(0, 30000, 61)) + [40962, 100000, 151296, 151297, 163842, 400000]
+    for other in (None, 1, 3000, 40962):
+        for swap in (False, True):
+            got = [size(*((other if other is not None else n, n) if swap else
+                          (n, other if other is not None else n)), precision) for n in ns]
+            assert got == sorted(got), (other, swap)
+
+
+# --- the plans of csrc/lddmm_common.cuh and csrc/pairs_sym.cuh, restated
+def _tri(j):
+    return j * (j - 1) // 2
+
+
+def _row_off(i, TT, TPB, B):
+    if B >= TPB:
+        return i * TT - (B // TPB) * _tri(i)
+    share = TPB // B
+    q, r = divmod(i, share)
+    return i * TT - (share * _tri(q) + q * r)
+
+
+def _cta_of(u, W, C):
+    return ((u + 1) * C - 1) // W
+
+
+def _max_slots(length, W, C):
+    return -(-(length - 1) * C // W) + 1
+
+
+def _sym_rows(n, TPB, B, wave):
+    """(slots, units, CTAs, tiles, row blocks) of make_sym_plan."""
+    nblk, TT = -(-n // B), -(-n // TPB)
+    U = _row_off(nblk, TT, TPB, B)
+    C = U if 2 * U < 3 * wave else wave
+    return _max_slots(TT, U, C), U, C, TT, nblk
+
+
+def _sym_upto(lo, hi, TPB, B, wave):
+    """Slots times points of sym_plan_upto."""
+    points = 2 * wave * B + 2 * hi
+    if 2 * _sym_rows(lo + 1, TPB, B, wave)[1] < 3 * wave:
+        points = max(points, 3 * wave * B)
+    return min(points, -(-hi // TPB) * hi)
+
+
+SHAPES = [(128, 32), (128, 64), (128, 128), (128, 256), (128, 512), (128, 768), (128, 1024), (64, 256), (128, 256)]
+
+
+@pytest.mark.parametrize('TPB,B', SHAPES)
+def test_slots_of_a_symmetric_plan(TPB, B):
+    """The slots reserved are those of the longest row, or one more; and the bound over a range of n holds each n's."""
+    for wave in (3, 148, 296, 444, 740, 1184):
+        ns = sorted(set(range(1, 4000, 173)) | {B - 1, B, B + 1, 8193, 10368, 16384, 20001, 40962})
+        need = {}
+        for n in ns:
+            S, U, C, TT, nblk = _sym_rows(n, TPB, B, wave)
+            real = max(_cta_of(_row_off(i + 1, TT, TPB, B) - 1, U, C) - _cta_of(_row_off(i, TT, TPB, B), U, C) + 1
+                       for i in range(nblk))
+            assert real <= S <= real + 1, (n, wave)
+            need[n] = S * n
+        for lo in (0, 1408, 8192, 16384):
+            for hi in ns:
+                inside = [need[n] for n in ns if lo < n <= hi]
+                assert not inside or max(inside) <= _sym_upto(lo, hi, TPB, B, wave), (lo, hi, wave)
+
+
+@pytest.mark.parametrize('TPB,B', [(128, 128), (128, 256), (128, 512), (128, 1024), (128, 64)])
+def test_slots_of_an_ordered_plan(TPB, B):
+    """Ordered sums and the triangles of the energies: the slots hold the longest row, and slots times targets of a
+    smaller ordered problem stay under the bound of the larger one."""
+    for wave in (5, 148, 444, 1184):
+        need = {}
+        ns = [1, 100, B, B + 1, 3000, 13000, 40962, 226301, 262144]
+        ts = [1, 2, 3, 24, 100, 161, 321, 7813]
+        for n in ns:
+            for tiles in ts:
+                gx = -(-n // B)
+                W = gx * tiles
+                C = min(W, wave)
+                S = _max_slots(tiles, W, C)
+                real = max(_cta_of((i + 1) * tiles - 1, W, C) - _cta_of(i * tiles, W, C) + 1 for i in range(gx))
+                assert real <= S <= real + 1
+                need[n, tiles] = S * n
+                self_tiles = -(-n // TPB)                        # an energy: the self part is a triangle
+                W = _row_off(gx, self_tiles + tiles, TPB, B)
+                C = min(W, wave)
+                off = [_row_off(i, self_tiles + tiles, TPB, B) for i in range(gx + 1)]
+                real = max(_cta_of(off[i + 1] - 1, W, C) - _cta_of(off[i], W, C) + 1 for i in range(gx))
+                assert real <= _max_slots(self_tiles + tiles, W, C)
+        for n in ns:
+            for tiles in ts:
+                bound = min(n * tiles, wave * B + 2 * n)
+                assert max(v for (k, t), v in need.items() if k <= n and t <= tiles) <= bound
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize('precision,nf', [(0, 1), (0, 10496), (0, 12800), (0, 14720), (0, 16500), (0, 20480),
                                           (0, 40960), (1, 1), (1, 6976), (1, 7232)])
@@ -68,3 +168,45 @@ def test_surface_calls_in_exactly_the_reported_scratch(precision, nf):
     for kind in (nat.DATA_VARIFOLD, nat.DATA_CURRENT, nat.DATA_MEASURE):
         for a, b in zip(calls(exact, kind), calls(2 * exact, kind)):
             assert torch.equal(a, b) and bool(torch.isfinite(a).all()), kind
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('precision', [0, 1], ids=['fp32c', 'fp64'])
+@pytest.mark.parametrize('kernel', [0, 19, 20], ids=['gauss', 'laplacian3', 'laplacian4'])
+def test_smaller_sets_in_the_scratch_of_the_largest(precision, kernel):
+    """Self-sums, shooting steps and ordered sums of every size up to n_max in exactly the bytes reported for n_max,
+    through the ranges where the launch shapes change."""
+    import torch
+    from base import _native as nat
+    lib = nat.lib()
+    rng = np.random.default_rng(kernel)
+    n_max = 20000 if precision == 0 else 9000
+    X = torch.from_numpy(rng.normal(size=(n_max, 3))).cuda()
+    A = torch.from_numpy(rng.normal(size=(n_max, 3)) / n_max).cuda()
+    out = [torch.empty((2 * n_max, 3), dtype=torch.float64, device='cuda') for _ in range(2)]
+    e = torch.zeros(1, dtype=torch.float64, device='cuda')
+    p = nat.ptr
+    for top in (n_max, n_max // 2):
+        nbytes = lib.lddmm_workspace_bytes(top, top, precision)
+        W = torch.empty(nbytes, dtype=torch.uint8, device='cuda')
+        end = (precision, p(W), nbytes, nat.stream_ptr())
+        ns = {1, 700, 1280, 1281, 1408, 1409, 2304, 2305, 3601, 4097, 4352, 5400, 6500, 7232, 8192, 8445, 8704, 9216, 9984,
+              10363, 10368, 10496, 13000, 15000, 16384, 16385, top}
+        for n in sorted(k for k in ns if k <= top):
+            rcs = {
+                'apply_k': lib.lddmm_apply_k(p(X), n, p(X), p(A), n, 0.5, kernel, None, p(out[0]), *end),
+                'ordered': lib.lddmm_apply_k(p(A), n, p(X), p(A), n, 0.5, kernel, None, p(out[0]), *end),
+                'diff_kt': lib.lddmm_apply_diff_kt(p(X), n, p(X), p(A), p(A), n, 0.5, kernel, 0, 1.0, None, p(out[0]),
+                                                   *end),
+                'forward': lib.lddmm_second_order_step(p(X), p(A), n, 0.5, kernel, 0.1, None, p(out[0]), p(out[1]), *end),
+                'adjoint': lib.lddmm_second_order_adjoint_step(p(X), p(A), p(A), p(A), n, 0.5, kernel, 0.1, None,
+                                                               p(out[0]), p(out[1]), *end),
+                'rows': lib.lddmm_second_order_adjoint_step_rows(p(X), p(A), p(A), p(A), n, 0, (n + 1) // 2, 0.5, kernel,
+                                                                 0.1, None, p(out[0]), p(out[1]), *end),
+                'first-order': lib.lddmm_first_order_gradient(p(X), p(A), n, 1, 0.5, kernel, 1.0, p(A), 1, None,
+                                                              p(out[0]), p(out[1]), *end),
+                'energy': lib.lddmm_first_order_shoot(p(X), p(A), n, 1, 0.5, kernel, 1.0, None, p(out[0]), p(e), *end),
+            }
+            assert not any(rcs.values()), (top, n, rcs)
+    torch.cuda.synchronize()
+    assert bool(torch.isfinite(out[0][:n_max // 2]).all())
