@@ -16,7 +16,8 @@
  *  - `precision`: LDDMM_FP32C = FP32 pair arithmetic with compensated (two-sum) accumulation across tiles and
  *    FP64 epilogues; LDDMM_FP64 = the same kernels in FP64 (the faithful baseline).
  *  - `workspace` / `workspace_bytes`: caller-provided device scratch of at least
- *    lddmm_workspace_bytes(n_max, m_max, precision) bytes. No entry point allocates memory.
+ *    lddmm_workspace_bytes(n_max, m_max, precision) bytes (or, for one size of call, lddmm_call_workspace_bytes). No
+ *    entry point allocates memory.
  *  - Calls are asynchronous on `stream`, launch no host synchronisation and are safe to capture in a CUDA graph.
  *  - Return value: LDDMM_OK or an error status; argument errors are detected before any launch.
  */
@@ -60,6 +61,13 @@ const char* lddmm_status_string(int status);
 /* Scratch size (bytes) sufficient for every entry point with at most n_max targets and m_max sources. */
 size_t lddmm_workspace_bytes(int64_t n_max, int64_t m_max, int precision);
 
+/* Scratch size (bytes) of calls with exactly n targets and m sources; at most lddmm_workspace_bytes(n, m, precision).
+ * self_sums = 0: calls that evaluate every ordered pair, that is K(y, x) a of two arrays, the derivative operators,
+ * divergence and K tensor, and steps on a part of the rows. self_sums = 1 (n == m): also K(x, x) a and whole shooting
+ * steps, sweeps and gradients. Those keep partial sums per pair of point blocks, which grow with n^2 (FP32 at 40,962
+ * points some 55 MB, FP64 170 MB; FP64 sets above 2 GiB of them are summed over ordered pairs). */
+size_t lddmm_call_workspace_bytes(int64_t n, int64_t m, int self_sums, int precision);
+
 /* ---------------------------------------------------------------------------------------------------------
  * Kernel operators (replace Kernel.* in base/kernelFunctions.py:452-674 and the numba / pykeops backends
  * ku.applyK / applyDiffKT / applyDDiffK / applykdiff1and2 / applyDiv / applyktensor in
@@ -68,9 +76,9 @@ size_t lddmm_workspace_bytes(int64_t n_max, int64_t m_max, int precision);
  * ------------------------------------------------------------------------------------------------------- */
 
 /* out(n,3) = K(y, x) a.  Kernel.applyK(x, a, firstVar=y)  base/kernelFunctions.py:452.
- * When y == x (the same pointer) and n == m, FP32 evaluates the self-sum once per unordered pair (symmetric
- * kernel; the workspace of lddmm_workspace_bytes(n, n, ...) covers it); results agree with the ordered-pair
- * evaluation to FP32 rounding. */
+ * When y == x (the same pointer) and n == m, the self-sum is evaluated once per unordered pair (symmetric kernel; its
+ * scratch is that of lddmm_workspace_bytes(n, n, ...) or lddmm_call_workspace_bytes(n, n, 1, ...)); results agree with
+ * the ordered-pair evaluation to the rounding of the precision. */
 int lddmm_apply_k(const double* y, int64_t n, const double* x, const double* a, int64_t m, double sigma, int kernel,
                   const double* origin, double* out, int precision, void* workspace, size_t workspace_bytes,
                   lddmm_stream_t stream);

@@ -30,6 +30,7 @@ SIGNATURES = {
     'lddmm_version': [],
     'lddmm_status_string': [_int],
     'lddmm_workspace_bytes': [_i64, _i64, _int],
+    'lddmm_call_workspace_bytes': [_i64, _i64, _int, _int],
     'lddmm_surface_workspace_bytes': [_i64, _i64, _int],
     'lddmm_apply_k': [_dp, _i64, _dp, _dp, _i64, _f64, _int, _hp, _dp, _int, _vp, _sz, _vp],
     'lddmm_apply_diff_kt': [_dp, _i64, _dp, _dp, _dp, _i64, _f64, _int, _int, _f64, _hp, _dp, _int, _vp, _sz, _vp],
@@ -76,7 +77,8 @@ OWN_ORIGIN_POINTS = {FP32C: 8192, FP64: 2304}       # LDDMM_OWN_ORIGIN_POINTS of
 LBFGS_MAX_PAIRS = 64        # LDDMM_LBFGS_MAX_PAIRS of the header
 _RESTYPES = {'lddmm_version': ctypes.c_char_p, 'lddmm_status_string': ctypes.c_char_p,
              'lddmm_mlp_workspace_bytes': ctypes.c_size_t,
-             'lddmm_workspace_bytes': ctypes.c_size_t, 'lddmm_surface_workspace_bytes': ctypes.c_size_t}
+             'lddmm_workspace_bytes': ctypes.c_size_t, 'lddmm_call_workspace_bytes': ctypes.c_size_t,
+             'lddmm_surface_workspace_bytes': ctypes.c_size_t}
 
 _lib = None
 _lock = threading.Lock()
@@ -174,19 +176,22 @@ class Workspace:
 WORKSPACE = Workspace()
 
 
-_WS_BYTES = {}   # (entry, n, m, precision, device) -> bytes: the library's answer depends on nothing else
+_WS_BYTES = {}   # (entry, arguments, device) -> bytes: the library's answer depends on nothing else
 
 
-def _ws_bytes(entry, n, m, precision):
-    key = (entry, int(n), int(m), int(precision), torch.cuda.current_device())
+def _ws_bytes(entry, *args):
+    key = (entry, *[int(v) for v in args], torch.cuda.current_device())
     nb = _WS_BYTES.get(key)
     if nb is None:
-        nb = _WS_BYTES[key] = getattr(lib(), entry)(key[1], key[2], key[3])
+        nb = _WS_BYTES[key] = getattr(lib(), entry)(*key[1:-1])
     return nb
 
 
-def workspace(n, m, precision=FP32C):
-    buf = WORKSPACE.get(_ws_bytes('lddmm_workspace_bytes', n, m, precision))
+def workspace(n, m, precision=FP32C, self_sums=None):
+    """Scratch of a call with n targets and m sources (pointer, size). self_sums: whether the call may be a self-sum or a
+    whole shooting step, whose scratch grows with n^2 (None: wherever n == m; False: the ordered sums)."""
+    both = n == m if self_sums is None else self_sums
+    buf = WORKSPACE.get(_ws_bytes('lddmm_call_workspace_bytes', n, m, both, precision))
     return ctypes.c_void_p(buf.data_ptr()), ctypes.c_size_t(buf.numel())
 
 

@@ -150,7 +150,7 @@ class Kernel(KernelSpec):
             origin = self._origin(Y, X)
         n, m = Y.shape[0], X.shape[0]
         out = torch.empty((n, 3), dtype=torch.float64, device=Y.device)
-        ws, wsb = nat.workspace(n, m, self.precision)
+        ws, wsb = nat.workspace(n, m, self.precision, self_sums=n == m and Y.data_ptr() == X.data_ptr())
         o = nat.origin_arg(origin)
         nat.check(nat.lib().lddmm_apply_k(nat.ptr(Y), n, nat.ptr(X), nat.ptr(A), m, float(sigma), self.code, o,
                                           nat.ptr(out), self.precision, ws, wsb, nat.stream_ptr()), 'applyK')
@@ -187,7 +187,7 @@ class Kernel(KernelSpec):
 
         def one(s):
             out = torch.empty(n, dtype=torch.float64, device=Y.device)
-            ws, wsb = nat.workspace(n, m, self.precision)
+            ws, wsb = nat.workspace(n, m, self.precision, self_sums=False)
             nat.check(nat.lib().lddmm_apply_k_tensor(nat.ptr(Y), n, nat.ptr(X), m, nat.ptr(AY), nat.ptr(AX),
                                                      nat.ptr(BY), nat.ptr(BX), float(s), o, nat.ptr(out),
                                                      self.precision, ws, wsb, nat.stream_ptr()), 'applyKTensor')
@@ -199,7 +199,7 @@ class Kernel(KernelSpec):
         """-(1/sigma^2) sum_l (D.(A1_k - A1_l)) K_kl A2_l for one width."""
         n = X.shape[0]
         out = torch.empty((n, 3), dtype=torch.float64, device=X.device)
-        ws, wsb = nat.workspace(n, n, self.precision)
+        ws, wsb = nat.workspace(n, n, self.precision, self_sums=False)
         o = nat.origin_arg(nat.centroid(X))
         nat.check(nat.lib().lddmm_apply_diff_k1and2(nat.ptr(X), nat.ptr(A1), nat.ptr(A2), n, float(sigma), self.code,
                                                     o, nat.ptr(out), self.precision, ws, wsb, nat.stream_ptr()),
@@ -291,7 +291,7 @@ class Kernel(KernelSpec):
 
         def one(s):
             out = torch.empty((n, 3), dtype=torch.float64, device=Y.device)
-            ws, wsb = nat.workspace(n, m, self.precision)
+            ws, wsb = nat.workspace(n, m, self.precision, self_sums=False)
             nat.check(nat.lib().lddmm_apply_diff_kt(nat.ptr(Y), n, nat.ptr(X), nat.ptr(P), nat.ptr(A), m, float(s),
                                                     self.code, mode, float(regweight), o, nat.ptr(out),
                                                     self.precision, ws, wsb, nat.stream_ptr()), 'applyDiffKT')
@@ -321,7 +321,7 @@ class Kernel(KernelSpec):
 
         def one(s):
             out = torch.empty((n, 1), dtype=torch.float64, device=Y.device)
-            ws, wsb = nat.workspace(n, m, self.precision)
+            ws, wsb = nat.workspace(n, m, self.precision, self_sums=False)
             nat.check(nat.lib().lddmm_apply_divergence(nat.ptr(Y), n, nat.ptr(X), nat.ptr(A), m, float(s), self.code,
                                                        o, nat.ptr(out), self.precision, ws, wsb, nat.stream_ptr()),
                       'applyDivergence')
@@ -339,7 +339,7 @@ class Kernel(KernelSpec):
 
         def one(s):
             out = torch.empty((N, 3), dtype=torch.float64, device=X.device)
-            ws, wsb = nat.workspace(N, N, self.precision)
+            ws, wsb = nat.workspace(N, N, self.precision, self_sums=False)
             nat.check(nat.lib().lddmm_apply_ddiff_k11and12(nat.ptr(X), nat.ptr(Nn), nat.ptr(A), nat.ptr(P), N,
                                                            float(s), self.code, o, nat.ptr(out), self.precision, ws,
                                                            wsb, nat.stream_ptr()), 'applyDDiffK11and12')

@@ -9,8 +9,9 @@
 
 namespace lddmm {
 
-size_t kernel_sums_ws_bytes(int64_t n, int64_t m, int precision);
-size_t shooting_ws_bytes(int64_t n, int precision);
+size_t ordered_ws_bytes(int64_t n, int64_t m, int precision, bool upto);
+size_t ordered_steps_ws_bytes(int64_t n, int64_t m, int precision, bool upto);
+size_t self_ws_bytes(int64_t n, int precision, bool upto);
 
 __device__ __forceinline__ double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -87,6 +88,17 @@ __global__ void diff_k_mat_kernel(const double* __restrict__ y, int n, const dou
   }
 }
 
+// `points` > 0: and self-sums and steps of that many (`upto`: of as many or fewer), with the per-point dot products of
+// the energies behind the pair partials.
+static size_t scratch_bytes(int64_t n, int64_t m, int64_t points, int precision, bool upto) {
+  size_t b = 0;
+  auto upd = [&](size_t v) { b = v > b ? v : b; };
+  upd(ordered_ws_bytes(n, m, precision, upto));
+  upd(ordered_steps_ws_bytes(n, m, precision, upto));
+  if (points > 0) upd(self_ws_bytes(points, precision, upto));
+  return ((b + 255) & ~(size_t)255) + (size_t)points * sizeof(double);
+}
+
 }  // namespace lddmm
 
 using namespace lddmm;
@@ -110,10 +122,13 @@ const char* lddmm_status_string(int status) {
 
 size_t lddmm_workspace_bytes(int64_t n_max, int64_t m_max, int precision) {
   if (n_max < 0 || m_max < 0 || (precision != kFP32Compensated && precision != kFP64)) return 0;
-  const size_t a = kernel_sums_ws_bytes(n_max, m_max, precision);
-  const int64_t nm = n_max > m_max ? n_max : m_max;
-  const size_t b = shooting_ws_bytes(nm, precision);
-  return a > b ? a : b;
+  // a self-sum or step of k points has k targets and k sources
+  return scratch_bytes(n_max, m_max, n_max < m_max ? n_max : m_max, precision, true);
+}
+
+size_t lddmm_call_workspace_bytes(int64_t n, int64_t m, int self_sums, int precision) {
+  if (n < 0 || m < 0 || (self_sums && n != m) || (precision != kFP32Compensated && precision != kFP64)) return 0;
+  return scratch_bytes(n, m, self_sums ? n : 0, precision, false);
 }
 
 int lddmm_apply_k_mat(const double* y, int64_t n, const double* x, int64_t m, const double* u, int64_t d,

@@ -66,27 +66,25 @@ int dispatch(int precision, int64_t n, int64_t m, double sigma, int kernel, cons
 }
 
 template <class Op, int TPB32, int RT32>
-size_t op_ws(int64_t n, int64_t m, int precision) {
-  return precision == kFP32Compensated ? pairs_ws_upto_any<Op, F2, TPB32, RT32>(n, m)
-                                       : pairs_ws_upto_any<Op, double, kTpb64, kRt64>(n, m);
+size_t op_ws(int64_t n, int64_t m, int precision, bool upto) {
+  if (precision == kFP32Compensated)
+    return upto ? pairs_ws_upto_any<Op, F2, TPB32, RT32>(n, m) : pairs_ws_bytes_any<Op, F2, TPB32, RT32>(n, m);
+  return upto ? pairs_ws_upto_any<Op, double, kTpb64, kRt64>(n, m) : pairs_ws_bytes_any<Op, double, kTpb64, kRt64>(n, m);
 }
 
 }  // namespace
 
-size_t kernel_sums_ws_bytes(int64_t n, int64_t m, int precision) {
+size_t ordered_ws_bytes(int64_t n, int64_t m, int precision, bool upto) {
   size_t b = 0;
   auto upd = [&](size_t v) { b = v > b ? v : b; };
-  upd(op_ws<OpK, kTpbLight, kRtLight>(n, m, precision));
-  upd(op_ws<OpDiffKT<0>, kTpbLight, kRtLight>(n, m, precision));
-  upd(op_ws<OpDiffKT<1>, kTpbLight, kRtLight>(n, m, precision));
-  upd(op_ws<OpDiffKT<2>, kTpbLight, kRtLight>(n, m, precision));
-  upd(op_ws<OpDDiffK, kTpbHeavy, kRtHeavy>(n, m, precision));
-  upd(op_ws<OpDiffK1and2, kTpbLight, kRtLight>(n, m, precision));
-  upd(op_ws<OpDiv, kTpbLight, kRtLight>(n, m, precision));
-  upd(op_ws<OpKTensor, kTpbLight, kRtLight>(n, m, precision));
-  if (n == m)
-    upd(precision == kFP32Compensated ? ksym_scratch_upto<OpKSym, OpKSymD, F2>(n)
-                                      : ksym_scratch_upto<OpKSym, OpKSymD, double>(n));
+  upd(op_ws<OpK, kTpbLight, kRtLight>(n, m, precision, upto));
+  upd(op_ws<OpDiffKT<0>, kTpbLight, kRtLight>(n, m, precision, upto));
+  upd(op_ws<OpDiffKT<1>, kTpbLight, kRtLight>(n, m, precision, upto));
+  upd(op_ws<OpDiffKT<2>, kTpbLight, kRtLight>(n, m, precision, upto));
+  upd(op_ws<OpDDiffK, kTpbHeavy, kRtHeavy>(n, m, precision, upto));
+  upd(op_ws<OpDiffK1and2, kTpbLight, kRtLight>(n, m, precision, upto));
+  upd(op_ws<OpDiv, kTpbLight, kRtLight>(n, m, precision, upto));
+  upd(op_ws<OpKTensor, kTpbLight, kRtLight>(n, m, precision, upto));
   return b;
 }
 

@@ -466,35 +466,6 @@ struct OpFOBwdSym {
   }
 };
 
-size_t shooting_ws_bytes(int64_t n, int precision) {
-  size_t b = 0;
-  auto upd = [&](size_t v) { b = v > b ? v : b; };
-  auto sym = [&](auto v) {
-    using V = decltype(v);
-    upd(sym_scratch_upto<OpSOFwdSym, V>(n));
-    upd(sym_scratch_upto<OpSOBwdSym, V>(n));
-    upd(sym_scratch_upto<OpFOBwdSym, V>(n));
-    upd(ksym_scratch_upto<OpKSym, OpKSymD, V>(n));
-  };
-  if (precision == kFP32Compensated) {
-    sym(F2{});
-    upd(pairs_ws_upto_any<OpSOFwd, F2, kTpbLight, kRtLight>(n, n));
-    upd(pairs_ws_upto<OpSOBwd, F2, kTpbHeavy, kRtAdjoint, Gauss>(n, n));
-    upd(pairs_ws_upto<OpSOBwd, F2, kTpbHeavy, kRtHeavy, Laplacian3>(n, n));
-    upd(pairs_ws_upto<OpSOBwd, F2, kTpbHeavy, kRtHeavy, Laplacian4>(n, n));
-    upd(pairs_ws_upto_any<OpFOBwd, F2, kTpbLight, kRtLight>(n, n));
-    upd(pairs_ws_upto_any<OpK, F2, kTpbLight, kRtLight>(n, n));
-  } else {
-    sym(0.0);
-    upd(pairs_ws_upto_any<OpSOFwd, double, kTpb64, kRt64>(n, n));
-    upd(pairs_ws_upto_any<OpSOBwd, double, kTpb64, kRt64>(n, n));
-    upd(pairs_ws_upto_any<OpFOBwd, double, kTpb64, kRt64>(n, n));
-    upd(pairs_ws_upto_any<OpK, double, kTpb64, kRt64>(n, n));
-  }
-  // per-point dot products for the FP64 energy reductions live after the pair partials
-  return ((b + 255) & ~(size_t)255) + (size_t)(n > 0 ? n : 0) * sizeof(double);
-}
-
 namespace {
 
 // Launch shapes per precision: light (forward / first-order) ops and the second-order adjoint step.
@@ -507,6 +478,54 @@ template <> struct StepShape<F2> {
 template <> struct StepShape<double> {
   static constexpr int kTpb = kTpb64, kRt = kRt64, kTpbH = kTpb64, kRtH = kRt64, kRtHL = kRt64;
 };
+
+}  // namespace
+
+// The steps evaluated per ordered pair: n targets (all points or a range of rows), m points.
+size_t ordered_steps_ws_bytes(int64_t n, int64_t m, int precision, bool upto) {
+  auto op = [&](auto v) {
+    using V = decltype(v);
+    constexpr int TPB = StepShape<V>::kTpb, RT = StepShape<V>::kRt;
+    size_t b = 0;
+    auto upd = [&](size_t w) { b = w > b ? w : b; };
+    upd(upto ? pairs_ws_upto_any<OpSOFwd, V, TPB, RT>(n, m) : pairs_ws_bytes_any<OpSOFwd, V, TPB, RT>(n, m));
+    upd(upto ? pairs_ws_upto_any<OpFOBwd, V, TPB, RT>(n, m) : pairs_ws_bytes_any<OpFOBwd, V, TPB, RT>(n, m));
+    upd(largest_by_family([&](auto fam) {
+      using Fam = decltype(fam);
+      constexpr int TPBH = StepShape<V>::kTpbH;
+      constexpr int R = std::is_same<Fam, Gauss>::value ? StepShape<V>::kRtH : StepShape<V>::kRtHL;
+      return upto ? pairs_ws_upto<OpSOBwd, V, TPBH, R, Fam>(n, m) : pairs_ws_bytes<OpSOBwd, V, TPBH, R, Fam>(n, m);
+    }));
+    return b;
+  };
+  return precision == kFP32Compensated ? op(F2{}) : op(0.0);
+}
+
+// Self-sums and whole shooting steps of n points (`upto`: of any number up to n) where the symmetric kernels take them.
+size_t self_ws_bytes(int64_t n, int precision, bool upto) {
+  auto op = [&](auto v) {
+    using V = decltype(v);
+    size_t b = 0;
+    auto upd = [&](size_t w) { b = w > b ? w : b; };
+    if (upto) {
+      upd(sym_scratch_upto<OpSOFwdSym, V>(n));
+      upd(sym_scratch_upto<OpSOBwdSym, V>(n));
+      upd(sym_scratch_upto<OpFOBwdSym, V>(n));
+      upd(ksym_scratch_upto<OpKSym, OpKSymD, V>(n));
+    } else {
+      for (const int family : {(int)kGauss, (int)kLaplacian0, (int)kLaplacianMax}) {
+        if (sym_takes<OpSOFwdSym, V>(n)) upd(sym_scratch<OpSOFwdSym, V>(n, family));
+        if (sym_takes<OpSOBwdSym, V>(n)) upd(sym_scratch<OpSOBwdSym, V>(n, family));
+        if (sym_takes<OpFOBwdSym, V>(n)) upd(sym_scratch<OpFOBwdSym, V>(n, family));
+        if (sym_takes<OpKSymD, V>(n)) upd(ksym_scratch<OpKSym, OpKSymD, V>(n, family));
+      }
+    }
+    return b;
+  };
+  return precision == kFP32Compensated ? op(F2{}) : op(0.0);
+}
+
+namespace {
 
 template <typename V>
 inline Frame frame(const double* origin, double sigma, int kernel) {

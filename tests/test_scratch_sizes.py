@@ -43,6 +43,24 @@ def test_workspace_bytes_never_falls_with_the_problem(precision):
             assert got == sorted(got), (other, swap)
 
 
+def test_ordered_sums_reserve_no_pair_partials():
+    """Scratch that grows with the square of the set is asked for by self-sums and shooting steps alone: ordered sums of
+    any size take tens of bytes per target, a wide sum of few sources in particular; and a call's own size is never above
+    that of the workspace that serves it."""
+    lib = _lib()
+    call, upto = lib.lddmm_call_workspace_bytes, lib.lddmm_workspace_bytes
+    assert upto(200000, 100, 1) < 200 << 20 and upto(100, 200000, 0) < 200 << 20
+    for precision in (0, 1):
+        for n in (1, 700, 1281, 4097, 8704, 10368, 13000, 40962, 150000, 200000):
+            # 12 sums of 8 bytes in at most (resident CTAs x block) / n + 2 slots
+            assert call(n, n, 0, precision) <= 96 * (2 * n + 148 * 8 * 1024) + 4096
+            assert call(n, 100, 0, precision) <= call(n, n, 0, precision)
+            assert call(n, n, 0, precision) <= call(n, n, 1, precision) <= upto(n, n, precision)
+            assert call(n, 100, 0, precision) <= upto(n, 100, precision)
+    assert call(300000, 300000, 1, 1) < 200 << 20          # above the symmetric FP64 kernels' bounds
+    assert call(10, 11, 1, 0) == 0 and call(10, 10, 0, 7) == 0
+
+
 # --- the plans of csrc/lddmm_common.cuh and csrc/pairs_sym.cuh, restated
 def _tri(j):
     return j * (j - 1) // 2
@@ -210,3 +228,25 @@ def test_smaller_sets_in_the_scratch_of_the_largest(precision, kernel):
             assert not any(rcs.values()), (top, n, rcs)
     torch.cuda.synchronize()
     assert bool(torch.isfinite(out[0][:n_max // 2]).all())
+
+
+@pytest.mark.gpu
+def test_ordered_fp64_sums_do_not_grow_the_workspace(monkeypatch):
+    """K(y, x) a and a derivative operator in FP64, and a self-sum after them in the same buffer."""
+    import torch
+    from base import _native as nat
+    from base.kernelFunctions import Kernel
+    monkeypatch.setattr(nat, 'WORKSPACE', nat.Workspace())
+    K = Kernel(name='gauss', sigma=0.5)
+    K.pk_dtype = 'float64'
+    rng = np.random.default_rng(0)
+    X = torch.from_numpy(rng.normal(size=(60000, 3))).cuda()
+    Y = X + 0.01
+    K.applyK(X[:100].contiguous(), X[:100].contiguous(), firstVar=Y)
+    K.applyK(X[:3000].contiguous(), X[:3000].contiguous(), firstVar=Y[:3000].contiguous())
+    K.applyDiffKT(X, X, X)
+    assert nat.WORKSPACE.get(1).numel() <= 64 << 20
+    Z = X[:5000].contiguous()
+    a = K.applyK(Z, Z)
+    b = K.applyK(Z, Z, firstVar=Z.clone())
+    assert float((a - b).norm() / b.norm()) < 1e-13
