@@ -190,11 +190,11 @@ class MomentumProposal:
 
     def adam(self, grads, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0):
         self.step += 1
-        params = (self.W + self.b)[:len(grads)]        # as many as there are gradients
-        n = len(params)
+        pairs = list(zip(self.W + self.b, grads))      # as many as there are gradients, from any iterable
+        n = len(pairs)
         if n == 0:
             return
-        grads = grads[:n]
+        params, grads = zip(*pairs)
         counts = (ctypes.c_int64 * n)(*[p.numel() for p in params])
         nat.check(nat.lib().lddmm_adam_steps(n, nat.ptrs(params), nat.ptrs(grads), nat.ptrs(self.m), nat.ptrs(self.v),
                                              nat.ptrs((list(self.Wb) + [None] * len(self.b))[:n]), counts, lr, beta1,
