@@ -94,6 +94,7 @@ constexpr int kRtKSymL = LDDMM_RT_KSYM_L;
 //                    45.6 (- 38.4)   13,000: 67 | 56 | 52 / 53 (- 54)   16,000: 98 | 81 | 79 / 70 (- 78)
 // and for the Laplacian of order 3: forward 10,242: 91 | 83 | 86 / 76 (- 82), 13,000: 139 | 123 | 122 / 141 (- 132);
 // adjoint 13,000: 227 | 208 / 230 (- 239), 16,000: 335 | 308 / 319; K a 10,242: 56 | 51 | 48 / 59 (- 53).
+// The bounds are in points, as measured on 148 SMs; on another chip they stay correct and may not be the fastest.
 // 2 targets up to kSplit2N: there the units of 64 points still have an SM each. Whole tiles are faster per pair and
 // their units four times longer, so between kWholeN and kSplitN they are taken where their units fill the resident CTAs
 // (10,242 and 16,000 points above, not 13,000), beyond kSplitN always. K a of the Gaussian keeps the split up to
@@ -108,8 +109,8 @@ constexpr int kRtKSym = LDDMM_RT_KSYM;
 constexpr int kTpb64 = LDDMM_TPB_64;
 constexpr int kRt64 = LDDMM_RT_64;
 // FP64 symmetric sums (pairs_kernel_sym with V = double), threads per CTA x targets per thread. 64 x 4 for K a, the
-// forward step and the first-order adjoint step, 128 x 2 for the adjoint step (17 target values per thread: 4 targets
-// would leave 1 CTA per SM). us at n = 10,242 / 40,962, 64 x 4 | 128 x 2 | 128 x 4: K a 113 / 1486 | 120 / 1593 | 111 /
+// forward step and the first-order adjoint step, 128 x 2 for the adjoint step (measured with 17 values per target, 13
+// since: 4 targets left 1 CTA per SM). us at n = 10,242 / 40,962, 64 x 4 | 128 x 2 | 128 x 4: K a 113 / 1486 | 120 / 1593 | 111 /
 // 1494; adjoint step 302 / 4218 | 291 / 4100 | 299 / 4232 (every ordered pair with exp(): K a 227 / 3111, adjoint step
 // 463 / 6606).
 constexpr int kTpbSym64 = 64, kRtSym64 = 4;

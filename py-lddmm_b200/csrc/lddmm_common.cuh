@@ -8,12 +8,13 @@
 // tile) units are split evenly over exactly one resident wave of CTAs (stream-K style, see SKPlan), so every
 // problem size keeps all 148 SMs equally busy.
 //
-// FP32 path: the pair arithmetic runs on Blackwell's packed FP32 instructions (fma/add/sub/mul .f32x2): one
-// instruction evaluates the same source against TWO targets of the thread, halving the issue slots of the FP32
-// work. Source fields are stored duplicated ((f, f) pairs) in shared memory so that a 16-byte LDS yields two
-// ready-to-use packed operands. Coordinates are centred on a caller-given origin and pre-scaled by
-// s = sqrt(log2(e)/2)/sigma so that exp(-|y-x|^2/(2 sigma^2)) = 2^-(|y'-x'|^2), one `ex2.approx.ftz` (MUFU)
-// per pair. Each tile is summed in plain FP32; tile sums are merged into a (hi, lo) pair by a two-sum
+// FP32 path: the pair arithmetic runs on Blackwell's packed FP32 instructions (fma/add/sub/mul .f32x2), halving the
+// issue slots of the FP32 work. In the ordered sums of this file an instruction evaluates the same source against TWO
+// targets of the thread; source fields are stored duplicated ((f, f) pairs) in shared memory so that a 16-byte LDS
+// yields two ready-to-use packed operands. (The symmetric sums of pairs_sym.cuh evaluate two sources against the same
+// target.) Coordinates are relative to an origin, the caller's or the target block's own (segment_origin), and
+// pre-scaled by s = sqrt(log2(e)/2)/sigma so that exp(-|y-x|^2/(2 sigma^2)) = 2^-(|y'-x'|^2), one `ex2.approx.ftz`
+// (MUFU) per pair. Each tile is summed in plain FP32; tile sums are merged into a (hi, lo) pair by a two-sum
 // (compensated accumulation across tiles). Chunk partials are reduced in FP64, in fixed order, by the epilogue
 // kernel, which applies the per-target constants and writes float64 outputs (and, for shooting steps, the
 // float64 Euler update of the state).
@@ -231,8 +232,7 @@ template <> struct VT<F2> {
     split(r2, a, b);
     return f2(ex2neg(a), ex2neg(b));
   }
-  // a scalar as the first lane of a value, and the sum of a value's lanes
-  static __device__ __forceinline__ F2 first(float a) { return f2(a, 0.f); }
+  // the sum of a value's lanes
   static __device__ __forceinline__ float hsum(F2 v) {
     float a, b;
     split(v, a, b);
@@ -254,8 +254,7 @@ template <> struct VT<double> {
   static __device__ __forceinline__ double dup(double a) { return a; }
   static __device__ __forceinline__ double pack(double a, double) { return a; }
   static __device__ __forceinline__ double expneg(double r2) { return exp2_neg(r2); }
-  // a scalar as the first lane of a value, and the sum of a value's lanes
-  static __device__ __forceinline__ double first(double a) { return a; }
+  // the sum of a value's lanes
   static __device__ __forceinline__ double hsum(double v) { return v; }
   static __device__ __forceinline__ double lane(double v, int) { return v; }
 };

@@ -355,7 +355,7 @@ struct GradReduce {
   const float* part[2 * kMaxLayers];
   float* out[2 * kMaxLayers];
   int count[2 * kMaxLayers], splits[2 * kMaxLayers], end[2 * kMaxLayers];  // end: running total of the counts
-  int segments, total;
+  int total;
   const float* row_loss;
   int rows;
   float w;
@@ -693,7 +693,6 @@ int lddmm_mlp_gradients(const int64_t* dims, int layers, const void* x, int64_t 
       cur = 1 - cur;
     }
   }
-  R.segments = at;
   R.row_loss = row_loss;
   R.rows = (int)M;
   R.w = w;
