@@ -176,27 +176,28 @@ class Workspace:
 WORKSPACE = Workspace()
 
 
-_WS_BYTES = {}   # (entry, arguments, device) -> bytes: the library's answer depends on nothing else
-
-
-def _ws_bytes(entry, *args):
-    key = (entry, *[int(v) for v in args], torch.cuda.current_device())
-    nb = _WS_BYTES.get(key)
-    if nb is None:
-        nb = _WS_BYTES[key] = getattr(lib(), entry)(*key[1:-1])
-    return nb
+_WS_BYTES = {}   # (n, m, self_sums or None for surfaces, precision, device) -> bytes: the library's answer depends on
+                 # nothing else
 
 
 def workspace(n, m, precision=FP32C, self_sums=None):
     """Scratch of a call with n targets and m sources (pointer, size). self_sums: whether the call may be a self-sum or a
     whole shooting step, whose scratch grows with n^2 (None: wherever n == m; False: the ordered sums)."""
     both = n == m if self_sums is None else self_sums
-    buf = WORKSPACE.get(_ws_bytes('lddmm_call_workspace_bytes', n, m, both, precision))
+    key = (n, m, both, precision, torch.cuda.current_device())
+    nb = _WS_BYTES.get(key)
+    if nb is None:
+        nb = _WS_BYTES[key] = lib().lddmm_call_workspace_bytes(int(n), int(m), int(both), int(precision))
+    buf = WORKSPACE.get(nb, key[4])
     return ctypes.c_void_p(buf.data_ptr()), ctypes.c_size_t(buf.numel())
 
 
 def surface_workspace(nf, nf1, precision=FP32C):
-    buf = WORKSPACE.get(_ws_bytes('lddmm_surface_workspace_bytes', nf, nf1, precision))
+    key = (nf, nf1, None, precision, torch.cuda.current_device())
+    nb = _WS_BYTES.get(key)
+    if nb is None:
+        nb = _WS_BYTES[key] = lib().lddmm_surface_workspace_bytes(int(nf), int(nf1), int(precision))
+    buf = WORKSPACE.get(nb, key[4])
     return ctypes.c_void_p(buf.data_ptr()), ctypes.c_size_t(buf.numel())
 
 
