@@ -35,7 +35,6 @@ struct OpK {
     const double* dotw = nullptr;
     double* dots = nullptr;
   };
-  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.y; }
   template <typename V> struct Tgt { V y0, y1, y2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {
@@ -162,7 +161,6 @@ struct OpDiffKT {
     Frame f;
     double w;  // regweight (lddmm)
   };
-  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.y; }
   template <typename V> struct Tgt { V y0, y1, y2, p0, p1, p2, a0, a1, a2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {
@@ -219,7 +217,6 @@ struct OpDDiffK {
     double* out;
     Frame f;
   };
-  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.x; }
   template <typename V> struct Tgt { V y0, y1, y2, n0, n1, n2, p0, p1, p2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {
@@ -271,7 +268,6 @@ struct OpDiffK1and2 {
     double* out;
     Frame f;
   };
-  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.x; }
   template <typename V> struct Tgt { V y0, y1, y2, b0, b1, b2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {
@@ -315,7 +311,6 @@ struct OpDiv {
     double* out;
     Frame f;
   };
-  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.y; }
   template <typename V> struct Tgt { V y0, y1, y2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {
@@ -347,7 +342,6 @@ struct OpKTensor {
     double* out;
     Frame f;
   };
-  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.y; }
   template <typename V> struct Tgt { V y0, y1, y2, b0, b1, b2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {

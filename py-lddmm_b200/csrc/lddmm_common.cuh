@@ -751,9 +751,6 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
   constexpr float kZeroR2 = Fam::template kCullR2<V>;
   using Un = Units<Op, TPB, TW * RT>;
   const int gx = (n + TW * RT - 1) / (TW * RT);
-  // (the culled ops' boxes are in the caller's frame, and so are their coordinates)
-  constexpr bool kOwn = SPLIT && !Culled<Op>::value;
-  __shared__ double org[3];
   __shared__ float tbox[6];  // the segment's target box, in shared memory (re-read per tile, not held in registers)
   VT<V>::setup();
   chain_wait();
@@ -768,13 +765,6 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
     const int j1 = first + (int)((u_end - off) < TT - first ? (u_end - off) : TT - first);
     const int slot = (int)blockIdx.x - sk_cta_of(off, W, C);
 
-    if constexpr (kOwn) {
-      const int b0 = tb * (TW * RT), b1 = b0 + TW * RT < n ? b0 + TW * RT : n;
-      double o[3];
-      segment_origin(P.f, Op::target_points(P), b0, b1 - 1, o);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) org[c] = o[c];
-    }
     typename Op::template Tgt<V> tgt[G];
     Comp<V> cmp[G][Op::NA];   // used when !kSm
     // target of (group g, lane k): base + (g * L + k) * TW
@@ -784,10 +774,7 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
       int i0 = base + (g * L) * TW, i1 = base + (g * L + L - 1) * TW;
       i0 = i0 < n ? i0 : n - 1;
       i1 = i1 < n ? i1 : n - 1;
-      if constexpr (kOwn)
-        Op::template load_target<V>(with_origin(P, org), i0, i1, tgt[g]);
-      else
-        Op::template load_target<V>(P, i0, i1, tgt[g]);
+      Op::template load_target<V>(P, i0, i1, tgt[g]);
 #pragma unroll
       for (int c = 0; c < Op::NA; ++c) {
         cmp[g][c].zero();
@@ -812,12 +799,7 @@ __global__ void __launch_bounds__(TPB, MinCtas<Op, V>::value)
         double f[2 * NU];
 #pragma unroll
         for (int q = 0; q < 2 * NU; ++q) f[q] = 0.0;
-        if (live) {
-          if constexpr (kOwn)
-            Op::source_fields(with_origin(P, org), l, f);
-          else
-            Op::source_fields(P, l, f);
-        }
+        if (live) Op::source_fields(P, l, f);
         if constexpr (Un::kTri) Op::weigh(f + 3, weight);
 #pragma unroll
         for (int q = 0; q < NU; ++q) {

@@ -23,7 +23,6 @@ struct OpSOFwd {
     double dt;
     int row0 = 0;
   };
-  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.x + 3 * (size_t)P.row0; }
   template <typename V> struct Tgt { V y0, y1, y2, a0, a1, a2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {
@@ -138,7 +137,6 @@ struct OpSOBwd {
     double dt;
     int row0 = 0;
   };
-  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.x + 3 * (size_t)P.row0; }
   template <typename V> struct Tgt { V y0, y1, y2, a0, a1, a2, b0, b1, b2, p0, p1, p2, q0, q1, q2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {
@@ -360,7 +358,6 @@ struct OpFOBwd {
     double dt, w;
     int euclidean;
   };
-  static __device__ __forceinline__ const double* target_points(const Params& P) { return P.x; }
   template <typename V> struct Tgt { V y0, y1, y2, p0, p1, p2, a0, a1, a2; };
   template <typename V>
   static __device__ __forceinline__ void load_target(const Params& P, int i0, int i1, Tgt<V>& t) {

@@ -1,0 +1,118 @@
+"""The origin that a block of a small set takes for itself when the caller gives none."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _errors(X, A, P, B, name, origin):
+    import torch
+    from base import _native as nat
+    from base import pointEvolution as evol
+    from base.kernelFunctions import Kernel
+    out = {}
+    for dtype, o in (('float32', origin), ('float64', nat.centroid(X))):
+        K = Kernel(name=name, sigma=1.0, order=3) if name == 'laplacian' else Kernel(name=name, sigma=1.0)
+        K.pk_dtype = dtype
+        xt, at = evol.shoot_second_order(X, A, K, 1.0, origin=o)
+        px, pa, _ = evol.second_order_adjoint(torch.stack([X, X]), torch.stack([A, A]), P, B, K, 1.0, origin=o,
+                                              with_da0=False)
+        f1, f0 = evol.first_order_gradient(torch.stack([X, X]), A[None].contiguous(), P, K, 0.5, euclidean=True,
+                                           origin=o)
+        out[dtype] = [K._apply_k(X, X, A, 1.0, o), xt[1] - X, at[1] - A, px[0] - P, pa[0] - B, f1[0] - P, f0[0]]
+    return [float((a - b).norm() / b.norm()) for a, b in zip(out['float32'], out['float64'])]
+
+
+@pytest.mark.parametrize('name', ['gauss', 'laplacian'])
+@pytest.mark.parametrize('n', [700, 1300, 2600, 5000, 8000])
+def test_scattered_sets_are_as_accurate_as_about_their_centroid(n, name):
+    """Points of a cube of 32 widths in random order: the FP32 errors of self-sums and steps without an origin against
+    those about the centroid. The rounding of a coordinate grows with its distance from the origin; the middle of a block
+    lies within an eighth of the half extent from the centre in the mean square, which adds 3 / 8^2 / 2 = 2.3% to the
+    error. Bound: 10% on the geometric mean of seven sums over three sets (their errors are sums of thousands of
+    roundings), where an origin at half the extent adds 30%."""
+    import torch
+    ratios = []
+    for seed in range(3):
+        r = np.random.default_rng(100 * seed + n)
+        X = torch.from_numpy(r.uniform(-16, 16, size=(n, 3))).cuda()
+        A, P, B = (torch.from_numpy(r.normal(size=(n, 3))).cuda() for _ in range(3))
+        own = _errors(X, A, P, B, name, None)
+        given = _errors(X, A, P, B, name, X.mean(0).tolist())
+        ratios += [a / b for a, b in zip(own, given)]
+    assert float(np.exp(np.mean(np.log(ratios)))) < 1.1, np.round(ratios, 2)
+
+
+@pytest.mark.parametrize('far', [1e3, -2e5, 1e30])
+@pytest.mark.parametrize('where', [0, 1, 20, 63, 64, 100, 127])
+def test_one_far_point_does_not_move_a_block(far, where):
+    """At any place of a block: the other points' sums are those of the set without it, whose blocks are as close to
+    their points. Bound 2e-5, that of the FP32 kernel sums; the far point is beyond the kernel's reach."""
+    import torch
+    from base.kernelFunctions import Kernel
+    r = np.random.default_rng(where)
+    x, a = r.normal(size=(700, 3)) + 40.0, r.normal(size=(700, 3))
+    x[where, 1] = far
+    K, K64 = Kernel(name='gauss', sigma=0.5), Kernel(name='gauss', sigma=0.5)
+    K.pk_dtype, K64.pk_dtype = 'float32', 'float64'
+    X, A = torch.from_numpy(x).cuda(), torch.from_numpy(a).cuda()
+    got, ref = K.applyK(X, A), K64.applyK(X, A)
+    keep = torch.arange(700, device='cuda') != where
+    assert float((got - ref)[keep].norm()) < 2e-5 * float(ref[keep].norm())
+    assert bool(torch.isfinite(got).all())
+
+
+@pytest.mark.parametrize('n', [1, 2, 3, 4, 5, 33, 65, 66, 67, 68])
+def test_blocks_of_few_points(n):
+    """Fewer points than groups in the last (or only) block, far from the coordinate origin."""
+    import torch
+    from base.kernelFunctions import Kernel
+    r = np.random.default_rng(n)
+    X = torch.from_numpy(r.normal(size=(n, 3)) - 5.0e4).cuda()
+    A = torch.from_numpy(r.normal(size=(n, 3))).cuda()
+    K, K64 = Kernel(name='gauss', sigma=0.5), Kernel(name='gauss', sigma=0.5)
+    K.pk_dtype, K64.pk_dtype = 'float32', 'float64'
+    got, ref = K.applyK(X, A), K64.applyK(X, A)
+    assert float((got - ref).norm()) < 2e-5 * float(ref.norm())
+
+
+@pytest.mark.parametrize('dtype', ['float32', 'float64'])
+def test_far_points_at_the_ends_and_the_middle_of_a_block(dtype):
+    """The three points that a block's reference is taken from may all be far ones (2e5 widths): the others' sums stay
+    those of the kernel tests (FP32 2e-5; FP64 coordinates at 2e5 widths round at 2^-53 x 2e5 of a width, 1e-10)."""
+    import torch
+    import oracle as O
+    from base.kernelFunctions import Kernel
+    r = np.random.default_rng(5)
+    x, a = r.normal(size=(640, 3)), r.normal(size=(640, 3))
+    far = np.zeros(640, dtype=bool)
+    for b in (32, 64, 128):
+        for k in range(0, 640, b):
+            far[[k, k + (b - 1) // 2, k + b - 1]] = k % 256 == 0
+    x[far, 0] += 2.0e5
+    K = Kernel(name='gauss', sigma=1.0)
+    K.pk_dtype = dtype
+    got, ref = K.applyK(x, a), O.apply_k(x, x, a, 1.0)
+    tol = 2e-5 if dtype == 'float32' else 1e-10
+    assert np.linalg.norm((got - ref)[~far]) < tol * np.linalg.norm(ref[~far])
+
+
+def test_ordered_fp64_sums_keep_the_callers_frame():
+    """K(y, x) a without an origin evaluates the coordinates as they are given: near targets among far ones keep the
+    rounding of their own distance (the bound of the exponential's range test), whatever block they are in."""
+    from base.kernelFunctions import Kernel
+    K = Kernel(name='gauss', sigma=0.5)
+    K.pk_dtype = 'float64'
+    rng = np.random.default_rng(3)
+    r = rng.uniform(0.0, 2.0, size=512)
+    far = np.zeros(512, dtype=bool)
+    for b in (32, 64, 128):
+        for k in range(0, 512, b):
+            far[[k, k + (b - 1) // 2, k + b - 1]] = True
+    y = np.zeros((512, 3))
+    y[:, 1] = np.where(far, 1.0e6 + r, r)
+    k = K.applyK(np.zeros((1, 3)), np.ones((1, 3)), firstVar=y)[:, 0]
+    t = 0.5 * (r / 0.5) ** 2
+    ref = np.exp(-t)
+    assert np.all(k[far] == 0)
+    assert np.all((np.abs(k - ref) <= (3.5 + 10 * t) * 2.0 ** -53 * ref)[~far])
