@@ -9,9 +9,9 @@
  *    with the reference's default `ms_exponent = -1` weighting; multi-scale kernels are one call per width.
  *  - `origin` (host pointer to 3 doubles, may be NULL): coordinates are taken relative to it before the conversion to
  *    the arithmetic of the sum. Results are translation invariant; pass the centroid of the points for best accuracy.
- *    With NULL it is 0, except that in the self-sums and shooting steps of small sets (at least up to
- *    LDDMM_OWN_ORIGIN_POINTS of the precision) every block of targets takes an origin of its own, the median of three
- *    of its points, which is as accurate and needs no centroid. The Gaussian FP32 expanded-distance kernels (ordered
+ *    With NULL it is 0, except that in the self-sums and whole shooting steps of small sets (at least up to
+ *    LDDMM_OWN_ORIGIN_POINTS of the precision) every block of targets takes an origin of its own, a middle of 32 of its
+ *    points, which is as accurate and needs no centroid. The Gaussian FP32 expanded-distance kernels (ordered
  *    K a, large K(x,x)a, surface terms) centre every target block on its own in either case.
  *  - `precision`: LDDMM_FP32C = FP32 pair arithmetic with compensated (two-sum) accumulation across tiles and
  *    FP64 epilogues; LDDMM_FP64 = the same kernels in FP64 (the faithful baseline).

@@ -335,20 +335,58 @@ __global__ void __launch_bounds__(TPB, kSymCtas<Op, V, RT>)
     const int slot = (int)blockIdx.x - sk_cta_of(off, U, C);
     const int base = i * B + (SPLIT ? lane : (int)threadIdx.x);
 
-    if constexpr (SPLIT) {
-      double o[3];
-      segment_origin(f, P.x, i * B, i * B + B < n ? i * B + B - 1 : n - 1, o);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) org[c] = o[c];
-    }
     typename Op::template SymTgt<V> tgt[RT];
+    // SPLIT: raw coordinates, loaded before the other fields; with nine of those (the second-order adjoint) and more than
+    // two targets they are loaded again when the origin is known (us held | again: adjoint of 2,562 points, 4 targets,
+    // 17.8 | 17.5, of 642, 2 targets, 9.5 | 9.75; forward of 2,562 12.4 | 13.0)
+    constexpr bool kHold = SPLIT && (Op::NSS < 12 || RT <= 2);
+    double xt[kHold ? RT : 1][3];
+    if constexpr (kHold) {
+#pragma unroll
+      for (int g = 0; g < RT; ++g) {
+        const int k = base + g * TW, kc = k < n ? k : n - 1;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) xt[g][c] = P.x[3 * (size_t)kc + c];
+      }
+    }
 #pragma unroll
     for (int g = 0; g < RT; ++g) {
       const int k = base + g * TW, kc = k < n ? k : n - 1;
-      if constexpr (SPLIT)
-        Op::template load_target_sym<V>(with_origin(P, org), kc, kc, k < n, k < n, tgt[g]);
-      else
-        Op::template load_target_sym<V>(P, kc, kc, k < n, k < n, tgt[g]);
+      Op::template load_target_sym<V>(P, kc, kc, k < n, k < n, tgt[g]);
+    }
+    if constexpr (SPLIT) {
+      // the segment's origin, a coordinate per warp, while the targets' other fields arrive; then their coordinates
+      static_assert(W >= 3, "a warp per coordinate");
+      if (warp < 3) {
+        const int last = i * B + B < n ? i * B + B - 1 : n - 1, count = last - i * B + 1;
+        constexpr int M = RT / 2;  // the middle 32 points, of a short block the first
+        const bool mid = count >= 32 * (M + 1);
+        double x;
+        if constexpr (kHold) {
+          const double x0 = warp == 0 ? xt[0][0] : warp == 1 ? xt[0][1] : xt[0][2];
+          const double xm = warp == 0 ? xt[M][0] : warp == 1 ? xt[M][1] : xt[M][2];
+          x = mid ? xm : x0;
+        } else {
+          const int k = base + (mid ? M * TW : 0);
+          x = P.x[3 * (size_t)(k < n ? k : n - 1) + warp];
+        }
+        const double o = segment_origin(f, P.x, i * B, last, warp, count >= 32, x);
+        if (lane == 0) org[warp] = o;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int g = 0; g < RT; ++g) {
+        if constexpr (kHold) {
+          tgt[g].y0 = VT<V>::dup((xt[g][0] - org[0]) * f.s);
+          tgt[g].y1 = VT<V>::dup((xt[g][1] - org[1]) * f.s);
+          tgt[g].y2 = VT<V>::dup((xt[g][2] - org[2]) * f.s);
+        } else {
+          const int k = base + g * TW, kc = k < n ? k : n - 1;
+          tgt[g].y0 = tgt_coord<V>(P.x, kc, kc, 0, org[0], f.s);
+          tgt[g].y1 = tgt_coord<V>(P.x, kc, kc, 1, org[1], f.s);
+          tgt[g].y2 = tgt_coord<V>(P.x, kc, kc, 2, org[2], f.s);
+        }
+      }
     }
 #pragma unroll
     for (int c = 0; c < H * NR; ++c) {
