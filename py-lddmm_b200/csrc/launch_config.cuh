@@ -94,6 +94,7 @@ constexpr int kRtKSymL = LDDMM_RT_KSYM_L;
 //                    45.6 (- 38.4)   13,000: 67 | 56 | 52 / 53 (- 54)   16,000: 98 | 81 | 79 / 70 (- 78)
 // and for the Laplacian of order 3: forward 10,242: 91 | 83 | 86 / 76 (- 82), 13,000: 139 | 123 | 122 / 141 (- 132);
 // adjoint 13,000: 227 | 208 / 230 (- 239), 16,000: 335 | 308 / 319; K a 10,242: 56 | 51 | 48 / 59 (- 53).
+// (Taken with a median of three points as a split block's origin; the middle of 32 adds 0.1-0.2 us to each split figure.)
 // The bounds are in points, as measured on 148 SMs; on another chip they stay correct and may not be the fastest.
 // 2 targets up to kSplit2N: there the units of 64 points still have an SM each. Whole tiles are faster per pair and
 // their units four times longer, so between kWholeN and kSplitN they are taken where their units fill the resident CTAs
