@@ -63,6 +63,10 @@ class SurfaceDataTerm:
         self.nf1 = self.faces1.shape[0]
         self.w = None if weights is None else nat.as_device(weights)
         self.w1 = None if target_weights is None else nat.as_device(target_weights)
+        if self.w is not None and self.w.numel() < self.nv and self.w.numel() <= self.faces_np.max(initial=-1):
+            raise ValueError('fewer weights than vertices')
+        if self.w1 is not None and self.w1.numel() < self.x1.shape[0] and self.w1.numel() <= f1.max(initial=-1):
+            raise ValueError('fewer target weights than target vertices')
         if self._with_gradient:
             self.vf_off, self.vf_items = vertex_face_table(self.faces_np, self.nv)
         elif self.faces_np.size and (self.faces_np.min() < 0 or self.faces_np.max() >= self.nv):
@@ -74,9 +78,16 @@ class SurfaceDataTerm:
     def _ws(self):
         return nat.surface_workspace(self.nf, self.nf1, self.precision)
 
+    def _deformed(self, xdef):
+        """xdef on the device, with a row for every vertex of the faces (the kernels do not check)."""
+        X = nat.as_device(xdef)
+        if X.numel() < 3 * self.nv and self.nf and X.numel() < 3 * (int(self.faces_np.max()) + 1):
+            raise ValueError('faces index outside the vertices')
+        return X
+
     def energy(self, xdef, with_norm0=False):
         """Device tensor (2,): [xNormDef, xNorm0 (or 0)] in FP64. xdef=None evaluates xNorm0 only."""
-        X = None if xdef is None else nat.as_device(xdef)
+        X = None if xdef is None else self._deformed(xdef)
         nv, nf = (0, 0) if X is None else (X.shape[0], self.nf)
         out = torch.zeros(2, dtype=torch.float64, device=self.x1.device)
         one = len(self.widths) == 1 and self.widths[0][1] == 1.0      # one width: no weighting pass
@@ -101,17 +112,19 @@ class SurfaceDataTerm:
 
     def gradient(self, xdef, with_weights=False):
         """Vertex gradient of xNormDef, (nv,3) FP64 device tensor (and (nv,) weight gradient if requested)."""
-        X = nat.as_device(xdef)
+        X = self._deformed(xdef)
+        nv = min(X.shape[0], self.nv)       # the table's vertices; further rows belong to no face
         one = len(self.widths) == 1 and self.widths[0][1] == 1.0      # one width: no weighting pass
-        make = torch.empty if one else torch.zeros
-        px = make((X.shape[0], 3), dtype=torch.float64, device=X.device)
-        pxw = make(X.shape[0], dtype=torch.float64, device=X.device) if with_weights else None
-        tmp = px if one else torch.empty_like(px)
-        tmpw = pxw if one or not with_weights else torch.empty_like(pxw)
+        make = torch.empty if nv == X.shape[0] else torch.zeros
+        out = make if one else torch.zeros
+        px = out((X.shape[0], 3), dtype=torch.float64, device=X.device)
+        pxw = out(X.shape[0], dtype=torch.float64, device=X.device) if with_weights else None
+        tmp = px if one else make(px.shape, dtype=px.dtype, device=px.device)
+        tmpw = pxw if one or not with_weights else make(pxw.shape, dtype=pxw.dtype, device=pxw.device)
         ws, wsb = self._ws()
         o = nat.origin_arg(self.origin)
         for s, wt in self.widths:
-            nat.check(nat.lib().lddmm_surface_gradient(self.kind, nat.ptr(X), X.shape[0], nat.ptr(self.faces),
+            nat.check(nat.lib().lddmm_surface_gradient(self.kind, nat.ptr(X), nv, nat.ptr(self.faces),
                                                        self.nf, nat.ptr(self.w), nat.ptr(self.vf_off),
                                                        nat.ptr(self.vf_items), nat.ptr(self.x1), self.x1.shape[0],
                                                        nat.ptr(self.faces1), self.nf1, nat.ptr(self.w1), float(s), o,
