@@ -697,14 +697,17 @@ constexpr int kRunRT = (kUseExpanded<Op, V, Fam> && RtXOf<Op>::value > 0) ? RtXO
 // Origin of a target block's coordinates in the split self-sums: the caller's, or a middle of the block's own points, so
 // that a caller whose points live on the device need not read a centroid back (one synchronisation per call before).
 // Coordinate by coordinate, on FP32 offsets of 32 points of the block from a reference (the median of its first, middle
-// and last point): the mean of the middle two of four lanes, the same of four such groups, and the mean of both
-// half warps. Far or non-finite points do not move it unless two of four are, several times over; in a block of a
-// scattered set it lies within an eighth of the half extent from the centre, so that coordinates round as about a common
-// centroid (Gaussian sums and steps of cubes of 32 widths in random order, 700 to 12,000 points: 0.99 of the errors about
-// the centroid; with the median of three points alone, 0.45 of the half extent, 1.2-1.5). A reference that is not finite
-// leaves the block in the caller's frame. It costs 0.2 us of a step (forward step of 2,562 points 12.37 -> 12.57 us),
-// where reading a centroid back costs a call 15. In the unsplit kernels, whose calls are long against that, the six more
-// registers cost 1-4% (forward step at 40,962 points 783 -> 792 us, FP64 first-order adjoint step 2458 -> 2569).
+// and last point): the mean of the middle two of four lanes eight apart, the same of four neighbouring groups, and the
+// mean of both halves. Far or non-finite points do not move it unless two of four are, several times over; a run of far
+// points in storage order, up to a quarter of the 32 (or of a shorter block), never does (with groups of four
+// neighbouring lanes six far points at 1e5 in a block of 32 moved it to 1.2e4: FP64 sums of the near ones 2e-13 instead
+// of 1e-16). In a block of a scattered set it lies within an eighth of the half extent from the centre, so that
+// coordinates round as about a common centroid (Gaussian sums and steps of cubes of 32 widths in random order, 700 to
+// 12,000 points: 0.99 of the errors about the centroid; with the median of three points alone, 0.45 of the half extent,
+// 1.2-1.5). A reference that is not finite leaves the block in the caller's frame. It costs 0.2 us of a step (forward
+// step of 2,562 points 12.37 -> 12.57 us), where reading a centroid back costs a call 15. In the unsplit kernels, whose
+// calls are long against that, the six more registers cost 1-4% (forward step at 40,962 points 783 -> 792 us, FP64
+// first-order adjoint step 2458 -> 2569).
 
 // the mean of the middle two of the values of lanes l, l ^ A, l ^ B and l ^ A ^ B
 template <int A, int B>
@@ -722,14 +725,14 @@ __device__ __forceinline__ double segment_origin(const Frame& f, const double* _
   if (!f.own) return given;
   const int count = last - first + 1;
   const double* p = points + c;
-  // fewer than 32 points: each in turn (four neighbouring lanes have four points)
-  if (!full) x = p[3 * (size_t)(first + (int)(threadIdx.x & 31) % count)];
+  // fewer than 32 points: spread evenly, so that lanes eight apart have different ones from four points on
+  if (!full) x = p[3 * (size_t)(first + (((int)(threadIdx.x & 31) * count) >> 5))];
   const double r0 = p[3 * (size_t)first], r1 = p[3 * (size_t)(first + (last - first) / 2)], r2 = p[3 * (size_t)last];
   const float f0 = (float)r0, f1 = (float)r1, f2 = (float)r2;
   const float fm = fmaxf(fminf(f0, f1), fminf(fmaxf(f0, f1), f2));
   const double m = fm == f0 ? r0 : fm == f1 ? r1 : r2;
-  float v = middle4_lanes<4, 8>(middle4_lanes<1, 2>((float)(x - m)));
-  v = 0.5f * (v + __shfl_xor_sync(0xffffffffu, v, 16));
+  float v = middle4_lanes<1, 2>(middle4_lanes<8, 16>((float)(x - m)));
+  v = 0.5f * (v + __shfl_xor_sync(0xffffffffu, v, 4));
   if (!isfinite(m)) return given;
   return count >= 4 && isfinite(v) ? m + (double)v : m;
 }

@@ -95,3 +95,27 @@ def test_far_points_at_the_ends_and_the_middle_of_a_block(dtype):
     got, ref = K.applyK(x, a), O.apply_k(x, x, a, 1.0)
     tol = 2e-5 if dtype == 'float32' else 1e-10
     assert np.linalg.norm((got - ref)[~far]) < tol * np.linalg.norm(ref[~far])
+
+
+@pytest.mark.parametrize('run', [2, 5, 6, 8])
+@pytest.mark.parametrize('start', [0, 3, 12, 24])
+@pytest.mark.parametrize('n', [300, 2000])
+def test_a_run_of_far_points_does_not_move_a_block(n, start, run):
+    """Far points in a row (1e9 and more, apart from each other), up to a quarter of the points that a block's origin is
+    taken from (32, or all of a shorter block): the FP64 sums of the others are those of
+    points within 16 of their origin. Coordinates of 27 widths' scale round at 27 x 2^-53, differences at 1.2e-14 at most,
+    and a term 2^-|d|^2 with |d| up to 5 at 2 x 5 x ln 2 of that: below 1e-13; bound 2e-13. About an origin that a far point
+    has moved by a sixteenth they would round at 1e-8."""
+    import torch
+    from base.kernelFunctions import Kernel
+    r = np.random.default_rng(start + 100 * run)
+    x, a = r.uniform(0, 16, size=(n, 3)), r.normal(size=(n, 3))
+    far = np.zeros(n, dtype=bool)
+    for b in range(0, n, 64):
+        far[b + start:b + start + min(run, min(n - b, 32) // 4)] = True
+    x[far, 0] += 1.0e9 * (1 + np.arange(int(far.sum())))
+    X, A = torch.from_numpy(x).cuda(), torch.from_numpy(a).cuda()
+    got = Kernel(name='gauss', sigma=0.5).applyK(X, A)[torch.from_numpy(~far).cuda()]
+    near, an = X[torch.from_numpy(~far).cuda()], A[torch.from_numpy(~far).cuda()]
+    ref = torch.exp(-2.0 * ((near[:, None] - near[None]) ** 2).sum(-1)) @ an
+    assert float((got - ref).norm()) < 2e-13 * float(ref.norm())
